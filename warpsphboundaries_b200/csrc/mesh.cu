@@ -18,14 +18,25 @@
 //    A_F(r) = -int_r^1 t F(t) dt of a profile F:   int_f F = sum_e w_e int_e (A_F(r) - A_F(|z|)) / (r^2 - z^2) ds,
 //    int_f u F = sum_e mu_e int_e A_F ds,  int_f u u^T F = sum_e mu_e (x) int_e u A_F ds - P int_f A_F
 //    (w_e: signed distance of the foot point to the edge line, mu_e: in-plane outward edge normal, P = I - N N^T).
-//  * edges.  Beyond the support the first integrand is -A_F(|z|) / rho^2: an angle.  Inside, every integrand is a
-//    smooth function of s along the edge (a divided difference of a Laurent polynomial in r = sqrt(c^2 + s^2)); it is
-//    integrated by 12-node Gauss-Legendre on panels split at the foot of the perpendicular, at the kernel's knot and
-//    at distances c 2^k from the foot (the dyadic grading of the reference's stable route, edge/warpbc.py:522-575),
-//    which keeps the branch points s = +-ic of r away from every panel: relative error below 1e-12.
+//  * edges.  Beyond the block's radius the first integrand is -A_F(|z|) / rho^2: an angle.  Inside, every integrand has
+//    a closed form in r = sqrt(c^2 + s^2), c^2 = z^2 + w^2, a = |z|: the line integrals of A_F are moments
+//    I_n = int r^n ds (n >= -1, -2, -3), and in the divided difference
+//      (r^(2m) - a^(2m)) / (r^2 - a^2)   = sum_(i<m) r^(2i) a^(2(m-1-i)),
+//      (r^(2m+1) - a^(2m+1)) / (r^2 - a^2) = sum_(i<m) r^(2i+1) a^(2(m-1-i)) + a^(2m) / (r + a),
+//    so a face needs its edges' w-weighted moments sum_e w_e I_n and Lambda = sum_e w_e int ds / (r + a) only, each
+//    potential one dot product with them (synthetic division by r^2 - a^2, once per face).  With
+//    Y = (s1 r0 - s0 r1) / c^2 (formed without cancellation), U = c^2 Y + c D, B = (r1 + c)(r0 + c), kappa = w / (c + a):
+//      int ds / r = asinh Y,                      int c ds / r^2 = 2 atan(U / (B + s0 s1)) = Theta,
+//      int ds / r^3 = Y / (r0 r1),                int w ds / (r (r + a)) = 2 atan(kappa U / (B + kappa^2 s0 s1)) = Omega,
+//      w int ds / (r + a) = w asinh Y - a Omega,  I_n = (E_n + n c^2 I_(n-2)) / (n + 1),  E_n = [s r^n],
+//      E_n = D/2 (r1^n + r0^n + S^2 / (r0 + r1) T_n),  T_n = (r1^n - r0^n) / (r1 - r0)      (D = s1 - s0, S = s1 + s0):
+//    sums of terms of one sign throughout, so a short edge keeps its relative accuracy.  The rounding of a channel is
+//    that of the potentials' monomial form (sum |c_n| / max |A|).
 //    Powers z^p multiply the profiles whose potentials hold r^-m (m <= p) so that every face term stays bounded as
 //    the query approaches the face plane.
-// The exact rational potentials are generated by warpsphboundaries_b200/kernels.py (mesh_tables, emit_mesh).
+//  * kernels of several pieces are sums of truncated blocks P(r) 1[r <= R] (the decomposition of the 2-D tables); every
+//    channel is the sum of its blocks' channels, so no integral crosses a knot.
+// The exact rational potentials are generated by warpsphboundaries_b200/kernels.py (mesh_blocks, emit_mesh).
 #include <algorithm>
 #include <cmath>
 #include <map>
@@ -58,10 +69,10 @@ struct Mesh {
 // candidate faces)
 enum : uint8_t { kCellEmpty = 1, kCellInside = 2, kCellNear = 4 };
 
-// per face: v0 v1 v2 (9), unit normal N (3), edge tangents t0 t1 t2 (9), edge normals mu_e = t_e x N (9),
-// edge lengths (3), box lo (3), box hi (3)
-constexpr int kFaceDoubles = 39;
-enum { kFV = 0, kFN = 9, kFT = 12, kFMU = 21, kFLEN = 30, kFLO = 33, kFHI = 36 };
+// per face, one 256-byte record: v0 v1 v2 (9), unit normal N (3), edge tangents t0 t1 t2 (9), edge lengths (3), box lo
+// (3), box hi (3), 2 unused; read by 32-byte loads
+constexpr int kFaceDoubles = 32;
+enum { kFV = 0, kFN = 9, kFT = 12, kFLEN = 21, kFLO = 24, kFHI = 27 };
 
 struct MeshView {
   const double* fdata;
@@ -246,26 +257,38 @@ __device__ __forceinline__ int cell_ordinal(int pref, int t) {
 
 // The faces of the 27 cells around the query's cell that come within h of the query (box first, then the exact
 // triangle distance, both tested by the lanes in parallel); a face listed in several of those cells is taken in one of
-// them only (the lowest corner of its box inside the 27-cell block).  Called by a whole warp with one query: the (cell, item) pairs of the block are flattened over the lanes (32 at a time, whatever
-// cell they belong to), and the faces that pass are visited one after the other, warp-uniformly, in cell order and
-// item order within a cell -- a fixed order, so the sums the visits accumulate do not depend on the launch.
-template <class Visit>
-__device__ __forceinline__ void for_candidates_warp(const MeshView& M, const double q[3], double h, int lane,
-                                                    Visit&& visit) {
-  const int cx = cell_coord(q[0], M.lo0, M.cell, M.nx), cy = cell_coord(q[1], M.lo1, M.cell, M.ny),
-            cz = cell_coord(q[2], M.lo2, M.cell, M.nz);
-  const int x0 = max(cx - 1, 0), x1 = min(cx + 1, M.nx - 1), y0 = max(cy - 1, 0), y1 = min(cy + 1, M.ny - 1),
-            z0 = max(cz - 1, 0), z1 = min(cz + 1, M.nz - 1);
-  if (x0 > x1 || y0 > y1 || z0 > z1) return;
-  const double h2 = h * h;
-  const int nxr = x1 - x0 + 1, nyr = y1 - y0 + 1;
-  int beg, pref;
-  const int total = block_cells(M, x0, x1, y0, y1, z0, z1, lane, [](int, int, int) { return true; }, beg, pref);
-  for (int base = 0; base < total; base += 32) {
+// them only (the lowest corner of its box inside the 27-cell block).  Held by a whole warp for one query: the (cell,
+// item) pairs of the block are flattened over the lanes, next() tests 32 of them (whatever cell they belong to) and
+// returns the mask of the lanes whose face f is within h -- in cell order and item order within a cell, a fixed order,
+// so the sums over the faces do not depend on the launch.
+struct FaceSearch {
+  double q[3], h;
+  int cx, cy, cz, x0, y0, z0, nxr, nyr, beg, pref, base, total;
+
+  __device__ __forceinline__ void start(const MeshView& M, const double* __restrict__ pos, double sup, int lane) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) q[a] = pos[a];
+    h = sup;
+    cx = cell_coord(q[0], M.lo0, M.cell, M.nx);
+    cy = cell_coord(q[1], M.lo1, M.cell, M.ny);
+    cz = cell_coord(q[2], M.lo2, M.cell, M.nz);
+    x0 = max(cx - 1, 0);
+    y0 = max(cy - 1, 0);
+    z0 = max(cz - 1, 0);
+    const int x1 = min(cx + 1, M.nx - 1), y1 = min(cy + 1, M.ny - 1), z1 = min(cz + 1, M.nz - 1);
+    nxr = x1 - x0 + 1;
+    nyr = y1 - y0 + 1;
+    base = total = 0;
+    if (x0 > x1 || y0 > y1 || z0 > z1) return;
+    total = block_cells(M, x0, x1, y0, y1, z0, z1, lane, [](int, int, int) { return true; }, beg, pref);
+  }
+
+  __device__ __forceinline__ unsigned next(const MeshView& M, int lane, int& f) {
     const int t = base + lane;
+    base += 32;
     const int o = cell_ordinal(pref, t);
     const int b = __shfl_sync(0xffffffffu, beg, o), p = __shfl_sync(0xffffffffu, pref, o);
-    int f = -1;
+    f = -1;
     bool hit = false;
     if (t < total) {
       const int i = x0 + o % nxr, j = y0 + (o / nxr) % nyr, k = z0 + o / (nxr * nyr);
@@ -276,12 +299,11 @@ __device__ __forceinline__ void for_candidates_warp(const MeshView& M, const dou
         double d2 = 0.0;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-          const double dl = F[kFLO + a] - q[a], dh = q[a] - F[kFHI + a];
-          const double d = fmax(0.0, fmax(dl, dh));
+          const double d = fmax(0.0, fmax(F[kFLO + a] - q[a], q[a] - F[kFHI + a]));
           d2 = fma(d, d, d2);
         }
-        if (d2 < h2) {
-          // the exact triangle distance (unit coordinates relative to the query, the operations of the visit's P)
+        if (d2 < h * h) {
+          // the exact triangle distance (unit coordinates relative to the query, the operations of the face integral's)
           const double ih = 1.0 / h;
           double P[3][3];
 #pragma unroll
@@ -292,16 +314,11 @@ __device__ __forceinline__ void for_candidates_warp(const MeshView& M, const dou
         }
       }
     }
-    unsigned m = __ballot_sync(0xffffffffu, hit);
-    while (m) {
-      const int bl = __ffs(m) - 1;
-      m &= m - 1;
-      visit(__shfl_sync(0xffffffffu, f, bl));
-    }
+    return __ballot_sync(0xffffffffu, hit);
   }
-}
+};
 
-// whether any face box comes within h of the query (the cells of for_candidates_warp, stopping at the first hit),
+// whether any face box comes within h of the query (the cells of FaceSearch, stopping at the first hit),
 // for a whole warp (every lane calls it with the same query): the (cell, item) pairs are flattened over the lanes.
 // A cell whose own box is h or more from the query is skipped: a face box within h of the query has its point nearest
 // to the query in a cell within h, and every cell its box overlaps lists the face (a relative margin far above the
@@ -342,49 +359,13 @@ __device__ __forceinline__ bool has_candidate_warp(const MeshView& M, const doub
   return false;
 }
 
-// ------------------------------------------------------------------------------------------ profiles
-template <class M, int Fn>
-__device__ __forceinline__ double fpoly(int p, double x) {
-  if constexpr (M::kPieces > 1) {
-    if (p) return MeshFn<M, Fn>::poly1(x);
+// ------------------------------------------------------------------------------------------ face integrals
+template <int I, int N, class Fn>
+__device__ __forceinline__ void static_for(Fn&& f) {
+  if constexpr (I < N) {
+    f(std::integral_constant<int, I>{});
+    static_for<I + 1, N>(f);
   }
-  return MeshFn<M, Fn>::poly0(x);
-}
-template <class M, int Fn>
-__device__ __forceinline__ double fdd(int p, double x, double a) {
-  if constexpr (M::kPieces > 1) {
-    if (p) return MeshFn<M, Fn>::dd1(x, a);
-  }
-  return MeshFn<M, Fn>::dd0(x, a);
-}
-// the divided difference fdd in two halves: the synthetic-division coefficients of piece p at a (kMeshDD slots), and
-// Horner's rule over them at x -- the same fma sequence as fdd, so the same value
-constexpr int kMeshDD = 24;
-template <class M, int Fn>
-__device__ __forceinline__ void fddb(int p, double a, double* b) {
-  static_assert(MeshFn<M, Fn>::kDD0 <= kMeshDD, "coefficient slots");
-  if constexpr (M::kPieces > 1) {
-    static_assert(MeshFn<M, Fn>::kDD1 <= kMeshDD, "coefficient slots");
-    if (p) {
-      MeshFn<M, Fn>::ddb1(a, b);
-      return;
-    }
-  }
-  MeshFn<M, Fn>::ddb0(a, b);
-}
-template <class M, int Fn>
-__device__ __forceinline__ double fddh(int p, double x, const double* b) {
-  if constexpr (M::kPieces > 1) {
-    if (p) return MeshFn<M, Fn>::ddh1(x, b);
-  }
-  return MeshFn<M, Fn>::ddh0(x, b);
-}
-template <class M, int Fn>
-__device__ __forceinline__ double fnu(int p) {
-  if constexpr (M::kPieces > 1) {
-    if (p) return MeshFn<M, Fn>::kNu1;
-  }
-  return MeshFn<M, Fn>::kNu0;
 }
 template <int K>
 __device__ __forceinline__ double zpow(double z) {
@@ -393,382 +374,229 @@ __device__ __forceinline__ double zpow(double z) {
   else if constexpr (K == 2) return z * z;
   else return z * z * z;
 }
-// sum_{i < m} x^i a^(m-1-i)
-template <int m>
-__device__ __forceinline__ double smix(double x, double a) {
-  if constexpr (m == 1) return 1.0;
-  else if constexpr (m == 2) return x + a;
-  else return fma(x, x + a, a * a);
-}
-template <class M>
-__device__ __forceinline__ int piece(double x) {
-  if constexpr (M::kPieces > 1) return x < M::kBreak ? 0 : 1;
-  return 0;
-}
 
-// A_F(r) (r inside the support); ir = 1 / r
-template <class M, int Fn>
-__device__ __forceinline__ double aval(double r, double ir) {
-  constexpr int m = MeshFn<M, Fn>::kNeg;
-  const int p = piece<M>(r);
-  double v = fpoly<M, Fn>(p, r);
-  if constexpr (m > 0) v = fma(fnu<M, Fn>(p), zpow<m>(ir), v);
-  return v;
-}
-
-// z^ZP A_F(|z|), |z| = a (0 outside the support); sg = sign(z)
-template <class M, int Fn, int ZP>
-__device__ __forceinline__ double aval_a(double a, double z, double sg) {
-  constexpr int m = MeshFn<M, Fn>::kNeg;
-  static_assert(ZP >= m, "z power must absorb the negative power");
-  if (a >= 1.0) return 0.0;
-  const int p = piece<M>(a);
-  double v = fpoly<M, Fn>(p, a) * zpow<ZP>(z);
-  if constexpr (m > 0) v += fnu<M, Fn>(p) * zpow<ZP - m>(z) * zpow<m>(sg);
-  return v;
-}
-
-// node quantities shared by the six divided differences: r, 1/r, 1/(r + a), 1/rho^2, and whether the segment
-// [a, r] crosses the kernel's knot
-struct Node {
-  double r, ir, irpa, irho2;
-  bool split;
+// coefficient n of potential f of block B, and the coefficient of its negative power
+template <class B, int f, int n>
+struct MeshC {
+  static constexpr double v = B::kC[f][n];
+};
+template <class B, int f>
+struct MeshNu {
+  static constexpr double v = B::kNu[f];
 };
 
-// z^ZP (A_F(r) - A_F(a)) / (r^2 - a^2) for a = |z| < r < 1.  Within one piece the divided difference of the
-// polynomial part comes from synthetic division (no cancellation between A(r) and A(a)); the negative power
-// nu r^-m gives -nu S_m(r, a) / (r^m a^m), whose 1 / a^m is absorbed by z^ZP.  Across the knot B the two pieces'
-// differences are weighted by (B - a) and (r - B) over r - a = rho^2 / (r + a).
-template <class M, int Fn, int ZP>
-__device__ __forceinline__ double dd2(const Node& nd, double a, double z, double sg, const double* fb) {
-  constexpr int m = MeshFn<M, Fn>::kNeg;
-  static_assert(ZP >= m, "z power must absorb the negative power");
-  const int pa = piece<M>(a);
-  if (!nd.split) {
-    double d0 = fddh<M, Fn>(pa, nd.r, fb + Fn * kMeshDD) * zpow<ZP>(z);
-    if constexpr (m > 0) d0 -= fnu<M, Fn>(pa) * smix<m>(nd.r, a) * zpow<m>(nd.ir) * zpow<ZP - m>(z) * zpow<m>(sg);
-    return d0 * nd.irpa;
-  }
-  constexpr double B = M::kBreak;
-  double d0 = fdd<M, Fn>(0, B, a) * zpow<ZP>(z);
-  if constexpr (m > 0) d0 -= fnu<M, Fn>(0) * smix<m>(B, a) * (1.0 / zpow<m>(B)) * zpow<ZP - m>(z) * zpow<m>(sg);
-  double d1 = fdd<M, Fn>(1, nd.r, B);
-  if constexpr (m > 0) d1 -= fnu<M, Fn>(1) * smix<m>(nd.r, B) * zpow<m>(nd.ir) * (1.0 / zpow<m>(B));
-  d1 *= zpow<ZP>(z);
-  return ((B - a) * d0 + (nd.r - B) * d1) * nd.irho2;
-}
+// the power z^p that multiplies each potential (rows of the block tables) and its one negative power r^-m
+constexpr int kZPow[6] = {1, 2, 3, 0, 0, 1};
+constexpr int kNeg[6] = {1, 2, 3, 0, 0, 1};
 
-__device__ __forceinline__ double angle_between(double w, double x0, double x1) {
-  return atan2(w * (x1 - x0), fma(w, w, x0 * x1));
-}
-
-// the 28 accumulators of one row (W~ units, unit support): M0, M1[3], M2[6] (00 01 02 11 12 22), G0[3],
-// G1[9] (i-major), H[6]
-enum { kAM0 = 0, kAM1 = 1, kAM2 = 4, kAG0 = 10, kAG1 = 13, kAH = 22 };
-struct Acc28 {
-  double v[28];
+// the face's sums over its edges that carry the edges' vectors: sum mu LK1, sum mu LK2, sum (mu mu w LK2b + sym(mu t)
+// TK2), sum mu LW, sum mu LL / 2 (LK1 = z int A_K1, LK2b = z int A_K2, LK2 = z LK2b, TK2 = z int s A_K2, LW = int A_W,
+// LL = int A_L); and J_F = sum_e w_e int z^p DD_F ds
+struct FaceSums {
+  double k1[3], k2[3], kk[6], lw[3], ll[3], J[6];
 };
 
-__device__ __forceinline__ void acc_zero(Acc28& A) {
-#pragma unroll
-  for (int i = 0; i < 28; ++i) A.v[i] = 0.0;
-}
-
-// per-edge integrals accumulated over the panels of one side of the foot point
-struct EdgeSums {
-  double J[6];   // w int z^p DD_F ds for A_K0 (p1) A_K1 (p2) A_K2 (p3) A_W A_L A2_K2 (p1)
-  double LK1, LK2, LK2b, TK2, LW, LL;   // int z A_K1, int z^2 A_K2, int z A_K2, int s z A_K2, int A_W, int A_L
-};
-
-// one quadrature node u (distance from the foot along the edge, s = sgn_side * u) with weight wt, in two parts that
-// each form r and 1 / r themselves, so that fewer values are live at once: the six divided differences (w != 0 only),
-// then the six potential sums (one loop over an edge's nodes calls both: measured 9.2 ms for the c3 leg against 9.7
-// ms with a loop for each)
-template <class M>
-__device__ __forceinline__ void node_eval_dd(double u, double wt, double c2, double a, double z, double sg, double w,
-                                             const double* fb, EdgeSums& S) {
-  const double rho2 = fma(u, u, w * w);
-  Node nd;
-  nd.r = sqrt(fma(u, u, c2));
-  nd.ir = 1.0 / nd.r;
-  nd.split = M::kPieces > 1 && a < M::kBreak && nd.r > M::kBreak;
-  nd.irpa = 1.0 / (nd.r + a);
-  nd.irho2 = nd.split ? 1.0 / rho2 : 0.0;
-  const double ww = w * wt;
-  S.J[0] = fma(ww, dd2<M, 0, 1>(nd, a, z, sg, fb), S.J[0]);
-  S.J[1] = fma(ww, dd2<M, 1, 2>(nd, a, z, sg, fb), S.J[1]);
-  S.J[2] = fma(ww, dd2<M, 2, 3>(nd, a, z, sg, fb), S.J[2]);
-  S.J[3] = fma(ww, dd2<M, 3, 0>(nd, a, z, sg, fb), S.J[3]);
-  S.J[4] = fma(ww, dd2<M, 4, 0>(nd, a, z, sg, fb), S.J[4]);
-  S.J[5] = fma(ww, dd2<M, 5, 1>(nd, a, z, sg, fb), S.J[5]);
-}
-
-template <class M>
-__device__ __forceinline__ void node_eval_pot(double u, double wt, double sgn_side, double c2, double z,
-                                              EdgeSums& S) {
-  const double s = sgn_side * u;
-  const double r = sqrt(fma(u, u, c2));
-  const double ir = 1.0 / r;
-  const double k1 = aval<M, 1>(r, ir) * z, k2 = aval<M, 2>(r, ir) * z;
-  S.LK1 = fma(wt, k1, S.LK1);
-  S.LK2b = fma(wt, k2, S.LK2b);
-  S.LK2 = fma(wt, k2 * z, S.LK2);
-  S.TK2 = fma(wt * s, k2, S.TK2);
-  S.LW = fma(wt, aval<M, 3>(r, ir), S.LW);
-  S.LL = fma(wt, aval<M, 4>(r, ir), S.LL);
-}
-
-// the panels of one edge (both sides of the foot of the perpendicular): [u0, u1] of distances from the foot, split
-// at the kernel's knot and at c 2^k (k >= 1); at most 26 panels a side (c 2^k runs from 2^-24 to 1).  A panel that
-// starts within 2c of the foot (the branch points of r sit at distance c from the foot) takes 16 Gauss-Legendre
-// nodes (relative error below 2e-15 on [0, 2c]), the graded ones further out 12 (below 1e-18 on [2^k c, 2^(k+1) c]).
-// A typical edge (side lengths up to 2c) is then 32 nodes: one round of the warp's lanes.
-constexpr int kMaxPanels = 64;
-struct PanelList {
-  double lo[kMaxPanels], hi[kMaxPanels], sg[kMaxPanels];
-  int off[kMaxPanels + 1];    // first node of each panel; off[np] = all nodes
-};
-
-// an edge of the face being evaluated, relative to the query in units of the support: tangent t and in-plane normal
-// mu, the foot's signed distance w to the edge line, the edge's ends lo, hi along t from the foot, c^2 = z^2 + w^2,
-// the part [s0, s1] inside the support, and its panel count
-struct EdgeGeo {
-  double t[3], mu[3], w, lo, hi, c2, s0, s1;
-  int np;
-};
-
-template <class M>
-__device__ int build_panels(PanelList& PL, double s0, double s1, double c) {
-  int np = 0, nodes = 0;
-  double knot = -1.0;
-  if constexpr (M::kPieces > 1) {
-    if (c < M::kBreak) knot = sqrt((M::kBreak - c) * (M::kBreak + c));
-  }
-  const double base = fmax(c, 1.0 / 16777216.0);
-  for (int side = 0; side < 2; ++side) {
-    const double sgn = side == 0 ? -1.0 : 1.0;
-    const double u0 = side == 0 ? fmax(-s1, 0.0) : fmax(s0, 0.0);
-    const double u1 = side == 0 ? -s0 : s1;
-    if (!(u1 > u0)) continue;
-    double d = 2.0 * base;
-    for (int it = 0; it < 64 && d <= u0; ++it) d *= 2.0;
-    double u = u0;
-    for (int it = 0; it < 96 && u < u1 && np < kMaxPanels; ++it) {
-      double nxt = fmin(u1, d);
-      if (knot > u && knot < nxt) nxt = knot;
-      PL.lo[np] = u;
-      PL.hi[np] = nxt;
-      PL.sg[np] = sgn;
-      PL.off[np] = nodes;
-      nodes += u < 2.0 * base ? 16 : 12;
-      ++np;
-      if (nxt >= d) d *= 2.0;
-      u = nxt;
-    }
-  }
-  PL.off[np] = nodes;
-  return np;
-}
-
-// the warp's sums of twelve values, in every lane: lanes 16 apart swap six values and keep the sums of the other six,
-// lanes 8 apart swap three, a butterfly over the last three lane bits completes each group of eight lanes' three sums,
-// and each total is broadcast from its group (a fixed order: deterministic)
-__device__ __forceinline__ void warp_sum12(double v[12]) {
-  const int lane = threadIdx.x & 31;
-  const bool up = (lane >> 4) & 1, b3 = (lane >> 3) & 1;
-  double a[6];
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    const double give = up ? v[k] : v[k + 6];
-    const double keep = up ? v[k + 6] : v[k];
-    a[k] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
-  }
-  double b[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const double give = b3 ? a[k] : a[k + 3];
-    const double keep = b3 ? a[k + 3] : a[k];
-    b[k] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
-  }
-#pragma unroll
-  for (int off = 4; off > 0; off >>= 1)
-#pragma unroll
-    for (int k = 0; k < 3; ++k) b[k] += __shfl_xor_sync(0xffffffffu, b[k], off);
-#pragma unroll
-  for (int x = 0; x < 12; ++x) v[x] = __shfl_sync(0xffffffffu, b[x % 3], 8 * (x / 3));
-}
-
-
-// Assembly (W~ units), per edge:  M0 += J0;  M1_i += N_i J1 + mu_i LK1;
-// M2_ij += N_i N_j (J2 + J5) + (N_i mu_j + mu_i N_j) LK2 + mu_i mu_j w LK2b + (mu_i t_j + mu_j t_i) TK2 / 2 - d_ij J5;
-// G0_i -= N_i J3;  G1_ij -= z N_i N_j J3 + mu_i N_j LW;  H_ij += z N_i N_j J4 + (N_i mu_j + mu_i N_j) LL / 2.
-// Lane k < 28 adds the term of accumulator k: every term is one bilinear form in the vectors N, mu, t whose
-// coefficients a lane selects by its accumulator's type, so all lanes run the same instructions.  The J terms multiply
-// face quantities (N, z) only, so they are added once per face with J summed over the face's edges; the LK / TK / LW
-// / LL terms, which carry the edge's mu and t, once per edge.
-enum { kTM0, kTM1, kTM2, kTG0, kTG1, kTH, kTNone };
-struct AccSlot {
-  int type, i, j;
-};
-
-__device__ __forceinline__ AccSlot acc_slot(int k) {
-  auto sym_i = [](int x) { return x < 3 ? 0 : (x < 5 ? 1 : 2); };
-  auto sym_j = [](int x) { return x < 3 ? x : (x < 5 ? x - 2 : 2); };
-  if (k == kAM0) return {kTM0, 0, 0};
-  if (k < kAM2) return {kTM1, k - kAM1, 0};
-  if (k < kAG0) return {kTM2, sym_i(k - kAM2), sym_j(k - kAM2)};
-  if (k < kAG1) return {kTG0, k - kAG0, 0};
-  if (k < kAH) return {kTG1, (k - kAG1) / 3, (k - kAG1) % 3};
-  if (k < 28) return {kTH, sym_i(k - kAH), sym_j(k - kAH)};
-  return {kTNone, 0, 0};
-}
-
-__device__ __forceinline__ double pick3(const double v[3], int i) { return i == 0 ? v[0] : (i == 1 ? v[1] : v[2]); }
-
-// the terms of accumulator sl with the edge's vectors mu, t (per edge)
-__device__ __forceinline__ double edge_term_mu(const AccSlot& sl, const double N[3], const double t[3],
-                                               const double mu[3], double w, const EdgeSums& S) {
-  const double Ni = pick3(N, sl.i), Nj = pick3(N, sl.j), mi = pick3(mu, sl.i), mj = pick3(mu, sl.j);
-  const double ti = pick3(t, sl.i), tj = pick3(t, sl.j);
-  const double X = Ni * mj + mi * Nj, MN = mi * Nj, MM = mi * mj, MT = 0.5 * (mi * tj + mj * ti);
-  const int ty = sl.type;
-  const double cMi = ty == kTM1 ? S.LK1 : 0.0;
-  const double cX = ty == kTM2 ? S.LK2 : (ty == kTH ? 0.5 * S.LL : 0.0);
-  const double cMN = ty == kTG1 ? -S.LW : 0.0;
-  const double cMM = ty == kTM2 ? w * S.LK2b : 0.0;
-  const double cMT = ty == kTM2 ? S.TK2 : 0.0;
-  return mi * cMi + X * cX + MN * cMN + MM * cMM + MT * cMT;
-}
-
-// the terms of accumulator sl with the J sums (face quantities N, z only: once per face, J summed over its edges)
-__device__ __forceinline__ double face_term_j(const AccSlot& sl, const double N[3], double z, const double J[6]) {
-  const double Ni = pick3(N, sl.i), Nj = pick3(N, sl.j);
-  const double NN = Ni * Nj, dij = sl.i == sl.j ? 1.0 : 0.0;
-  const int ty = sl.type;
-  const double cC = ty == kTM0 ? J[0] : 0.0;
-  const double cNi = ty == kTM1 ? J[1] : (ty == kTG0 ? -J[3] : 0.0);
-  const double cNN = ty == kTM2 ? J[2] + J[5] : (ty == kTG1 ? -z * J[3] : (ty == kTH ? z * J[4] : 0.0));
-  const double cD = ty == kTM2 ? -J[5] : 0.0;
-  return cC + Ni * cNi + NN * cNN + dij * cD;
-}
-
-// the contribution of face f to the row's accumulators (lane k < 28 holds accumulator k in acc), computed by the
-// whole warp: the geometry is the same in every lane, the quadrature nodes of an edge (12 or 16 per panel) are spread over the lanes and
-// their sums reduced by a fixed butterfly, then lane k adds the edge's term of accumulator k (slot: this lane's).
-// Everything is linear in the per-edge integrals.  Faces that do not meet the support contribute exactly nothing:
-// the candidate search visits only faces within the support.  q in world units, ih = 1 / support.
-template <class M>
-__device__ void face_contrib_warp(const MeshView& Mv, int f, const double q[3], double ih, PanelList* PL3,
-                                  EdgeGeo* G3, double* FB, int lane, const AccSlot& slot, double& acc) {
-  const double* F = Mv.fdata + (int64_t)f * kFaceDoubles;
-  double P[3][3];
-#pragma unroll
-  for (int v = 0; v < 3; ++v)
-#pragma unroll
-    for (int k = 0; k < 3; ++k) P[v][k] = (F[kFV + 3 * v + k] - q[k]) * ih;
-  const double N[3] = {F[kFN], F[kFN + 1], F[kFN + 2]};
-  const double z = N[0] * P[0][0] + N[1] * P[0][1] + N[2] * P[0][2];
+// one block's contribution to the sums of the face F (query q, 1 / support ih; z = signed distance of the query to the
+// face plane in supports, N its normal)
+template <class B>
+__device__ __forceinline__ void face_block(const double* __restrict__ F, const double q[3], double ih,
+                                           const double N[3], double z, FaceSums& A) {
+  constexpr double R = B::kR;
   const double a = fabs(z), sg = z > 0.0 ? 1.0 : (z < 0.0 ? -1.0 : 0.0);
-  // the three edges' geometry and panel lists, lane e for edge e, side by side (the previous face's lists are read)
-  __syncwarp();
-  if (lane < 3) {
-    const int e = lane;
-    EdgeGeo& ge = G3[e];
-    // the edge's first vertex relative to the query: the same operations as P[e]
-    const double pe[3] = {(F[kFV + 3 * e] - q[0]) * ih, (F[kFV + 3 * e + 1] - q[1]) * ih,
-                          (F[kFV + 3 * e + 2] - q[2]) * ih};
+  if (!(a < R)) return;                 // no point of the plane within R: no chord, and the potentials vanish at |z|
+  double M[B::kLine + 1];               // sum_e w_e I_n
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      ge.t[k] = F[kFT + 3 * e + k];
-      ge.mu[k] = F[kFMU + 3 * e + k];
-    }
-    const double len = F[kFLEN + e] * ih;
-    ge.w = ge.mu[0] * pe[0] + ge.mu[1] * pe[1] + ge.mu[2] * pe[2];
-    ge.lo = ge.t[0] * pe[0] + ge.t[1] * pe[1] + ge.t[2] * pe[2];
-    ge.hi = ge.lo + len;
-    ge.c2 = fma(z, z, ge.w * ge.w);
-    const double c = sqrt(ge.c2);
-    double s0 = 0.0, s1 = 0.0;
-    if (c < 1.0) {
-      const double L = sqrt((1.0 - c) * (1.0 + c));
-      s0 = fmax(ge.lo, -L);
-      s1 = fmin(ge.hi, L);
-    }
-    ge.s0 = s0;
-    ge.s1 = s1;
-    ge.np = s1 > s0 ? build_panels<M>(PL3[e], s0, s1, c) : 0;
-  } else if (lane == 3) {
-    // the synthetic-division coefficients of the six divided differences at a = |z| (a face constant), once per face
-    // instead of once per node
-    const int pa = piece<M>(a);
-    fddb<M, 0>(pa, a, FB);
-    fddb<M, 1>(pa, a, FB + kMeshDD);
-    fddb<M, 2>(pa, a, FB + 2 * kMeshDD);
-    fddb<M, 3>(pa, a, FB + 3 * kMeshDD);
-    fddb<M, 4>(pa, a, FB + 4 * kMeshDD);
-    fddb<M, 5>(pa, a, FB + 5 * kMeshDD);
-  }
-  __syncwarp();
-  double Jf[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};          // the face's J sums over its edges
-  double out = 0.0;                                       // the face's summed angles beyond the support
+  for (int n = 0; n <= B::kLine; ++n) M[n] = 0.0;
+  double lam = 0.0, om = 0.0, th = 0.0, s3 = 0.0, out = 0.0;
+  const double zz = z * z;
+#pragma unroll 1
   for (int e = 0; e < 3; ++e) {
-    const EdgeGeo& ge = G3[e];
-    const PanelList& PL = PL3[e];
-    const double t[3] = {ge.t[0], ge.t[1], ge.t[2]}, mu[3] = {ge.mu[0], ge.mu[1], ge.mu[2]};
-    const double w = ge.w, lo = ge.lo, hi = ge.hi, c2 = ge.c2, s0 = ge.s0, s1 = ge.s1;
-    EdgeSums S;
-#pragma unroll
-    for (int i = 0; i < 6; ++i) S.J[i] = 0.0;
-    S.LK1 = S.LK2 = S.LK2b = S.TK2 = S.LW = S.LL = 0.0;
-    if (s1 > s0) {
-      const int np = ge.np;
-      int p = 0;
-      for (int k = lane; k < PL.off[np]; k += 32) {
-        while (k >= PL.off[p + 1]) ++p;
-        const int g = k - PL.off[p];
-        const bool n16 = PL.off[p + 1] - PL.off[p] == 16;
-        const double xg = n16 ? kTriGx16[g] : kRadialGx[g], wg = n16 ? kTriGw16[g] : kRadialGw[g];
-        const double x0 = PL.lo[p], x1 = PL.hi[p];
-        const double hc = 0.5 * (x1 - x0);
-        const double u = fma(hc, xg, 0.5 * (x1 + x0)), wt = wg * hc;
-        if (w != 0.0) node_eval_dd<M>(u, wt, c2, a, z, sg, w, FB, S);
-        node_eval_pot<M>(u, wt, PL.sg[p], c2, z, S);
-      }
-      double v[12] = {S.J[0], S.J[1], S.J[2], S.J[3], S.J[4], S.J[5], S.LK1, S.LK2, S.LK2b, S.TK2, S.LW, S.LL};
-      warp_sum12(v);
-#pragma unroll
-      for (int i = 0; i < 6; ++i) S.J[i] = v[i];
-      S.LK1 = v[6];
-      S.LK2 = v[7];
-      S.LK2b = v[8];
-      S.TK2 = v[9];
-      S.LW = v[10];
-      S.LL = v[11];
+    const double P[3] = {(F[kFV + 3 * e] - q[0]) * ih, (F[kFV + 3 * e + 1] - q[1]) * ih,
+                         (F[kFV + 3 * e + 2] - q[2]) * ih};
+    const double t[3] = {F[kFT + 3 * e], F[kFT + 3 * e + 1], F[kFT + 3 * e + 2]};
+    const double mu[3] = {t[1] * N[2] - t[2] * N[1], t[2] * N[0] - t[0] * N[2], t[0] * N[1] - t[1] * N[0]};
+    const double w = mu[0] * P[0] + mu[1] * P[1] + mu[2] * P[2];
+    const double lo = t[0] * P[0] + t[1] * P[1] + t[2] * P[2], hi = lo + F[kFLEN + e] * ih;
+    const double c2 = fma(w, w, zz) + 1e-200, c = sqrt(c2);
+    double s0 = 0.0, s1 = 0.0;
+    if (c < R) {
+      const double L = sqrt((R - c) * (R + c));
+      s0 = fmax(lo, -L);
+      s1 = fmin(hi, L);
     }
-    if (w != 0.0) {
-      if (s1 > s0) {
-        if (lo < s0) out += angle_between(w, lo, s0);
-        if (s1 < hi) out += angle_between(w, s1, hi);
+    const bool in = s1 > s0;
+    // the angle under which the foot of the query sees the part of the edge beyond R: the parts' unit rotations
+    // multiplied (their sum lies in (-pi, pi), with the sign of w)
+    if (w != 0.0 && (!in || lo < s0 || s1 < hi)) {
+      const double ww = w * w;
+      double x, y;
+      if (!in) {
+        x = fma(lo, hi, ww);
+        y = w * (hi - lo);
       } else {
-        out += angle_between(w, lo, hi);
+        const bool l = lo < s0, r = s1 < hi;
+        const double xl = l ? fma(lo, s0, ww) : 1.0, yl = l ? w * (s0 - lo) : 0.0;
+        const double xr = r ? fma(s1, hi, ww) : 1.0, yr = r ? w * (hi - s1) : 0.0;
+        x = xl * xr - yl * yr;
+        y = xl * yr + yl * xr;
       }
+      out += atan2(y, x);
     }
+    if (!in) continue;
+    const double r0 = lo < s0 ? R : sqrt(fma(s0, s0, c2)), r1 = s1 < hi ? R : sqrt(fma(s1, s1, c2));
+    const double D = s1 - s0, S = s1 + s0;
+    const bool same = s0 > 0.0 || s1 < 0.0;                       // the chord on one side of the foot
+    const double Y = (same ? D * S : s1 * r0 - s0 * r1) / (same ? s1 * r0 + s0 * r1 : c2);
+    const double as = asinh(Y), U = fma(Y, c2, c * D), Bc = (r1 + c) * (r0 + c), s01 = s0 * s1, ic = 1.0 / c;
+    const double kap = w / (c + a);
+    const double Om = 2.0 * atan(kap * U / fmax(fma(kap * kap, s01, Bc), 1e-300));
+    const double Th = 2.0 * atan(U / fmax(Bc + s01, 1e-300));
+    const double ir = 1.0 / (r0 * r1), Y3 = Y * ir;
+    om += Om;
+    lam += w * as - a * Om;
+    th += w * ic * Th;
+    s3 += a * w * Y3;
+    const double sr = S / (r0 + r1), qs = S * sr, eh = 0.5 * D;
+    double pb = r1, pa = r0, T = 1.0, nc2 = c2;
+    double Im = D;                                                // I_(n-1), I_n
+    double I = 0.5 * fma(eh, (r1 + r0) + qs, c2 * as);
+    M[0] = fma(w, D, M[0]);
+    M[1] = fma(w, I, M[1]);
+    // the four line integrals of the potentials and (A2_K2(r1) - A2_K2(r0)) / (r1 - r0)
+    double k1 = fma(MeshC<B, 1, 0>::v, D, MeshNu<B, 1>::v * Th * ic), k2 = fma(MeshC<B, 2, 0>::v, D, MeshNu<B, 2>::v * Y3);
+    double lw = MeshC<B, 3, 0>::v * D, ll = MeshC<B, 4, 0>::v * D, t2 = MeshC<B, 5, 1>::v - MeshNu<B, 5>::v * ir;
+    if constexpr (MeshC<B, 1, 1>::v != 0.0) k1 = fma(MeshC<B, 1, 1>::v, I, k1);
+    if constexpr (MeshC<B, 2, 1>::v != 0.0) k2 = fma(MeshC<B, 2, 1>::v, I, k2);
+    if constexpr (MeshC<B, 3, 1>::v != 0.0) lw = fma(MeshC<B, 3, 1>::v, I, lw);
+    if constexpr (MeshC<B, 4, 1>::v != 0.0) ll = fma(MeshC<B, 4, 1>::v, I, ll);
+    static_for<2, B::kTop + 1>([&](auto nn) {
+      constexpr int n = decltype(nn)::value;
+      T = fma(r1, T, pa);
+      if constexpr (MeshC<B, 5, n>::v != 0.0) t2 = fma(MeshC<B, 5, n>::v, T, t2);
+      pa *= r0;
+      if constexpr (n <= B::kLine) {
+        pb *= r1;
+        nc2 += c2;
+        const double In = fma(nc2, Im, eh * fma(qs, T, pb + pa)) * (1.0 / (n + 1));
+        M[n] = fma(w, In, M[n]);
+        if constexpr (MeshC<B, 1, n>::v != 0.0) k1 = fma(MeshC<B, 1, n>::v, In, k1);
+        if constexpr (MeshC<B, 2, n>::v != 0.0) k2 = fma(MeshC<B, 2, n>::v, In, k2);
+        if constexpr (MeshC<B, 3, n>::v != 0.0) lw = fma(MeshC<B, 3, n>::v, In, lw);
+        if constexpr (MeshC<B, 4, n>::v != 0.0) ll = fma(MeshC<B, 4, n>::v, In, ll);
+        Im = I;
+        I = In;
+      }
+    });
+    const double lk1 = z * k1, lk2b = z * k2, lk2 = z * lk2b, hk = 0.5 * z * (D * sr * t2), wk = w * lk2b, hl = 0.5 * ll;
 #pragma unroll
-    for (int i = 0; i < 6; ++i) Jf[i] += S.J[i];
-    // assembly of the terms with the edge's vectors: lane k adds its accumulator's (the sums are in every lane)
-    if (lane < 28) acc += edge_term_mu(slot, N, t, mu, w, S);
+    for (int i = 0; i < 3; ++i) {
+      A.k1[i] = fma(mu[i], lk1, A.k1[i]);
+      A.k2[i] = fma(mu[i], lk2, A.k2[i]);
+      A.lw[i] = fma(mu[i], lw, A.lw[i]);
+      A.ll[i] = fma(mu[i], hl, A.ll[i]);
+    }
+    int k = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = i; j < 3; ++j, ++k)
+        A.kk[k] += mu[i] * (mu[j] * wk + t[j] * hk) + t[i] * (mu[j] * hk);
   }
-  // the J terms multiply face quantities only: the face's three edges summed, with the angle part of the edges
-  // beyond the support (a face constant times the summed angle) taken once
-  if (out != 0.0) {
-    Jf[0] -= aval_a<M, 0, 1>(a, z, sg) * out;
-    Jf[1] -= aval_a<M, 1, 2>(a, z, sg) * out;
-    Jf[2] -= aval_a<M, 2, 3>(a, z, sg) * out;
-    Jf[3] -= aval_a<M, 3, 0>(a, z, sg) * out;
-    Jf[4] -= aval_a<M, 4, 0>(a, z, sg) * out;
-    Jf[5] -= aval_a<M, 5, 1>(a, z, sg) * out;
+  static_for<0, 6>([&](auto ff) {
+    constexpr int f = decltype(ff)::value, p = kZPow[f], m = kNeg[f];
+    constexpr int top = f == 5 ? B::kTop : B::kLine;
+    double J = 0.0, Aa = 0.0, b = 0.0;
+    // even powers, then odd ones: synthetic division in r^2 by r^2 - z^2
+    static_for<0, top / 2>([&](auto kk) {
+      constexpr int i = top / 2 - decltype(kk)::value;
+      b = fma(zz, b, MeshC<B, f, 2 * i>::v);
+      J = fma(b, M[2 * i - 2], J);
+    });
+    Aa = fma(zz, b, MeshC<B, f, 0>::v);
+    b = 0.0;
+    static_for<0, (top + 1) / 2 - 1>([&](auto kk) {
+      constexpr int i = (top + 1) / 2 - 1 - decltype(kk)::value;
+      b = fma(zz, b, MeshC<B, f, 2 * i + 1>::v);
+      J = fma(b, M[2 * i - 1], J);
+    });
+    b = fma(zz, b, MeshC<B, f, 1>::v);
+    J = fma(b, lam, J) * zpow<p>(z);
+    Aa = fma(a, b, Aa) * zpow<p>(z);                             // z^p A_F(|z|)
+    if constexpr (m > 0) {
+      constexpr double nu = MeshNu<B, f>::v;
+      const double zr = zpow<p - m>(z);
+      if constexpr (m == 1) J -= nu * sg * zr * om;
+      if constexpr (m == 2) J -= nu * sg * sg * zr * th;            // (a query in the face's plane: no r^-m term)
+      if constexpr (m == 3) J -= nu * sg * zr * (s3 + om);
+      Aa += nu * zr * zpow<m>(sg);
+    }
+    A.J[f] += J - Aa * out;
+  });
+}
+
+template <class M, int B = 0>
+__device__ __forceinline__ void face_blocks(const double* __restrict__ F, const double q[3], double ih,
+                                            const double N[3], double z, FaceSums& A) {
+  if constexpr (B < M::kBlocks) {
+    face_block<typename M::template Block<B>>(F, q, ih, N, z, A);
+    face_blocks<M, B + 1>(F, q, ih, N, z, A);
   }
-  if (lane < 28) acc += face_term_j(slot, N, z, Jf);
+}
+
+// The 28 accumulators of a row (W~ units, unit support): M0, M1[3], M2[6] (00 01 02 11 12 22), G0[3], G1[9] (i-major),
+// H[6]; face f adds  M0 += J0;  M1_i += N_i J1 + k1_i;
+// M2_ij += N_i N_j (J2 + J5) + N_i k2_j + k2_i N_j + kk_ij - d_ij J5;
+// G0_i -= N_i J3;  G1_ij -= z N_i N_j J3 + lw_i N_j;  H_ij += z N_i N_j J4 + N_i ll_j + ll_i N_j.
+template <class M>
+__device__ __forceinline__ void face_channels(const double* __restrict__ F, const double q[3], double ih, double* o) {
+  const double N[3] = {F[kFN], F[kFN + 1], F[kFN + 2]};
+  const double z = N[0] * ((F[kFV] - q[0]) * ih) + N[1] * ((F[kFV + 1] - q[1]) * ih) + N[2] * ((F[kFV + 2] - q[2]) * ih);
+  FaceSums A;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) A.k1[i] = A.k2[i] = A.lw[i] = A.ll[i] = 0.0;
+#pragma unroll
+  for (int i = 0; i < 6; ++i) A.kk[i] = A.J[i] = 0.0;
+  face_blocks<M>(F, q, ih, N, z, A);
+  o[0] = A.J[0];
+  const double j25 = A.J[2] + A.J[5], z3 = z * A.J[3], z4 = z * A.J[4];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    o[1 + i] = fma(N[i], A.J[1], A.k1[i]);
+    o[10 + i] = -N[i] * A.J[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) o[13 + 3 * i + j] = -N[j] * fma(z3, N[i], A.lw[i]);
+  }
+  int k = 0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = i; j < 3; ++j, ++k) {
+      const double NN = N[i] * N[j];
+      o[4 + k] = fma(NN, j25, N[i] * A.k2[j] + A.k2[i] * N[j]) + (i == j ? A.kk[k] - A.J[5] : A.kk[k]);
+      o[22 + k] = fma(NN, z4, N[i] * A.ll[j] + A.ll[i] * N[j]);
+    }
+}
+
+// what the accumulator k of a row becomes: its power of the support, and whether the indicator's constants enter (M0;
+// the diagonal of M2; the diagonal of G1, which takes the row's M0)
+struct Channel {
+  int hpow;
+  bool m0, m2, g1;
+};
+__device__ __forceinline__ Channel channel_of(int k) {
+  return {k == 0 ? 0 : (k < 4 ? 1 : (k < 10 ? 2 : (k < 13 ? -1 : (k < 22 ? 0 : -2)))), k == 0,
+          k == 4 || k == 7 || k == 9, k == 13 || k == 17 || k == 21};
+}
+template <class M>
+__device__ __forceinline__ double channel_value(const Channel& c, double acc, double acc0, double ind, double h,
+                                                double ih) {
+  const double ip = kInvPi, m0 = acc0 * ip + ind * 4.0 * M::kQ0;
+  double v = c.m0 ? m0 : acc * ip + (c.g1 ? m0 : 0.0) + (c.m2 ? ind * (4.0 / 3.0) * M::kQ2 : 0.0);
+  if (c.hpow == 1) v *= h;
+  if (c.hpow == 2) v *= h * h;
+  if (c.hpow == -1) v *= ih;
+  if (c.hpow == -2) v *= ih * ih;
+  return v;
 }
 
 // ------------------------------------------------------------------------------------------ kernels
@@ -870,28 +698,6 @@ __global__ void __launch_bounds__(kMeshThreads) k_mesh_rownear(MeshView M, const
   }
 }
 
-template <class M>
-__device__ __forceinline__ void write_row(double* __restrict__ out, int64_t row, const Acc28& A, double ind, double h) {
-  const double ip = kInvPi;
-  const double M0 = A.v[kAM0] * ip + ind * 4.0 * M::kQ0;
-  const double m2c = ind * (4.0 / 3.0) * M::kQ2;
-  const double h2 = h * h, ih = 1.0 / h, ih2 = ih * ih;
-  double* o = out + row * 28;
-  o[0] = M0;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) o[1 + i] = A.v[kAM1 + i] * ip * h;
-#pragma unroll
-  for (int k = 0; k < 6; ++k) o[4 + k] = (A.v[kAM2 + k] * ip + (k == 0 || k == 3 || k == 5 ? m2c : 0.0)) * h2;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) o[10 + i] = A.v[kAG0 + i] * ip * ih;
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) o[13 + 3 * i + j] = A.v[kAG1 + 3 * i + j] * ip + (i == j ? M0 : 0.0);
-#pragma unroll
-  for (int k = 0; k < 6; ++k) o[22 + k] = A.v[kAH + k] * ip * ih2;
-}
-
 // rows without faces in their support: whole-support constants inside, zeros outside, NaN for invalid rows.  Each
 // thread builds its row in shared memory (stride 29 doubles against bank conflicts) and the block writes its
 // contiguous slab of 128 x 28 outputs coalesced.
@@ -908,9 +714,8 @@ __global__ void __launch_bounds__(kMeshThreads) k_mesh_rows(const double* __rest
     if (ind[row] < 0) {
       for (int k = 0; k < 28; ++k) mine[k] = __longlong_as_double(0x7ff8000000000000LL);
     } else {
-      Acc28 A;
-      acc_zero(A);
-      write_row<M>(mine, 0, A, (double)ind[row], sup[row]);
+      const double id = (double)ind[row], h = sup[row];
+      for (int k = 0; k < 28; ++k) mine[k] = channel_value<M>(channel_of(k), 0.0, 0.0, id, h, 1.0 / h);
     }
   }
   __syncthreads();
@@ -919,49 +724,92 @@ __global__ void __launch_bounds__(kMeshThreads) k_mesh_rows(const double* __rest
     out[row0 * 28 + k] = s_rows[(k / 28) * kRowStride + k % 28];
 }
 
-// one warp per work row; warps take rows from a counter (rows differ in their number of faces), and the row's
-// result does not depend on which warp computes it
-// 4 resident CTAs per SM (at most 128 registers a thread): with the divided-difference coefficients formed once per
-// face the c3 leg measured 8.14 ms on B200 against 8.26 ms with 3 CTAs (before that change 3 CTAs were best: 9.0 ms
-// against 9.9 ms with 2 and 10.2 ms with 4)
-#ifndef WSB_MESH_MIN_BLOCKS
-#define WSB_MESH_MIN_BLOCKS 4
-#endif
+// The rows with faces.  A warp takes rows in turn, its lanes search a row's faces together (FaceSearch), and
+// the (row, face) pairs wait in the warp's queue until there are 32: then every lane integrates one pair, whatever row
+// it belongs to, so the lanes stay full although a row has some 20 faces.  The 28 terms of each pair go through shared
+// memory to the lanes k < 28, which add accumulator k of the row pair after pair in queue order -- the row's face order
+// -- and finish the row at its last pair: the result does not depend on the other rows of the queue.
+// On the 2^21-particle scene of 20480 faces (w4, 129 562 rows, 2.6 M pairs) this takes 1.33 ms on B200 against 7.0 ms with
+// a warp per row, the quadrature nodes of one edge after the other over its lanes: 0.45 Kflop an edge instead of some
+// 15 Kflop, and no reduction over the lanes.
+constexpr int kEvalWarps = kMeshThreads / 32;
+constexpr int kEvalBlocks = 3;        // resident CTAs per SM (168 registers)
+constexpr int kPairStride = 29;       // doubles per pair in shared memory (28 and one against bank conflicts)
+
 template <class M>
-__global__ void __launch_bounds__(kMeshThreads, WSB_MESH_MIN_BLOCKS) k_mesh_eval(MeshView Mv, const double* __restrict__ pos,
-                                                           const double* __restrict__ sup,
-                                                           const int32_t* __restrict__ ind,
-                                                           const int32_t* __restrict__ work,
-                                                           const int32_t* __restrict__ nwork,
-                                                           int32_t* __restrict__ grab, double* __restrict__ out) {
-  __shared__ PanelList pl[kMeshThreads / 32][3];
-  __shared__ EdgeGeo eg[kMeshThreads / 32][3];
-  __shared__ double fb[kMeshThreads / 32][6 * kMeshDD];
-  __shared__ double acc[kMeshThreads / 32][28];
+__global__ void __launch_bounds__(kMeshThreads, kEvalBlocks) k_mesh_eval(MeshView Mv, const double* __restrict__ pos,
+                                                                        const double* __restrict__ sup,
+                                                                        const int32_t* __restrict__ ind,
+                                                                        const int32_t* __restrict__ work,
+                                                                        const int32_t* __restrict__ nwork,
+                                                                        double* __restrict__ out) {
+  __shared__ double s_val[kEvalWarps][32 * kPairStride];
+  __shared__ int2 s_queue[kEvalWarps][64];             // (row, face), the row's last pair marked by ~face
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const AccSlot aslot = acc_slot(lane);                  // the accumulator this lane assembles
+  double* const val = s_val[wib];
+  int2* const queue = s_queue[wib];
+  const Channel ch = channel_of(lane);
   const int nw = *nwork;
-  for (int it = 0; it < (1 << 30); ++it) {
-    int slot = 0;
-    if (lane == 0) slot = atomicAdd(grab, 1);
-    slot = __shfl_sync(0xffffffffu, slot, 0);
-    if (slot >= nw) break;
-    const int64_t row = work[slot];
-    const double q[3] = {pos[3 * row], pos[3 * row + 1], pos[3 * row + 2]};
-    const double h = sup[row], ih = 1.0 / h;
-    double mine = 0.0;                                   // accumulator `lane` of the row (lanes < 28)
-    for_candidates_warp(Mv, q, h, lane, [&](int f) {
-      face_contrib_warp<M>(Mv, f, q, ih, pl[wib], eg[wib], fb[wib], lane, aslot, mine);
-    });
-    if (lane < 28) acc[wib][lane] = mine;
+  int qn = 0;
+  double acc = 0.0;                                    // accumulator `lane` of the queue's first row
+  // integrates the first m pairs of the queue and finishes the rows that end among them
+  auto flush = [&](int m) {
     __syncwarp();
-    if (lane == 0) {
-      Acc28 A;
+    if (lane < m) {
+      const int2 p = queue[lane];
+      const int64_t row = p.x;
+      const double qp[3] = {pos[3 * row], pos[3 * row + 1], pos[3 * row + 2]};
+      double o[28];
+      face_channels<M>(Mv.fdata + (int64_t)(p.y < 0 ? ~p.y : p.y) * kFaceDoubles, qp, 1.0 / sup[row], o);
 #pragma unroll
-      for (int i = 0; i < 28; ++i) A.v[i] = acc[wib][i];
-      write_row<M>(out, row, A, (double)ind[row], h);
+      for (int k = 0; k < 28; ++k) val[lane * kPairStride + k] = o[k];
     }
     __syncwarp();
+    for (int k = 0; k < m; ++k) {
+      if (lane < 28) acc += val[k * kPairStride + lane];
+      const int2 p = queue[k];
+      if (p.y < 0) {
+        const double acc0 = __shfl_sync(0xffffffffu, acc, 0), h = sup[p.x];
+        if (lane < 28) out[(int64_t)p.x * 28 + lane] = channel_value<M>(ch, acc, acc0, (double)ind[p.x], h, 1.0 / h);
+        acc = 0.0;
+      }
+    }
+    // the pairs that stay move to the front
+    const int2 p = lane + m < 64 ? queue[lane + m] : make_int2(0, 0);
+    __syncwarp();
+    queue[lane] = p;
+    __syncwarp();
+    qn -= m;
+  };
+  const int warps = gridDim.x * kEvalWarps;
+  int it = blockIdx.x * kEvalWarps + wib - warps, row = 0;
+  bool any = false;                                    // the searched row has pairs
+  FaceSearch fs;
+  fs.base = fs.total = 0;
+  for (;;) {
+    // fill the queue past 32 pairs: the first 32 then never hold the last pair of a row whose search goes on, which may
+    // still have to be marked
+    while (qn <= 32 && it < nw) {
+      if (fs.base < fs.total) {
+        int f;
+        const unsigned mask = fs.next(Mv, lane, f);
+        if ((mask >> lane) & 1u) queue[qn + __popc(mask & ((1u << lane) - 1))] = make_int2(row, f);
+        qn += __popc(mask);
+        any = any || mask;
+        continue;
+      }
+      if (any) {
+        __syncwarp();
+        if (lane == 0) queue[qn - 1].y = ~queue[qn - 1].y;
+        any = false;
+      }
+      it += warps;
+      if (it >= nw) break;
+      row = work[it];
+      fs.start(Mv, pos + 3 * (int64_t)row, sup[row], lane);
+    }
+    if (qn == 0) break;
+    flush(min(qn, 32));
   }
 }
 
@@ -992,7 +840,7 @@ int launch_mesh(const Mesh* m, const double* pos, const double* sup, int64_t n, 
                 int32_t* work, int32_t* nwork, int32_t* near, cudaStream_t st) {
   const MeshView v = view_of(m);
   const unsigned grid = (unsigned)((n + kMeshThreads - 1) / kMeshThreads);
-  WSB_CUDA(cudaMemsetAsync(nwork, 0, 3 * sizeof(int32_t), st));      // work rows, grab counter, listed rows
+  WSB_CUDA(cudaMemsetAsync(nwork, 0, 3 * sizeof(int32_t), st));      // work rows, (unused), listed rows
   k_mesh_rowinfo<<<grid, kMeshThreads, 0, st>>>(v, pos, sup, n, ind, near, nwork + 2);
   WSB_CUDA(cudaGetLastError());
   const unsigned grid_near = (unsigned)std::min<int64_t>((n + kMeshThreads / 32 - 1) / (kMeshThreads / 32), 8192);
@@ -1000,10 +848,10 @@ int launch_mesh(const Mesh* m, const double* pos, const double* sup, int64_t n, 
   WSB_CUDA(cudaGetLastError());
   k_mesh_rows<M><<<grid, kMeshThreads, 0, st>>>(sup, n, ind, out);
   WSB_CUDA(cudaGetLastError());
-  // enough warps to fill the GPU; each loops over rows taken from the counter
-  const int64_t warps = std::min<int64_t>(n, (int64_t)148 * 64);
-  const unsigned egrid = (unsigned)((warps * 32 + kMeshThreads - 1) / kMeshThreads);
-  k_mesh_eval<M><<<egrid, kMeshThreads, 0, st>>>(v, pos, sup, ind, work, nwork, nwork + 1, out);
+  // the resident warps, striding over the work rows (no more warps than rows)
+  const unsigned egrid =
+      (unsigned)std::min<int64_t>((n + kEvalWarps - 1) / kEvalWarps, (int64_t)148 * kEvalBlocks);
+  k_mesh_eval<M><<<egrid, kMeshThreads, 0, st>>>(v, pos, sup, ind, work, nwork, out);
   WSB_CUDA(cudaGetLastError());
   return WSB_OK;
 }
@@ -1074,12 +922,7 @@ extern "C" int wsb_mesh_create(const double* verts, int64_t n_verts, const int32
       double t[3] = {B[0] - A[0], B[1] - A[1], B[2] - A[2]};
       const double len = std::sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
       for (int k = 0; k < 3; ++k) t[k] /= len;
-      const double* n = F + kFN;
-      const double mu[3] = {t[1] * n[2] - t[2] * n[1], t[2] * n[0] - t[0] * n[2], t[0] * n[1] - t[1] * n[0]};
-      for (int k = 0; k < 3; ++k) {
-        F[kFT + 3 * e + k] = t[k];
-        F[kFMU + 3 * e + k] = mu[k];
-      }
+      for (int k = 0; k < 3; ++k) F[kFT + 3 * e + k] = t[k];
       F[kFLEN + e] = len;
     }
     for (int k = 0; k < 3; ++k) {
@@ -1218,7 +1061,7 @@ extern "C" int wsb_mesh_channels(const wsb_mesh* m, int kernel, const double* po
   const size_t s = al256(sizeof(int32_t) * (size_t)n);
   int32_t* work = (int32_t*)base;
   int32_t* ind = inside ? inside : (int32_t*)(base + s);
-  int32_t* nwork = (int32_t*)(base + 2 * s);     // [3]: work rows, grab counter, listed rows
+  int32_t* nwork = (int32_t*)(base + 2 * s);     // [3]: work rows, (unused), listed rows
   int32_t* near = (int32_t*)(base + 2 * s + 256);
   cudaStream_t st = (cudaStream_t)stream;
   switch (kernel) {

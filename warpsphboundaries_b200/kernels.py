@@ -350,7 +350,7 @@ def emit_header() -> str:
     """the generated C++ header with every kernel's block profiles as literal code."""
     out = ["// GENERATED by warpsphboundaries_b200/kernels.py (emit_header); do not edit by hand.",
            "// Exact rational kernel profiles rounded once to double; see that module for the algebra.",
-           "#pragma once", "", "namespace wsb {", ""]
+           "#pragma once", "", "#include <tuple>", "", "namespace wsb {", ""]
     out.append(f"constexpr int kNumKernels = {len(KERNEL_IDS)};")
     # the largest A_n index any kernel needs: forward max_degree, adjoint needs c up to deg+2 (s^2 W) on A
     amax = max(max(kernel(n).max_degree, max(len(b.c) + 1 for b in kernel(n).blocks)) for n in KERNEL_IDS)
@@ -746,6 +746,7 @@ def radial(name: str):
 
 # ------------------------------------------------------------------ 3-D closed surfaces (face -> edge reductions)
 MESH_FUNCS = ("A_K0", "A_K1", "A_K2", "A_W", "A_L", "A2_K2")
+MESH_NEGATIVE = (1, 2, 3, 0, 0, 1)      # the one negative power r^-m of each potential
 
 
 def _leval(d, x):
@@ -753,135 +754,75 @@ def _leval(d, x):
     return sum((c * F(x) ** e for e, c in d.items() if c), F(0))
 
 
-def _compact_potential(bounds, fp):
-    """per piece the Laurent polynomial A_p with A' = r f and A(r) = -int_r^1 t f(t) dt (zero from r = 1 on)."""
-    prims = []
-    for f in fp:
-        prim = {}
-        for n, c in f.items():
-            if n + 2 == 0:
-                raise AssertionError("logarithmic term in a compact potential")
-            prim[n + 2] = prim.get(n + 2, F(0)) + c / (n + 2)
-        prims.append(prim)
-    out = []
-    for p, ((lo, hi), prim) in enumerate(zip(bounds, prims)):
-        tail = sum((_leval(prims[q], bounds[q][1]) - _leval(prims[q], bounds[q][0]) for q in range(p + 1, len(bounds))),
-                   F(0))
-        d = dict(prim)
-        d[0] = d.get(0, F(0)) - _leval(prim, hi) - tail
-        out.append({e: c for e, c in d.items() if c})
-    return out
+def _block_potential(f, R):
+    """A with A' = r f and A(r) = -int_r^R t f(t) dt (a Laurent polynomial; the block's potential is zero from R on)."""
+    out = {}
+    for n, c in f.items():
+        if n + 2 == 0:
+            raise AssertionError("logarithmic term in a compact potential")
+        out[n + 2] = out.get(n + 2, F(0)) + c / (n + 2)
+    out[0] = out.get(0, F(0)) - _leval(out, R)
+    return {e: c for e, c in out.items() if c}
 
 
 @lru_cache(maxsize=None)
-def mesh_tables(name: str):
-    """exact tables of the closed-surface reduction of `name` (unit support, W~ = c3*pi * shape = pi * W):
-    {"bounds": [(lo, hi)] per piece, "Q": (Q0(1), Q1(1), Q2(1)) with Q_k(r) = int_0^r t^(2+k) W~ dt,
-     "funcs": {name: [Laurent dict per piece]} for the compact potentials
-        A_K0, A_K1, A_K2  of K_k(r) = (Q_k(r) - Q_k(1)) / r^(3+k)   (volume potentials of the value moments),
-        A_W, A_L          of W~ and L = W~'/r,
+def mesh_blocks(name: str):
+    """exact tables of the closed-surface reduction of `name` (unit support, W~ = c3*pi * shape = pi * W), one entry per
+    truncated block P(r) 1[r <= R] of W~ (their sum is W~, so every channel is the sum of the blocks' channels):
+    {"R": R, "Q": (Q0, Q1, Q2) with Q_k = int_0^R t^(2+k) P, "funcs": {name: Laurent dict} for the compact potentials
+        A_K0, A_K1, A_K2  of K_k(r) = (int_0^r t^(2+k) P - Q_k) / r^(3+k)   (volume potentials of the value moments),
+        A_W, A_L          of P and L = P'/r,
         A2_K2             of r -> A_K2(r) (the trace term of the in-plane second moment)}."""
     raw = _pieces(name)
     c3pi = radial(name)[1]
-    bounds = [(lo, hi) for lo, hi, _ in raw]
-    Wp = [{n: c3pi * c for n, c in enumerate(co) if c} for _, _, co in raw]
-    Lp = [{n - 2: n * c for n, c in w.items() if n >= 1} for w in Wp]
-    Q, K = [], []
-    for k in range(3):
-        pieces, acc = [], F(0)
-        for (lo, hi), w in zip(bounds, Wp):
-            prim = {n + 3 + k: c / (n + 3 + k) for n, c in w.items()}
-            d = dict(prim)
-            d[0] = d.get(0, F(0)) + acc - _leval(prim, lo)
-            pieces.append(d)
-            acc += _leval(prim, hi) - _leval(prim, lo)
-        Q.append(acc)
-        Kk = []
-        for d in pieces:
-            kd = {}
-            for e, c in d.items():
-                kd[e - 3 - k] = kd.get(e - 3 - k, F(0)) + c
-            kd[-3 - k] = kd.get(-3 - k, F(0)) - acc
-            Kk.append({e: c for e, c in kd.items() if c})
-        K.append(Kk)
-    funcs = {"A_K0": _compact_potential(bounds, K[0]), "A_K1": _compact_potential(bounds, K[1]),
-             "A_K2": _compact_potential(bounds, K[2]), "A_W": _compact_potential(bounds, Wp),
-             "A_L": _compact_potential(bounds, Lp)}
-    funcs["A2_K2"] = _compact_potential(bounds, funcs["A_K2"])
-    for fname, pcs in funcs.items():
-        negs = {e for d in pcs for e in d if e < 0}
-        if len(negs) > 1:
-            raise AssertionError(f"{name} {fname}: more than one negative power {negs}")
-    return {"bounds": bounds, "Q": tuple(Q), "funcs": funcs}
-
-
-def mesh_negative_power(name, fname):
-    pcs = mesh_tables(name)["funcs"][fname]
-    negs = {e for d in pcs for e in d if e < 0}
-    return -min(negs) if negs else 0
-
-
-def _emit_dd(coeffs, x, a):
-    """C++ statements computing (P(x) - P(a)) / (x - a) into `dd` for P = sum coeffs[n] x^n (n >= 0): the synthetic
-    division by (x - a) evaluated by Horner's rule, no cancellation between P(x) and P(a)."""
-    cs = list(coeffs)
-    while len(cs) > 1 and cs[-1] == 0:
-        cs.pop()
-    D = len(cs) - 1
-    if D < 1:
-        return ["dd = 0.0;"]
-    out = [f"double b = {_lit(cs[D])}; dd = b;"]
-    for j in range(D - 2, -1, -1):
-        out.append(f"b = fma({a}, b, {_lit(cs[j + 1])}); dd = fma(dd, {x}, b);")
-    return out
+    out = []
+    for j in range(len(raw) - 1, -1, -1):             # outer piece first, then the differences at the inner knots
+        _, R, c = raw[j]
+        co = list(c) if j == len(raw) - 1 else _padd(list(c), [-x for x in raw[j + 1][2]])
+        P = {n: c3pi * x for n, x in enumerate(_trim(co)) if x}
+        Q, K = [], []
+        for k in range(3):
+            q = {n + 3 + k: x / (n + 3 + k) for n, x in P.items()}
+            Q.append(_leval(q, R))
+            K.append({**{e - 3 - k: x for e, x in q.items()}, -3 - k: -Q[k]})
+        funcs = {f"A_K{k}": _block_potential(K[k], R) for k in range(3)}
+        funcs["A_W"] = _block_potential(P, R)
+        funcs["A_L"] = _block_potential({n - 2: n * x for n, x in P.items() if n}, R)
+        funcs["A2_K2"] = _block_potential(funcs["A_K2"], R)
+        for fname, m in zip(MESH_FUNCS, MESH_NEGATIVE):
+            if any(e < 0 and e != -m for e in funcs[fname]):
+                raise AssertionError(f"{name} {fname}: an unexpected negative power")
+        out.append({"R": R, "Q": tuple(Q), "funcs": funcs})
+    return tuple(out)
 
 
 def emit_mesh() -> list:
-    """generated device code of the closed-surface family: per kernel and compact potential the polynomial part's value
-    and divided difference per piece, the negative power and its coefficient."""
-    import numpy as np
-    x8, w8 = np.polynomial.legendre.leggauss(8)
-    out = ["// ---- 3-D closed surfaces: compact potentials (unit support, W~ = c3*pi * shape); function ids:",
-           "//      0 A_K0, 1 A_K1, 2 A_K2, 3 A_W, 4 A_L, 5 A2_K2",
-           "template <class M, int Fn> struct MeshFn;",
-           "static __device__ const double kMeshGx8[8] = {" + ", ".join(repr(float(x)) for x in x8) + "};",
-           "static __device__ const double kMeshGw8[8] = {" + ", ".join(repr(float(x)) for x in w8) + "};"]
+    """generated tables of the closed-surface family: per kernel and block the radius, the coefficients of the six
+    compact potentials (powers 0, 1, ... of r) and the coefficients of their negative powers."""
+    out = ["// ---- 3-D closed surfaces: compact potentials per truncated block (unit support, W~ = c3*pi * shape); rows:",
+           "//      0 A_K0, 1 A_K1, 2 A_K2, 3 A_W, 4 A_L, 5 A2_K2"]
     for name in RADIAL_KERNELS:
-        t = mesh_tables(name)
-        bounds = t["bounds"]
-        out.append(f"struct Mesh_{name} {{")
-        out.append(f"  static constexpr int kPieces = {len(bounds)};")
-        out.append(f"  static constexpr double kBreak = {_lit(bounds[0][1]) if len(bounds) > 1 else '2.0'};   // end of the inner piece")
-        out.append(f"  static constexpr double kQ0 = {_lit(t['Q'][0])}, kQ1 = {_lit(t['Q'][1])}, kQ2 = {_lit(t['Q'][2])};")
-        out.append("};")
-        for fi, fname in enumerate(MESH_FUNCS):
-            pcs = t["funcs"][fname]
-            m = mesh_negative_power(name, fname)
-            out.append(f"template <> struct MeshFn<Mesh_{name}, {fi}> {{   // {fname}")
-            out.append(f"  static constexpr int kNeg = {m};")
-            for p, d in enumerate(pcs):
-                poly = [d.get(n, F(0)) for n in range(max([e for e in d if e >= 0], default=0) + 1)]
-                nu = d.get(-m, F(0)) if m else F(0)
-                out.append(f"  static constexpr double kNu{p} = {_lit(nu)};")
-                out.append(f"  __host__ __device__ static __forceinline__ double poly{p}(double x) {{ return {_horner(poly, 'x')}; }}")
-                body = " ".join(_emit_dd(poly, "x", "a"))
-                out.append(f"  __host__ __device__ static __forceinline__ double dd{p}(double x, double a) {{ double dd; {body} return dd; }}")
-                # the same divided difference in two halves: the synthetic-division coefficients b (they depend on a
-                # only, so a caller forms them once per a) and Horner's rule over b at x -- the same fma sequence
-                cs = list(poly)
-                while len(cs) > 1 and cs[-1] == 0:
-                    cs.pop()
-                D = len(cs) - 1
-                out.append(f"  static constexpr int kDD{p} = {max(D, 0)};")
-                if D >= 1:
-                    bs = [f"b[0] = {_lit(cs[D])};"] + [f"b[{k}] = fma(a, b[{k - 1}], {_lit(cs[D - k])});"
-                                                       for k in range(1, D)]
-                    hs = ["double dd = b[0];"] + [f"dd = fma(dd, x, b[{k}]);" for k in range(1, D)]
-                else:
-                    bs, hs = [], ["double dd = 0.0;"]
-                out.append(f"  __host__ __device__ static __forceinline__ void ddb{p}(double a, double* b) {{ {' '.join(bs)} }}")
-                out.append(f"  __host__ __device__ static __forceinline__ double ddh{p}(double x, const double* b) {{ {' '.join(hs)} return dd; }}")
+        blocks = mesh_blocks(name)
+        for b, t in enumerate(blocks):
+            fs = [t["funcs"][f] for f in MESH_FUNCS]
+            top = max(max(f) for f in fs)
+            line = max(max(f) for f in fs[:5])
+            out.append(f"struct MeshBlock_{name}_{b} {{")
+            out.append(f"  static constexpr double kR = {_lit(t['R'])};")
+            out.append(f"  static constexpr int kTop = {top};      // highest power of A2_K2")
+            out.append(f"  static constexpr int kLine = {line};     // highest power of the other potentials")
+            out.append("  static constexpr double kNu[6] = {" +
+                       ", ".join(_lit(f.get(-m, F(0)) if m else F(0)) for f, m in zip(fs, MESH_NEGATIVE)) + "};")
+            out.append("  static constexpr double kC[6][kTop + 1] = {" + ", ".join(
+                "{" + ", ".join(_lit(f.get(n, F(0))) for n in range(top + 1)) + "}" for f in fs) + "};")
             out.append("};")
+        q = [sum(t["Q"][k] for t in blocks) for k in range(3)]
+        out.append(f"struct Mesh_{name} {{")
+        out.append(f"  static constexpr int kBlocks = {len(blocks)};")
+        out.append(f"  static constexpr double kQ0 = {_lit(q[0])}, kQ2 = {_lit(q[2])};")
+        out.append("  template <int B> using Block = std::tuple_element_t<B, std::tuple<" +
+                   ", ".join(f"MeshBlock_{name}_{b}" for b in range(len(blocks))) + ">>;")
+        out.append("};")
     out.append("")
     return out
 
