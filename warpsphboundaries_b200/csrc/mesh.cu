@@ -26,9 +26,9 @@
 //    so a face needs its edges' w-weighted moments sum_e w_e I_n and Lambda = sum_e w_e int ds / (r + a) only, each
 //    potential one dot product with them (synthetic division by r^2 - a^2, once per face).  With
 //    Y = (s1 r0 - s0 r1) / c^2 (formed without cancellation), U = c^2 Y + c D, B = (r1 + c)(r0 + c), kappa = w / (c + a):
-//      int ds / r = asinh Y,                      int c ds / r^2 = 2 atan(U / (B + s0 s1)) = Theta,
+//      int ds / r = log1p(2 U / ((r1 - s1 + c) (r0 + s0 + c))) = L,   int c ds / r^2 = 2 atan(U / (B + s0 s1)) = Theta,
 //      int ds / r^3 = Y / (r0 r1),                int w ds / (r (r + a)) = 2 atan(kappa U / (B + kappa^2 s0 s1)) = Omega,
-//      w int ds / (r + a) = w asinh Y - a Omega,  I_n = (E_n + n c^2 I_(n-2)) / (n + 1),  E_n = [s r^n],
+//      w int ds / (r + a) = w L - a Omega,  I_n = (E_n + n c^2 I_(n-2)) / (n + 1),  E_n = [s r^n],
 //      E_n = D/2 (r1^n + r0^n + S^2 / (r0 + r1) T_n),  T_n = (r1^n - r0^n) / (r1 - r0)      (D = s1 - s0, S = s1 + s0):
 //    sums of terms of one sign throughout, so a short edge keeps its relative accuracy.  The rounding of a channel is
 //    that of the potentials' monomial form (sum |c_n| / max |A|).
@@ -39,7 +39,6 @@
 // The exact rational potentials are generated by warpsphboundaries_b200/kernels.py (mesh_blocks, emit_mesh).
 #include <algorithm>
 #include <cmath>
-#include <map>
 #include <vector>
 
 #include "common.cuh"
@@ -55,43 +54,41 @@ struct Mesh {
   int32_t nx = 1, ny = 1, nz = 1;
   int64_t n_items = 0, n_col_items = 0;
   double* fdata = nullptr;     // [n_faces * kFaceDoubles]
-  int32_t* fcell = nullptr;    // [n_faces * 3] lowest cell of the face's box
-  int32_t* fvid = nullptr;     // [n_faces * 3] vertex ids
-  int32_t* cstart = nullptr;   // [nx*ny*nz + 1]
-  int32_t* citems = nullptr;   // faces per cell
-  int32_t* colstart = nullptr; // [nx*ny + 1] faces per (x, y) column
+  int32_t words = 1;           // 64-bit words of a row's hit mask (at most kMaxWords)
+  int64_t* nstart = nullptr;   // [nx*ny*nz + 1]
+  int32_t* nitems = nullptr;   // per cell the faces a query of the cell may reach (each once)
+  double col = 1;              // size of an (x, y) column: half a cell (a cell where that would list too many faces)
+  int32_t ncx = 1, ncy = 1;
+  int32_t* colstart = nullptr; // [ncx*ncy + 1] faces per column
   int32_t* colitems = nullptr;
   uint8_t* cflag = nullptr;    // [nx*ny*nz] kCellEmpty | kCellInside | kCellNear
 };
 
 // per-cell flags: no face box meets the cell (so the surface does not cross it and every point of it has the inside
-// status of its centre); that status; a face box meets one of the 27 cells around it (a query in the cell may have
-// candidate faces)
+// status of its centre); that status; the cell's face list is not empty (a query in the cell may have candidate faces)
 enum : uint8_t { kCellEmpty = 1, kCellInside = 2, kCellNear = 4 };
 
 // per face, one 256-byte record: v0 v1 v2 (9), unit normal N (3), edge tangents t0 t1 t2 (9), edge lengths (3), box lo
-// (3), box hi (3), 2 unused; read by 32-byte loads
+// (3), box hi (3), the edges that run from the lower to the higher vertex id (bits 0-2, as a number), 1 unused
 constexpr int kFaceDoubles = 32;
-enum { kFV = 0, kFN = 9, kFT = 12, kFLEN = 21, kFLO = 24, kFHI = 27 };
+enum { kFV = 0, kFN = 9, kFT = 12, kFLEN = 21, kFLO = 24, kFHI = 27, kFORD = 30 };
 
 struct MeshView {
   const double* fdata;
-  const int32_t* fcell;
-  const int32_t* fvid;
-  const int32_t* cstart;
-  const int32_t* citems;
+  const int64_t* nstart;
+  const int32_t* nitems;
   const int32_t* colstart;
   const int32_t* colitems;
   const uint8_t* cflag;
-  double lo0, lo1, lo2, cell;
-  int32_t nx, ny, nz;
+  double lo0, lo1, lo2, cell, col;
+  int32_t nx, ny, nz, ncx, ncy;
 };
 
 namespace {
 
 MeshView view_of(const Mesh* m) {
-  return MeshView{m->fdata, m->fcell, m->fvid, m->cstart, m->citems, m->colstart, m->colitems, m->cflag,
-                  m->lo[0], m->lo[1], m->lo[2], m->cell, m->nx, m->ny, m->nz};
+  return MeshView{m->fdata, m->nstart, m->nitems, m->colstart, m->colitems, m->cflag,
+                  m->lo[0], m->lo[1], m->lo[2], m->cell, m->col, m->nx, m->ny, m->nz, m->ncx, m->ncy};
 }
 
 __device__ __forceinline__ int cell_coord(double x, double lo, double cell, int n) {
@@ -115,53 +112,43 @@ __device__ __forceinline__ double edge_fn(double ax, double ay, double bx, doubl
 // lies above z)
 __device__ __forceinline__ bool column_cross(const MeshView& M, int f, double x, double y, double z) {
   const double* F = M.fdata + (int64_t)f * kFaceDoubles;
-  const double nzf = F[kFN + 2];
+  double V[12];                                     // the vertices and the normal, loaded together
+#pragma unroll
+  for (int k = 0; k < 3; ++k) ld4_nc(F + 4 * k, V[4 * k], V[4 * k + 1], V[4 * k + 2], V[4 * k + 3]);
+  const int ord = (int)F[kFORD];
+  const double nzf = V[kFN + 2];
   if (nzf == 0.0) return false;                     // vertical face: its projection has no interior
-  const int* vid = M.fvid + 3 * f;
   const double sgn = nzf > 0.0 ? 1.0 : -1.0;        // counter-clockwise projection for N.z > 0
+  bool owns = true;
+#pragma unroll
   for (int e = 0; e < 3; ++e) {
-    const int a = e, b = (e + 1) % 3;
-    const bool fwd = vid[a] < vid[b];
-    const double* A = F + kFV + 3 * (fwd ? a : b);
-    const double* B = F + kFV + 3 * (fwd ? b : a);
-    double E = edge_fn(A[0], A[1], B[0], B[1], x, y);
-    if (!fwd) E = -E;
+    const double ax = V[3 * e], ay = V[3 * e + 1], bx = V[3 * ((e + 1) % 3)], by = V[3 * ((e + 1) % 3) + 1];
+    const bool fwd = (ord >> e) & 1;
+    double E = fwd ? edge_fn(ax, ay, bx, by, x, y) : -edge_fn(bx, by, ax, ay, x, y);
     E *= sgn;
-    if (E < 0.0) return false;
+    if (E < 0.0) owns = false;
     if (E == 0.0) {
-      const double* P0 = F + kFV + 3 * a;
-      const double* P1 = F + kFV + 3 * b;
-      const double dx = (P1[0] - P0[0]) * sgn, dy = (P1[1] - P0[1]) * sgn;
-      if (!(dy > 0.0 || (dy == 0.0 && dx < 0.0))) return false;
+      const double dx = (bx - ax) * sgn, dy = (by - ay) * sgn;
+      if (!(dy > 0.0 || (dy == 0.0 && dx < 0.0))) owns = false;
     }
   }
-  const double zt = F[kFV + 2] - (F[kFN] * (x - F[kFV]) + F[kFN + 1] * (y - F[kFV + 1])) / nzf;
-  return zt > z;
+  const double zt = V[2] - (V[kFN] * (x - V[0]) + V[kFN + 1] * (y - V[1])) / nzf;
+  return owns && zt > z;
+}
+
+// the column of (x, y), -1 outside the grid (no face above or below)
+__device__ __forceinline__ int column_of(const MeshView& M, double x, double y) {
+  const int ix = cell_coord(x, M.lo0, M.col, M.ncx), iy = cell_coord(y, M.lo1, M.col, M.ncy);
+  return ix < 0 || iy < 0 || ix >= M.ncx || iy >= M.ncy ? -1 : iy * M.ncx + ix;
 }
 
 __device__ int mesh_inside(const MeshView& M, double x, double y, double z) {
-  const int ix = cell_coord(x, M.lo0, M.cell, M.nx), iy = cell_coord(y, M.lo1, M.cell, M.ny);
-  if (ix < 0 || iy < 0 || ix >= M.nx || iy >= M.ny) return 0;
-  const int col = iy * M.nx + ix;
+  const int col = column_of(M, x, y);
+  if (col < 0) return 0;
   int parity = 0;
   for (int k = M.colstart[col]; k < M.colstart[col + 1]; ++k)
     if (column_cross(M, M.colitems[k], x, y, z)) parity ^= 1;
   return parity;
-}
-
-// mesh_inside for a whole warp (every lane calls it with the same point): the lanes test the column's faces 32 at a
-// time; the parity of the crossings (an integer count) is the same as the serial walk's
-__device__ __forceinline__ int mesh_inside_warp(const MeshView& M, double x, double y, double z, int lane) {
-  const int ix = cell_coord(x, M.lo0, M.cell, M.nx), iy = cell_coord(y, M.lo1, M.cell, M.ny);
-  if (ix < 0 || iy < 0 || ix >= M.nx || iy >= M.ny) return 0;
-  const int col = iy * M.nx + ix;
-  const int e = M.colstart[col + 1];
-  int crossings = 0;
-  for (int base = M.colstart[col]; base < e; base += 32) {
-    const int k = base + lane;
-    crossings += __popc(__ballot_sync(0xffffffffu, k < e && column_cross(M, M.colitems[k], x, y, z)));
-  }
-  return crossings & 1;
 }
 
 // squared distance from the origin to the triangle P (unit coordinates relative to the query)
@@ -215,149 +202,115 @@ __device__ __forceinline__ double tri_dist2(const double P[3][3]) {
 }
 
 // ------------------------------------------------------------------------------------------ candidate faces
-// The cells of the block x0..x1, y0..y1, z0..z1 (at most 27) for a warp: lane l < number of cells takes cell ordinal
-// l (z outermost, then y, then x -- the order of nested loops) and returns its first item (beg) and the exclusive
-// prefix of the items of the cells before it (pref; a cell `keep` rejects has none).  Returns the block's total.
-template <class Keep>
-__device__ __forceinline__ int block_cells(const MeshView& M, int x0, int x1, int y0, int y1, int z0, int z1, int lane,
-                                           Keep&& keep, int& beg, int& pref) {
-  const int nxr = x1 - x0 + 1, nyr = y1 - y0 + 1, nc = nxr * nyr * (z1 - z0 + 1);
-  int cnt = 0;
-  beg = 0;
-  if (lane < nc) {
-    const int i = x0 + lane % nxr, j = y0 + (lane / nxr) % nyr, k = z0 + lane / (nxr * nyr);
-    if (keep(i, j, k)) {
-      const int c = (k * M.ny + j) * M.nx + i;
-      beg = M.cstart[c];
-      cnt = M.cstart[c + 1] - beg;
-    }
-  }
-  int inc = cnt;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += v;
-  }
-  pref = inc - cnt;
-  return __shfl_sync(0xffffffffu, inc, 31);
-}
+// the faces by cell as the host counts them: every cell lists the faces whose box overlaps it
+struct BoxLists {
+  const int32_t* start;   // [nx*ny*nz + 1]
+  const int32_t* items;
+  const int32_t* fcell;   // [n_faces * 3] lowest cell of the face's box
+};
 
-// the cell ordinal of flattened item t (< total): the last lane whose prefix is <= t (prefixes do not decrease with
-// the lane; an empty cell shares the next cell's prefix, lanes past the cells hold the total), by a binary search over
-// the lanes; every lane of the warp takes part
-__device__ __forceinline__ int cell_ordinal(int pref, int t) {
-  int lo = 0;
+// The candidate list of one cell, once per mesh, by a warp: the faces listed in the 27 cells around it whose box comes
+// within a cell's size (>= every support) of the cell's box -- each face once (a face listed in several of the 27 cells
+// is taken in the lowest of them inside the block), in cell order and item order within a cell.  The margin of 1e-6
+// is far above the rounding of the cell boxes: a face is only left out when clearly beyond reach.  Writes the list to
+// `dst` when it is given; returns its length.
+__device__ __forceinline__ int cell_faces(const MeshView& M, const BoxLists& L, int64_t c, int lane, int32_t* dst) {
+  const int cx = (int)(c % M.nx), cy = (int)((c / M.nx) % M.ny), cz = (int)(c / ((int64_t)M.nx * M.ny));
+  const double b[3] = {fma((double)cx, M.cell, M.lo0), fma((double)cy, M.cell, M.lo1), fma((double)cz, M.cell, M.lo2)};
+  const double reach2 = M.cell * M.cell * (1.0 + 1e-6);
+  int len = 0;
+  for (int k = max(cz - 1, 0); k <= min(cz + 1, M.nz - 1); ++k)
+    for (int j = max(cy - 1, 0); j <= min(cy + 1, M.ny - 1); ++j) {
+      const int64_t r0 = ((int64_t)k * M.ny + j) * M.nx;
+      for (int i = max(cx - 1, 0); i <= min(cx + 1, M.nx - 1); ++i) {
+        const int e = L.start[r0 + i + 1];
+        for (int base = L.start[r0 + i]; base < e; base += 32) {
+          bool take = false;
+          int f = 0;
+          if (base + lane < e) {
+            f = L.items[base + lane];
+            const int32_t* fc = L.fcell + 3 * (int64_t)f;
+            if (max(fc[0], cx - 1) == i && max(fc[1], cy - 1) == j && max(fc[2], cz - 1) == k) {
+              const double* F = M.fdata + (int64_t)f * kFaceDoubles;
+              double d2 = 0.0;
 #pragma unroll
-  for (int step = 16; step > 0; step >>= 1) {
-    const int pv = __shfl_sync(0xffffffffu, pref, lo + step);
-    if (pv <= t) lo += step;
-  }
-  return lo;
-}
-
-// The faces of the 27 cells around the query's cell that come within h of the query (box first, then the exact
-// triangle distance, both tested by the lanes in parallel); a face listed in several of those cells is taken in one of
-// them only (the lowest corner of its box inside the 27-cell block).  Held by a whole warp for one query: the (cell,
-// item) pairs of the block are flattened over the lanes, next() tests 32 of them (whatever cell they belong to) and
-// returns the mask of the lanes whose face f is within h -- in cell order and item order within a cell, a fixed order,
-// so the sums over the faces do not depend on the launch.
-struct FaceSearch {
-  double q[3], h;
-  int cx, cy, cz, x0, y0, z0, nxr, nyr, beg, pref, base, total;
-
-  __device__ __forceinline__ void start(const MeshView& M, const double* __restrict__ pos, double sup, int lane) {
-#pragma unroll
-    for (int a = 0; a < 3; ++a) q[a] = pos[a];
-    h = sup;
-    cx = cell_coord(q[0], M.lo0, M.cell, M.nx);
-    cy = cell_coord(q[1], M.lo1, M.cell, M.ny);
-    cz = cell_coord(q[2], M.lo2, M.cell, M.nz);
-    x0 = max(cx - 1, 0);
-    y0 = max(cy - 1, 0);
-    z0 = max(cz - 1, 0);
-    const int x1 = min(cx + 1, M.nx - 1), y1 = min(cy + 1, M.ny - 1), z1 = min(cz + 1, M.nz - 1);
-    nxr = x1 - x0 + 1;
-    nyr = y1 - y0 + 1;
-    base = total = 0;
-    if (x0 > x1 || y0 > y1 || z0 > z1) return;
-    total = block_cells(M, x0, x1, y0, y1, z0, z1, lane, [](int, int, int) { return true; }, beg, pref);
-  }
-
-  __device__ __forceinline__ unsigned next(const MeshView& M, int lane, int& f) {
-    const int t = base + lane;
-    base += 32;
-    const int o = cell_ordinal(pref, t);
-    const int b = __shfl_sync(0xffffffffu, beg, o), p = __shfl_sync(0xffffffffu, pref, o);
-    f = -1;
-    bool hit = false;
-    if (t < total) {
-      const int i = x0 + o % nxr, j = y0 + (o / nxr) % nyr, k = z0 + o / (nxr * nyr);
-      f = M.citems[b + (t - p)];
-      const int* fc = M.fcell + 3 * f;
-      if (max(fc[0], cx - 1) == i && max(fc[1], cy - 1) == j && max(fc[2], cz - 1) == k) {
-        const double* F = M.fdata + (int64_t)f * kFaceDoubles;
-        double d2 = 0.0;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          const double d = fmax(0.0, fmax(F[kFLO + a] - q[a], q[a] - F[kFHI + a]));
-          d2 = fma(d, d, d2);
-        }
-        if (d2 < h * h) {
-          // the exact triangle distance (unit coordinates relative to the query, the operations of the face integral's)
-          const double ih = 1.0 / h;
-          double P[3][3];
-#pragma unroll
-          for (int v = 0; v < 3; ++v)
-#pragma unroll
-            for (int a = 0; a < 3; ++a) P[v][a] = (F[kFV + 3 * v + a] - q[a]) * ih;
-          hit = tri_dist2(P) < 1.0;
+              for (int a = 0; a < 3; ++a) {
+                const double d = fmax(0.0, fmax(F[kFLO + a] - (b[a] + M.cell), b[a] - F[kFHI + a]));
+                d2 = fma(d, d, d2);
+              }
+              take = d2 < reach2;
+            }
+          }
+          const unsigned m = __ballot_sync(0xffffffffu, take);
+          if (dst && take) dst[len + __popc(m & ((1u << lane) - 1))] = f;
+          len += __popc(m);
         }
       }
     }
-    return __ballot_sync(0xffffffffu, hit);
+  return len;
+}
+
+// whether face f comes within h of the query (unit coordinates relative to the query, the operations of the face
+// integral's)
+__device__ __forceinline__ bool face_within(const MeshView& M, int f, const double q[3], double ih) {
+  const double* F = M.fdata + (int64_t)f * kFaceDoubles;
+  double v[12];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) ld4_nc(F + kFV + 4 * k, v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+  double P[3][3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) P[k][a] = (v[3 * k + a] - q[a]) * ih;
+  return tri_dist2(P) < 1.0;
+}
+
+// The items that a warp's batch of rows brings, flattened over the lanes: lane r < kRows holds the length of its row's
+// items and the exclusive prefix of the lengths before it (lanes past the batch: the total).  Unsigned: a round may
+// start past the last item.
+template <int kRows>
+struct Flat {
+  unsigned len, pref, total;
+  __device__ __forceinline__ void set(unsigned length, int lane) {
+    len = length;
+    unsigned inc = length;
+#pragma unroll
+    for (int o = 1; o < kRows; o <<= 1) {
+      const unsigned v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    total = __shfl_sync(0xffffffffu, inc, kRows - 1);
+    pref = lane < kRows ? inc - len : total;
+  }
+  // the batch row of item t (the last lane whose prefix is <= t) and the item's place in it; every lane takes part
+  __device__ __forceinline__ int row_of(unsigned t, unsigned& place) const {
+    int r = 0;
+#pragma unroll
+    for (int step = kRows / 2; step > 0; step >>= 1)
+      if (__shfl_sync(0xffffffffu, pref, r + step) <= t) r += step;
+    place = t - __shfl_sync(0xffffffffu, pref, r);
+    return r;
+  }
+  // of the round that starts at item `base`: the first of lane r's items in it, the lane that holds it, how many
+  __device__ __forceinline__ int part(unsigned base, unsigned& place, int& lane0) const {
+    const int64_t a = max((int64_t)pref - base, (int64_t)0), b = min((int64_t)pref + len - base, (int64_t)32);
+    lane0 = (int)a;
+    place = (unsigned)(base + a - pref);
+    return (int)(b - a);
   }
 };
 
-// whether any face box comes within h of the query (the cells of FaceSearch, stopping at the first hit),
-// for a whole warp (every lane calls it with the same query): the (cell, item) pairs are flattened over the lanes.
-// A cell whose own box is h or more from the query is skipped: a face box within h of the query has its point nearest
-// to the query in a cell within h, and every cell its box overlaps lists the face (a relative margin far above the
-// rounding of the cell boxes: a cell is only skipped when clearly out of reach).
-__device__ __forceinline__ bool has_candidate_warp(const MeshView& M, const double q[3], double h, int lane) {
-  const int cx = cell_coord(q[0], M.lo0, M.cell, M.nx), cy = cell_coord(q[1], M.lo1, M.cell, M.ny),
-            cz = cell_coord(q[2], M.lo2, M.cell, M.nz);
-  const int x0 = max(cx - 1, 0), x1 = min(cx + 1, M.nx - 1), y0 = max(cy - 1, 0), y1 = min(cy + 1, M.ny - 1),
-            z0 = max(cz - 1, 0), z1 = min(cz + 1, M.nz - 1);
-  if (x0 > x1 || y0 > y1 || z0 > z1) return false;
-  const double h2 = h * h;
-  auto gap2 = [&](double x, double lo, int i) {
-    const double a = fma((double)i, M.cell, lo), d = fmax(0.0, fmax(a - x, x - (a + M.cell)));
-    return d * d;
-  };
-  auto reach = [&](int i, int j, int k) {
-    return gap2(q[0], M.lo0, i) + gap2(q[1], M.lo1, j) + gap2(q[2], M.lo2, k) < h2 * (1.0 + 1e-9);
-  };
-  int beg, pref;
-  const int total = block_cells(M, x0, x1, y0, y1, z0, z1, lane, reach, beg, pref);
-  for (int base = 0; base < total; base += 32) {
-    const int t = base + lane;
-    const int o = cell_ordinal(pref, t);
-    const int b = __shfl_sync(0xffffffffu, beg, o), p = __shfl_sync(0xffffffffu, pref, o);
-    bool hit = false;
-    if (t < total) {
-      const double* F = M.fdata + (int64_t)M.citems[b + (t - p)] * kFaceDoubles;
-      double d2 = 0.0;
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        const double d = fmax(0.0, fmax(F[kFLO + a] - q[a], q[a] - F[kFHI + a]));
-        d2 = fma(d, d, d2);
-      }
-      hit = d2 < h2;
-    }
-    if (__any_sync(0xffffffffu, hit)) return true;
-  }
-  return false;
-}
+// a row with faces, as the integration reads it: the query, its support, its list and the hits among the list's first
+// 64 x words faces (a word of the mask each 64); faces beyond are tested when they are integrated
+constexpr int kMaxWords = 8;
+struct __align__(32) MeshRow {
+  double q[3], h;
+  int64_t first;        // first item of the list
+  int32_t len, tag;     // its length; row | inside << 30
+  int32_t at, pad[3];   // the row's place in the masks
+};
+static_assert(sizeof(MeshRow) == 64, "row record layout");
+constexpr int kRowMask = (1 << 30) - 1;
 
 // ------------------------------------------------------------------------------------------ face integrals
 template <int I, int N, class Fn>
@@ -407,7 +360,8 @@ __device__ __forceinline__ void face_block(const double* __restrict__ F, const d
   double M[B::kLine + 1];               // sum_e w_e I_n
 #pragma unroll
   for (int n = 0; n <= B::kLine; ++n) M[n] = 0.0;
-  double lam = 0.0, om = 0.0, th = 0.0, s3 = 0.0, out = 0.0;
+  double lam = 0.0, om = 0.0, th = 0.0, s3 = 0.0, ox = 1.0, oy = 0.0;
+  float turn = 0.0f;
   const double zz = z * z;
 #pragma unroll 1
   for (int e = 0; e < 3; ++e) {
@@ -425,8 +379,9 @@ __device__ __forceinline__ void face_block(const double* __restrict__ F, const d
       s1 = fmin(hi, L);
     }
     const bool in = s1 > s0;
-    // the angle under which the foot of the query sees the part of the edge beyond R: the parts' unit rotations
-    // multiplied (their sum lies in (-pi, pi), with the sign of w)
+    // the angle under which the foot of the query sees the part of the edge beyond R: the parts' rotations multiplied
+    // (their sum lies in (-pi, pi), with the sign of w), and those of the three edges: one atan2 a face; the float sum
+    // of the edges' angles tells the full turns
     if (w != 0.0 && (!in || lo < s0 || s1 < hi)) {
       const double ww = w * w;
       double x, y;
@@ -440,26 +395,33 @@ __device__ __forceinline__ void face_block(const double* __restrict__ F, const d
         x = xl * xr - yl * yr;
         y = xl * yr + yl * xr;
       }
-      out += atan2(y, x);
+      const double m = 1.0 / (fabs(x) + fabs(y));
+      x *= m;
+      y *= m;
+      turn += atan2f((float)y, (float)x);
+      const double t0 = ox * x - oy * y;
+      oy = ox * y + oy * x;
+      ox = t0;
     }
     if (!in) continue;
     const double r0 = lo < s0 ? R : sqrt(fma(s0, s0, c2)), r1 = s1 < hi ? R : sqrt(fma(s1, s1, c2));
     const double D = s1 - s0, S = s1 + s0;
     const bool same = s0 > 0.0 || s1 < 0.0;                       // the chord on one side of the foot
     const double Y = (same ? D * S : s1 * r0 - s0 * r1) / (same ? s1 * r0 + s0 * r1 : c2);
-    const double as = asinh(Y), U = fma(Y, c2, c * D), Bc = (r1 + c) * (r0 + c), s01 = s0 * s1, ic = 1.0 / c;
-    const double kap = w / (c + a);
+    const double U = fma(Y, c2, c * D), Bc = (r1 + c) * (r0 + c), s01 = s0 * s1, ca = c + a;
+    const double as = log1p(2.0 * U / ((r1 - s1 + c) * (r0 + s0 + c)));
+    const double ica = 1.0 / (c * ca), ic = ica * ca, kap = w * (ica * c);
+    const double rr = r0 * r1, rs = r0 + r1, irs = 1.0 / (rr * rs), ir = irs * rs, Y3 = Y * ir;
     const double Om = 2.0 * atan(kap * U / fmax(fma(kap * kap, s01, Bc), 1e-300));
     const double Th = 2.0 * atan(U / fmax(Bc + s01, 1e-300));
-    const double ir = 1.0 / (r0 * r1), Y3 = Y * ir;
     om += Om;
     lam += w * as - a * Om;
     th += w * ic * Th;
     s3 += a * w * Y3;
-    const double sr = S / (r0 + r1), qs = S * sr, eh = 0.5 * D;
+    const double sr = S * (irs * rr), qs = S * sr, eh = 0.5 * D;
     double pb = r1, pa = r0, T = 1.0, nc2 = c2;
     double Im = D;                                                // I_(n-1), I_n
-    double I = 0.5 * fma(eh, (r1 + r0) + qs, c2 * as);
+    double I = 0.5 * fma(eh, rs + qs, c2 * as);
     M[0] = fma(w, D, M[0]);
     M[1] = fma(w, I, M[1]);
     // the four line integrals of the potentials and (A2_K2(r1) - A2_K2(r0)) / (r1 - r0)
@@ -501,6 +463,11 @@ __device__ __forceinline__ void face_block(const double* __restrict__ F, const d
 #pragma unroll
       for (int j = i; j < 3; ++j, ++k)
         A.kk[k] += mu[i] * (mu[j] * wk + t[j] * hk) + t[i] * (mu[j] * hk);
+  }
+  double out = 0.0;
+  if (turn != 0.0f) {
+    out = atan2(oy, ox);
+    out += kTwoPi * rint((turn - out) * (1.0 / kTwoPi));
   }
   static_for<0, 6>([&](auto ff) {
     constexpr int f = decltype(ff)::value, p = kZPow[f], m = kNeg[f];
@@ -602,214 +569,366 @@ __device__ __forceinline__ double channel_value(const Channel& c, double acc, do
 // ------------------------------------------------------------------------------------------ kernels
 constexpr int kMeshThreads = 128;
 
+// the length of every cell's candidate list (fill == 0), then the lists (fill == 1): a warp per cell, once per mesh
+__global__ void __launch_bounds__(kMeshThreads) k_mesh_lists(MeshView M, BoxLists L, int fill, int32_t* __restrict__ len,
+                                                            int32_t* __restrict__ items) {
+  const int lane = threadIdx.x & 31;
+  const int64_t n = (int64_t)M.nx * M.ny * M.nz, warps = (int64_t)gridDim.x * (kMeshThreads / 32);
+  for (int64_t c = (int64_t)blockIdx.x * (kMeshThreads / 32) + threadIdx.x / 32; c < n; c += warps) {
+    if (fill) {
+      if (M.nstart[c + 1] > M.nstart[c]) cell_faces(M, L, c, lane, items + M.nstart[c]);
+    } else {
+      const int m = cell_faces(M, L, c, lane, nullptr);
+      if (lane == 0) {
+        len[c] = m;
+        if (m) atomicMax(&len[n], m);                  // the longest list, after the lengths
+      }
+    }
+  }
+}
+
+// exclusive prefix sums of the list lengths (64-bit: the lists of a mesh far finer than its supports may pass 2^31
+// faces), one block, 1024 lengths at a time
+constexpr int kPrefixThreads = 1024;
+__global__ void __launch_bounds__(kPrefixThreads) k_mesh_prefix(const int32_t* __restrict__ len, int64_t n,
+                                                               int64_t* __restrict__ start) {
+  __shared__ int64_t s_warp[kPrefixThreads / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int64_t carry = 0;
+  for (int64_t base = 0; base < n; base += kPrefixThreads) {
+    const int64_t k = base + threadIdx.x;
+    const int64_t v = k < n ? len[k] : 0;
+    int64_t x = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int64_t y = __shfl_up_sync(0xffffffffu, x, d);
+      if (lane >= d) x += y;
+    }
+    if (lane == 31) s_warp[wid] = x;
+    __syncthreads();
+    int64_t before = 0, total = 0;
+    for (int w = 0; w < kPrefixThreads / 32; ++w) {
+      if (w < wid) before += s_warp[w];
+      total += s_warp[w];
+    }
+    if (k < n) start[k] = carry + before + x - v;
+    carry += total;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) start[n] = carry;
+}
+
 // the per-cell flags, once per mesh: emptiness, the inside status of an empty cell's centre (the column parity test),
-// whether any of the 27 cells around holds a face
-__global__ void k_mesh_cellflags(MeshView M, uint8_t* __restrict__ flags) {
+// whether the cell's candidate list holds a face
+__global__ void k_mesh_cellflags(MeshView M, BoxLists L, const int32_t* __restrict__ len, uint8_t* __restrict__ flags) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nxy = (int64_t)M.nx * M.ny;
   if (c >= nxy * M.nz) return;
   const int i = (int)(c % M.nx), j = (int)((c / M.nx) % M.ny), k = (int)(c / nxy);
-  uint8_t f = 0;
-  if (M.cstart[c] == M.cstart[c + 1]) {
+  uint8_t f = len[c] > 0 ? kCellNear : 0;
+  if (L.start[c] == L.start[c + 1]) {
     f |= kCellEmpty;
     const double x = M.lo0 + (i + 0.5) * M.cell, y = M.lo1 + (j + 0.5) * M.cell, z = M.lo2 + (k + 0.5) * M.cell;
     if (mesh_inside(M, x, y, z)) f |= kCellInside;
   }
-  for (int dk = -1; dk <= 1; ++dk)
-    for (int dj = -1; dj <= 1; ++dj)
-      for (int di = -1; di <= 1; ++di) {
-        const int a = i + di, b = j + dj, e = k + dk;
-        if (a < 0 || b < 0 || e < 0 || a >= M.nx || b >= M.ny || e >= M.nz) continue;
-        const int64_t n = ((int64_t)e * M.ny + b) * M.nx + a;
-        if (M.cstart[n] != M.cstart[n + 1]) f |= kCellNear;
-      }
   flags[c] = f;
 }
 
-// Per query, first pass: the cell's flags settle the rows away from the surface (inside status of an empty cell, no
-// faces within the support when no face box meets the 27 cells around); the others are appended to `near`, so the
-// second pass runs the parity walk and the face search on full warps of such rows.  Invalid rows (a support above the
-// grid cell would reach faces outside the 27-cell block, non-finite input) are marked -1 and come back as NaN.
-__global__ void __launch_bounds__(kMeshThreads) k_mesh_rowinfo(MeshView M, const double* __restrict__ pos,
+__device__ __forceinline__ int64_t cell_of_query(const MeshView& M, const double q[3]) {
+  const int cx = cell_coord(q[0], M.lo0, M.cell, M.nx), cy = cell_coord(q[1], M.lo1, M.cell, M.ny),
+            cz = cell_coord(q[2], M.lo2, M.cell, M.nz);
+  if (cx < 0 || cy < 0 || cz < 0 || cx >= M.nx || cy >= M.ny || cz >= M.nz) return -1;
+  return ((int64_t)cz * M.ny + cy) * M.nx + cx;
+}
+
+// First pass, one thread per query: the cell's flags settle the rows away from the surface (outside the grid, which
+// reaches a cell past the surface's box: outside the solid, no face within the support; an empty candidate list: the
+// cell is empty and its centre's status holds); the others are appended to `near` for the second pass.  Invalid rows (a
+// support above the grid cell would reach faces beyond the lists, non-finite input) are marked -1 and come back as NaN.
+// Every row's constants -- whole-support values inside, zeros outside, NaN -- are built in shared memory (stride 29
+// doubles against bank conflicts) and the block writes its contiguous slab of 128 x 28 outputs coalesced (the second
+// pass overwrites its rows).  One global atomic a block for the list: one a warp took 54 us for 2^21 rows, the row
+// constants in a kernel of their own another 75.
+constexpr int kRowStride = 29;
+
+template <class M>
+__global__ void __launch_bounds__(kMeshThreads) k_mesh_rowinfo(MeshView Mv, const double* __restrict__ pos,
                                                               const double* __restrict__ sup, int64_t n,
                                                               int32_t* __restrict__ ind, int32_t* __restrict__ near,
-                                                              int32_t* __restrict__ nnear) {
-  const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+                                                              int32_t* __restrict__ nnear, double* __restrict__ out) {
+  __shared__ double s_rows[kMeshThreads * kRowStride];
+  __shared__ int32_t s_count[kMeshThreads / 32 + 1];
+  const int64_t row0 = (int64_t)blockIdx.x * kMeshThreads;
+  const int64_t row = row0 + threadIdx.x;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   bool listed = false;
   if (row < n) {
     const double q[3] = {pos[3 * row], pos[3 * row + 1], pos[3 * row + 2]};
     const double h = sup[row];
-    const bool ok = h > 0.0 && h <= M.cell && isfinite(q[0]) && isfinite(q[1]) && isfinite(q[2]);
-    if (!ok) {
-      ind[row] = -1;
-    } else {
-      const int cx = cell_coord(q[0], M.lo0, M.cell, M.nx), cy = cell_coord(q[1], M.lo1, M.cell, M.ny),
-                cz = cell_coord(q[2], M.lo2, M.cell, M.nz);
-      const bool in_grid = cx >= 0 && cy >= 0 && cz >= 0 && cx < M.nx && cy < M.ny && cz < M.nz;
-      // more than a cell outside the grid along some axis (cell_coord gives -2 or n + 1): the grid reaches a cell
-      // (>= the support) past the surface's box, so no face is within the support and the query is outside the solid
-      const bool far = cx == -2 || cy == -2 || cz == -2 || cx == M.nx + 1 || cy == M.ny + 1 || cz == M.nz + 1;
-      const uint8_t f = in_grid ? M.cflag[((int64_t)cz * M.ny + cy) * M.nx + cx] : (uint8_t)(far ? 0 : kCellNear);
-      if (!(f & kCellNear)) {
-        ind[row] = (f & kCellInside) ? 1 : 0;     // no face box in the 27 cells: the cell is empty as well
-      } else {
-        listed = true;
-      }
+    const bool ok = h > 0.0 && h <= Mv.cell && isfinite(q[0]) && isfinite(q[1]) && isfinite(q[2]);
+    int in = ok ? 0 : -1;
+    if (ok) {
+      const int64_t c = cell_of_query(Mv, q);
+      const uint8_t f = c >= 0 ? Mv.cflag[c] : (uint8_t)0;
+      listed = f & kCellNear;
+      in = !listed && (f & kCellInside) ? 1 : 0;
     }
+    if (!listed) ind[row] = in;
+    double* const mine = s_rows + threadIdx.x * kRowStride;
+    const double id = in < 0 ? __longlong_as_double(0x7ff8000000000000LL) : (double)in, ih = 1.0 / h;
+    for (int k = 0; k < 28; ++k)
+      mine[k] = in < 0 ? id : channel_value<M>(channel_of(k), 0.0, 0.0, id, h, ih);
   }
   const unsigned mask = __ballot_sync(0xffffffffu, listed);
-  if (mask) {
-    const int lane = threadIdx.x & 31;
-    const int leader = __ffs(mask) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(nnear, __popc(mask));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (listed) near[base + __popc(mask & ((1u << lane) - 1))] = (int32_t)row;
-  }
-}
-
-// Second pass over the listed rows: the inside test (the cell's flag where the cell is empty, the parity walk
-// otherwise) and whether any face is within the support; rows with faces are appended to `work`
-__global__ void __launch_bounds__(kMeshThreads) k_mesh_rownear(MeshView M, const double* __restrict__ pos,
-                                                              const double* __restrict__ sup,
-                                                              const int32_t* __restrict__ near,
-                                                              const int32_t* __restrict__ nnear,
-                                                              int32_t* __restrict__ ind, int32_t* __restrict__ work,
-                                                              int32_t* __restrict__ nwork) {
-  // one warp per listed row (the warps of the grid stride over them): the column's faces and the candidate cells'
-  // items are tested 32 at a time
-  const int lane = threadIdx.x & 31;
-  const int64_t m = *nnear;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x / 32);
-  for (int64_t t = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; t < m; t += warps) {
-    const int32_t row = near[t];
-    const double q[3] = {pos[3 * row], pos[3 * row + 1], pos[3 * row + 2]};
-    const double h = sup[row];
-    const int cx = cell_coord(q[0], M.lo0, M.cell, M.nx), cy = cell_coord(q[1], M.lo1, M.cell, M.ny),
-              cz = cell_coord(q[2], M.lo2, M.cell, M.nz);
-    const bool in_grid = cx >= 0 && cy >= 0 && cz >= 0 && cx < M.nx && cy < M.ny && cz < M.nz;
-    const uint8_t f = in_grid ? M.cflag[((int64_t)cz * M.ny + cy) * M.nx + cx] : (uint8_t)0;
-    const int inside = (f & kCellEmpty) ? ((f & kCellInside) ? 1 : 0) : mesh_inside_warp(M, q[0], q[1], q[2], lane);
-    const bool has = has_candidate_warp(M, q, h, lane);
-    if (lane == 0) {
-      ind[row] = inside;
-      if (has) work[atomicAdd(nwork, 1)] = row;     // (the order is irrelevant: each row is computed alone)
-    }
-  }
-}
-
-// rows without faces in their support: whole-support constants inside, zeros outside, NaN for invalid rows.  Each
-// thread builds its row in shared memory (stride 29 doubles against bank conflicts) and the block writes its
-// contiguous slab of 128 x 28 outputs coalesced.
-constexpr int kRowStride = 29;
-
-template <class M>
-__global__ void __launch_bounds__(kMeshThreads) k_mesh_rows(const double* __restrict__ sup, int64_t n,
-                                                           const int32_t* __restrict__ ind, double* __restrict__ out) {
-  __shared__ double s_rows[kMeshThreads * kRowStride];
-  const int64_t row0 = (int64_t)blockIdx.x * kMeshThreads;
-  const int64_t row = row0 + threadIdx.x;
-  double* const mine = s_rows + threadIdx.x * kRowStride;
-  if (row < n) {
-    if (ind[row] < 0) {
-      for (int k = 0; k < 28; ++k) mine[k] = __longlong_as_double(0x7ff8000000000000LL);
-    } else {
-      const double id = (double)ind[row], h = sup[row];
-      for (int k = 0; k < 28; ++k) mine[k] = channel_value<M>(channel_of(k), 0.0, 0.0, id, h, 1.0 / h);
-    }
-  }
+  if (lane == 0) s_count[wid] = __popc(mask);
   __syncthreads();
+  if (threadIdx.x == 0) {
+    int total = 0;
+    for (int w = 0; w < kMeshThreads / 32; ++w) {
+      const int v = s_count[w];
+      s_count[w] = total;
+      total += v;
+    }
+    s_count[kMeshThreads / 32] = total ? atomicAdd(nnear, total) : 0;
+  }
   const int rows = (int)min((int64_t)kMeshThreads, n - row0);
   for (int k = threadIdx.x; k < rows * 28; k += kMeshThreads)
     out[row0 * 28 + k] = s_rows[(k / 28) * kRowStride + k % 28];
+  __syncthreads();
+  if (listed) near[s_count[kMeshThreads / 32] + s_count[wid] + __popc(mask & ((1u << lane) - 1))] = (int32_t)row;
 }
 
-// The rows with faces.  A warp takes rows in turn, its lanes search a row's faces together (FaceSearch), and
-// the (row, face) pairs wait in the warp's queue until there are 32: then every lane integrates one pair, whatever row
-// it belongs to, so the lanes stay full although a row has some 20 faces.  The 28 terms of each pair go through shared
-// memory to the lanes k < 28, which add accumulator k of the row pair after pair in queue order -- the row's face order
-// -- and finish the row at its last pair: the result does not depend on the other rows of the queue.
-// On the 2^21-particle scene of 20480 faces (w4, 129 562 rows, 2.6 M pairs) this takes 1.33 ms on B200 against 7.0 ms with
-// a warp per row, the quadrature nodes of one edge after the other over its lanes: 0.45 Kflop an edge instead of some
-// 15 Kflop, and no reduction over the lanes.
-constexpr int kEvalWarps = kMeshThreads / 32;
+// Second pass, the listed rows.  A warp takes up to eight rows at a time: lane r loads row r and its list, then the
+// inside tests (the cell's flag where the cell is empty, the column parity otherwise) and the face search run over the
+// eight rows' items flattened on the lanes, so the chain of loads from a row to its faces is paid once for eight rows
+// and the rounds are full although a list holds some 40 faces.  A row's hits are kept as a mask over its list; rows with
+// hits are appended to `rows`, the others get their constants.
+// (2^21 particles, 20480 faces: 0.21 ms on B200; a warp per row over the 27 cells' box lists, in which a face of the
+// cell's size is met six times, and the inside test a warp per row: 1.3 ms, half of it a second search in the
+// integration.  A kernel of its own, 8 CTAs per SM, because it waits for loads: inside the integration's kernel, at 3
+// CTAs per SM, the search of 20011 near rows took 109 us of 169, here 49.)
+constexpr int kBatch = 8;
+constexpr int kSearchBlocks = 8;
+
+// rows per batch: as many as the warps' even share allows (a share of 12 rows in two batches of 6, not 8 and 4)
+__device__ __forceinline__ int batch_rows(int n, int warps, int most) {
+  const int share = (n + warps - 1) / warps, nb = (share + most - 1) / most;
+  return nb ? (share + nb - 1) / nb : 1;
+}
+
+template <class M>
+__global__ void __launch_bounds__(kMeshThreads, kSearchBlocks)
+    k_mesh_search(MeshView Mv, const double* __restrict__ pos, const double* __restrict__ sup,
+                  const int32_t* __restrict__ near, int32_t* __restrict__ counts, int words, int32_t* __restrict__ ind,
+                  MeshRow* __restrict__ rows, uint64_t* __restrict__ mask, double* __restrict__ out) {
+  __shared__ double s_row[kMeshThreads / 32][kBatch][4];      // the batch's queries and 1 / support
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const Channel ch = channel_of(lane);
+  const int n = counts[0], warps = gridDim.x * (kMeshThreads / 32), per = batch_rows(n, warps, kBatch);
+  for (int it = (blockIdx.x * (kMeshThreads / 32) + wib) * per; it < n; it += warps * per) {
+    const bool mine = lane < per && it + lane < n;
+    MeshRow row{};
+    int cbeg = 0, clen = 0, inside = 0;
+    __syncwarp();
+    if (mine) {
+      const int64_t i = near[it + lane];
+      row.q[0] = pos[3 * i];
+      row.q[1] = pos[3 * i + 1];
+      row.q[2] = pos[3 * i + 2];
+      row.h = sup[i];
+      const int64_t c = cell_of_query(Mv, row.q);      // listed: inside the grid
+      const uint8_t fl = Mv.cflag[c];
+      row.first = Mv.nstart[c];
+      row.len = (int)(Mv.nstart[c + 1] - row.first);
+      row.tag = (int)i;
+      if (fl & kCellEmpty) {
+        inside = (fl & kCellInside) ? 1 : 0;
+      } else {
+        const int col = column_of(Mv, row.q[0], row.q[1]);
+        if (col >= 0) {
+          cbeg = Mv.colstart[col];
+          clen = Mv.colstart[col + 1] - cbeg;
+        }
+      }
+#pragma unroll
+      for (int a = 0; a < 3; ++a) s_row[wib][lane][a] = row.q[a];
+      s_row[wib][lane][3] = 1.0 / row.h;
+    }
+    __syncwarp();
+    Flat<kBatch> flat;
+    unsigned place;
+    int r, lane0;
+    flat.set(clen, lane);
+    for (unsigned base = 0; base < flat.total; base += 32) {
+      r = flat.row_of(base + lane, place);
+      const int beg = __shfl_sync(0xffffffffu, cbeg, r);
+      const double* q = s_row[wib][r];
+      const bool cross = base + lane < flat.total && column_cross(Mv, Mv.colitems[beg + place], q[0], q[1], q[2]);
+      const unsigned m = __ballot_sync(0xffffffffu, cross);
+      const int cnt = flat.part(base, place, lane0);
+      if (cnt > 0) inside ^= __popc((m >> lane0) & (0xffffffffu >> (32 - cnt))) & 1;
+    }
+    if (mine) {
+      ind[row.tag] = inside;
+      row.tag |= inside << 30;
+    }
+    flat.set(row.len, lane);
+    // the mask is built in the listed row's place (it + lane): the place among the rows with faces is not known yet
+    row.at = it + lane;
+    uint64_t* const words_r = mask + (int64_t)row.at * words;
+    uint64_t word = 0;
+    bool any = false;
+    for (unsigned base = 0; base < flat.total; base += 32) {
+      r = flat.row_of(base + lane, place);
+      const int64_t beg = __shfl_sync(0xffffffffu, row.first, r);
+      const double* q = s_row[wib][r];
+      const bool hit = base + lane < flat.total && face_within(Mv, Mv.nitems[beg + place], q, q[3]);
+      const unsigned m = __ballot_sync(0xffffffffu, hit);
+      const int cnt = flat.part(base, place, lane0);
+      if (cnt > 0) {
+        const uint64_t bits = (m >> lane0) & (0xffffffffu >> (32 - cnt));
+        const int at = (int)(place & 63u), w = (int)(place >> 6);
+        any = any || bits;
+        word |= bits << at;
+        if (at + cnt >= 64 || place + cnt == flat.len) {       // the word is full, or the list ends
+          if (w < words) words_r[w] = word;
+          word = at + cnt > 64 ? bits >> (64 - at) : 0;
+          if (at + cnt > 64 && place + cnt == flat.len && w + 1 < words) words_r[w + 1] = word;
+        }
+      }
+    }
+    // rows with faces: their records; the others: the constants
+    const unsigned with = __ballot_sync(0xffffffffu, mine && any);
+    int slot = 0;
+    if (lane == 0 && with) slot = atomicAdd(&counts[1], __popc(with));
+    slot = __shfl_sync(0xffffffffu, slot, 0);
+    if (mine && any) rows[slot + __popc(with & ((1u << lane) - 1))] = row;
+    for (unsigned none = __ballot_sync(0xffffffffu, mine && !any); none; none &= none - 1) {
+      const int b = __ffs(none) - 1, tag = __shfl_sync(0xffffffffu, row.tag, b);
+      const double h = __shfl_sync(0xffffffffu, row.h, b);
+      if (lane < 28)
+        out[(int64_t)(tag & kRowMask) * 28 + lane] = channel_value<M>(ch, 0.0, 0.0, (double)(tag >> 30), h, 1.0 / h);
+    }
+  }
+}
+
+// the place of the k-th set bit (k = 0, 1, ...) of m, which has more than k
+__device__ __forceinline__ int select_bit(uint64_t m, int k) {
+  unsigned x = (unsigned)m;
+  int c = __popc(x), at = 0;
+  if (k >= c) {
+    k -= c;
+    x = (unsigned)(m >> 32);
+    at = 32;
+  }
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1) {
+    c = __popc(x & ((1u << w) - 1));
+    if (k >= c) {
+      k -= c;
+      x >>= w;
+      at += w;
+    }
+  }
+  return at;
+}
+
+// Third pass, the rows with faces: the (row, face) pairs of up to 32 rows flattened on a warp's lanes, every lane one
+// pair, whatever row it belongs to, so the lanes stay full although a row has some 20 faces.  The 28 terms of each pair
+// go through shared memory to the lanes k < 28, which add accumulator k of the row pair after pair in the list's order
+// and finish the row when the next row's first pair comes: the result does not depend on the other rows.
+// On the 2^21-particle scene of 20480 faces (w4, 129 562 rows, 2.6 M pairs): 0.43 ms on B200, 20011 near queries (w2) 0.10 ms; 12 warps per
+// SM, bound by the latency of the float64 chains (24 % of the pipe, issue 31 %; 4 CTAs at 128 registers: no gain).  Before, a warp took one row and
+// spread the quadrature nodes of one edge after the other over its lanes (7.0 ms with the search).
 constexpr int kEvalBlocks = 3;        // resident CTAs per SM (168 registers)
+constexpr int kEvalRows = 32;
 constexpr int kPairStride = 29;       // doubles per pair in shared memory (28 and one against bank conflicts)
 
 template <class M>
-__global__ void __launch_bounds__(kMeshThreads, kEvalBlocks) k_mesh_eval(MeshView Mv, const double* __restrict__ pos,
-                                                                        const double* __restrict__ sup,
-                                                                        const int32_t* __restrict__ ind,
-                                                                        const int32_t* __restrict__ work,
-                                                                        const int32_t* __restrict__ nwork,
-                                                                        double* __restrict__ out) {
-  __shared__ double s_val[kEvalWarps][32 * kPairStride];
-  __shared__ int2 s_queue[kEvalWarps][64];             // (row, face), the row's last pair marked by ~face
+__global__ void __launch_bounds__(kMeshThreads, kEvalBlocks)
+    k_mesh_eval(MeshView Mv, const MeshRow* __restrict__ rows, const uint64_t* __restrict__ mask, int words,
+                const int32_t* __restrict__ nrows, double* __restrict__ out) {
+  __shared__ double s_val[kMeshThreads / 32][32 * kPairStride];
+  __shared__ double s_h[kMeshThreads / 32][32];               // the round's supports and tags
+  __shared__ int32_t s_tag[kMeshThreads / 32][32];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   double* const val = s_val[wib];
-  int2* const queue = s_queue[wib];
   const Channel ch = channel_of(lane);
-  const int nw = *nwork;
-  int qn = 0;
-  double acc = 0.0;                                    // accumulator `lane` of the queue's first row
-  // integrates the first m pairs of the queue and finishes the rows that end among them
-  auto flush = [&](int m) {
-    __syncwarp();
-    if (lane < m) {
-      const int2 p = queue[lane];
-      const int64_t row = p.x;
-      const double qp[3] = {pos[3 * row], pos[3 * row + 1], pos[3 * row + 2]};
-      double o[28];
-      face_channels<M>(Mv.fdata + (int64_t)(p.y < 0 ? ~p.y : p.y) * kFaceDoubles, qp, 1.0 / sup[row], o);
+  const int n = *nrows, warps = gridDim.x * (kMeshThreads / 32), per = batch_rows(n, warps, kEvalRows);
+  for (int it = (blockIdx.x * (kMeshThreads / 32) + wib) * per; it < n; it += warps * per) {
+    unsigned pairs = 0;
+    if (lane < per && it + lane < n) {
+      const MeshRow& row = rows[it + lane];
+      const uint64_t* m = mask + (int64_t)row.at * words;
+      const int full = min(words, (row.len + 63) / 64);
+      for (int w = 0; w < full; ++w) pairs += __popcll(m[w]);
+      pairs += max(row.len - 64 * words, 0);
+    }
+    Flat<kEvalRows> flat;
+    flat.set(pairs, lane);
+    int f = -1, r = 0;
+    // this lane's pair of the round at `base`: its row and its face (~face: beyond the mask, still to be tested)
+    auto fetch = [&](unsigned base) {
+      unsigned k;
+      r = flat.row_of(base + lane, k);
+      if (base + lane >= flat.total) return;
+      const MeshRow& row = rows[it + r];
+      const uint64_t* m = mask + (int64_t)row.at * words;
+      const int full = min(words, (row.len + 63) / 64);
+      for (int w = 0; w < full; ++w) {
+        const uint64_t bits = m[w];
+        const unsigned c = __popcll(bits);
+        if (k < c) {
+          f = Mv.nitems[row.first + 64 * w + select_bit(bits, (int)k)];
+          return;
+        }
+        k -= c;
+      }
+      f = ~Mv.nitems[row.first + 64 * words + k];
+    };
+    fetch(0);
+    int cur = -1;
+    double acc = 0.0, h = 1.0;                                // accumulator `lane` of the row `cur`, its support
+    auto finish = [&]() {
+      const double a0 = __shfl_sync(0xffffffffu, acc, 0);
+      if (cur >= 0 && lane < 28)
+        out[(int64_t)(cur & kRowMask) * 28 + lane] = channel_value<M>(ch, acc, a0, (double)(cur >> 30), h, 1.0 / h);
+    };
+    for (unsigned base = 0; base < flat.total; base += 32) {
+      const int f0 = f, r0 = r;
+      if (base + 32 < flat.total) fetch(base + 32);           // (the next round's loads run ahead of the integration)
+      if (base + lane < flat.total) {
+        const MeshRow& row = rows[it + r0];
+        double q[3], hr;
+        ld4_nc(row.q, q[0], q[1], q[2], hr);
+        const double ih = 1.0 / hr;
+        s_tag[wib][lane] = row.tag;
+        s_h[wib][lane] = hr;
+        double o[28];
+        if (f0 >= 0 || face_within(Mv, ~f0, q, ih)) {
+          face_channels<M>(Mv.fdata + (int64_t)(f0 < 0 ? ~f0 : f0) * kFaceDoubles, q, ih, o);
+        } else {
 #pragma unroll
-      for (int k = 0; k < 28; ++k) val[lane * kPairStride + k] = o[k];
-    }
-    __syncwarp();
-    for (int k = 0; k < m; ++k) {
-      if (lane < 28) acc += val[k * kPairStride + lane];
-      const int2 p = queue[k];
-      if (p.y < 0) {
-        const double acc0 = __shfl_sync(0xffffffffu, acc, 0), h = sup[p.x];
-        if (lane < 28) out[(int64_t)p.x * 28 + lane] = channel_value<M>(ch, acc, acc0, (double)ind[p.x], h, 1.0 / h);
-        acc = 0.0;
+          for (int k = 0; k < 28; ++k) o[k] = 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < 28; ++k) val[lane * kPairStride + k] = o[k];
       }
-    }
-    // the pairs that stay move to the front
-    const int2 p = lane + m < 64 ? queue[lane + m] : make_int2(0, 0);
-    __syncwarp();
-    queue[lane] = p;
-    __syncwarp();
-    qn -= m;
-  };
-  const int warps = gridDim.x * kEvalWarps;
-  int it = blockIdx.x * kEvalWarps + wib - warps, row = 0;
-  bool any = false;                                    // the searched row has pairs
-  FaceSearch fs;
-  fs.base = fs.total = 0;
-  for (;;) {
-    // fill the queue past 32 pairs: the first 32 then never hold the last pair of a row whose search goes on, which may
-    // still have to be marked
-    while (qn <= 32 && it < nw) {
-      if (fs.base < fs.total) {
-        int f;
-        const unsigned mask = fs.next(Mv, lane, f);
-        if ((mask >> lane) & 1u) queue[qn + __popc(mask & ((1u << lane) - 1))] = make_int2(row, f);
-        qn += __popc(mask);
-        any = any || mask;
-        continue;
+      __syncwarp();
+      const int cnt = (int)min(flat.total - base, 32u);
+      for (int k = 0; k < cnt; ++k) {
+        const int tag = s_tag[wib][k];
+        if (tag != cur) {
+          finish();
+          cur = tag;
+          h = s_h[wib][k];
+          acc = 0.0;
+        }
+        if (lane < 28) acc += val[k * kPairStride + lane];
       }
-      if (any) {
-        __syncwarp();
-        if (lane == 0) queue[qn - 1].y = ~queue[qn - 1].y;
-        any = false;
-      }
-      it += warps;
-      if (it >= nw) break;
-      row = work[it];
-      fs.start(Mv, pos + 3 * (int64_t)row, sup[row], lane);
+      __syncwarp();
     }
-    if (qn == 0) break;
-    flush(min(qn, 32));
+    finish();
   }
 }
 
@@ -828,30 +947,81 @@ int upload_vec(T** dst, const std::vector<T>& src) {
 }
 
 void free_mesh(Mesh* m) {
-  void* ptrs[] = {m->fdata, m->fcell, m->fvid, m->cstart, m->citems, m->colstart, m->colitems, m->cflag};
+  void* ptrs[] = {m->fdata, m->nstart, m->nitems, m->colstart, m->colitems, m->cflag};
   for (void* p : ptrs)
     if (p) cudaFree(p);
 }
 
 inline size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
+// the candidate lists and flags of every cell: lengths, their prefix sums, the lists, the flags
+int mesh_lists(Mesh* m, const BoxLists& L, int64_t ncells, int32_t** len) {
+  WSB_CUDA(cudaMalloc((void**)len, sizeof(int32_t) * (size_t)(ncells + 1)));
+  WSB_CUDA(cudaMemset(*len + ncells, 0, sizeof(int32_t)));
+  WSB_CUDA(cudaMalloc((void**)&m->nstart, sizeof(int64_t) * (size_t)(ncells + 1)));
+  WSB_CUDA(cudaMalloc((void**)&m->cflag, (size_t)ncells));
+  constexpr int W = kMeshThreads / 32;
+  const unsigned grid = (unsigned)std::min<int64_t>((ncells + W - 1) / W, 148 * 64);
+  k_mesh_lists<<<grid, kMeshThreads>>>(view_of(m), L, 0, *len, nullptr);
+  k_mesh_prefix<<<1, kPrefixThreads>>>(*len, ncells, m->nstart);
+  int64_t total = 0;
+  int32_t longest = 0;
+  WSB_CUDA(cudaMemcpy(&longest, *len + ncells, sizeof(longest), cudaMemcpyDeviceToHost));
+  if (longest > (1 << 26))   // the passes flatten up to 32 lists in 32 bits
+    return fail(WSB_ERR_SIZE, "wsb_mesh_create: more than 2^26 faces within reach of one cell");
+  m->words = std::min(kMaxWords, std::max(1, (longest + 63) / 64));
+  WSB_CUDA(cudaMemcpy(&total, m->nstart + ncells, sizeof(total), cudaMemcpyDeviceToHost));
+  WSB_CUDA(cudaMalloc((void**)&m->nitems, sizeof(int32_t) * (size_t)std::max<int64_t>(total, 1)));
+  k_mesh_lists<<<grid, kMeshThreads>>>(view_of(m), L, 1, *len, m->nitems);
+  k_mesh_cellflags<<<(unsigned)((ncells + 255) / 256), 256>>>(view_of(m), L, *len, m->cflag);
+  WSB_CUDA(cudaGetLastError());
+  WSB_CUDA(cudaDeviceSynchronize());
+  return WSB_OK;
+}
+
+// the workspace of n queries: the listed rows, their number and that of the rows with faces, the indicator (where the
+// caller wants none), the rows with faces and their masks
+struct MeshWork {
+  int32_t *near, *counts, *ind;
+  MeshRow* rows;
+  uint64_t* mask;
+  size_t total;
+};
+MeshWork carve_mesh(const Mesh* m, int64_t n, void* base) {
+  MeshWork w{};
+  const uintptr_t p = ((uintptr_t)base + 255) & ~(uintptr_t)255;
+  const size_t k = (size_t)std::max<int64_t>(n, 1);
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    const size_t o = off;
+    off += al256(bytes);
+    return (void*)(p + o);
+  };
+  w.counts = (int32_t*)take(2 * sizeof(int32_t));
+  w.near = (int32_t*)take(k * sizeof(int32_t));
+  w.ind = (int32_t*)take(k * sizeof(int32_t));
+  w.rows = (MeshRow*)take(k * sizeof(MeshRow));
+  w.mask = (uint64_t*)take(k * m->words * sizeof(uint64_t));
+  w.total = off + 256;
+  return w;
+}
+
 template <class M>
 int launch_mesh(const Mesh* m, const double* pos, const double* sup, int64_t n, double* out, int32_t* ind,
-                int32_t* work, int32_t* nwork, int32_t* near, cudaStream_t st) {
+                const MeshWork& w, cudaStream_t st) {
   const MeshView v = view_of(m);
   const unsigned grid = (unsigned)((n + kMeshThreads - 1) / kMeshThreads);
-  WSB_CUDA(cudaMemsetAsync(nwork, 0, 3 * sizeof(int32_t), st));      // work rows, (unused), listed rows
-  k_mesh_rowinfo<<<grid, kMeshThreads, 0, st>>>(v, pos, sup, n, ind, near, nwork + 2);
+  WSB_CUDA(cudaMemsetAsync(w.counts, 0, 2 * sizeof(int32_t), st));
+  k_mesh_rowinfo<M><<<grid, kMeshThreads, 0, st>>>(v, pos, sup, n, ind, w.near, w.counts, out);
   WSB_CUDA(cudaGetLastError());
-  const unsigned grid_near = (unsigned)std::min<int64_t>((n + kMeshThreads / 32 - 1) / (kMeshThreads / 32), 8192);
-  k_mesh_rownear<<<grid_near, kMeshThreads, 0, st>>>(v, pos, sup, near, nwork + 2, ind, work, nwork);
+  const int warps = kMeshThreads / 32;
+  const auto grid_of = [&](int blocks) {           // the resident warps, striding over the rows; no more warps than rows
+    return (unsigned)std::min<int64_t>((n + warps - 1) / warps, (int64_t)148 * blocks);
+  };
+  k_mesh_search<M><<<grid_of(kSearchBlocks), kMeshThreads, 0, st>>>(v, pos, sup, w.near, w.counts, m->words, ind, w.rows,
+                                                                    w.mask, out);
   WSB_CUDA(cudaGetLastError());
-  k_mesh_rows<M><<<grid, kMeshThreads, 0, st>>>(sup, n, ind, out);
-  WSB_CUDA(cudaGetLastError());
-  // the resident warps, striding over the work rows (no more warps than rows)
-  const unsigned egrid =
-      (unsigned)std::min<int64_t>((n + kEvalWarps - 1) / kEvalWarps, (int64_t)148 * kEvalBlocks);
-  k_mesh_eval<M><<<egrid, kMeshThreads, 0, st>>>(v, pos, sup, ind, work, nwork, out);
+  k_mesh_eval<M><<<grid_of(kEvalBlocks), kMeshThreads, 0, st>>>(v, w.rows, w.mask, m->words, w.counts + 1, out);
   WSB_CUDA(cudaGetLastError());
   return WSB_OK;
 }
@@ -874,29 +1044,38 @@ extern "C" int wsb_mesh_create(const double* verts, int64_t n_verts, const int32
     return fail(WSB_ERR_ARG, "wsb_mesh_create: support_max must be positive and finite");
   for (int64_t i = 0; i < 3 * n_verts; ++i)
     if (!std::isfinite(verts[i])) return fail(WSB_ERR_ARG, "wsb_mesh_create: non-finite vertex");
-  // watertight, consistently oriented 2-manifold: every undirected edge twice, once in each direction
-  std::map<std::pair<int32_t, int32_t>, int> dir;
-  for (int64_t f = 0; f < n_faces; ++f) {
-    const int32_t* v = faces + 3 * f;
-    for (int k = 0; k < 3; ++k)
-      if (v[k] < 0 || v[k] >= n_verts) return fail(WSB_ERR_ARG, "wsb_mesh_create: face index out of range");
-    if (v[0] == v[1] || v[1] == v[2] || v[0] == v[2]) return fail(WSB_ERR_ARG, "wsb_mesh_create: repeated vertex");
-    for (int k = 0; k < 3; ++k) {
-      const int32_t a = v[k], b = v[(k + 1) % 3];
-      const auto key = std::make_pair(std::min(a, b), std::max(a, b));
-      const int bit = a < b ? 1 : 2;
-      int& d = dir[key];
-      if (d & bit) return fail(WSB_ERR_ARG, "wsb_mesh_create: surface must be watertight and consistently oriented");
-      d |= bit;
+  // watertight, consistently oriented 2-manifold: every undirected edge twice, once in each direction (an open-addressing
+  // table of the undirected edges, at most half full: 3 n_faces / 2 edges of a closed surface, 3 n_faces of any other)
+  {
+    size_t cap = 16;
+    while (cap < (size_t)n_faces * 6) cap *= 2;
+    std::vector<uint64_t> keys(cap, ~0ull);
+    std::vector<uint8_t> dir(cap, 0);
+    for (int64_t f = 0; f < n_faces; ++f) {
+      const int32_t* v = faces + 3 * f;
+      for (int k = 0; k < 3; ++k)
+        if (v[k] < 0 || v[k] >= n_verts) return fail(WSB_ERR_ARG, "wsb_mesh_create: face index out of range");
+      if (v[0] == v[1] || v[1] == v[2] || v[0] == v[2]) return fail(WSB_ERR_ARG, "wsb_mesh_create: repeated vertex");
+      for (int k = 0; k < 3; ++k) {
+        const int32_t a = v[k], b = v[(k + 1) % 3];
+        const uint64_t key = ((uint64_t)(uint32_t)std::min(a, b) << 32) | (uint32_t)std::max(a, b);
+        size_t h = (size_t)((key * 0x9E3779B97F4A7C15ull) >> 20) & (cap - 1);
+        while (keys[h] != key && keys[h] != ~0ull) h = (h + 1) & (cap - 1);
+        keys[h] = key;
+        const uint8_t bit = a < b ? 1 : 2;
+        if (dir[h] & bit)
+          return fail(WSB_ERR_ARG, "wsb_mesh_create: surface must be watertight and consistently oriented");
+        dir[h] |= bit;
+      }
     }
+    for (size_t h = 0; h < cap; ++h)
+      if (keys[h] != ~0ull && dir[h] != 3)
+        return fail(WSB_ERR_ARG, "wsb_mesh_create: surface must be watertight and consistently oriented");
   }
-  for (const auto& kv : dir)
-    if (kv.second != 3) return fail(WSB_ERR_ARG, "wsb_mesh_create: surface must be watertight and consistently oriented");
   // face records, box, signed volume (relative to the first vertex: outward normals give a positive volume)
   double vol6 = 0.0;
   const double* o = verts;
   std::vector<double> hf((size_t)n_faces * kFaceDoubles);
-  std::vector<int32_t> hvid((size_t)n_faces * 3);
   double blo[3] = {INFINITY, INFINITY, INFINITY}, bhi[3] = {-INFINITY, -INFINITY, -INFINITY};
   for (int64_t f = 0; f < n_faces; ++f) {
     const int32_t* v = faces + 3 * f;
@@ -923,6 +1102,7 @@ extern "C" int wsb_mesh_create(const double* verts, int64_t n_verts, const int32
       const double len = std::sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
       for (int k = 0; k < 3; ++k) t[k] /= len;
       for (int k = 0; k < 3; ++k) F[kFT + 3 * e + k] = t[k];
+      if (v[e] < v[(e + 1) % 3]) F[kFORD] += (double)(1 << e);
       F[kFLEN + e] = len;
     }
     for (int k = 0; k < 3; ++k) {
@@ -930,7 +1110,6 @@ extern "C" int wsb_mesh_create(const double* verts, int64_t n_verts, const int32
       F[kFHI + k] = std::max(P[0][k], std::max(P[1][k], P[2][k]));
       blo[k] = std::min(blo[k], F[kFLO + k]);
       bhi[k] = std::max(bhi[k], F[kFHI + k]);
-      hvid[3 * f + k] = v[k];
     }
   }
   if (!(vol6 > 0.0)) return fail(WSB_ERR_ARG, "wsb_mesh_create: surface must have positive signed volume");
@@ -951,8 +1130,8 @@ extern "C" int wsb_mesh_create(const double* verts, int64_t n_verts, const int32
     const int64_t i = (int64_t)std::floor((x - lo[k]) / cell);
     return std::min<int64_t>(std::max<int64_t>(i, 0), n3[k] - 1);
   };
-  const int64_t ncell = nx * ny * nz, ncol = nx * ny;
-  std::vector<int64_t> cnt(ncell + 1, 0), ccnt(ncol + 1, 0);
+  const int64_t ncell = nx * ny * nz;
+  std::vector<int64_t> cnt(ncell + 1, 0), ccnt;
   std::vector<int32_t> fcell((size_t)n_faces * 3);
   std::vector<int64_t> range((size_t)n_faces * 6);
   for (int64_t f = 0; f < n_faces; ++f) {
@@ -965,9 +1144,36 @@ extern "C" int wsb_mesh_create(const double* verts, int64_t n_verts, const int32
     for (int64_t kz = range[6 * f + 4]; kz <= range[6 * f + 5]; ++kz)
       for (int64_t jy = range[6 * f + 2]; jy <= range[6 * f + 3]; ++jy)
         for (int64_t ix = range[6 * f]; ix <= range[6 * f + 1]; ++ix) ++cnt[(kz * ny + jy) * nx + ix + 1];
-    for (int64_t jy = range[6 * f + 2]; jy <= range[6 * f + 3]; ++jy)
-      for (int64_t ix = range[6 * f]; ix <= range[6 * f + 1]; ++ix) ++ccnt[jy * nx + ix + 1];
   }
+  // (x, y) columns of half a cell: the inside test meets 24 faces a column on the 20480-face scene instead of 46 with
+  // whole cells; whole cells where faces far larger than a cell would list more than 2^28 items
+  double col = 0.0;
+  int64_t ncx = 0, ncy = 0;
+  auto crange = [&](int64_t f, int64_t r[4]) {
+    const double* F = hf.data() + f * kFaceDoubles;
+    for (int k = 0; k < 2; ++k) {
+      const int64_t top = (k == 0 ? ncx : ncy) - 1;
+      r[2 * k] = std::min<int64_t>(std::max<int64_t>((int64_t)std::floor((F[kFLO + k] - lo[k]) / col), 0), top);
+      r[2 * k + 1] = std::min<int64_t>(std::max<int64_t>((int64_t)std::floor((F[kFHI + k] - lo[k]) / col), 0), top);
+    }
+  };
+  for (int split = 2; split >= 1; --split) {
+    col = cell / split;
+    ncx = nx * split;
+    ncy = ny * split;
+    ccnt.assign((size_t)(ncx * ncy) + 1, 0);
+    int64_t total = 0;
+    for (int64_t f = 0; f < n_faces; ++f) {
+      int64_t r[4];
+      crange(f, r);
+      total += (r[1] - r[0] + 1) * (r[3] - r[2] + 1);
+      if (split > 1 && total > ((int64_t)1 << 28)) break;
+      for (int64_t jy = r[2]; jy <= r[3]; ++jy)
+        for (int64_t ix = r[0]; ix <= r[1]; ++ix) ++ccnt[jy * ncx + ix + 1];
+    }
+    if (split == 1 || total <= ((int64_t)1 << 28)) break;
+  }
+  const int64_t ncol = ncx * ncy;
   for (int64_t c = 0; c < ncell; ++c) cnt[c + 1] += cnt[c];
   for (int64_t c = 0; c < ncol; ++c) ccnt[c + 1] += ccnt[c];
   if (cnt[ncell] > INT32_MAX || ccnt[ncol] > INT32_MAX)
@@ -975,14 +1181,16 @@ extern "C" int wsb_mesh_create(const double* verts, int64_t n_verts, const int32
   std::vector<int32_t> items((size_t)cnt[ncell]), citems((size_t)ccnt[ncol]);
   std::vector<int32_t> start(cnt.begin(), cnt.end()), cstart(ccnt.begin(), ccnt.end());
   {
-    std::vector<int64_t> cur(cnt.begin(), cnt.end() - 1), ccur(ccnt.begin(), ccnt.end() - 1);
+    std::vector<int64_t>&cur = cnt, &ccur = ccnt;      // (the starts are copied: the counts serve as fill cursors)
     for (int64_t f = 0; f < n_faces; ++f) {
       for (int64_t kz = range[6 * f + 4]; kz <= range[6 * f + 5]; ++kz)
         for (int64_t jy = range[6 * f + 2]; jy <= range[6 * f + 3]; ++jy)
           for (int64_t ix = range[6 * f]; ix <= range[6 * f + 1]; ++ix)
             items[cur[(kz * ny + jy) * nx + ix]++] = (int32_t)f;
-      for (int64_t jy = range[6 * f + 2]; jy <= range[6 * f + 3]; ++jy)
-        for (int64_t ix = range[6 * f]; ix <= range[6 * f + 1]; ++ix) citems[ccur[jy * nx + ix]++] = (int32_t)f;
+      int64_t r[4];
+      crange(f, r);
+      for (int64_t jy = r[2]; jy <= r[3]; ++jy)
+        for (int64_t ix = r[0]; ix <= r[1]; ++ix) citems[ccur[jy * ncx + ix]++] = (int32_t)f;
     }
   }
   WSB_CUDA(cudaSetDevice(device));
@@ -996,25 +1204,27 @@ extern "C" int wsb_mesh_create(const double* verts, int64_t n_verts, const int32
   m->nx = (int32_t)nx;
   m->ny = (int32_t)ny;
   m->nz = (int32_t)nz;
+  m->col = col;
+  m->ncx = (int32_t)ncx;
+  m->ncy = (int32_t)ncy;
   m->n_items = (int64_t)items.size();
   m->n_col_items = (int64_t)citems.size();
+  // the cells' candidate lists and flags, from the box lists (device copies for the length of this call)
+  const int64_t ncells = (int64_t)m->nx * m->ny * m->nz;
+  int32_t *d_start = nullptr, *d_items = nullptr, *d_fcell = nullptr, *d_len = nullptr;
   int rc;
-  if ((rc = upload_vec(&m->fdata, hf)) || (rc = upload_vec(&m->fcell, fcell)) || (rc = upload_vec(&m->fvid, hvid)) ||
-      (rc = upload_vec(&m->cstart, start)) || (rc = upload_vec(&m->citems, items)) ||
-      (rc = upload_vec(&m->colstart, cstart)) || (rc = upload_vec(&m->colitems, citems)) ||
-      (rc = upload_vec(&m->cflag, std::vector<uint8_t>((size_t)m->nx * m->ny * m->nz, 0)))) {
+  if ((rc = upload_vec(&m->fdata, hf)) || (rc = upload_vec(&m->colstart, cstart)) ||
+      (rc = upload_vec(&m->colitems, citems)) || (rc = upload_vec(&d_start, start)) ||
+      (rc = upload_vec(&d_items, items)) || (rc = upload_vec(&d_fcell, fcell))) {
+  } else {
+    rc = mesh_lists(m, BoxLists{d_start, d_items, d_fcell}, ncells, &d_len);
+  }
+  for (void* p : {(void*)d_start, (void*)d_items, (void*)d_fcell, (void*)d_len})
+    if (p) cudaFree(p);
+  if (rc) {
     free_mesh(m);
     delete m;
     return rc;
-  }
-  const int64_t ncells = (int64_t)m->nx * m->ny * m->nz;
-  k_mesh_cellflags<<<(unsigned)((ncells + 255) / 256), 256>>>(view_of(m), m->cflag);
-  cudaError_t e = cudaDeviceSynchronize();
-  if (e == cudaSuccess) e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    free_mesh(m);
-    delete m;
-    return cuda_fail(e, "wsb_mesh_create: cell flags");
   }
   *out = static_cast<wsb_mesh*>(m);
   return WSB_OK;
@@ -1030,7 +1240,7 @@ extern "C" int wsb_mesh_destroy(wsb_mesh* m) {
 
 extern "C" size_t wsb_mesh_workspace_size(const wsb_mesh* m, int64_t n) {
   if (!m || n < 0) return 0;
-  return al256(sizeof(int32_t) * (size_t)std::max<int64_t>(n, 1)) * 3 + 256;
+  return carve_mesh(m, n, nullptr).total;
 }
 
 extern "C" int wsb_mesh_inside(const wsb_mesh* m, const double* pos, int64_t n, int32_t* inside, void* stream) {
@@ -1057,17 +1267,13 @@ extern "C" int wsb_mesh_channels(const wsb_mesh* m, int kernel, const double* po
   if (workspace_bytes < wsb_mesh_workspace_size(m, n))
     return fail(WSB_ERR_SIZE, "wsb_mesh_channels: workspace smaller than wsb_mesh_workspace_size");
   WSB_CUDA(cudaSetDevice(m->device));
-  char* base = (char*)workspace;
-  const size_t s = al256(sizeof(int32_t) * (size_t)n);
-  int32_t* work = (int32_t*)base;
-  int32_t* ind = inside ? inside : (int32_t*)(base + s);
-  int32_t* nwork = (int32_t*)(base + 2 * s);     // [3]: work rows, (unused), listed rows
-  int32_t* near = (int32_t*)(base + 2 * s + 256);
+  const MeshWork w = carve_mesh(m, n, workspace);
+  int32_t* ind = inside ? inside : w.ind;
   cudaStream_t st = (cudaStream_t)stream;
   switch (kernel) {
-    case WSB_KERNEL_CUBIC: return launch_mesh<Mesh_cubic>(m, pos, sup, n, out, ind, work, nwork, near, st);
-    case WSB_KERNEL_W2: return launch_mesh<Mesh_w2>(m, pos, sup, n, out, ind, work, nwork, near, st);
-    case WSB_KERNEL_W4: return launch_mesh<Mesh_w4>(m, pos, sup, n, out, ind, work, nwork, near, st);
-    default: return launch_mesh<Mesh_w6>(m, pos, sup, n, out, ind, work, nwork, near, st);
+    case WSB_KERNEL_CUBIC: return launch_mesh<Mesh_cubic>(m, pos, sup, n, out, ind, w, st);
+    case WSB_KERNEL_W2: return launch_mesh<Mesh_w2>(m, pos, sup, n, out, ind, w, st);
+    case WSB_KERNEL_W4: return launch_mesh<Mesh_w4>(m, pos, sup, n, out, ind, w, st);
+    default: return launch_mesh<Mesh_w6>(m, pos, sup, n, out, ind, w, st);
   }
 }
