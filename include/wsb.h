@@ -225,6 +225,14 @@ int wsb_aggregate_backward(const wsb_surface* s, int kernel, const double* pos, 
 int wsb_signed_distance(const wsb_surface* s, const double* lpos, int64_t m, double norm_support, double* d,
                         double* cp, double* n_loc, int32_t* edge, void* stream);
 
+/* The same for one surface of a posed body at world points, in one pass: pos [2m] world, pose (cx, cy, cos, sin) on the
+ * device; keeps the nearest so far in best [m], normal [2m] (world frame) and, where given, body_index [m] -- a point
+ * is overwritten where the signed distance is below best, every point with `first` != 0 (nothing before: best may be
+ * uninitialised; a point without a distance gets infinity, a zero normal and -1).  Replaces the loop over bodies and
+ * representations of Scene.signed_distance (src/warpSPHBoundaries/scene/scene.py:1312-1372). */
+int wsb_body_distance(const wsb_surface* s, const double* pos, int64_t m, const double* pose, double norm_support,
+                      int first, int64_t body, double* best, double* normal, int64_t* body_index, void* stream);
+
 /* Rigid-body fields of B bodies at world points x [n*2]: body [b] = (cx, cy, cos, sin, vx, vy, omega, ax, ay, alpha)
  * (device [B*10]); writes rel, local, velocity, acceleration [B*n*2] (any may be NULL).  Replaces BodyKinematics
  * (src/warpSPHBoundaries/scene/scene.py:1155-1225) and Body.velocityAt / accelerationAt (scene.py:934-939, 1063-1067). */

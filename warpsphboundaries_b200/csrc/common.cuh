@@ -60,6 +60,11 @@ struct Surface {
   int32_t* bitems = nullptr;    // [n_bitems]
   double4* erec = nullptr;      // [n_edges] (ax, ay, bx, by) by edge id
   double4* brec = nullptr;      // [n_bitems] the records of the y-bin items, bin order
+  // bounding-box tree over the edges (signed distance), one allocation: node boxes by level, edge records and ids in
+  // tree order
+  double4* tbox = nullptr;
+  double4* trec = nullptr;      // [n_edges]
+  int32_t* tid = nullptr;       // [n_edges]
   // host copies (tests, signed distance set-up)
   std::string err;
 };

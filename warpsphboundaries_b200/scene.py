@@ -920,42 +920,46 @@ class Scene:
         normal from the wall into the fluid (scene.py:1312-1372)."""
         pts = points.to(self.device, F64).contiguous()
         M = len(pts)
-        bidx = torch.full((M,), -1, dtype=torch.long, device=self.device)
-        best = torch.full((M,), float("inf"), dtype=F64, device=self.device)
-        normal = torch.zeros((M, 2), dtype=F64, device=self.device)
-        hit = torch.zeros(M, dtype=torch.bool, device=self.device)
+        best = torch.empty(M, dtype=F64, device=self.device)
+        normal = torch.empty((M, 2), dtype=F64, device=self.device)
+        bidx = torch.empty(M, dtype=torch.long, device=self.device) if want_body else None
+        first = True                                   # nothing written yet: the first representation assigns
+
+        def clear():
+            best.fill_(float("inf"))
+            normal.zero_()
+            if want_body:
+                bidx.fill_(-1)
+
         for bi, bd in enumerate(self.bodies):
             if body is not None and bi != body:
                 continue
-            lp = bd.toLocal(pts).contiguous()
             for rep in bd.reps:
                 if isinstance(rep, SdfRep):
                     rep = rep.lowered(0.0, self.device)        # the exact distance to its polygon form
                 if isinstance(rep, (BoxRep, ImplicitRep, DiskArrayRep)):
                     # the shape's own closed form and normals (scene.py:1351-1353, 1360-1362)
-                    d, nl = rep.signed(lp)
+                    if first:
+                        clear()
+                        first = False
+                    d, nl = rep.signed(bd.toLocal(pts).contiguous())
                     n = bd.pose.vecToWorld(nl)
                     better = d < best
                     best = torch.where(better, d, best)
                     normal = torch.where(better[:, None], n, normal)
-                    bidx = torch.where(better, torch.full_like(bidx, bi), bidx)
-                    hit |= True
+                    if want_body:
+                        bidx = torch.where(better, torch.full_like(bidx, bi), bidx)
                     continue
                 if not isinstance(rep, SurfaceRep):
                     continue
                 ns = rep.native(supportMax, self.device) if supportMax is not None else rep._default_native(self.device)
-                d = torch.empty(M, dtype=F64, device=self.device)
-                cp = torch.empty((M, 2), dtype=F64, device=self.device)
-                nl = torch.empty((M, 2), dtype=F64, device=self.device)
-                ed = torch.empty(M, dtype=torch.int32, device=self.device)
-                check(lib.wsb_signed_distance(ns.handle, ptr(lp), M, float(supportMax) if supportMax else 0.0, ptr(d),
-                                              ptr(cp), ptr(nl), ptr(ed), _stream()), "wsb_signed_distance")
-                n = bd.pose.vecToWorld(nl)
-                better = d < best
-                best = torch.where(better, d, best)
-                normal = torch.where(better[:, None], n, normal)
-                bidx = torch.where(better, torch.full_like(bidx, bi), bidx)
-                hit |= True
+                check(lib.wsb_body_distance(ns.handle, ptr(pts), M, ptr(bd.pose_tensor(self.device)),
+                                            float(supportMax) if supportMax else 0.0, int(first), bi, ptr(best),
+                                            ptr(normal), ptr(bidx), _stream()), "wsb_body_distance")
+                first = False
+        hit = torch.full((M,), not first, dtype=torch.bool, device=self.device)
+        if first:
+            clear()
         if want_body:
             return best, normal, hit, bidx
         return best, normal, hit
