@@ -40,103 +40,107 @@ struct Disks {
 
 constexpr int kDiskThreads = 128;
 
-// the sum over the warp's lanes, in a fixed butterfly order, on every lane
-__device__ __forceinline__ double warp_allsum(double v) {
+constexpr int kDiskBlocks = 4;    // resident CTAs per SM of the arc pass (128 registers)
+
+// the arc of a disk's circle inside the support, u in [0, U] and its mirror image (U < 0: none): D = centre distance, R =
+// radius (h = 1), base = the distance of the singularity of the integrand from u = 0, knots = the angles where r crosses a
+// block radius, ascending (U where there is none)
+struct DiskArc {
+  double D, R, U, base, knots[kDiskMaxKnots];
+};
+
+template <int KID>
+__device__ __forceinline__ DiskArc disk_arc(double D, double R) {
+  DiskArc a;
+  a.D = D;
+  a.R = R;
+  const double dm = D - R;
+  // (D = 0: a concentric circle, one panel: the singularity distance is infinite)
+  a.U = D + R <= 1.0 ? 0.5 * kTwoPi : 2.0 * asin(fmin(1.0, sqrt((1.0 - dm * dm) / (4.0 * D * R))));
+  const double x = 0.5 * dm * dm / (D * R);                    // acosh(1 + x): the distance of the singularity
+  a.base = fmax(log1p(x + sqrt(x * (x + 2.0))), 0x1p-24);
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  return v;
+  for (int k = 0; k < kDiskMaxKnots; ++k) a.knots[k] = a.U;
+  double radii[kDiskMaxKnots];
+  const int nr = disk_knots<KID>(radii);
+  // (ascending radii give ascending angles)
+#pragma unroll
+  for (int k = 0; k < kDiskMaxKnots; ++k)
+    if (k < nr && fabs(dm) < radii[k] && radii[k] < D + R) {
+      const double kn = 2.0 * asin(fmin(1.0, sqrt((radii[k] * radii[k] - dm * dm) / (4.0 * D * R))));
+      if (kn > 0.0 && kn < a.U) a.knots[k] = kn;
+    }
+  return a;
 }
 
-// The seven non-zero channels of one disk in its aligned frame (before 1/pi): lam, m1_x, G_x, g1_xx, g1_yy, m2_xx,
-// m2_yy.  D = centre distance, R = radius (h = 1), D < 1 + R.  Called by a whole warp with the same (D, R): lane q
-// takes node q of every panel, the eight sums are reduced by a fixed butterfly, every lane returns the totals.
+// The panels of an arc: [0, U] split at the doublings 2 base, 4 base, ... and at the knots.  A panel that starts within
+// 2 base of u = 0 takes 24 Gauss-Legendre nodes, as two items of 12 (six node pairs about the panel's middle each), a
+// farther one, whose singularities lie at least its own length away (Bernstein parameter >= 5.8), 12 nodes: one item.
+struct DiskPanels {
+  double lo, hi, d;
+  __device__ __forceinline__ void first(const DiskArc& a) {
+    hi = 0.0;
+    d = 2.0 * a.base;
+    next(a);
+  }
+  __device__ __forceinline__ void next(const DiskArc& a) {
+    lo = hi;
+    double nxt = fmin(a.U, d);
+#pragma unroll
+    for (int k = kDiskMaxKnots - 1; k >= 0; --k)
+      if (a.knots[k] > lo && a.knots[k] < nxt) nxt = a.knots[k];
+    if (nxt >= d) d *= 2.0;
+    hi = nxt;
+  }
+  __device__ __forceinline__ int items(const DiskArc& a) const { return lo < 2.0 * a.base ? 2 : 1; }
+};
+constexpr int kMaxDiskPanels = 160;
+
+// the sums over the 12 nodes of one item, mirror image included: lam, m1, G, g1_xx, g1_yy, m2_xx, m2_yy, int F2 / r^2
 template <int KID>
-__device__ void disk_pair(double D, double R, int lane, double out[7]) {
-  double lam = 0.0, m1 = 0.0, G = 0.0, gxx = 0.0, gyy = 0.0, mxx = 0.0, myy = 0.0, SF = 0.0;
-  const double dm = D - R;
-  // the arc of the disk's circle inside the support: u in [0, U] (and its mirror image)
-  if (fabs(dm) < 1.0) {   // (D = 0: a concentric circle, one panel: the singularity distance is infinite)
-    const double U = D + R <= 1.0 ? 0.5 * kTwoPi : 2.0 * asin(fmin(1.0, sqrt((1.0 - dm * dm) / (4.0 * D * R))));
-    const double x = 0.5 * dm * dm / (D * R);                  // acosh(1 + x): the distance of the singularity
-    const double base = fmax(log1p(x + sqrt(x * (x + 2.0))), 0x1p-24);
-    double radii[kDiskMaxKnots], knots[kDiskMaxKnots];
-    const int nr = disk_knots<KID>(radii);
-    int nk = 0;
-    for (int k = 0; k < nr; ++k) {
-      const double Rb = radii[k];
-      if (fabs(dm) < Rb && Rb < D + R) {
-        const double kn = 2.0 * asin(fmin(1.0, sqrt((Rb * Rb - dm * dm) / (4.0 * D * R))));
-        if (kn > 0.0 && kn < U) knots[nk++] = kn;
-      }
-    }
-    for (int a = 1; a < nk; ++a)                                   // ascending (at most kDiskMaxKnots knots)
-      for (int b = a; b > 0 && knots[b] < knots[b - 1]; --b) {
-        const double t = knots[b];
-        knots[b] = knots[b - 1];
-        knots[b - 1] = t;
-      }
-    auto node = [&](double uu, double wq) {
-      double sh, ch;
-      sincos(0.5 * uu, &sh, &ch);                                  // one half-angle evaluation per node
-      const double s2 = sh * sh, su = 2.0 * sh * ch, cu = fma(-2.0, s2, 1.0);
-      const double yx = fma(2.0 * R, s2, dm), yy = R * su, nx = -cu, ny = su;
+__device__ __forceinline__ void disk_item(const DiskArc& a, const DiskPanels& p, int half, double s[8]) {
+  const double D = a.D, R = a.R, dm = D - R, DR4 = 4.0 * D * R;
+  const double hc = 0.5 * (p.hi - p.lo), mc = 0.5 * (p.hi + p.lo);
+  const bool near = p.lo < 2.0 * a.base;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) s[k] = 0.0;
+  // nodes come in pairs about the panel's middle: the half angles from one sincos a pair and one for the middle
+  double sm, cm;
+  sincos(0.5 * mc, &sm, &cm);
+  for (int q = 0; q < 6; ++q) {
+    const double x = near ? kQuadGx[12 + 6 * half + q] : kQuadFx[6 + q];
+    const double wg = near ? kQuadGw[12 + 6 * half + q] : kQuadFw[6 + q];
+    double sx, cx;
+    sincos(0.5 * hc * x, &sx, &cx);
+    const double w = 2.0 * R * hc * wg, sc = sm * cx, cs = cm * sx, cc = cm * cx, ss = sm * sx;
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+      const double sh = side ? sc + cs : sc - cs, ch = side ? cc - ss : cc + ss;
+      const double s2 = sh * sh, su = 2.0 * sh * ch, nx = fma(2.0, s2, -1.0);
+      const double yx = fma(2.0 * R, s2, dm), yy = R * su;
       const double yn = fma(2.0 * D, s2, -dm);
-      const double r = sqrt(fma(4.0 * D * R, s2, dm * dm));
+      const double r2 = fma(DR4, s2, dm * dm), r = sqrt(r2);
       double P, Fl, F2l;
-      disk_profile<KID>(r, 1.0 / (r * r), P, Fl, F2l);
-      const double F1 = Fl * r * r;
-      const double w = 2.0 * R * wq;
-      lam = fma(w * Fl, yn, lam);
-      m1 = fma(w * F1, nx, m1);
-      G = fma(-w * P, nx, G);
-      gxx = fma(-w * P * yx, nx, gxx);
-      gyy = fma(-w * P * yy, ny, gyy);
-      mxx = fma(w * F1 * yx, nx, mxx);
-      myy = fma(w * F1 * yy, ny, myy);
-      SF = fma(w * F2l, yn, SF);
-    };
-    // the panel after u: up to the doubling bound d or the next knot, whichever is first
-    double d = 2.0 * base;
-    int ki = 0;
-    auto next_panel = [&](double u) {
-      double nxt = fmin(U, d);
-      while (ki < nk && knots[ki] <= u) ++ki;
-      if (ki < nk && knots[ki] < nxt) nxt = knots[ki];
-      if (nxt >= d) d *= 2.0;
-      return nxt;
-    };
-    // panels next to the nearest point (start below 2 * base) take 24 nodes on lanes 0-23; farther panels, whose
-    // singularities lie at least their own length away (Bernstein parameter >= 5.8), 12 nodes, two panels at a time
-    // (lanes 0-11 and 12-23)
-    double u = 0.0;
-    for (int it = 0; it < 160 && u < U; ++it) {
-      const double a0 = u, a1 = next_panel(u);
-      if (a0 < 2.0 * base) {
-        const double hc = 0.5 * (a1 - a0), mc = 0.5 * (a1 + a0);
-        if (lane < kQuadGauss) node(fma(hc, kQuadGx[lane], mc), hc * kQuadGw[lane]);
-        u = a1;
-        continue;
-      }
-      const double b1 = a1 < U ? next_panel(a1) : a1;
-      const bool second = lane >= kQuadGaussFar;
-      const double lo = second ? a1 : a0, hi = second ? b1 : a1;
-      const int q = second ? lane - kQuadGaussFar : lane;
-      if (q < kQuadGaussFar && hi > lo) {
-        const double hc = 0.5 * (hi - lo), mc = 0.5 * (hi + lo);
-        node(fma(hc, kQuadFx[q], mc), hc * kQuadFw[q]);
-      }
-      u = b1;
+      disk_profile<KID>(r, P, Fl, F2l);
+      const double wF1 = w * Fl * r2, wP = w * P, xx = yx * nx, yy2 = yy * su;
+      s[0] = fma(w * Fl, yn, s[0]);
+      s[1] = fma(wF1, nx, s[1]);
+      s[2] = fma(-wP, nx, s[2]);
+      s[3] = fma(-wP, xx, s[3]);
+      s[4] = fma(-wP, yy2, s[4]);
+      s[5] = fma(wF1, xx, s[5]);
+      s[6] = fma(wF1, yy2, s[6]);
+      s[7] = fma(w * F2l, yn, s[7]);
     }
   }
-  lam = warp_allsum(lam);
-  m1 = warp_allsum(m1);
-  G = warp_allsum(G);
-  gxx = warp_allsum(gxx);
-  gyy = warp_allsum(gyy);
-  mxx = warp_allsum(mxx);
-  myy = warp_allsum(myy);
-  SF = warp_allsum(SF);
-  // the arc of the support circle inside the disk: |phi| < beta
+}
+
+// The seven non-zero channels of one disk in its aligned frame (before 1/pi): lam, m1_x, G_x, g1_xx, g1_yy, m2_xx, m2_yy,
+// from the sums over the disk's arc (zero where the circle does not meet the support) and the arc of the support circle
+// inside the disk, |phi| < beta, in closed form
+template <int KID>
+__device__ __forceinline__ void disk_channels(double D, double R, const double s[8], double out[7]) {
+  double lam = s[0], m1 = s[1], G = s[2], gxx = s[3], gyy = s[4], mxx = s[5], myy = s[6], SF = s[7];
   double beta = -1.0;
   if (R >= D + 1.0)
     beta = 0.5 * kTwoPi;
@@ -144,9 +148,10 @@ __device__ void disk_pair(double D, double R, int lane, double out[7]) {
     beta = 2.0 * asin(fmin(1.0, sqrt((R * R - (D - 1.0) * (D - 1.0)) / (4.0 * D))));
   if (beta > 0.0) {
     double P1, Fl1, F2l1;
-    disk_profile<KID>(1.0, 1.0, P1, Fl1, F2l1);
-    const double sb = sin(beta), s2b = sin(2.0 * beta);
-    const double cxx = beta + 0.5 * s2b, cyy = beta - 0.5 * s2b;
+    disk_profile<KID>(1.0, P1, Fl1, F2l1);
+    double sb, cb;
+    sincos(beta, &sb, &cb);
+    const double cxx = fma(sb, cb, beta), cyy = fma(-sb, cb, beta);
     lam += 2.0 * beta * Fl1;
     m1 += 2.0 * sb * Fl1;
     G -= 2.0 * sb * P1;
@@ -165,6 +170,40 @@ __device__ void disk_pair(double D, double R, int lane, double out[7]) {
   out[6] = myy - SF;
 }
 
+// the channels of one disk added to the row's, the aligned frame's x axis along (ca, sa)
+__device__ __forceinline__ void disk_add(const double o[7], double ca, double sa, double acc[12]) {
+  acc[0] += o[0];
+  acc[1] += ca * o[1];
+  acc[2] += sa * o[1];
+  acc[3] += ca * o[2];
+  acc[4] += sa * o[2];
+  const double dg = o[3] - o[4], dmm = o[5] - o[6];
+  acc[5] += ca * ca * o[3] + sa * sa * o[4];
+  acc[6] += ca * sa * dg;
+  acc[7] += ca * sa * dg;
+  acc[8] += sa * sa * o[3] + ca * ca * o[4];
+  acc[9] += ca * ca * o[5] + sa * sa * o[6];
+  acc[10] += ca * sa * dmm;
+  acc[11] += sa * sa * o[5] + ca * ca * o[6];
+}
+
+// a disk of the particle's cell in units of the support: within reach (D < 1 + R), its circle meeting the support
+// (|D - R| < 1); a disk that is neither is either out of reach or covers the support
+struct DiskAt {
+  double vx, vy, D, R;
+  bool reach, arc;
+};
+__device__ __forceinline__ DiskAt disk_at(const double4& e, double lx, double ly, double ih) {
+  DiskAt t;
+  t.vx = (e.x - lx) * ih;
+  t.vy = (e.y - ly) * ih;
+  t.R = e.z * ih;
+  t.D = sqrt(t.vx * t.vx + t.vy * t.vy);
+  t.reach = t.D < 1.0 + t.R;
+  t.arc = t.reach && fabs(t.D - t.R) < 1.0;
+  return t;
+}
+
 // the body-frame position of particle i and its cell (false outside the grid or outside `allowed`)
 __device__ __forceinline__ bool disk_row(const double* __restrict__ pos, const int32_t* __restrict__ allowed,
                                          const double* __restrict__ pose, int64_t i, int32_t nx, int32_t ny,
@@ -177,8 +216,10 @@ __device__ __forceinline__ bool disk_row(const double* __restrict__ pos, const i
   return true;
 }
 
-// Pass 1, one thread per particle: a particle that reaches no disk gets its zero channels (when the call assigns);
-// the others are appended to the work list (warp-aggregated).
+// Pass 1, one thread per particle: a particle that no circle meets gets its channels at once (zeros when the call
+// assigns, the whole-support values of the disks that cover it); the others are listed -- those with one arc from the
+// front of `work`, those with more from its back, so that a warp of the second pass holds equal rows (warp-aggregated).
+template <int KID>
 __global__ void __launch_bounds__(kDiskThreads) k_disk_rows(const int32_t* __restrict__ cstart,
                                                            const double4* __restrict__ items, int32_t nx,
                                                            int32_t ny, double lo_x, double lo_y, double cell,
@@ -186,85 +227,153 @@ __global__ void __launch_bounds__(kDiskThreads) k_disk_rows(const int32_t* __res
                                                            const double* __restrict__ sup,
                                                            const int32_t* __restrict__ allowed, int64_t n,
                                                            const double* __restrict__ pose, bool assign,
-                                                           int32_t* __restrict__ work, int32_t* __restrict__ nwork,
+                                                           int32_t* __restrict__ work, int32_t* __restrict__ counts,
                                                            double* lam, double* G, double* cov, double* m1,
                                                            double* m2) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  bool has = false;
+  int arcs = 0;
   if (i < n) {
-    double lx, ly;
+    double lx, ly, covered = 0.0;
     int32_t cid;
     if (disk_row(pos, allowed, pose, i, nx, ny, lo_x, lo_y, cell, lx, ly, cid)) {
       const double ih = 1.0 / sup[i];
-      for (int32_t k = cstart[cid]; k < cstart[cid + 1] && !has; ++k) {
-        const double4 e = items[k];
-        const double vx = (e.x - lx) * ih, vy = (e.y - ly) * ih;
-        has = sqrt(vx * vx + vy * vy) < 1.0 + e.z * ih;
+      for (int32_t k = cstart[cid]; k < cstart[cid + 1]; ++k) {
+        const DiskAt t = disk_at(items[k], lx, ly, ih);
+        arcs += t.arc ? 1 : 0;
+        covered += t.reach && !t.arc ? 1.0 : 0.0;
       }
     }
-    if (!has && assign) {
+    if (arcs == 0 && (assign || covered > 0.0)) {
       double acc[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+      if (covered > 0.0) {                                   // (any disk that covers the support gives the same values)
+        const double zero[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        double o[7];
+        disk_channels<KID>(0.0, 2.0, zero, o);
+        acc[0] = covered * kInvPi * o[0];
+        acc[5] = acc[8] = covered * kInvPi * o[3];
+        acc[9] = acc[11] = covered * kInvPi * o[5];
+      }
       const double c = pose[2], s = pose[3];
       const double rot[4] = {c, -s, s, c};
-      write_outputs(acc, sup[i], rot, i, lam, G, cov, m1, m2, true);
+      write_outputs(acc, sup[i], rot, i, lam, G, cov, m1, m2, assign);
     }
   }
-  const unsigned ballot = __ballot_sync(0xffffffffu, has);
+  const unsigned one = __ballot_sync(0xffffffffu, arcs == 1), more = __ballot_sync(0xffffffffu, arcs > 1);
   const int lane = threadIdx.x & 31;
   int base = 0;
-  if (lane == 0 && ballot) base = atomicAdd(nwork, __popc(ballot));
-  base = __shfl_sync(0xffffffffu, base, 0);
-  if (has) work[base + __popc(ballot & ((1u << lane) - 1))] = (int32_t)i;
+  if (lane == 0 && one) base = atomicAdd(&counts[0], __popc(one));
+  if (lane == 1 && more) base = atomicAdd(&counts[1], __popc(more));
+  const int b0 = __shfl_sync(0xffffffffu, base, 0), b1 = __shfl_sync(0xffffffffu, base, 1);
+  const unsigned below = (1u << lane) - 1;
+  if (arcs == 1) work[b0 + __popc(one & below)] = (int32_t)i;
+  if (arcs > 1) work[n - 1 - (b1 + __popc(more & below))] = (int32_t)i;
 }
 
-// Pass 2, one warp per listed particle (grid-stride): every disk of the particle's cell within reach, in cell-list
-// order, integrated by the whole warp, rotated from its aligned frame and summed; lane 0 scales, rotates to the world
-// frame and writes.  Each particle is one warp's work in a fixed order: the result does not depend on the list order.
+// Pass 2, the listed particles, 32 to a warp, lane r for particle r: the disks of its cell in cell-list order -- one that
+// covers the support adds its constants, one with an arc waits for the warp: the arcs of the 32 particles are cut into
+// items of 12 quadrature nodes, flattened on the lanes (1 to some 20 panels an arc: a lane per arc would wait for the
+// longest), and lane r adds up its arc's items in order, so a particle's result does not depend on its neighbours.
+// On B200, 1024 disks and 2^20 particles (w4, 0.52 M arcs): 0.25 ms, 52 % of the FP64 pipe.  A warp per particle, the nodes of one panel after the
+// other over its lanes and eight butterfly sums per disk, took 1.25 ms; a thread per particle 4.79.
 template <int KID>
-__global__ void __launch_bounds__(kDiskThreads, 4) k_disk_warp(const int32_t* __restrict__ cstart,
-                                                           const double4* __restrict__ items, int32_t nx,
-                                                           int32_t ny, double lo_x, double lo_y, double cell,
-                                                           const double* __restrict__ pos,
-                                                           const double* __restrict__ sup,
-                                                           const int32_t* __restrict__ work,
-                                                           const int32_t* __restrict__ nwork_p,
-                                                           const double* __restrict__ pose, bool assign, double* lam,
-                                                           double* G, double* cov, double* m1, double* m2) {
-  const int lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(kDiskThreads, kDiskBlocks)
+    k_disk_arcs(const int32_t* __restrict__ cstart, const double4* __restrict__ items, int32_t nx, int32_t ny, double lo_x,
+                double lo_y, double cell, const double* __restrict__ pos, const double* __restrict__ sup,
+                const int32_t* __restrict__ work, const int32_t* __restrict__ counts, int64_t n,
+                const double* __restrict__ pose, bool assign, double* lam, double* G, double* cov, double* m1,
+                double* m2) {
+  __shared__ DiskArc s_arc[kDiskThreads / 32][32];
+  __shared__ double s_sum[kDiskThreads / 32][32][9];          // an item's eight sums (9: against bank conflicts)
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int64_t n0 = counts[0], n1 = counts[1], b0 = (n0 + 31) / 32, batches = b0 + (n1 + 31) / 32;
   const int64_t warps = (int64_t)gridDim.x * (kDiskThreads / 32);
-  const int64_t nwork = *nwork_p;
-  for (int64_t j = (int64_t)blockIdx.x * (kDiskThreads / 32) + threadIdx.x / 32; j < nwork; j += warps) {
-    const int64_t i = work[j];
-    double lx, ly;
-    int32_t cid = 0;
-    disk_row(pos, nullptr, pose, i, nx, ny, lo_x, lo_y, cell, lx, ly, cid);   // listed: inside the grid
-    const double h = sup[i], ih = 1.0 / h;
-    double acc[12];
+  for (int64_t b = (int64_t)blockIdx.x * (kDiskThreads / 32) + wib; b < batches; b += warps) {
+    const int64_t j = b < b0 ? b * 32 + lane : (b - b0) * 32 + lane;
+    const bool mine = j < (b < b0 ? n0 : n1);
+    const int64_t i = mine ? work[b < b0 ? j : n - 1 - j] : 0;
+    double lx = 0.0, ly = 0.0, h = 1.0, acc[12];
+    int32_t cid = 0, k = 0, k1 = 0;
 #pragma unroll
     for (int c = 0; c < 12; ++c) acc[c] = 0.0;
-    for (int32_t k = cstart[cid]; k < cstart[cid + 1]; ++k) {
-      const double4 e = items[k];
-      const double vx = (e.x - lx) * ih, vy = (e.y - ly) * ih, R = e.z * ih;
-      const double D = sqrt(vx * vx + vy * vy);
-      if (!(D < 1.0 + R)) continue;
-      double o[7];
-      disk_pair<KID>(D, R, lane, o);
-      const double ca = D > 0.0 ? vx / D : 1.0, sa = D > 0.0 ? vy / D : 0.0;
-      acc[0] += o[0];
-      acc[1] += ca * o[1];
-      acc[2] += sa * o[1];
-      acc[3] += ca * o[2];
-      acc[4] += sa * o[2];
-      const double dg = o[3] - o[4], dmm = o[5] - o[6];
-      acc[5] += ca * ca * o[3] + sa * sa * o[4];
-      acc[6] += ca * sa * dg;
-      acc[7] += ca * sa * dg;
-      acc[8] += sa * sa * o[3] + ca * ca * o[4];
-      acc[9] += ca * ca * o[5] + sa * sa * o[6];
-      acc[10] += ca * sa * dmm;
-      acc[11] += sa * sa * o[5] + ca * ca * o[6];
+    if (mine) {
+      disk_row(pos, nullptr, pose, i, nx, ny, lo_x, lo_y, cell, lx, ly, cid);   // listed: inside the grid
+      h = sup[i];
+      k = cstart[cid];
+      k1 = cstart[cid + 1];
     }
-    if (lane == 0) {
+    const double ih = 1.0 / h;
+    for (;;) {
+      // up to the lane's next arc
+      DiskAt t;
+      t.arc = false;
+      while (k < k1) {
+        t = disk_at(items[k++], lx, ly, ih);
+        if (t.arc) break;
+        if (t.reach) {
+          const double zero[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+          double o[7];
+          disk_channels<KID>(t.D, t.R, zero, o);
+          disk_add(o, t.D > 0.0 ? t.vx / t.D : 1.0, t.D > 0.0 ? t.vy / t.D : 0.0, acc);
+        }
+      }
+      if (!__any_sync(0xffffffffu, t.arc)) break;
+      // the arc's items: counted by walking its panels
+      int count = 0;
+      if (t.arc) {
+        const DiskArc a = disk_arc<KID>(t.D, t.R);
+        s_arc[wib][lane] = a;
+        DiskPanels p;
+        p.first(a);
+        count = p.items(a);
+        for (int it = 0; it < kMaxDiskPanels && p.hi < a.U; ++it) {
+          p.next(a);
+          count += p.items(a);
+        }
+      }
+      int inc = count;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      const int total = __shfl_sync(0xffffffffu, inc, 31), pref = inc - count;
+      __syncwarp();
+      double s[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) s[c] = 0.0;
+      for (int base = 0; base < total; base += 32) {
+        const int item = base + lane;
+        int r = 0;                                            // the last lane whose prefix is <= item
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1)
+          if (__shfl_sync(0xffffffffu, pref, r + step) <= item) r += step;
+        int at = item - __shfl_sync(0xffffffffu, pref, r);
+        if (item < total) {
+          const DiskArc a = s_arc[wib][r];
+          DiskPanels p;
+          p.first(a);
+          while (at >= p.items(a)) {                          // (at is below the arc's count: the walk ends in its panels)
+            at -= p.items(a);
+            p.next(a);
+          }
+          double v[8];
+          disk_item<KID>(a, p, at, v);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) s_sum[wib][lane][c] = v[c];
+        }
+        __syncwarp();
+        for (int q = max(pref - base, 0); q < min(pref + count - base, 32); ++q)
+#pragma unroll
+          for (int c = 0; c < 8; ++c) s[c] += s_sum[wib][q][c];
+        __syncwarp();
+      }
+      if (t.arc) {
+        double o[7];
+        disk_channels<KID>(t.D, t.R, s, o);
+        disk_add(o, t.D > 0.0 ? t.vx / t.D : 1.0, t.D > 0.0 ? t.vy / t.D : 0.0, acc);
+      }
+    }
+    if (mine) {
 #pragma unroll
       for (int c = 0; c < 12; ++c) acc[c] *= kInvPi;
       const double c = pose[2], s = pose[3];
@@ -569,19 +678,21 @@ extern "C" int wsb_disk_aggregate(const wsb_disks* d_, int kernel, const double*
   double* M1 = (out_mask & WSB_OUT_M1) ? m1 : nullptr;
   double* M2 = (out_mask & WSB_OUT_M2) ? m2 : nullptr;
   int32_t* work = static_cast<int32_t*>(workspace);
-  int32_t* nwork = reinterpret_cast<int32_t*>(static_cast<char*>(workspace) + need - 256);
-  WSB_CUDA(cudaMemsetAsync(nwork, 0, sizeof(int32_t), st));
+  int32_t* counts = reinterpret_cast<int32_t*>(static_cast<char*>(workspace) + need - 256);
+  WSB_CUDA(cudaMemsetAsync(counts, 0, 2 * sizeof(int32_t), st));
   const unsigned grid = (unsigned)((n + kDiskThreads - 1) / kDiskThreads);
-  k_disk_rows<<<grid, kDiskThreads, 0, st>>>(d->cstart, d->items, d->nx, d->ny, d->lo_x, d->lo_y, d->cell, pos, sup,
-                                             allowed, n, pose, assign, work, nwork, L, Gp, C, M1, M2);
-  // warps per listed particle, grid-stride: at most 16 blocks of 4 warps per SM, never more warps than particles
+  // the resident warps, striding over batches of 32 listed particles; no more warps than batches
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device);
-  const int64_t wgrid = std::min<int64_t>((n + 3) / 4, (int64_t)sms * 16);
+  constexpr int W = kDiskThreads / 32;
+  const int64_t batches = (n + 31) / 32 + 1;
+  const unsigned wgrid = (unsigned)std::min<int64_t>((batches + W - 1) / W, (int64_t)sms * kDiskBlocks);
   auto launch = [&](auto kid) {
-    k_disk_warp<decltype(kid)::value><<<(unsigned)wgrid, kDiskThreads, 0, st>>>(
-        d->cstart, d->items, d->nx, d->ny, d->lo_x, d->lo_y, d->cell, pos, sup, work, nwork, pose, assign, L, Gp, C,
-        M1, M2);
+    constexpr int K = decltype(kid)::value;
+    k_disk_rows<K><<<grid, kDiskThreads, 0, st>>>(d->cstart, d->items, d->nx, d->ny, d->lo_x, d->lo_y, d->cell, pos, sup,
+                                                  allowed, n, pose, assign, work, counts, L, Gp, C, M1, M2);
+    k_disk_arcs<K><<<wgrid, kDiskThreads, 0, st>>>(d->cstart, d->items, d->nx, d->ny, d->lo_x, d->lo_y, d->cell, pos,
+                                                   sup, work, counts, n, pose, assign, L, Gp, C, M1, M2);
   };
   switch (kernel) {
     case 0: launch(std::integral_constant<int, 0>{}); break;

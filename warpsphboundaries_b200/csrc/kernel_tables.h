@@ -1857,10 +1857,9 @@ template <> __device__ __forceinline__ void Cheb_lw4::potentials<0>(float x, flo
 }
 
 // ---- disk element: pi*W, M/r^2 and the second potential of every exact kernel, summed over its blocks
-template <int KID> __device__ __forceinline__ void disk_profile(double r, double ir2, double& P, double& Fl,
-                                                             double& F2l);
+template <int KID> __device__ __forceinline__ void disk_profile(double r, double& P, double& Fl, double& F2l);
 template <int KID> __device__ __forceinline__ int disk_knots(double* out);
-template <> __device__ __forceinline__ void disk_profile<0>(double r, double ir2, double& P, double& Fl, double& F2l) {   // cubic
+template <> __device__ __forceinline__ void disk_profile<0>(double r, double& P, double& Fl, double& F2l) {   // cubic
   P = 0.0;
   Fl = 0.0;
   F2l = 0.25;
@@ -1869,6 +1868,7 @@ template <> __device__ __forceinline__ void disk_profile<0>(double r, double ir2
     Fl += fma(fma(fma(-2.2857142857142856, r, 8.571428571428571), r, -11.428571428571429), r, 5.714285714285714);
     F2l += fma(fma(fma(fma(fma(-0.32653061224489793, r, 1.4285714285714286), r, -2.2857142857142856), r, 1.4285714285714286), r, 0.0), r, -0.2857142857142857);
   } else {
+    const double ir2 = 1.0 / (r * r);
     Fl += 0.5714285714285714 * ir2;
     F2l += -0.04081632653061224 * ir2;
   }
@@ -1877,6 +1877,7 @@ template <> __device__ __forceinline__ void disk_profile<0>(double r, double ir2
     Fl += fma(fma(fma(9.142857142857142, r, -17.142857142857142), r, 11.428571428571429), r, -2.857142857142857);
     F2l += fma(fma(fma(fma(fma(1.3061224489795917, r, -2.857142857142857), r, 2.2857142857142856), r, -0.7142857142857143), r, 0.0), r, 0.03571428571428571);
   } else {
+    const double ir2 = 1.0 / (r * r);
     Fl += -0.07142857142857142 * ir2;
     F2l += 0.0012755102040816326 * ir2;
   }
@@ -1885,7 +1886,7 @@ template <> __device__ __forceinline__ int disk_knots<0>(double* out) {
   out[0] = 0.5;
   return 1;
 }
-template <> __device__ __forceinline__ void disk_profile<1>(double r, double ir2, double& P, double& Fl, double& F2l) {   // w2
+template <> __device__ __forceinline__ void disk_profile<1>(double r, double& P, double& Fl, double& F2l) {   // w2
   P = 0.0;
   Fl = 0.0;
   F2l = 0.25;
@@ -1894,6 +1895,7 @@ template <> __device__ __forceinline__ void disk_profile<1>(double r, double ir2
     Fl += fma(fma(fma(fma(fma(4.0, r, -17.5), r, 28.0), r, -17.5), r, 0.0), r, 3.5);
     F2l += fma(fma(fma(fma(fma(fma(fma(0.4444444444444444, r, -2.1875), r, 4.0), r, -2.9166666666666665), r, 0.0), r, 0.875), r, 0.0), r, -0.25);
   } else {
+    const double ir2 = 1.0 / (r * r);
     Fl += 0.5 * ir2;
     F2l += -0.034722222222222224 * ir2;
   }
@@ -1901,7 +1903,7 @@ template <> __device__ __forceinline__ void disk_profile<1>(double r, double ir2
 template <> __device__ __forceinline__ int disk_knots<1>(double* out) {
   return 0;
 }
-template <> __device__ __forceinline__ void disk_profile<2>(double r, double ir2, double& P, double& Fl, double& F2l) {   // w4
+template <> __device__ __forceinline__ void disk_profile<2>(double r, double& P, double& Fl, double& F2l) {   // w4
   P = 0.0;
   Fl = 0.0;
   F2l = 0.25;
@@ -1910,6 +1912,7 @@ template <> __device__ __forceinline__ void disk_profile<2>(double r, double ir2
     Fl += fma(fma(fma(fma(fma(fma(fma(fma(10.5, r, -64.0), r, 157.5), r, -192.0), r, 105.0), r, 0.0), r, -21.0), r, 0.0), r, 4.5);
     F2l += fma(fma(fma(fma(fma(fma(fma(fma(fma(fma(0.875, r, -5.818181818181818), r, 15.75), r, -21.333333333333332), r, 13.125), r, 0.0), r, -3.5), r, 0.0), r, 1.125), r, 0.0), r, -0.25);
   } else {
+    const double ir2 = 1.0 / (r * r);
     Fl += 0.5 * ir2;
     F2l += -0.026515151515151516 * ir2;
   }
@@ -1917,7 +1920,7 @@ template <> __device__ __forceinline__ void disk_profile<2>(double r, double ir2
 template <> __device__ __forceinline__ int disk_knots<2>(double* out) {
   return 0;
 }
-template <> __device__ __forceinline__ void disk_profile<3>(double r, double ir2, double& P, double& Fl, double& F2l) {   // w6
+template <> __device__ __forceinline__ void disk_profile<3>(double r, double& P, double& Fl, double& F2l) {   // w6
   P = 0.0;
   Fl = 0.0;
   F2l = 0.25;
@@ -1926,6 +1929,7 @@ template <> __device__ __forceinline__ void disk_profile<3>(double r, double ir2
     Fl += fma(fma(fma(fma(fma(fma(fma(fma(fma(fma(fma(27.428571428571427, r, -214.5), r, 713.1428571428571), r, -1287.0), r, 1307.4285714285713), r, -643.5), r, 0.0), r, 122.57142857142857), r, 0.0), r, -30.642857142857142), r, 0.0), r, 5.571428571428571);
     F2l += fma(fma(fma(fma(fma(fma(fma(fma(fma(fma(fma(fma(fma(1.8285714285714285, r, -15.321428571428571), r, 54.857142857142854), r, -107.25), r, 118.85714285714286), r, -64.35), r, 0.0), r, 15.321428571428571), r, 0.0), r, -5.107142857142857), r, 0.0), r, 1.3928571428571428), r, 0.0), r, -0.25);
   } else {
+    const double ir2 = 1.0 / (r * r);
     Fl += 0.5 * ir2;
     F2l += -0.02142857142857143 * ir2;
   }
@@ -1933,7 +1937,7 @@ template <> __device__ __forceinline__ void disk_profile<3>(double r, double ir2
 template <> __device__ __forceinline__ int disk_knots<3>(double* out) {
   return 0;
 }
-template <> __device__ __forceinline__ void disk_profile<4>(double r, double ir2, double& P, double& Fl, double& F2l) {   // quartic
+template <> __device__ __forceinline__ void disk_profile<4>(double r, double& P, double& Fl, double& F2l) {   // quartic
   P = 0.0;
   Fl = 0.0;
   F2l = 0.25;
@@ -1942,6 +1946,7 @@ template <> __device__ __forceinline__ void disk_profile<4>(double r, double ir2
     Fl += fma(fma(fma(fma(3.2579232693911595, r, -15.638031693077565), r, 29.321309424520432), r, -26.063386155129276), r, 9.773769808173478);
     F2l += fma(fma(fma(fma(fma(fma(0.40724040867389494, r, -2.2340045275825093), r, 4.886884904086739), r, -5.212677231025855), r, 2.4434424520433695), r, 0.0), r, -0.3257923269391159);
   } else {
+    const double ir2 = 1.0 / (r * r);
     Fl += 0.6515846538782318 * ir2;
     F2l += -0.03490632074347671 * ir2;
   }
@@ -1950,6 +1955,7 @@ template <> __device__ __forceinline__ void disk_profile<4>(double r, double ir2
     Fl += fma(fma(fma(fma(-16.289616346955796, r, 46.914095079232695), r, -52.77835696413678), r, 28.148457047539615), r, -6.333402835696414);
     F2l += fma(fma(fma(fma(fma(fma(-2.0362020433694745, r, 6.702013582747528), r, -8.79639282735613), r, 5.629691409507923), r, -1.5833507089241035), r, 0.0), r, 0.07600083402835696);
   } else {
+    const double ir2 = 1.0 / (r * r);
     Fl += -0.15200166805671392 * ir2;
     F2l += 0.0029314607410937687 * ir2;
   }
@@ -1958,6 +1964,7 @@ template <> __device__ __forceinline__ void disk_profile<4>(double r, double ir2
     Fl += fma(fma(fma(fma(32.57923269391159, r, -31.27606338615513), r, 11.728523769808174), r, -2.085070892410342), r, 0.15638031693077564);
     F2l += fma(fma(fma(fma(fma(fma(4.072404086738949, r, -4.468009055165019), r, 1.9547539616346956), r, -0.4170141784820684), r, 0.03909507923269391), r, 0.0), r, -0.0002085070892410342);
   } else {
+    const double ir2 = 1.0 / (r * r);
     Fl += 0.0004170141784820684 * ir2;
     F2l += -8.936018110330037e-07 * ir2;
   }
@@ -1967,7 +1974,7 @@ template <> __device__ __forceinline__ int disk_knots<4>(double* out) {
   out[1] = 0.6;
   return 2;
 }
-template <> __device__ __forceinline__ void disk_profile<5>(double r, double ir2, double& P, double& Fl, double& F2l) {   // quintic
+template <> __device__ __forceinline__ void disk_profile<5>(double r, double& P, double& Fl, double& F2l) {   // quintic
   P = 0.0;
   Fl = 0.0;
   F2l = 0.25;
@@ -1976,6 +1983,7 @@ template <> __device__ __forceinline__ void disk_profile<5>(double r, double ir2
     Fl += fma(fma(fma(fma(fma(-4.575313807531381, r, 26.689330543933053), r, -64.05439330543933), r, 80.06799163179916), r, -53.37866108786611), r, 16.013598326359833);
     F2l += fma(fma(fma(fma(fma(fma(fma(-0.5083682008368201, r, 3.3361663179916317), r, -9.150627615062762), r, 13.344665271966527), r, -10.675732217573222), r, 4.003399581589958), r, 0.0), r, -0.38127615062761505);
   } else {
+    const double ir2 = 1.0 / (r * r);
     Fl += 0.7625523012552301 * ir2;
     F2l += -0.03177301255230126 * ir2;
   }
@@ -1984,6 +1992,7 @@ template <> __device__ __forceinline__ void disk_profile<5>(double r, double ir2
     Fl += fma(fma(fma(fma(fma(27.451882845188283, r, -106.75732217573221), r, 170.81171548117155), r, -142.34309623430963), r, 63.26359832635983), r, -12.652719665271967);
     F2l += fma(fma(fma(fma(fma(fma(fma(3.0502092050209204, r, -13.344665271966527), r, 24.401673640167363), r, -23.723849372384937), r, 12.652719665271967), r, -3.1631799163179917), r, 0.0), r, 0.13389121338912133);
   } else {
+    const double ir2 = 1.0 / (r * r);
     Fl += -0.26778242677824265 * ir2;
     F2l += 0.004958933829226716 * ir2;
   }
@@ -1992,6 +2001,7 @@ template <> __device__ __forceinline__ void disk_profile<5>(double r, double ir2
     Fl += fma(fma(fma(fma(fma(-68.6297071129707, r, 133.44665271966528), r, -106.75732217573221), r, 44.48221757322176), r, -9.884937238493723), r, 0.9884937238493724);
     F2l += fma(fma(fma(fma(fma(fma(fma(-7.625523012552302, r, 16.68083158995816), r, -15.251046025104603), r, 7.4137029288702925), r, -1.9769874476987448), r, 0.2471234309623431), r, 0.0), r, -0.002615062761506276);
   } else {
+    const double ir2 = 1.0 / (r * r);
     Fl += 0.005230125523012552 * ir2;
     F2l += -2.4213544088021077e-05 * ir2;
   }
@@ -2001,7 +2011,7 @@ template <> __device__ __forceinline__ int disk_knots<5>(double* out) {
   out[1] = 0.6666666666666666;
   return 2;
 }
-template <> __device__ __forceinline__ void disk_profile<6>(double r, double ir2, double& P, double& Fl, double& F2l) {   // poly6
+template <> __device__ __forceinline__ void disk_profile<6>(double r, double& P, double& Fl, double& F2l) {   // poly6
   P = 0.0;
   Fl = 0.0;
   F2l = 0.25;
@@ -2010,6 +2020,7 @@ template <> __device__ __forceinline__ void disk_profile<6>(double r, double ir2
     Fl += fma(fma(fma(fma(fma(fma(-0.5, r, 0.0), r, 2.0), r, 0.0), r, -3.0), r, 0.0), r, 2.0);
     F2l += fma(fma(fma(fma(fma(fma(fma(fma(-0.05, r, 0.0), r, 0.25), r, 0.0), r, -0.5), r, 0.0), r, 0.5), r, 0.0), r, -0.25);
   } else {
+    const double ir2 = 1.0 / (r * r);
     Fl += 0.5 * ir2;
     F2l += -0.05 * ir2;
   }
@@ -2017,7 +2028,7 @@ template <> __device__ __forceinline__ void disk_profile<6>(double r, double ir2
 template <> __device__ __forceinline__ int disk_knots<6>(double* out) {
   return 0;
 }
-template <> __device__ __forceinline__ void disk_profile<7>(double r, double ir2, double& P, double& Fl, double& F2l) {   // cone
+template <> __device__ __forceinline__ void disk_profile<7>(double r, double& P, double& Fl, double& F2l) {   // cone
   P = 0.0;
   Fl = 0.0;
   F2l = 0.25;
@@ -2026,6 +2037,7 @@ template <> __device__ __forceinline__ void disk_profile<7>(double r, double ir2
     Fl += fma(-1.0, r, 1.5);
     F2l += fma(fma(fma(-0.2, r, 0.375), r, 0.0), r, -0.25);
   } else {
+    const double ir2 = 1.0 / (r * r);
     Fl += 0.5 * ir2;
     F2l += -0.075 * ir2;
   }
@@ -2033,7 +2045,7 @@ template <> __device__ __forceinline__ void disk_profile<7>(double r, double ir2
 template <> __device__ __forceinline__ int disk_knots<7>(double* out) {
   return 0;
 }
-template <> __device__ __forceinline__ void disk_profile<8>(double r, double ir2, double& P, double& Fl, double& F2l) {   // lw2
+template <> __device__ __forceinline__ void disk_profile<8>(double r, double& P, double& Fl, double& F2l) {   // lw2
   P = 0.0;
   Fl = 0.0;
   F2l = 0.25;
@@ -2042,6 +2054,7 @@ template <> __device__ __forceinline__ void disk_profile<8>(double r, double ir2
     Fl += fma(fma(fma(-2.0, r, 7.5), r, -10.0), r, 5.0);
     F2l += fma(fma(fma(fma(fma(-0.2857142857142857, r, 1.25), r, -2.0), r, 1.25), r, 0.0), r, -0.25);
   } else {
+    const double ir2 = 1.0 / (r * r);
     Fl += 0.5 * ir2;
     F2l += -0.03571428571428571 * ir2;
   }
@@ -2049,7 +2062,7 @@ template <> __device__ __forceinline__ void disk_profile<8>(double r, double ir2
 template <> __device__ __forceinline__ int disk_knots<8>(double* out) {
   return 0;
 }
-template <> __device__ __forceinline__ void disk_profile<9>(double r, double ir2, double& P, double& Fl, double& F2l) {   // lw4
+template <> __device__ __forceinline__ void disk_profile<9>(double r, double& P, double& Fl, double& F2l) {   // lw4
   P = 0.0;
   Fl = 0.0;
   F2l = 0.25;
@@ -2058,6 +2071,7 @@ template <> __device__ __forceinline__ void disk_profile<9>(double r, double ir2
     Fl += fma(fma(fma(fma(fma(fma(-5.833333333333333, r, 32.0), r, -70.0), r, 74.66666666666667), r, -35.0), r, 0.0), r, 4.666666666666667);
     F2l += fma(fma(fma(fma(fma(fma(fma(fma(-0.5833333333333334, r, 3.5555555555555554), r, -8.75), r, 10.666666666666666), r, -5.833333333333333), r, 0.0), r, 1.1666666666666667), r, 0.0), r, -0.25);
   } else {
+    const double ir2 = 1.0 / (r * r);
     Fl += 0.5 * ir2;
     F2l += -0.027777777777777776 * ir2;
   }

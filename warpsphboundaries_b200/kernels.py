@@ -537,13 +537,12 @@ def emit_disk() -> list:
     truncated blocks (a block past its radius R continues as M(R)/r^2 and MPsi(R)/r^2), and disk_knots<KID> the
     block radii below 1 (where the profiles have kinks)."""
     out = ["// ---- disk element: pi*W, M/r^2 and the second potential of every exact kernel, summed over its blocks",
-           "template <int KID> __device__ __forceinline__ void disk_profile(double r, double ir2, double& P, double& Fl,",
-           "                                                             double& F2l);",
+           "template <int KID> __device__ __forceinline__ void disk_profile(double r, double& P, double& Fl, double& F2l);",
            "template <int KID> __device__ __forceinline__ int disk_knots(double* out);"]
     for kid in range(len(KERNEL_IDS)):
         k = kernel(KERNEL_NAMES[kid])
         half = sum((b.Mhat for b in k.blocks), F(0)) / 2
-        body = [f"template <> __device__ __forceinline__ void disk_profile<{kid}>(double r, double ir2, double& P, "
+        body = [f"template <> __device__ __forceinline__ void disk_profile<{kid}>(double r, double& P, "
                 f"double& Fl, double& F2l) {{   // {k.name}",
                 f"  P = 0.0;", f"  Fl = 0.0;", f"  F2l = {_lit(half)};"]
         for b in k.blocks:
@@ -552,6 +551,7 @@ def emit_disk() -> list:
             body.append(f"    Fl += {_horner(b.flam, 'r')};")
             body.append(f"    F2l += {_horner(b.fpsi, 'r')};")
             body.append("  } else {")
+            body.append("    const double ir2 = 1.0 / (r * r);")
             body.append(f"    Fl += {_lit(b.Mhat)} * ir2;")
             body.append(f"    F2l += {_lit(b.MPhat)} * ir2;")
             body.append("  }")
