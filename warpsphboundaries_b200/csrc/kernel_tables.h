@@ -2196,13 +2196,43 @@ __host__ __device__ __forceinline__ T ipow(T x) {
 }
 __host__ __device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
 __host__ __device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
-constexpr int kRadialGauss = 12;
-static __device__ const double kRadialGx[kRadialGauss] = {-0.9815606342467192, -0.9041172563704748, -0.7699026741943047, -0.5873179542866175, -0.3678314989981802, -0.1252334085114689, 0.1252334085114689, 0.3678314989981802, 0.5873179542866175, 0.7699026741943047, 0.9041172563704748, 0.9815606342467192};
-static __device__ const double kRadialGw[kRadialGauss] = {0.04717533638651141, 0.10693932599531907, 0.16007832854334642, 0.20316742672306573, 0.2334925365383546, 0.2491470458134027, 0.2491470458134027, 0.2334925365383546, 0.20316742672306573, 0.16007832854334642, 0.10693932599531907, 0.04717533638651141};
+// the Gauss-Legendre rules of the family
+template <int N> __device__ __forceinline__ double radial_gx(int g);
+template <int N> __device__ __forceinline__ double radial_gw(int g);
+static __device__ const double kRadialGx4[4] = {-0.8611363115940526, -0.33998104358485626, 0.33998104358485626, 0.8611363115940526};
+template <> __device__ __forceinline__ double radial_gx<4>(int g) { return kRadialGx4[g]; }
+static __device__ const double kRadialGw4[4] = {0.34785484513745357, 0.6521451548625464, 0.6521451548625464, 0.34785484513745357};
+template <> __device__ __forceinline__ double radial_gw<4>(int g) { return kRadialGw4[g]; }
+static __device__ const double kRadialGx5[5] = {-0.906179845938664, -0.5384693101056831, 0.0, 0.5384693101056831, 0.906179845938664};
+template <> __device__ __forceinline__ double radial_gx<5>(int g) { return kRadialGx5[g]; }
+static __device__ const double kRadialGw5[5] = {0.23692688505618928, 0.4786286704993663, 0.5688888888888887, 0.4786286704993663, 0.23692688505618928};
+template <> __device__ __forceinline__ double radial_gw<5>(int g) { return kRadialGw5[g]; }
+static __device__ const double kRadialGx6[6] = {-0.9324695142031519, -0.6612093864662645, -0.2386191860831969, 0.2386191860831969, 0.6612093864662645, 0.9324695142031519};
+template <> __device__ __forceinline__ double radial_gx<6>(int g) { return kRadialGx6[g]; }
+static __device__ const double kRadialGw6[6] = {0.17132449237917027, 0.3607615730481387, 0.46791393457269104, 0.46791393457269104, 0.3607615730481387, 0.17132449237917027};
+template <> __device__ __forceinline__ double radial_gw<6>(int g) { return kRadialGw6[g]; }
+static __device__ const double kRadialGx7[7] = {-0.9491079123427586, -0.7415311855993945, -0.4058451513773972, 0.0, 0.4058451513773972, 0.7415311855993945, 0.9491079123427586};
+template <> __device__ __forceinline__ double radial_gx<7>(int g) { return kRadialGx7[g]; }
+static __device__ const double kRadialGw7[7] = {0.12948496616886973, 0.27970539148927687, 0.3818300505051187, 0.4179591836734693, 0.3818300505051187, 0.27970539148927687, 0.12948496616886973};
+template <> __device__ __forceinline__ double radial_gw<7>(int g) { return kRadialGw7[g]; }
+static __device__ const double kRadialGx8[8] = {-0.9602898564975362, -0.7966664774136267, -0.525532409916329, -0.18343464249564978, 0.18343464249564978, 0.525532409916329, 0.7966664774136267, 0.9602898564975362};
+template <> __device__ __forceinline__ double radial_gx<8>(int g) { return kRadialGx8[g]; }
+static __device__ const double kRadialGw8[8] = {0.10122853629037706, 0.22238103445337443, 0.3137066458778869, 0.36268378337836166, 0.36268378337836166, 0.3137066458778869, 0.22238103445337443, 0.10122853629037706};
+template <> __device__ __forceinline__ double radial_gw<8>(int g) { return kRadialGw8[g]; }
+static __device__ const double kRadialGx10[10] = {-0.9739065285171717, -0.8650633666889845, -0.6794095682990244, -0.4333953941292472, -0.14887433898163122, 0.14887433898163122, 0.4333953941292472, 0.6794095682990244, 0.8650633666889845, 0.9739065285171717};
+template <> __device__ __forceinline__ double radial_gx<10>(int g) { return kRadialGx10[g]; }
+static __device__ const double kRadialGw10[10] = {0.06667134430868814, 0.1494513491505804, 0.219086362515982, 0.2692667193099965, 0.2955242247147528, 0.2955242247147528, 0.2692667193099965, 0.219086362515982, 0.1494513491505804, 0.06667134430868814};
+template <> __device__ __forceinline__ double radial_gw<10>(int g) { return kRadialGw10[g]; }
+static __device__ const double kRadialGx12[12] = {-0.9815606342467192, -0.9041172563704748, -0.7699026741943047, -0.5873179542866175, -0.3678314989981802, -0.1252334085114689, 0.1252334085114689, 0.3678314989981802, 0.5873179542866175, 0.7699026741943047, 0.9041172563704748, 0.9815606342467192};
+template <> __device__ __forceinline__ double radial_gx<12>(int g) { return kRadialGx12[g]; }
+static __device__ const double kRadialGw12[12] = {0.04717533638651141, 0.10693932599531907, 0.16007832854334642, 0.20316742672306573, 0.2334925365383546, 0.2491470458134027, 0.2491470458134027, 0.2334925365383546, 0.20316742672306573, 0.16007832854334642, 0.10693932599531907, 0.04717533638651141};
+template <> __device__ __forceinline__ double radial_gw<12>(int g) { return kRadialGw12[g]; }
 struct Rad_cubic {   // c3*pi = 16
   static constexpr int kPieces = 2;
   static constexpr double kLo[kPieces] = {0.0, 0.5};
   static constexpr double kHi[kPieces] = {0.5, 1.0};
+  static constexpr int kCap[kPieces] = {6, 12};
+  static constexpr int kBall[kPieces] = {4, 12};
   template <typename T> __host__ __device__ static __forceinline__ void full(T* v) {
     v[0] = T(1.0); v[1] = T(0.0); v[2] = T(0.075); v[3] = T(0.075); v[4] = T(0.0); v[5] = T(1.0); v[6] = T(1.0); v[7] = T(0.0); v[8] = T(0.0);
   }
@@ -2236,6 +2266,8 @@ struct Rad_w2 {   // c3*pi = 21/2
   static constexpr int kPieces = 1;
   static constexpr double kLo[kPieces] = {0.0};
   static constexpr double kHi[kPieces] = {1.0};
+  static constexpr int kCap[kPieces] = {7};
+  static constexpr int kBall[kPieces] = {5};
   template <typename T> __host__ __device__ static __forceinline__ void full(T* v) {
     v[0] = T(1.0); v[1] = T(0.0); v[2] = T(0.06666666666666667); v[3] = T(0.06666666666666667); v[4] = T(0.0); v[5] = T(1.0); v[6] = T(1.0); v[7] = T(0.0); v[8] = T(0.0);
   }
@@ -2257,6 +2289,8 @@ struct Rad_w4 {   // c3*pi = 495/32
   static constexpr int kPieces = 1;
   static constexpr double kLo[kPieces] = {0.0};
   static constexpr double kHi[kPieces] = {1.0};
+  static constexpr int kCap[kPieces] = {8};
+  static constexpr int kBall[kPieces] = {7};
   template <typename T> __host__ __device__ static __forceinline__ void full(T* v) {
     v[0] = T(1.0); v[1] = T(0.0); v[2] = T(0.05128205128205128); v[3] = T(0.05128205128205128); v[4] = T(0.0); v[5] = T(1.0); v[6] = T(1.0); v[7] = T(0.0); v[8] = T(0.0);
   }
@@ -2278,6 +2312,8 @@ struct Rad_w6 {   // c3*pi = 1365/64
   static constexpr int kPieces = 1;
   static constexpr double kLo[kPieces] = {0.0};
   static constexpr double kHi[kPieces] = {1.0};
+  static constexpr int kCap[kPieces] = {10};
+  static constexpr int kBall[kPieces] = {8};
   template <typename T> __host__ __device__ static __forceinline__ void full(T* v) {
     v[0] = T(1.0); v[1] = T(0.0); v[2] = T(0.041666666666666664); v[3] = T(0.041666666666666664); v[4] = T(0.0); v[5] = T(1.0); v[6] = T(1.0); v[7] = T(0.0); v[8] = T(0.0);
   }

@@ -9,12 +9,14 @@
 // radius R whose surface is at signed distance d), and integrating the monomials over the cap gives
 //   a0 = 2 pi (1 + cap), a1 = pi (cap^2 - 1), at = pi (cap - cap^3/3 + 2/3), an = 2 pi (cap^3 + 1) / 3.
 // The reference integrates products of linear factors in Bernstein form; here each radial sub-interval (per kernel
-// piece: the full-ball region [0, min(1, -d)] and the cap region [|d|, min(1, 2R + d)]) is integrated by 12-node
-// Gauss-Legendre, which is exact for the polynomial integrands (degree <= 18) and leaves < 1e-17 relative on cubic's
-// outer Laurent piece (r >= 1/2).  Cancellation is avoided by factoring the angular terms:
-//   u = 1 + cap = (r - d)(2R + d - r) / (2 D r),  v = 1 - cap = (r + d)(r + d + 2R) / (2 D r)   (sphere)
-//   u = (r - d) / r,                              v = (r + d) / r                               (half-space)
-//   a0 = 2u, a1 = -u v, at = u^2 (1 + v) / 3, an = 2/3 u (cap^2 - cap + 1)          (times pi; pi cancels against W)
+// piece: the full-ball region [0, min(1, -d)] and the cap region [|d|, min(1, 2R + d)]) is integrated by the
+// Gauss-Legendre rule that is exact for its polynomial integrands (w2 7 nodes in the cap region, w4 8, w6 10; 12 nodes
+// leave < 1e-17 relative on cubic's outer Laurent piece, r >= 1/2).  Cancellation is avoided by factoring the angular
+// terms, with the factor r kept inside so that no node divides:
+//   ru = r (1 + cap) = (r - d)(2R + d - r) / (2 D),  rv = r (1 - cap) = (r + d)(r + d + 2R) / (2 D)   (sphere)
+//   ru = r - d,                                      rv = r + d                                       (half-space)
+//   r a0 = 2 ru, r^2 a1 = -ru rv, r^3 at = ru^2 (r + rv) / 3, r^3 an = 2/3 ru (rc^2 - r rc + r^2), rc = r cap
+//   (times pi; pi cancels against W)
 // and the kernel profiles W, W'/r and (W'/r)' are evaluated as r^p (hi - r)^k g(r) with exact factors.
 #include "common.cuh"
 
@@ -34,23 +36,24 @@ struct Inv9 {
 
 // one piece's contribution: the full-ball region [lo, hi] (cap = 1) and the cap region [clo, chi]
 template <class KR, int P, typename T>
-__device__ __forceinline__ void radial_piece(T d, T R, T D, bool sphere, T full_end, T cap_end, Inv9<T>& acc) {
+__device__ __forceinline__ void radial_piece(T d, T R, T inv2D, bool sphere, T full_end, T cap_end, Inv9<T>& acc) {
   const T plo = T(KR::kLo[P]), phi = T(KR::kHi[P]);
   {
+    constexpr int N = KR::kBall[P];
     const T lo = plo, hi = fmin(phi, full_end);
     if (hi > lo) {
       const T c = T(0.5) * (hi + lo), hw = T(0.5) * (hi - lo);
       T s0 = 0, s2 = 0, s5 = 0, s7 = 0;
 #pragma unroll
-      for (int g = 0; g < kRadialGauss; ++g) {
-        const T r = fma_t(hw, T(kRadialGx[g]), c), wg = T(kRadialGw[g]);
+      for (int g = 0; g < N; ++g) {
+        const T r = fma_t(hw, T(radial_gx<N>(g)), c), wg = T(radial_gw<N>(g));
         T w, l, dl;
         KR::template eval<P, T>(r, w, l, dl);
-        const T r2 = r * r, r3 = r2 * r, r4 = r2 * r2;
-        s0 = fma_t(wg, r2 * w, s0);
-        s2 = fma_t(wg, r4 * w, s2);
-        s5 = fma_t(wg, r4 * l, s5);
-        s7 = fma_t(wg, fma_t(T(4), r2 * l, T(4.0 / 3.0) * r3 * dl), s7);
+        const T r2 = wg * r * r, r3 = r2 * r, r4 = r3 * r;
+        s0 = fma_t(r2, w, s0);
+        s2 = fma_t(r4, w, s2);
+        s5 = fma_t(r4, l, s5);
+        s7 = fma_t(T(4) * r2, l, fma_t(T(4.0 / 3.0) * r3, dl, s7));
       }
       acc.v[0] += hw * T(4) * s0;
       acc.v[2] += hw * T(4.0 / 3.0) * s2;
@@ -62,50 +65,44 @@ __device__ __forceinline__ void radial_piece(T d, T R, T D, bool sphere, T full_
     }
   }
   {
+    constexpr int N = KR::kCap[P];
     const T lo = fmax(plo, fabs(d)), hi = fmin(phi, cap_end);
     if (hi > lo) {
       const T c = T(0.5) * (hi + lo), hw = T(0.5) * (hi - lo);
-      T s[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-      const T inv2D = sphere ? T(1) / (T(2) * D) : T(0);
+      T s[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
-      for (int g = 0; g < kRadialGauss; ++g) {
-        const T r = fma_t(hw, T(kRadialGx[g]), c), wg = T(kRadialGw[g]);
+      for (int g = 0; g < N; ++g) {
+        const T r = fma_t(hw, T(radial_gx<N>(g)), c), wg = T(radial_gw<N>(g));
         T w, l, dl;
         KR::template eval<P, T>(r, w, l, dl);
-        const T ir = T(1) / r;
-        T u, v;
+        T ru = r - d, rv = r + d;
         if (sphere) {
-          u = (r - d) * ((R - r) + (R + d)) * inv2D * ir;
-          v = (r + d) * ((r + d) + T(2) * R) * inv2D * ir;
-        } else {
-          u = (r - d) * ir;
-          v = (r + d) * ir;
+          ru *= ((R - r) + (R + d)) * inv2D;
+          rv *= (rv + T(2) * R) * inv2D;
         }
-        const T cap = T(0.5) * (u - v);
-        const T a0 = T(2) * u, a1 = -u * v, at = u * u * (T(1) + v) * T(1.0 / 3.0),
-                an = T(2.0 / 3.0) * u * fma_t(cap, cap - T(1), T(1));
-        const T r2 = r * r, r3 = r2 * r, r4 = r2 * r2;
-        const T ww = wg * w, wl = wg * l;
-        s[0] = fma_t(ww, r2 * a0, s[0]);
-        s[1] = fma_t(ww, r3 * a1, s[1]);
-        s[2] = fma_t(ww, r4 * at, s[2]);
-        s[3] = fma_t(ww, r4 * an, s[3]);
-        s[4] = fma_t(wl, r3 * a1, s[4]);
-        s[5] = fma_t(wl, r4 * at, s[5]);
-        s[6] = fma_t(wl, r4 * an, s[6]);
-        const T base = wl * r2 * a0, wdl = wg * dl * r3;
-        s[7] += fma_t(wdl, at, base);
-        s[8] += fma_t(wdl, an, base);
+        const T rc = T(0.5) * (ru - rv), a1 = ru * rv, at = ru * ru * (r + rv), an = ru * fma_t(rc, rc - r, r * r);
+        const T wr = wg * r, ww = wr * w, wl = wr * l, wd = wg * dl;
+        s[0] = fma_t(ww, ru, s[0]);
+        s[1] = fma_t(ww, a1, s[1]);
+        s[2] = fma_t(ww, at, s[2]);
+        s[3] = fma_t(ww, an, s[3]);
+        s[4] = fma_t(wl, a1, s[4]);
+        s[5] = fma_t(wl, at, s[5]);
+        s[6] = fma_t(wl, an, s[6]);
+        s[7] = fma_t(wl, ru, s[7]);
+        s[8] = fma_t(wd, at, s[8]);
+        s[9] = fma_t(wd, an, s[9]);
       }
-      acc.v[0] += hw * s[0];
-      acc.v[1] += hw * s[1];
-      acc.v[2] += hw * s[2];
-      acc.v[3] += hw * s[3];
-      acc.v[4] -= hw * s[4];
-      acc.v[5] -= hw * s[5];
-      acc.v[6] -= hw * s[6];
-      acc.v[7] += hw * s[7];
-      acc.v[8] += hw * s[8];
+      const T h3 = hw * T(1.0 / 3.0);
+      acc.v[0] += T(2) * hw * s[0];
+      acc.v[1] -= hw * s[1];
+      acc.v[2] += h3 * s[2];
+      acc.v[3] += T(2) * h3 * s[3];
+      acc.v[4] += hw * s[4];
+      acc.v[5] -= h3 * s[5];
+      acc.v[6] -= T(2) * h3 * s[6];
+      acc.v[7] += fma_t(T(2) * hw, s[7], h3 * s[8]);
+      acc.v[8] += fma_t(T(2) * hw, s[7], T(2) * h3 * s[9]);
     }
   }
 }
@@ -124,8 +121,9 @@ __device__ __forceinline__ void radial_invariants(T d, T R, bool sphere, Inv9<T>
   }
   if (d >= T(1)) return;                       // the support does not reach the solid
   const T full_end = fmin(T(1), fmax(T(0), -d));
-  radial_piece<KR, 0, T>(d, R, R + d, sphere, full_end, cap_end, acc);
-  if constexpr (KR::kPieces > 1) radial_piece<KR, 1, T>(d, R, R + d, sphere, full_end, cap_end, acc);
+  const T inv2D = sphere ? T(1) / (T(2) * (R + d)) : T(0);
+  radial_piece<KR, 0, T>(d, R, inv2D, sphere, full_end, cap_end, acc);
+  if constexpr (KR::kPieces > 1) radial_piece<KR, 1, T>(d, R, inv2D, sphere, full_end, cap_end, acc);
   static_assert(KR::kPieces <= 2, "radial kernels have at most two pieces");
 }
 
@@ -133,9 +131,36 @@ constexpr int kRadialThreads = 128;
 
 __device__ __forceinline__ double pick3(int i, double x, double y, double z) { return i == 0 ? x : (i == 1 ? y : z); }
 
-// one thread per row; the block's rows are contiguous, so their outputs [row0 .. row0 + 128) x n_requests are one
-// contiguous range: each thread writes its row into shared memory, then the block stores the range coalesced
-template <class KR, typename T>
+// the 28 baseline requests of a row in their order, from its invariants and normal
+__device__ __forceinline__ void baseline_row(const double inv[9], const double n[3], double* o) {
+  o[0] = inv[0];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    o[1 + i] = inv[1] * n[i];
+    o[10 + i] = inv[4] * n[i];
+  }
+  const double dm = inv[3] - inv[2], dg = inv[6] - inv[5], dh = inv[8] - inv[7];
+  int k = 0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = i; j < 3; ++j, ++k) {
+      o[4 + k] = dm * n[i] * n[j] + (i == j ? inv[2] : 0.0);
+      o[22 + k] = dh * n[i] * n[j] + (i == j ? inv[7] : 0.0);
+    }
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) o[13 + 3 * i + j] = dg * n[i] * n[j] + (i == j ? inv[5] : 0.0);
+}
+
+// One thread per row; the block's rows are contiguous, so their outputs [row0 .. row0 + 128) x n_requests (and their
+// invariants, x 9) are one contiguous range each: every thread puts its row into shared memory (odd strides against bank
+// conflicts), then the block stores the range coalesced.  FULL: the 28 baseline requests in their order -- written
+// straight from the invariants; other sets look up each request's row of the table (half of the instructions of a full
+// row before).  2^21 sphere rows (w4) on B200: 0.136 ms (5.0 TB/s of DRAM traffic) with 8 + 7 nodes a row and no division in a node; 0.47 ms with 12 + 12
+// nodes, a division each, and the table for every set.
+template <class KR, typename T, bool FULL>
 __global__ void __launch_bounds__(kRadialThreads, 6) k_radial(const double* __restrict__ dist,
                                                               const double* __restrict__ radii,
                                                               const double* __restrict__ normals,
@@ -143,18 +168,19 @@ __global__ void __launch_bounds__(kRadialThreads, 6) k_radial(const double* __re
                                                               int sphere, RadialRequests req,
                                                               double* __restrict__ out, double* __restrict__ inv_out,
                                                               int32_t* __restrict__ status) {
-  __shared__ double stage[kRadialThreads * 28];
+  __shared__ double stage[kRadialThreads * 29];
   const int64_t row0 = (int64_t)blockIdx.x * kRadialThreads;
   const int64_t row = row0 + threadIdx.x;
-  const int nreq = req.n;
+  const int nreq = FULL ? 28 : req.n, stride = nreq | 1;
+  const int rows_here = (int)(n - row0 < kRadialThreads ? n - row0 : kRadialThreads);
+  double inv[9];
   if (row < n) {
     const double h = supports[row], dd = dist[row];
     const double Rr = sphere ? radii[row] : 0.0;
-    const double nx = normals[3 * row], ny = normals[3 * row + 1], nz = normals[3 * row + 2];
-    const bool ok = h > 0.0 && isfinite(h) && isfinite(dd) && isfinite(nx) && isfinite(ny) && isfinite(nz) &&
+    const double nrm[3] = {normals[3 * row], normals[3 * row + 1], normals[3 * row + 2]};
+    const bool ok = h > 0.0 && isfinite(h) && isfinite(dd) && isfinite(nrm[0]) && isfinite(nrm[1]) && isfinite(nrm[2]) &&
                     (!sphere || (Rr > 0.0 && isfinite(Rr) && dd >= -Rr));
     Inv9<T> acc;
-    double inv[9];
     if (ok) {
       radial_invariants<KR, T>(T(dd / h), T(Rr / h), sphere != 0, acc);
       const double ih = 1.0 / h;
@@ -166,35 +192,68 @@ __global__ void __launch_bounds__(kRadialThreads, 6) k_radial(const double* __re
       for (int j = 0; j < 9; ++j) inv[j] = __longlong_as_double(0x7ff8000000000000LL);
     }
     if (status) status[row] = ok ? 0 : 1;
-    if (inv_out) {
+    double* const mine = stage + threadIdx.x * stride;
+    if constexpr (FULL) {
+      double o[28];
+      baseline_row(inv, nrm, o);
 #pragma unroll
-      for (int j = 0; j < 9; ++j) inv_out[row * 9 + j] = inv[j];
-    }
+      for (int c = 0; c < 28; ++c) mine[c] = o[c];
+    } else {
 #pragma unroll 4
-    for (int c = 0; c < nreq; ++c) {
-      const int degree = req.meta[c][0], i = req.meta[c][1], j = req.meta[c][2], order = req.meta[c][3];
-      const double ni = pick3(i, nx, ny, nz), nj = pick3(j, nx, ny, nz);
-      double v;
-      if (degree == 0 && order == 0) {
-        v = inv[0];
-      } else if (degree == 1 && order == 0) {
-        v = inv[1] * ni;
-      } else if (degree == 0 && order == 1) {
-        v = inv[4] * ni;
-      } else {
-        // tangent / axial pair of the second-order entry: m2 (2, 3), g1 (5, 6), Hessian (7, 8)
-        const double tan = order == 0 ? inv[2] : (order == 1 ? inv[5] : inv[7]);
-        const double axi = order == 0 ? inv[3] : (order == 1 ? inv[6] : inv[8]);
-        v = (axi - tan) * ni * nj + (i == j ? tan : 0.0);
+      for (int c = 0; c < nreq; ++c) {
+        const int degree = req.meta[c][0], i = req.meta[c][1], j = req.meta[c][2], order = req.meta[c][3];
+        const double ni = pick3(i, nrm[0], nrm[1], nrm[2]), nj = pick3(j, nrm[0], nrm[1], nrm[2]);
+        double v;
+        if (degree == 0 && order == 0) {
+          v = inv[0];
+        } else if (degree == 1 && order == 0) {
+          v = inv[1] * ni;
+        } else if (degree == 0 && order == 1) {
+          v = inv[4] * ni;
+        } else {
+          // tangent / axial pair of the second-order entry: m2 (2, 3), g1 (5, 6), Hessian (7, 8)
+          const double tan = order == 0 ? inv[2] : (order == 1 ? inv[5] : inv[7]);
+          const double axi = order == 0 ? inv[3] : (order == 1 ? inv[6] : inv[8]);
+          v = (axi - tan) * ni * nj + (i == j ? tan : 0.0);
+        }
+        mine[c] = v;
       }
-      stage[threadIdx.x * nreq + c] = v;
     }
   }
   __syncthreads();
-  const int64_t rows_here = n - row0 < kRadialThreads ? n - row0 : kRadialThreads;
-  const int count = (int)rows_here * nreq;
-  double* dst = out + row0 * nreq;
-  for (int k = threadIdx.x; k < count; k += kRadialThreads) dst[k] = stage[k];
+  for (int k = threadIdx.x; k < rows_here * nreq; k += kRadialThreads)
+    out[row0 * nreq + k] = stage[k / nreq * stride + k % nreq];
+  if (inv_out) {
+    __syncthreads();
+    if (row < n) {
+#pragma unroll
+      for (int j = 0; j < 9; ++j) stage[threadIdx.x * 9 + j] = inv[j];
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < rows_here * 9; k += kRadialThreads) inv_out[row0 * 9 + k] = stage[k];
+  }
+}
+
+// whether the requests are the 28 baseline requests in their order: value moments of degree 0, 1, 2, first-derivative
+// moments of degree 0 and 1 per axis, the Hessian's upper triangle
+bool is_baseline(const RadialRequests& req) {
+  if (req.n != 28) return false;
+  int c = 0;
+  bool same = true;
+  auto row = [&](int degree, int i, int j, int order) {
+    const signed char* m = req.meta[c++];
+    same = same && m[0] == degree && m[1] == i && m[2] == j && m[3] == order;
+  };
+  row(0, 0, 0, 0);
+  for (int i = 0; i < 3; ++i) row(1, i, 0, 0);
+  for (int i = 0; i < 3; ++i)
+    for (int j = i; j < 3; ++j) row(2, i, j, 0);
+  for (int j = 0; j < 3; ++j) row(0, j, 0, 1);
+  for (int i = 0; i < 3; ++i)
+    for (int j = 0; j < 3; ++j) row(1, i, j, 1);
+  for (int i = 0; i < 3; ++i)
+    for (int j = i; j < 3; ++j) row(0, i, j, 2);
+  return same;
 }
 
 template <typename T>
@@ -203,11 +262,18 @@ int launch_radial(int kernel, const double* d, const double* r, const double* nr
                   cudaStream_t st) {
   const unsigned grid = (unsigned)((n + kRadialThreads - 1) / kRadialThreads);
   constexpr int B = kRadialThreads;
+  auto launch = [&](auto kr) {
+    using KR = decltype(kr);
+    if (is_baseline(req))
+      k_radial<KR, T, true><<<grid, B, 0, st>>>(d, r, nrm, h, n, sphere, req, out, inv, status);
+    else
+      k_radial<KR, T, false><<<grid, B, 0, st>>>(d, r, nrm, h, n, sphere, req, out, inv, status);
+  };
   switch (kernel) {
-    case WSB_KERNEL_CUBIC: k_radial<Rad_cubic, T><<<grid, B, 0, st>>>(d, r, nrm, h, n, sphere, req, out, inv, status); break;
-    case WSB_KERNEL_W2: k_radial<Rad_w2, T><<<grid, B, 0, st>>>(d, r, nrm, h, n, sphere, req, out, inv, status); break;
-    case WSB_KERNEL_W4: k_radial<Rad_w4, T><<<grid, B, 0, st>>>(d, r, nrm, h, n, sphere, req, out, inv, status); break;
-    case WSB_KERNEL_W6: k_radial<Rad_w6, T><<<grid, B, 0, st>>>(d, r, nrm, h, n, sphere, req, out, inv, status); break;
+    case WSB_KERNEL_CUBIC: launch(Rad_cubic{}); break;
+    case WSB_KERNEL_W2: launch(Rad_w2{}); break;
+    case WSB_KERNEL_W4: launch(Rad_w4{}); break;
+    case WSB_KERNEL_W6: launch(Rad_w6{}); break;
     default: return fail(WSB_ERR_UNSUPPORTED, "wsb_radial_channels: the radial family serves cubic, w2, w4, w6");
   }
   WSB_CUDA(cudaGetLastError());

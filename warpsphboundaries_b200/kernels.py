@@ -683,10 +683,23 @@ def plane_channels(name):
 # ------------------------------------------------------------------ 3-D radial profiles (solid half-space / sphere)
 RADIAL_KERNELS = ("cubic", "w2", "w4", "w6")
 _PUBLISHED_C3PI = {"cubic": F(16), "w2": F(21, 2), "w4": F(495, 32), "w6": F(1365, 64)}
-# Gauss-Legendre order of every radial sub-interval: exact for polynomial integrands up to degree 2 * 12 - 1 = 23
-# (the highest is r^4 W a_t of w6, degree 18); cubic's outer Laurent piece lives on r >= 1/2, where 12 nodes leave a
-# relative error below 1e-17.
+# Gauss-Legendre order of a radial sub-interval holding a Laurent profile (cubic's outer piece, r >= 1/2): 12 nodes leave
+# a relative error below 1e-17.  Polynomial integrands take the order that is exact for their degree (radial_orders).
 RADIAL_GAUSS = 12
+
+
+def radial_orders(name):
+    """per piece (cap, ball): Gauss-Legendre nodes that integrate the shell integrands exactly -- with W of degree m the cap
+    integrands reach degree m + 7 (r (r u)^2 (r + r v) W with r u, r v quadratic in r), the whole-shell ones m + 4; a
+    piece whose W'/r has negative powers takes RADIAL_GAUSS nodes."""
+    out = []
+    for lo, hi, W, L, dL in radial(name)[0]:
+        deg = lambda f: f.p + f.k + len(f.g) - 1
+        if min(W.p, L.p, dL.p) < 0:
+            out.append((RADIAL_GAUSS, RADIAL_GAUSS))
+        else:
+            out.append(((deg(W) + 8 + 1) // 2, (deg(W) + 5 + 1) // 2))
+    return out
 
 
 @dataclass(frozen=True)
@@ -891,7 +904,6 @@ def emit_triangle() -> list:
 def emit_radial() -> list:
     """generated device code of the radial family: per kernel the pieces and W, W'/r, (W'/r)' in factored form."""
     import numpy as np
-    xg, wg = np.polynomial.legendre.leggauss(RADIAL_GAUSS)
     out = ["// ---- 3-D radial family (solid half-space / sphere), unit support; W = c3*pi * shape, L = W'/r, dL = L'",
            "template <int K, typename T>",
            "__host__ __device__ __forceinline__ T ipow(T x) {",
@@ -902,15 +914,23 @@ def emit_radial() -> list:
            "}",
            "__host__ __device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }",
            "__host__ __device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }",
-           f"constexpr int kRadialGauss = {RADIAL_GAUSS};",
-           "static __device__ const double kRadialGx[kRadialGauss] = {" + ", ".join(repr(float(x)) for x in xg) + "};",
-           "static __device__ const double kRadialGw[kRadialGauss] = {" + ", ".join(repr(float(x)) for x in wg) + "};"]
+           "// the Gauss-Legendre rules of the family"]
+    orders = sorted({n for name in RADIAL_KERNELS for pair in radial_orders(name) for n in pair})
+    out.append("template <int N> __device__ __forceinline__ double radial_gx(int g);")
+    out.append("template <int N> __device__ __forceinline__ double radial_gw(int g);")
+    for n in orders:
+        xg, wg = np.polynomial.legendre.leggauss(n)
+        for c, v in (("x", xg), ("w", wg)):
+            out.append(f"static __device__ const double kRadialG{c}{n}[{n}] = {{" + ", ".join(repr(float(a)) for a in v) + "};")
+            out.append(f"template <> __device__ __forceinline__ double radial_g{c}<{n}>(int g) {{ return kRadialG{c}{n}[g]; }}")
     for name in RADIAL_KERNELS:
         pcs, c3pi = radial(name)
         out.append(f"struct Rad_{name} {{   // c3*pi = {c3pi}")
         out.append(f"  static constexpr int kPieces = {len(pcs)};")
         out.append("  static constexpr double kLo[kPieces] = {" + ", ".join(_lit(p[0]) for p in pcs) + "};")
         out.append("  static constexpr double kHi[kPieces] = {" + ", ".join(_lit(p[1]) for p in pcs) + "};")
+        out.append("  static constexpr int kCap[kPieces] = {" + ", ".join(str(o[0]) for o in radial_orders(name)) + "};")
+        out.append("  static constexpr int kBall[kPieces] = {" + ", ".join(str(o[1]) for o in radial_orders(name)) + "};")
         # whole-support constants (the region of the support inside the solid is the full ball)
         full = _radial_full(name)
         out.append("  template <typename T> __host__ __device__ static __forceinline__ void full(T* v) {")
