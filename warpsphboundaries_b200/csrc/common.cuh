@@ -29,6 +29,9 @@ int cuda_fail(cudaError_t e, const char* where);
     if (e__ != cudaSuccess) return cuda_fail(e__, #call); \
   } while (0)
 
+// a cell that lists this many edges or more is long: the rows of such cells are split over several lanes
+constexpr int kLongList = 32;
+
 // ----------------------------------------------------------------------------------------------- surface
 struct Surface {
   int device = 0;
@@ -54,8 +57,9 @@ struct Surface {
   double* cind = nullptr;       // [nx*ny] winding + background at the cell centre
   int32_t* cok = nullptr;       // [nx*ny] 1 where the centre's winding is certain (clear of every edge line it tests)
   int32_t* cempty = nullptr;    // [nx*ny]
-  int32_t* ccompact = nullptr;  // [nx*ny] index of a cell among the cells with edges (cell order), -1 for an empty one
+  int32_t* ccompact = nullptr;  // [nx*ny] index of a cell among the cells with edges (longest list first), -1 for an empty one
   int32_t n_nonempty = 0;       // cells with edges
+  int32_t n_long = 0;           // of those, cells of kLongList edges or more
   int32_t* bstart = nullptr;    // [nb+1]
   int32_t* bitems = nullptr;    // [n_bitems]
   double4* erec = nullptr;      // [n_edges] (ax, ay, bx, by) by edge id
@@ -136,7 +140,7 @@ struct SurfView {        // the device pointers and scalars a kernel needs (pass
   const int32_t* bitems;
   const double4* brec;
   const double4* erec;
-  int32_t nx, ny, nb, K, nne;
+  int32_t nx, ny, nb, K, nne, nlc;
   double lo_x, lo_y, cell, y0, dy;
   double background;
 };

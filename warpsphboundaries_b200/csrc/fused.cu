@@ -19,6 +19,10 @@ constexpr int kKeys = 65;          // count keys: 0..63 rows with pairs (63 - mi
 
 static inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
+// a work row of this many pairs or more is split over eight lanes in the pair pass, a shorter one over two; a quadrature
+// kernel's pair costs several closed forms
+constexpr int kLongPairs = 32, kLongQuad = 16;
+
 constexpr int kMaxPackStaged = 4;   // kernels of the largest pack: channel sums a staged work row holds
 
 // the neighbour mask of a row covers the first kMaskBits candidates of its cell; later candidates (cells holding more
@@ -51,7 +55,7 @@ struct Workspace {
   int32_t* khist;    // [kKeys] rows per key   } zeroed together
   int32_t* kcur;     // [kKeys] fill cursors   }
   WorkRec* wrec;     // [n] work rows by decreasing pair count (slots < nwork used)
-  int32_t* nwork;    // [1] number of rows with pairs
+  int32_t* nwork;    // [3] number of rows with pairs, of those with kLongPairs or more, kLongQuad or more (first in wrec)
   size_t total;
   // optional staging region after `total` (a workspace of total + staging bytes): the channel sums of every work row,
   // [slot][kernel][12], written by the pair pass and expanded to the outputs by k_agg_expand; nullptr without it
@@ -81,7 +85,7 @@ static Workspace carve(const Surface* s, int64_t n, void* base) {
   w.khist = (int32_t*)take(sizeof(int32_t) * 2 * kKeys);
   w.kcur = w.khist + kKeys;
   w.wrec = (WorkRec*)take(sizeof(WorkRec) * std::max<int64_t>(n, 1));
-  w.nwork = (int32_t*)take(sizeof(int32_t));
+  w.nwork = (int32_t*)take(3 * sizeof(int32_t));
   w.total = off;
   w.staging = align256(sizeof(double) * 12 * kMaxPackStaged * std::max<int64_t>(n, 1));
   w.wacc = nullptr;
@@ -202,72 +206,62 @@ __device__ __forceinline__ double4 ldg4(const double4* p) {
   return make_double4(a.x, a.y, b.x, b.y);
 }
 
-constexpr int kStageRecs = 768;   // candidate records a row-info block stages in shared memory (24 KiB)
-
 // Per sorted row: its number of neighbour pairs (float-prefiltered exact predicate over its cell's candidates) as a
 // radix key with the neighbour mask, and its winding indicator -- both kernel independent, computed once per position
-// set.
+// set.  The buckets run from the longest candidate list to the shortest, so the rows of a warp have lists of one length;
+// the rows of long lists (kLongList candidates or more, a bucket range of the surface) come first and are split over
+// eight lanes: cells of small polygons list ten times the mean, and launches of a few hundred thousand rows waited for
+// their rows' serial walk.  The others take short_lanes each: one where the rows fill the GPU, more in launches that leave
+// it idle (info_lanes; the results are integers and do not depend on it).  (B200: 300 001 rows, cells of up to 161 candidates, 22 us against
+// 103 with a lane per row in cell order; 2^20 rows 58 against 66; four lanes for every row 41 and 80.)
+constexpr int kListLanes = 8;
+constexpr int kInfoWarps = kThreads / 32;
 
-__global__ void __launch_bounds__(kThreads) k_agg_rowinfo(SurfView S, const double* __restrict__ sup,
-                                                         const int32_t* __restrict__ key,
-                                                         const double* __restrict__ lpos,
-                                                         const int32_t* __restrict__ offs,
-                                                         const int32_t* __restrict__ order, int64_t n,
-                                                         double* __restrict__ ind, int32_t* __restrict__ flag,
-                                                         int32_t* __restrict__ rkey, uint64_t* __restrict__ mask,
-                                                         int32_t* __restrict__ khist) {
+__global__ void __launch_bounds__(kThreads, 6) k_agg_rowinfo(SurfView S, const double* __restrict__ sup,
+                                                            const int32_t* __restrict__ key,
+                                                            const double* __restrict__ lpos,
+                                                            const int32_t* __restrict__ offs,
+                                                            const int32_t* __restrict__ order, int64_t n,
+                                                            double* __restrict__ ind, int32_t* __restrict__ flag,
+                                                            int32_t* __restrict__ rkey, uint64_t* __restrict__ mask,
+                                                            int32_t* __restrict__ khist, int short_lanes) {
   pdl_wait();      // the preceding kernel of the stream has completed and its writes are visible
   pdl_trigger();   // the next kernel of the stream may be scheduled into the SMs this grid frees
-  // The block's rows are consecutive in cell order, so the candidates of all their cells are one contiguous range of
-  // the cell-list records: it is staged in shared memory with coalesced loads when it fits, and every row's pass
-  // over its cell's candidates reads it there.
-  __shared__ double4 s_rec[kStageRecs];
-  __shared__ int32_t s_lo, s_hi;
   __shared__ int32_t s_hist[kKeys - 1];
-  const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (threadIdx.x == 0) {
-    s_lo = INT32_MAX;
-    s_hi = -1;
-  }
   for (int k = threadIdx.x; k < kKeys - 1; k += kThreads) s_hist[k] = 0;
-  // sorted rows: the rows in cells with candidates (k_agg_prep settles all others)
-  int32_t i = 0, b = 0;
-  const bool cand = j < (int64_t)offs[S.nne];
-  if (cand) {
-    i = order[j];
-    b = key[i];
-  }
   __syncthreads();
-  if (cand) {
-    atomicMin(&s_lo, b);
-    atomicMax(&s_hi, b);
-  }
-  __syncthreads();
-  int r0 = 0;
-  bool staged = false;
-  if (s_hi >= 0) {
-    r0 = S.cstart[s_lo];
-    const int r1 = S.cstart[s_hi + 1];
-    staged = r1 - r0 <= kStageRecs;
-    if (staged)
-      for (int k = threadIdx.x; k < r1 - r0; k += kThreads) s_rec[k] = ldg4(S.crec + r0 + k);
-  }
-  __syncthreads();
-  int cnt = 0;
-  if (j < n) {
+  // sorted rows: the rows in cells with candidates (k_agg_prep settles all others), those of long lists first
+  const int64_t nrows = offs[S.nne], nlong = offs[S.nlc];
+  constexpr int kLongRows = 32 / kListLanes;
+  const int short_rows = 32 / short_lanes;
+  const int64_t tlong = (nlong + kLongRows - 1) / kLongRows, tasks = tlong + (nrows - nlong + short_rows - 1) / short_rows;
+  const int lane = threadIdx.x & 31;
+  for (int64_t task = (int64_t)blockIdx.x * kInfoWarps + threadIdx.x / 32; task < tasks;
+       task += (int64_t)gridDim.x * kInfoWarps) {
+    const bool lng = task < tlong;
+    const int G = lng ? kListLanes : short_lanes, sub = lane % G;
+    const int64_t j = lng ? task * kLongRows + lane / kListLanes : nlong + (task - tlong) * short_rows + lane / G;
+    const bool cand = j < (lng ? nlong : nrows);
+    int32_t i = 0, b = 0;
+    double lx = 0.0, ly = 0.0, h = 1.0;
+    int cnt = 0, cross = 0;
+    bool degenerate = false;
+    uint64_t m0 = 0, m1 = 0;                        // the neighbour mask, bit k: candidate k of the cell
     if (cand) {
-      const double lx = lpos[2 * i], ly = lpos[2 * i + 1], h = sup[i];
+      i = order[j];
+      b = key[i];
+      lx = lpos[2 * i];
+      ly = lpos[2 * i + 1];
+      h = sup[i];
       // one pass over the cell's candidates: the neighbour count and the signed crossings of the segment from the
       // cell centre (whose exact winding is stored) to the row; an uncertain orientation falls back to the ray cast
-      const int64_t cx = b / S.ny, cy = b % S.ny;
+      const int32_t cx = b / S.ny, cy = b % S.ny;
       const double rx = __dadd_rn(S.lo_x, __dmul_rn(__dadd_rn((double)cx, 0.5), S.cell));
       const double ry = __dadd_rn(S.lo_y, __dmul_rn(__dadd_rn((double)cy, 0.5), S.cell));
-      bool degenerate = S.cok[b] == 0;
-      int cross = 0;
-      uint64_t m0 = 0, m1 = 0;
+      degenerate = S.cok[b] == 0;
       const int k0 = S.cstart[b], k1 = S.cstart[b + 1];
-      for (int k = k0; k < k1; ++k) {
-        const double4 e = staged ? s_rec[k - r0] : ldg4(S.crec + k);
+      for (int k = k0 + sub; k < k1; k += G) {
+        const double4 e = ldg4(S.crec + k);
         if (seg_within_fast(lx, ly, e.x, e.y, e.z, e.w, h)) {
           ++cnt;
           const int r = k - k0;
@@ -278,19 +272,36 @@ __global__ void __launch_bounds__(kThreads) k_agg_rowinfo(SurfView S, const doub
         }
         if (!degenerate) cross += segment_crossing(rx, ry, lx, ly, e, &degenerate);
       }
-      reinterpret_cast<ulonglong2*>(mask)[j] = make_ulonglong2(m0, m1);
-      const double w = degenerate ? indicator_at(S, lx, ly, h, true, b) : S.cind[b] + (double)cross;
-      ind[i] = w;
-      flag[i] = cnt > 0 ? 2 : 1;
     }
-    rkey[j] = cnt > 0 ? 63 - min(cnt, 63) : kKeys - 1;
+    if (G > 1) {                                    // the group's counts and mask
+      int bad = degenerate ? 1 : 0;
+      for (int o = 1; o < G; o <<= 1) {
+        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+        cross += __shfl_xor_sync(0xffffffffu, cross, o);
+        bad |= __shfl_xor_sync(0xffffffffu, bad, o);
+        m0 |= __shfl_xor_sync(0xffffffffu, m0, o);
+        m1 |= __shfl_xor_sync(0xffffffffu, m1, o);
+      }
+      degenerate = bad != 0;
+    }
+    const bool mine = cand && sub == 0;
+    if (mine) {
+      reinterpret_cast<ulonglong2*>(mask)[j] = make_ulonglong2(m0, m1);
+      ind[i] = degenerate ? indicator_at(S, lx, ly, h, true, b) : S.cind[b] + (double)cross;
+      flag[i] = cnt > 0 ? 2 : 1;
+      rkey[j] = cnt > 0 ? 63 - min(cnt, 63) : kKeys - 1;
+    }
+    // histogram of the keys of the rows with pairs (the rows without are never scattered, so their key is not
+    // counted): warp-aggregated into the block's counts
+    const int ckey = mine && cnt > 0 ? 63 - min(cnt, 63) : -1;
+    const unsigned peers = __match_any_sync(0xffffffffu, ckey);
+    if (ckey >= 0 && lane == __ffs(peers) - 1) atomicAdd(&s_hist[ckey], __popc(peers));
   }
-  // histogram of the keys of the rows with pairs (the rows without are never scattered, so their key is not
-  // counted): warp-aggregated into the block's counts, then one global add per key the block has -- a global atomic
-  // per warp and key would serialise on the few hot keys of millions of rows
-  const int ckey = j < n && cnt > 0 ? 63 - min(cnt, 63) : -1;
-  const unsigned peers = __match_any_sync(0xffffffffu, ckey);
-  if (ckey >= 0 && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&s_hist[ckey], __popc(peers));
+  // the positions past the sorted rows hold no row
+  for (int64_t j = nrows + blockIdx.x * (int64_t)kThreads + threadIdx.x; j < n; j += (int64_t)gridDim.x * kThreads)
+    rkey[j] = kKeys - 1;
+  // one global add per key the block has: a global atomic per warp and key would serialise on the few hot keys of
+  // millions of rows
   __syncthreads();
   for (int k = threadIdx.x; k < kKeys - 1; k += kThreads)
     if (s_hist[k]) atomicAdd(&khist[k], s_hist[k]);
@@ -381,18 +392,9 @@ __device__ __forceinline__ void pack_blocks_at(const PairGeo& g, double lo, doub
     using KT = typename Pack::template Kern<K>;
     if constexpr (B < KT::kBlocks) {
       if constexpr (KT::kR[B] == Pack::kRadii.r[D]) {
-        if constexpr (KT::kQuad) {
-          // a quadrature kernel contributes its gradient channels only: G = -n int W ds (no indicator term, W and
-          // W' vanish at the support edge)
-          const double W0 = quad_chord<KT>(lo, hi, g.z);
-          const SmemAcc a{acc_t + K * 12 * kThreads};
-          a[3] -= g.n0 * W0;
-          a[4] -= g.n1 * W0;
-        } else {
-          BlockSums S;
-          KT::template sums<B>(A, rlo, rhi, S);
-          add_block(g, S, dang, SmemAcc{acc_t + K * 12 * kThreads});
-        }
+        BlockSums S;
+        KT::template sums<B>(A, rlo, rhi, S);
+        add_block(g, S, dang, SmemAcc{acc_t + K * 12 * kThreads});
       }
       pack_blocks_at<Pack, D, K, B + 1>(g, lo, hi, A, rlo, rhi, dang, acc_t);
     } else {
@@ -426,8 +428,7 @@ __device__ __forceinline__ void pack_pair(const PairGeo& g, double* acc_t) {
 // 8-node Gauss-Legendre on panels graded from the foot of the perpendicular -- 0, |z|, 2|z|, 4|z|, ... up to the
 // chord end, the reference's stable route (src/warpSPHBoundaries/edge/warpbc.py:519-575) without its cap on the
 // panel count -- the node radius shared by every block of the pack; the odd chord sums come from the potentials M,
-// MPsi at the chord ends; the edge-frame combination and the row sums stay in float64.  The tensile (quadrature)
-// kernels keep their float64 chord quadrature.  Float slot of (kernel K, block B): K * kF32MaxBlocks + B.
+// MPsi at the chord ends; the edge-frame combination and the row sums stay in float64.  Float slot of (kernel K, block B): K * kF32MaxBlocks + B.
 constexpr int kF32MaxBlocks = 3;
 
 template <class Pack, int D, int K, int B>
@@ -435,7 +436,7 @@ __device__ __forceinline__ void f32_node(float x, float w, float* q) {
   if constexpr (K < Pack::kN) {
     using KT = typename Pack::template Kern<K>;
     if constexpr (B < KT::kBlocks) {
-      if constexpr (!KT::kQuad && KT::kR[B] == Pack::kRadii.r[D]) {
+      if constexpr (KT::kR[B] == Pack::kRadii.r[D]) {
         static_assert(B < kF32MaxBlocks, "blocks per kernel");
         constexpr int o = 4 * (K * kF32MaxBlocks + B);
         float P, Psi, Fl, Fp;
@@ -460,27 +461,21 @@ __device__ __forceinline__ void f32_finish(const PairGeo& g, const float* q, dou
     if constexpr (B < KT::kBlocks) {
       if constexpr (KT::kR[B] == Pack::kRadii.r[D]) {
         const SmemAcc a{acc_t + K * 12 * kThreads};
-        if constexpr (KT::kQuad) {
-          const double W0 = quad_chord<KT>(lo, hi, g.z);
-          a[3] -= g.n0 * W0;
-          a[4] -= g.n1 * W0;
-        } else {
-          constexpr int o = 4 * (K * kF32MaxBlocks + B);
-          constexpr float s2R = (float)(2.0 / KT::kR[B]);
-          float Mh, MPh, Ml, MPl;
-          ChebOf<KT>::template potentials<B>(fminf(fmaf((float)rhi, s2R, -1.0f), 1.0f), Mh, MPh);
-          ChebOf<KT>::template potentials<B>(fminf(fmaf((float)rlo, s2R, -1.0f), 1.0f), Ml, MPl);
-          BlockSums S;
-          S.W0 = (double)q[o];
-          S.P0 = (double)q[o + 1];
-          S.Lreg = (double)q[o + 2];
-          S.Preg = (double)q[o + 3];
-          S.W1 = (double)Mh - (double)Ml;
-          S.P1 = (double)MPh - (double)MPl;
-          S.Mhat = ChebOf<KT>::kMhat[B];
-          S.MPhat = ChebOf<KT>::kMPhat[B];
-          add_block(g, S, dang, a);
-        }
+        constexpr int o = 4 * (K * kF32MaxBlocks + B);
+        constexpr float s2R = (float)(2.0 / KT::kR[B]);
+        float Mh, MPh, Ml, MPl;
+        ChebOf<KT>::template potentials<B>(fminf(fmaf((float)rhi, s2R, -1.0f), 1.0f), Mh, MPh);
+        ChebOf<KT>::template potentials<B>(fminf(fmaf((float)rlo, s2R, -1.0f), 1.0f), Ml, MPl);
+        BlockSums S;
+        S.W0 = (double)q[o];
+        S.P0 = (double)q[o + 1];
+        S.Lreg = (double)q[o + 2];
+        S.Preg = (double)q[o + 3];
+        S.W1 = (double)Mh - (double)Ml;
+        S.P1 = (double)MPh - (double)MPl;
+        S.Mhat = ChebOf<KT>::kMhat[B];
+        S.MPhat = ChebOf<KT>::kMPhat[B];
+        add_block(g, S, dang, a);
       }
       f32_finish<Pack, D, K, B + 1>(g, q, lo, hi, rlo, rhi, dang, acc_t);
     } else {
@@ -536,6 +531,118 @@ __device__ __forceinline__ void pack_pair_f32(const PairGeo& g, double* acc_t) {
   }
 }
 
+// ------------------------------------------------------------------------------------------------ quadrature kernels
+// A quadrature kernel (W^5 of the tensile group) contributes its gradient channels only, G = -n int W ds, in every
+// precision by the float64 chord quadrature (quad_chord's panels).  A chord has 1 to some 30 panels, so a lane per chord
+// waits for the longest of the warp (108 nodes against 33 on average among 64 star polygons): here a warp cuts its 32
+// chords into items of 10 nodes (half of a panel next to the foot) or 12 (a panel further out), flattens them on the
+// lanes and adds every chord's items in order.  300 001 rows, w2p5, the pair pass: 142 us against 490.
+struct ChordPanels {
+  double lo, hi, base;      // the chord and its distance (at least 2^-24) from the foot
+  double a, b, end, d;      // the panel [a, b] of distances from the foot, the side's end, the next doubling
+  int side;
+  bool ok;                  // there is a panel
+  __device__ __forceinline__ bool open(int s) {
+    side = s;
+    a = s == 0 ? fmax(-hi, 0.0) : fmax(lo, 0.0);
+    end = s == 0 ? -lo : hi;
+    if (!(end > a)) return false;
+    d = 2.0 * base;
+    for (int it = 0; it < 64 && d <= a; ++it) d *= 2.0;
+    b = fmin(end, d);
+    return true;
+  }
+  __device__ __forceinline__ void first(double l, double h, double z) {
+    lo = l;
+    hi = h;
+    base = fmax(fabs(z), 0x1p-24);
+    ok = open(0) || open(1);
+  }
+  __device__ __forceinline__ void next() {
+    a = b;
+    if (b >= d) d *= 2.0;
+    if (a < end)
+      b = fmin(end, d);
+    else
+      ok = side == 0 && open(1);
+  }
+  __device__ __forceinline__ int items() const { return a < 2.0 * base ? 2 : 1; }
+};
+constexpr int kMaxChordPanels = 128;
+
+// int W ds over each lane's chord [lo, hi] at distance z of the edge line (none where !have), by the whole warp
+template <class KT>
+__device__ __forceinline__ double quad_chord_warp(bool have, double lo, double hi, double z) {
+  __shared__ double s_chord[kThreads / 32][32][3];
+  __shared__ double s_item[kThreads / 32][32];
+  static_assert(kQuadGaussChord == 20 && kQuadGaussFar == 12, "items of 10 and 12 nodes");
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  ChordPanels p;
+  int count = 0;
+  if (have) {
+    s_chord[wib][lane][0] = lo;
+    s_chord[wib][lane][1] = hi;
+    s_chord[wib][lane][2] = z;
+    p.first(lo, hi, z);
+    for (int it = 0; it < kMaxChordPanels && p.ok; ++it) {
+      count += p.items();
+      p.next();
+    }
+  }
+  int inc = count;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  const int total = __shfl_sync(0xffffffffu, inc, 31), pref = inc - count;
+  __syncwarp();
+  double sum = 0.0;
+  for (int base = 0; base < total; base += 32) {
+    const int item = base + lane;
+    int r = 0;                                              // the chord of the item: the last lane whose prefix is <= it
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+      if (__shfl_sync(0xffffffffu, pref, r + step) <= item) r += step;
+    int at = item - __shfl_sync(0xffffffffu, pref, r);
+    if (item < total) {
+      const double zc = s_chord[wib][r][2], zz = zc * zc;
+      p.first(s_chord[wib][r][0], s_chord[wib][r][1], zc);
+      while (at >= p.items()) {                             // (at is below the chord's count: the walk ends in its panels)
+        at -= p.items();
+        p.next();
+      }
+      const bool near = p.items() == 2;
+      const double hc = 0.5 * (p.b - p.a), mc = 0.5 * (p.b + p.a);
+      const double* gx = near ? kQuadCx + 10 * at : kQuadFx;
+      const double* gw = near ? kQuadCw + 10 * at : kQuadFw;
+      double ps = 0.0;
+      for (int k = 0; k < (near ? 10 : 12); ++k) {
+        const double x = fma(hc, gx[k], mc);
+        ps = fma(gw[k], KT::poly(fmin(sqrt(fma(x, x, zz)), 1.0)), ps);
+      }
+      s_item[wib][lane] = hc * ps;
+    }
+    __syncwarp();
+    for (int q = max(pref - base, 0); q < min(pref + count - base, 32); ++q) sum += s_item[wib][q];
+    __syncwarp();
+  }
+  return sum;
+}
+
+// the pairs of a warp (none where !have) of a pack that is one quadrature kernel; every lane takes part
+template <class KT>
+__device__ __forceinline__ void quad_pairs(bool have, const PairGeo& g, double* acc_t) {
+  double lo = 0.0, hi = 0.0, rlo, rhi, zz;
+  have = have && clip_chord(g, KT::kR[0], lo, hi, rlo, rhi, zz);
+  const double W0 = quad_chord_warp<KT>(have, lo, hi, g.z);
+  if (have) {
+    const SmemAcc a{acc_t};
+    a[3] -= g.n0 * W0;
+    a[4] -= g.n1 * W0;
+  }
+}
+
 // the outputs of a row of a quadrature kernel: its gradient channels G (scaled, rotated); the other outputs are not
 // defined for it and are written as NaN
 template <int VEC = 0>
@@ -584,15 +691,14 @@ __device__ __forceinline__ void pack_constant_row(int64_t i, double w, double h,
 
 // a work row, every kernel of the pack: the G lanes' sums combined by an xor butterfly (every lane of the warp takes
 // part), then the lane that writes adds the indicator terms and stores the outputs
-template <class Pack, int G, int K>
-__device__ __forceinline__ void pack_finish(const double* acc_t, bool write, int64_t i, double w, double h,
+template <class Pack, int K>
+__device__ __forceinline__ void pack_finish(const double* acc_t, int G, bool write, int64_t i, double w, double h,
                                             const double* pose, bool assign, const PackOut& o) {
   if constexpr (K < Pack::kN) {
     using KT = typename Pack::template Kern<K>;
     double acc[12];
 #pragma unroll
     for (int c = 0; c < 12; ++c) acc[c] = acc_t[(K * 12 + c) * kThreads];
-#pragma unroll
     for (int off = 1; off < G; off <<= 1) {
 #pragma unroll
       for (int c = 0; c < 12; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], off);
@@ -606,18 +712,17 @@ __device__ __forceinline__ void pack_finish(const double* acc_t, bool write, int
       else
         finish_row(acc, w, KT::kMass, KT::kPlane2, h, pose, i, assign, o.lam[K], o.G[K], o.cov[K], o.m1[K], o.m2[K]);
     }
-    pack_finish<Pack, G, K + 1>(acc_t, write, i, w, h, pose, assign, o);
+    pack_finish<Pack, K + 1>(acc_t, G, write, i, w, h, pose, assign, o);
   }
 }
 
 // a work row's channel sums (the G lanes' sums by the xor butterfly, x 1/pi) into its staging slot [kernel][12]
-template <class Pack, int G, int K>
-__device__ __forceinline__ void pack_stage(const double* acc_t, bool write, double* dst) {
+template <class Pack, int K>
+__device__ __forceinline__ void pack_stage(const double* acc_t, int G, bool write, double* dst) {
   if constexpr (K < Pack::kN) {
     double acc[12];
 #pragma unroll
     for (int c = 0; c < 12; ++c) acc[c] = acc_t[(K * 12 + c) * kThreads];
-#pragma unroll
     for (int off = 1; off < G; off <<= 1) {
 #pragma unroll
       for (int c = 0; c < 12; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], off);
@@ -627,39 +732,49 @@ __device__ __forceinline__ void pack_stage(const double* acc_t, bool write, doub
 #pragma unroll
       for (int c = 0; c < 6; ++c) d2[c] = make_double2(__dmul_rn(acc[2 * c], kInvPi), __dmul_rn(acc[2 * c + 1], kInvPi));
     }
-    pack_stage<Pack, G, K + 1>(acc_t, write, dst);
+    pack_stage<Pack, K + 1>(acc_t, G, write, dst);
   }
 }
 
-// Rows with neighbour pairs (compacted, by decreasing pair count), then the rows without: the first
-// ceil(nwork G / kThreads) blocks take the work rows, the next ceil(n / kThreads) blocks the constant rows (one row a
-// thread, coalesced), so the constant rows' stores overlap the last wave of pair blocks instead of running as a launch
-// of their own; the grid is sized for nwork = n and blocks past both ranges return.  A group of G adjacent lanes owns
-// one work row and splits its neighbours: the row's neighbour mask (set by k_agg_rowinfo) lists them among the first
-// kMaskBits candidates of its cell, and lane g takes those of rank g, g + G, ... in candidate order; candidates past
-// the mask are split g, g + G, ... and found by the float-prefiltered predicate.  Work rows are sorted by pair count,
-// so the lanes of a warp evaluate nearly the same number of closed forms.  The G partial sums are combined by an xor
-// butterfly (the same additions on every lane, commutative, so the result is deterministic and identical on the G
-// lanes).  The channel sums live in shared memory ([kernel][channel][thread]), which keeps the registers for the
-// closed form.
-template <class Pack, int PREC, int G, int MINB, bool STAGED>
+// Rows with neighbour pairs (compacted, by decreasing pair count), then the rows without: the first blocks take the work
+// rows, a warp's rows at a time, the next ceil(n / kThreads) blocks the constant rows (one row a thread, coalesced), so
+// the constant rows' stores overlap the last wave of pair blocks instead of running as a launch of their own; the grid is
+// sized for nwork = n in pairs of lanes and blocks past both ranges return.  A group of G adjacent lanes owns one work
+// row and splits its neighbours: the row's neighbour mask (set by k_agg_rowinfo) lists them among the first kMaskBits
+// candidates of its cell, and lane g takes those of rank g, g + G, ... in candidate order; candidates past the mask are
+// split g, g + G, ... and found by the float-prefiltered predicate.  G = 2, and 8 for the rows of kLongPairs pairs or
+// more (kLongQuad for a quadrature kernel), which come first: two lanes would evaluate some 46 pairs one after the other
+// on small polygons, and launches of a few hundred thousand rows waited for them.  (B200, 300 001 rows of the delta+ groups:
+// 100 -> 37 us; 2^20 rows, w4 109 -> 82 us, four kernels 204 -> 203.  From 16 pairs on: 36 / 87 / 219; from 48: 52 / 81 /
+// 200; w2p5 144 from 16 pairs on, 199 from 32, 247 from 48.)  G follows from the row alone.  Work rows are sorted by pair
+// count, so the lanes of a warp evaluate nearly the same number of closed forms.  The G partial sums are combined by an
+// xor butterfly (the same additions on every lane, commutative, so the result is deterministic and identical on the G
+// lanes).  The channel sums live in shared memory ([kernel][channel][thread]), which keeps the registers for the closed
+// form.
+constexpr int kShortLanes = 2, kLongLanes = 8;
+
+template <class Pack, int PREC, int MINB, bool STAGED>
 __global__ void __launch_bounds__(kThreads, MINB) k_agg_pairs(SurfView S, const double* __restrict__ sup,
                                                              const WorkRec* __restrict__ wrec,
                                                              const int32_t* __restrict__ nwork_p, int64_t n,
                                                              const double* __restrict__ ind,
                                                              const int32_t* __restrict__ flag,
                                                              const double* __restrict__ pose, bool assign,
-                                                             const PackOut out, double* __restrict__ wacc) {
+                                                             const PackOut out, double* __restrict__ wacc,
+                                                             int64_t pair_blocks) {
   pdl_wait();      // the preceding kernel of the stream has completed and its writes are visible
   pdl_trigger();   // the next kernel of the stream may be scheduled into the SMs this grid frees
-  static_assert(G == 1 || G == 2 || G == 4 || G == 8 || G == 16, "lanes per row");
   static_assert(Pack::kN >= 1 && Pack::kN <= kMaxPack, "pack size");
+  constexpr bool kQuadPack = Pack::kN == 1 && Pack::template Kern<0>::kQuad;
   // dynamic shared memory: the channel sums [kernel][channel][thread], then each thread's next edge record
   extern __shared__ double4 s_dyn[];
   double* const s_acc = reinterpret_cast<double*>(s_dyn + kThreads);
   double4* const s_next = s_dyn;
-  const int64_t nwork = *nwork_p;
-  const int64_t wblocks = (nwork + kThreads / G - 1) / (kThreads / G);
+  // a warp's task: 32 / G rows; the long rows' tasks first
+  constexpr int kWarps = kThreads / 32, kLongRows = 32 / kLongLanes, kShortRows = 32 / kShortLanes;
+  const int64_t nwork = nwork_p[0], nlong = nwork_p[kQuadPack ? 2 : 1], tlong = (nlong + kLongRows - 1) / kLongRows;
+  const int64_t tasks = tlong + (nwork - nlong + kShortRows - 1) / kShortRows;
+  const int64_t wblocks = min((tasks + kWarps - 1) / kWarps, pair_blocks);
   if ((int64_t)blockIdx.x >= wblocks) {                             // a tail block: constant rows
     if constexpr (STAGED) return;                                   // (staged: k_agg_expand writes every row)
     const int64_t i = ((int64_t)blockIdx.x - wblocks) * kThreads + threadIdx.x;
@@ -669,82 +784,91 @@ __global__ void __launch_bounds__(kThreads, MINB) k_agg_pairs(SurfView S, const 
     }
     return;
   }
-  const int64_t w = (int64_t)blockIdx.x * (blockDim.x / G) + threadIdx.x / G;
-  const int sub = threadIdx.x % G;
-  const bool ok = w < nwork;
-  int32_t i = 0;
-  int kb = 0, kt = 0, e1 = 0;
-  uint64_t mk0 = 0, mk1 = 0;
-  double lx = 0.0, ly = 0.0, h = 1.0;
-  if (ok) {
-    const WorkRec r = load_workrec(wrec + w);
-    i = r.row;
-    lx = r.lx;
-    ly = r.ly;
-    h = r.h;
-    kb = r.kb;
-    e1 = r.ke;
-    kt = kb + kMaskBits + sub;                                      // past the mask: lane sub scans kt, kt + G, ...
-    mk0 = r.m0;
-    mk1 = r.m1;
-  }
-  // lane sub takes the neighbours of rank sub, sub + G, ... of the mask (in candidate order), then its share of the
-  // candidates past the mask by the predicate
-  for (int s = 0; s < sub; ++s) pop_bit(mk0, mk1);
-  int nb = pop_bit(mk0, mk1);
-  const double ih = 1.0 / h;
-  double* const acc_t = s_acc + threadIdx.x;
+  // (more tasks than warps only where more than a quarter of all rows are long)
+  for (int64_t task = (int64_t)blockIdx.x * kWarps + threadIdx.x / 32; task < tasks; task += wblocks * kWarps) {
+    const bool lng = task < tlong;
+    const int G = lng ? kLongLanes : kShortLanes, lane = threadIdx.x & 31;
+    const int64_t w = lng ? task * kLongRows + lane / kLongLanes : nlong + (task - tlong) * kShortRows + lane / kShortLanes;
+    const int sub = lane % G;
+    const bool ok = w < (lng ? nlong : nwork);
+    int32_t i = 0;
+    int kb = 0, kt = 0, e1 = 0;
+    uint64_t mk0 = 0, mk1 = 0;
+    double lx = 0.0, ly = 0.0, h = 1.0;
+    if (ok) {
+      const WorkRec r = load_workrec(wrec + w);
+      i = r.row;
+      lx = r.lx;
+      ly = r.ly;
+      h = r.h;
+      kb = r.kb;
+      e1 = r.ke;
+      kt = kb + kMaskBits + sub;                                    // past the mask: lane sub scans kt, kt + G, ...
+      mk0 = r.m0;
+      mk1 = r.m1;
+    }
+    // lane sub takes the neighbours of rank sub, sub + G, ... of the mask (in candidate order), then its share of the
+    // candidates past the mask by the predicate
+    for (int s = 0; s < sub; ++s) pop_bit(mk0, mk1);
+    int nb = pop_bit(mk0, mk1);
+    const double ih = 1.0 / h;
+    double* const acc_t = s_acc + threadIdx.x;
 #pragma unroll
-  for (int c = 0; c < Pack::kN * 12; ++c) acc_t[c * kThreads] = 0.0;
-  // the next neighbour's (or tail candidate's) record is copied into the thread's shared-memory slot one step ahead
-  // (cp.async), so its latency hides behind the current pair's closed form
-  const double4 zero = make_double4(0.0, 0.0, 0.0, 0.0);
-  double4* const slot = s_next + threadIdx.x;
-  if (nb >= 0)
-    cp_async_rec(slot, S.crec + kb + nb);
-  else if (kt < e1)
-    cp_async_rec(slot, S.crec + kt);
-  while (__any_sync(0xffffffffu, nb >= 0 || kt < e1)) {
-    double4 e = zero;
-    bool have = false;
-    if (nb >= 0) {
-      cp_async_wait_all();
-      e = *slot;
-      have = true;
-      for (int s = 1; s < G; ++s) pop_bit(mk0, mk1);
-      nb = pop_bit(mk0, mk1);
-      if (nb >= 0)
-        cp_async_rec(slot, S.crec + kb + nb);
-      else if (kt < e1)
-        cp_async_rec(slot, S.crec + kt);
-    } else {
-      while (kt < e1) {
+    for (int c = 0; c < Pack::kN * 12; ++c) acc_t[c * kThreads] = 0.0;
+    // the next neighbour's (or tail candidate's) record is copied into the thread's shared-memory slot one step ahead
+    // (cp.async), so its latency hides behind the current pair's closed form
+    const double4 zero = make_double4(0.0, 0.0, 0.0, 0.0);
+    double4* const slot = s_next + threadIdx.x;
+    if (nb >= 0)
+      cp_async_rec(slot, S.crec + kb + nb);
+    else if (kt < e1)
+      cp_async_rec(slot, S.crec + kt);
+    while (__any_sync(0xffffffffu, nb >= 0 || kt < e1)) {
+      double4 e = zero;
+      bool have = false;
+      if (nb >= 0) {
         cp_async_wait_all();
         e = *slot;
-        kt += G;
-        if (kt < e1) cp_async_rec(slot, S.crec + kt);
-        if (seg_within_fast(lx, ly, e.x, e.y, e.z, e.w, h)) {
-          have = true;
-          break;
+        have = true;
+        for (int s = 1; s < G; ++s) pop_bit(mk0, mk1);
+        nb = pop_bit(mk0, mk1);
+        if (nb >= 0)
+          cp_async_rec(slot, S.crec + kb + nb);
+        else if (kt < e1)
+          cp_async_rec(slot, S.crec + kt);
+      } else {
+        while (kt < e1) {
+          cp_async_wait_all();
+          e = *slot;
+          kt += G;
+          if (kt < e1) cp_async_rec(slot, S.crec + kt);
+          if (seg_within_fast(lx, ly, e.x, e.y, e.z, e.w, h)) {
+            have = true;
+            break;
+          }
+        }
+      }
+      __syncwarp();
+      if constexpr (kQuadPack) {
+        PairGeo g{};
+        have = have && pair_geo_row(lx, ly, h, ih, e, g);
+        quad_pairs<typename Pack::template Kern<0>>(have, g, acc_t);
+      } else if (have) {
+        PairGeo g;
+        if (pair_geo_row(lx, ly, h, ih, e, g)) {
+          if constexpr (PREC == WSB_PREC_FP32)
+            pack_pair_f32<Pack, 0>(g, acc_t);
+          else
+            pack_pair<Pack, PREC, 0>(g, acc_t);
         }
       }
     }
-    __syncwarp();
-    if (have) {
-      PairGeo g;
-      if (pair_geo_row(lx, ly, h, ih, e, g)) {
-        if constexpr (PREC == WSB_PREC_FP32)
-          pack_pair_f32<Pack, 0>(g, acc_t);
-        else
-          pack_pair<Pack, PREC, 0>(g, acc_t);
-      }
-    }
+    const bool write = ok && sub == 0;
+    if constexpr (STAGED)
+      pack_stage<Pack, 0>(acc_t, G, write, wacc + w * (Pack::kN * 12));
+    else
+      pack_finish<Pack, 0>(acc_t, G, write, i, write ? ind[i] : 0.0, h, pose, assign, out);
   }
-  const bool write = ok && sub == 0;
-  if constexpr (STAGED)
-    pack_stage<Pack, G, 0>(acc_t, write, wacc + w * (Pack::kN * 12));
-  else
-    pack_finish<Pack, G, 0>(acc_t, write, i, write ? ind[i] : 0.0, h, pose, assign, out);
 }
 
 // Staged expansion: one thread per row, consecutive rows in consecutive threads, so every output array is written in
@@ -832,11 +956,10 @@ constexpr size_t pack_smem_bytes() {
 template <class Pack, int PREC>
 static int launch_pack(const SurfView& v, const double* sup, const Workspace& w, int64_t n, const double* pose,
                        bool assign, const PackOut& out, cudaStream_t st) {
-  constexpr int G = 2;
   constexpr size_t smem = pack_smem_bytes<Pack>();
   const bool staged = w.wacc != nullptr;
-  auto kern = staged ? k_agg_pairs<Pack, PREC, G, pack_min_blocks(Pack::kN), true>
-                     : k_agg_pairs<Pack, PREC, G, pack_min_blocks(Pack::kN), false>;
+  auto kern = staged ? k_agg_pairs<Pack, PREC, pack_min_blocks(Pack::kN), true>
+                     : k_agg_pairs<Pack, PREC, pack_min_blocks(Pack::kN), false>;
   if (smem > 48 * 1024) {       // above the default limit: opt in once per device for this instantiation
     static std::atomic<uint64_t> opted[2] = {{0}, {0}};
     int dev = 0;
@@ -848,10 +971,12 @@ static int launch_pack(const SurfView& v, const double* sup, const Workspace& w,
     }
   }
   const unsigned rows = (unsigned)((n + kThreads - 1) / kThreads);
-  const unsigned grid = (unsigned)((n * G + kThreads - 1) / kThreads) + (staged ? 0u : rows);
+  const unsigned pair_blocks = (unsigned)((n * kShortLanes + kThreads - 1) / kThreads);
+  const unsigned grid = pair_blocks + (staged ? 0u : rows);
   if (g_pair_ev[0]) WSB_CUDA(cudaEventRecord(g_pair_ev[0], st));
   WSB_CUDA(launch_dep(kern, grid, kThreads, smem, st, v, sup, (const WorkRec*)w.wrec, (const int32_t*)w.nwork, n,
-                      (const double*)w.ind, (const int32_t*)w.flag, pose, assign, out, w.wacc));
+                      (const double*)w.ind, (const int32_t*)w.flag, pose, assign, out, w.wacc,
+                      (int64_t)pair_blocks));
   if (g_pair_ev[1]) WSB_CUDA(cudaEventRecord(g_pair_ev[1], st));
   if (staged) {
     const int vec = pack_out_vec(out, Pack::kN);
@@ -1108,9 +1233,13 @@ __global__ void k_key_scatter(SurfView S, const int32_t* __restrict__ rkey, int6
     const int tot_a = __shfl_sync(0xffffffffu, sa, 31), tot_b = __shfl_sync(0xffffffffu, sb, 31);
     s_pre[l] = sa - a;
     s_pre[l + 32] = tot_a + sb - b;
+    // (the first key of a shorter row: the prefix up to it counts the long ones)
+    constexpr int ka = kWork - kLongPairs, kb = kWork - kLongQuad;
+    if (blockIdx.x == 0 && l == ka % 32) nwork[1] = ka < 32 ? sa - a : tot_a + sb - b;
+    if (blockIdx.x == 0 && l == kb % 32) nwork[2] = kb < 32 ? sa - a : tot_a + sb - b;
     if (l == 0) {
       s_pre[kWork] = tot_a + tot_b;
-      if (blockIdx.x == 0) *nwork = tot_a + tot_b;                  // rows with key < 64
+      if (blockIdx.x == 0) nwork[0] = tot_a + tot_b;                // rows with key < 64
     }
   }
   for (int k = threadIdx.x; k < kWork; k += kThreads) s_cnt[k] = 0;
@@ -1353,6 +1482,14 @@ static cudaError_t launch_dep(void (*k)(P...), unsigned grid, unsigned block, si
   return cudaLaunchKernelEx(&cfg, k, std::forward<A>(a)...);
 }
 
+// lanes per row of a short list, by the launch's lanes in waves of the row-info kernel (6 CTAs on 148 SMs; a third of the
+// rows of a domain are in cells with edges).  B200, one lane against the choice: 4096 rows of a 256-gon (30 candidates
+// each) 17.3 against 8.0 us, 2^18 rows 26 against 16, 300 001 rows 31 against 22; 2^20 rows 58 with one, 74 with two.
+static int info_lanes(int64_t n) {
+  const int64_t wave = (int64_t)148 * 6 * kThreads;
+  return n * 8 <= 4 * wave ? 8 : (n * 4 <= 10 * wave ? 4 : (n * 2 <= 10 * wave ? 2 : 1));
+}
+
 static int sort_rows(const Surface* s, const double* pos, const double* sup, const int32_t* allowed, int64_t n,
                      const double* pose, const double* obb, int unbounded, const Workspace& w, cudaStream_t st) {
   const int64_t nbk = (int64_t)s->n_nonempty + 2;   // buckets: the cells with edges
@@ -1365,8 +1502,9 @@ static int sort_rows(const Surface* s, const double* pos, const double* sup, con
   WSB_CUDA(launch_dep(k_scan_block, 1, kScanThreads, 0, st, (const int32_t*)w.counts, w.offs, nbk + 1));
   WSB_CUDA(launch_dep(k_agg_scatter, grid, kThreads, 0, st, v, (const int32_t*)w.key, n, (const int32_t*)w.offs,
                       w.cursor, w.order));
-  WSB_CUDA(launch_dep(k_agg_rowinfo, grid, kThreads, 0, st, v, sup, (const int32_t*)w.key, (const double*)w.lpos,
-                      (const int32_t*)w.offs, (const int32_t*)w.order, n, w.ind, w.flag, w.rkey, w.mask, w.khist));
+  const int lanes = info_lanes(n);
+  WSB_CUDA(launch_dep(k_agg_rowinfo, (unsigned)((n * lanes + kThreads - 1) / kThreads), kThreads, 0, st, v, sup, (const int32_t*)w.key, (const double*)w.lpos,
+                      (const int32_t*)w.offs, (const int32_t*)w.order, n, w.ind, w.flag, w.rkey, w.mask, w.khist, lanes));
   WSB_CUDA(launch_dep(k_key_scatter, grid, kThreads, 0, st, v, (const int32_t*)w.rkey, n, (const int32_t*)w.khist,
                       w.kcur, (const int32_t*)w.order, w.key, (const double*)w.lpos, sup, (const uint64_t*)w.mask,
                       w.wrec, w.nwork));

@@ -40,6 +40,7 @@ SurfView view_of(const Surface* s) {
   v.cempty = s->cempty;
   v.ccompact = s->ccompact;
   v.nne = s->n_nonempty;
+  v.nlc = s->n_long;
   v.bstart = s->bstart;
   v.bitems = s->bitems;
   v.brec = s->brec;
@@ -210,8 +211,16 @@ extern "C" int wsb_surface_create(const double* verts, int64_t n_verts, const in
   std::vector<int32_t> cempty(ncells);
   for (int64_t c = 0; c < ncells; ++c) cempty[c] = (start[c + 1] == start[c]) ? 1 : 0;
   std::vector<int32_t> ccompact(ncells);
-  int32_t nne = 0;
-  for (int64_t c = 0; c < ncells; ++c) ccompact[c] = cempty[c] ? -1 : nne++;
+  // the cells with edges in decreasing order of their lists' length (a counting sort; cell order within a length)
+  int32_t nne = 0, nlc = 0;
+  {
+    std::vector<int32_t> of((size_t)K + 2, 0);
+    for (int64_t c = 0; c < ncells; ++c) ++of[K - (start[c + 1] - start[c]) + 1];
+    for (int32_t k = 0; k <= K; ++k) of[k + 1] += of[k];
+    nne = of[K];
+    nlc = of[std::max(0, K - kLongList + 1)];
+    for (int64_t c = 0; c < ncells; ++c) ccompact[c] = cempty[c] ? -1 : of[K - (start[c + 1] - start[c])]++;
+  }
   // ---- y bins (scene.py:297-314)
   const int32_t nb = std::max<int32_t>(1, (int32_t)std::sqrt((double)n_edges) * 2);
   double ylo_min = INFINITY, yhi_max = -INFINITY;
@@ -242,6 +251,7 @@ extern "C" int wsb_surface_create(const double* verts, int64_t n_verts, const in
   s->cell = cell;
   s->K = K;
   s->n_nonempty = nne;
+  s->n_long = nlc;
   s->n_items = n_items;
   s->nb = nb;
   s->y0 = y0;
