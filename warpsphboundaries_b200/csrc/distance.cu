@@ -191,7 +191,7 @@ __device__ __forceinline__ Group group_of() {
           0xffu << (lane / kGroup * kGroup)};
 }
 
-__global__ void __launch_bounds__(kDistThreads) k_signed_distance(SurfView S, const TreeView T,
+__global__ void __launch_bounds__(kDistThreads, 16) k_signed_distance(SurfView S, const TreeView T,
                                                                  const double* __restrict__ lpos, int64_t m,
                                                                  double norm_support, double* d, double* cp, double* nl,
                                                                  int32_t* edge) {
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(kDistThreads) k_signed_distance(SurfView S, co
 // One surface of a body in one pass over world points: into the body frame, the signed distance, the normal back to the
 // world frame, and the nearest body so far kept (d < best; `first`: nothing before).  The frame changes are the rounded
 // operations of Pose.toLocal / vecToWorld (scene.py:75-90).
-__global__ void __launch_bounds__(kDistThreads) k_body_distance(SurfView S, const TreeView T,
+__global__ void __launch_bounds__(kDistThreads, 16) k_body_distance(SurfView S, const TreeView T,
                                                                const double* __restrict__ pos, int64_t m,
                                                                const double* __restrict__ pose, double norm_support,
                                                                int first, int64_t body, double* best, double* normal,
