@@ -753,6 +753,69 @@ __device__ __forceinline__ void pack_stage(const double* acc_t, int G, bool writ
 // form.
 constexpr int kShortLanes = 2, kLongLanes = 8;
 
+// the pairs of a warp's rows (every lane takes part; lane `sub` of the G that share a row; no row: kb = e1 = 0, an empty
+// mask): the channel sums of the lane's share into acc_t
+template <class Pack, int PREC>
+__device__ __forceinline__ void pair_walk(const SurfView& S, int G, int sub, double lx, double ly, double h, int kb, int e1,
+                                          uint64_t mk0, uint64_t mk1, double* acc_t, double4* slot) {
+  constexpr bool kQuadPack = Pack::kN == 1 && Pack::template Kern<0>::kQuad;
+  int kt = kb + kMaskBits + sub;                                    // past the mask: lane sub scans kt, kt + G, ...
+  // lane sub takes the neighbours of rank sub, sub + G, ... of the mask (in candidate order), then its share of the
+  // candidates past the mask by the predicate
+  for (int s = 0; s < sub; ++s) pop_bit(mk0, mk1);
+  int nb = pop_bit(mk0, mk1);
+  const double ih = 1.0 / h;
+#pragma unroll
+  for (int c = 0; c < Pack::kN * 12; ++c) acc_t[c * kThreads] = 0.0;
+  // the next neighbour's (or tail candidate's) record is copied into the thread's shared-memory slot one step ahead
+  // (cp.async), so its latency hides behind the current pair's closed form
+  const double4 zero = make_double4(0.0, 0.0, 0.0, 0.0);
+  if (nb >= 0)
+    cp_async_rec(slot, S.crec + kb + nb);
+  else if (kt < e1)
+    cp_async_rec(slot, S.crec + kt);
+  while (__any_sync(0xffffffffu, nb >= 0 || kt < e1)) {
+    double4 e = zero;
+    bool have = false;
+    if (nb >= 0) {
+      cp_async_wait_all();
+      e = *slot;
+      have = true;
+      for (int s = 1; s < G; ++s) pop_bit(mk0, mk1);
+      nb = pop_bit(mk0, mk1);
+      if (nb >= 0)
+        cp_async_rec(slot, S.crec + kb + nb);
+      else if (kt < e1)
+        cp_async_rec(slot, S.crec + kt);
+    } else {
+      while (kt < e1) {
+        cp_async_wait_all();
+        e = *slot;
+        kt += G;
+        if (kt < e1) cp_async_rec(slot, S.crec + kt);
+        if (seg_within_fast(lx, ly, e.x, e.y, e.z, e.w, h)) {
+          have = true;
+          break;
+        }
+      }
+    }
+    __syncwarp();
+    if constexpr (kQuadPack) {
+      PairGeo g{};
+      have = have && pair_geo_row(lx, ly, h, ih, e, g);
+      quad_pairs<typename Pack::template Kern<0>>(have, g, acc_t);
+    } else if (have) {
+      PairGeo g;
+      if (pair_geo_row(lx, ly, h, ih, e, g)) {
+        if constexpr (PREC == WSB_PREC_FP32)
+          pack_pair_f32<Pack, 0>(g, acc_t);
+        else
+          pack_pair<Pack, PREC, 0>(g, acc_t);
+      }
+    }
+  }
+}
+
 template <class Pack, int PREC, int MINB, bool STAGED>
 __global__ void __launch_bounds__(kThreads, MINB) k_agg_pairs(SurfView S, const double* __restrict__ sup,
                                                              const WorkRec* __restrict__ wrec,
@@ -791,83 +854,190 @@ __global__ void __launch_bounds__(kThreads, MINB) k_agg_pairs(SurfView S, const 
     const int64_t w = lng ? task * kLongRows + lane / kLongLanes : nlong + (task - tlong) * kShortRows + lane / kShortLanes;
     const int sub = lane % G;
     const bool ok = w < (lng ? nlong : nwork);
-    int32_t i = 0;
-    int kb = 0, kt = 0, e1 = 0;
-    uint64_t mk0 = 0, mk1 = 0;
-    double lx = 0.0, ly = 0.0, h = 1.0;
-    if (ok) {
-      const WorkRec r = load_workrec(wrec + w);
-      i = r.row;
-      lx = r.lx;
-      ly = r.ly;
-      h = r.h;
-      kb = r.kb;
-      e1 = r.ke;
-      kt = kb + kMaskBits + sub;                                    // past the mask: lane sub scans kt, kt + G, ...
-      mk0 = r.m0;
-      mk1 = r.m1;
-    }
-    // lane sub takes the neighbours of rank sub, sub + G, ... of the mask (in candidate order), then its share of the
-    // candidates past the mask by the predicate
-    for (int s = 0; s < sub; ++s) pop_bit(mk0, mk1);
-    int nb = pop_bit(mk0, mk1);
-    const double ih = 1.0 / h;
+    WorkRec r{};
+    r.h = 1.0;
+    if (ok) r = load_workrec(wrec + w);
     double* const acc_t = s_acc + threadIdx.x;
-#pragma unroll
-    for (int c = 0; c < Pack::kN * 12; ++c) acc_t[c * kThreads] = 0.0;
-    // the next neighbour's (or tail candidate's) record is copied into the thread's shared-memory slot one step ahead
-    // (cp.async), so its latency hides behind the current pair's closed form
-    const double4 zero = make_double4(0.0, 0.0, 0.0, 0.0);
-    double4* const slot = s_next + threadIdx.x;
-    if (nb >= 0)
-      cp_async_rec(slot, S.crec + kb + nb);
-    else if (kt < e1)
-      cp_async_rec(slot, S.crec + kt);
-    while (__any_sync(0xffffffffu, nb >= 0 || kt < e1)) {
-      double4 e = zero;
-      bool have = false;
-      if (nb >= 0) {
-        cp_async_wait_all();
-        e = *slot;
-        have = true;
-        for (int s = 1; s < G; ++s) pop_bit(mk0, mk1);
-        nb = pop_bit(mk0, mk1);
-        if (nb >= 0)
-          cp_async_rec(slot, S.crec + kb + nb);
-        else if (kt < e1)
-          cp_async_rec(slot, S.crec + kt);
-      } else {
-        while (kt < e1) {
-          cp_async_wait_all();
-          e = *slot;
-          kt += G;
-          if (kt < e1) cp_async_rec(slot, S.crec + kt);
-          if (seg_within_fast(lx, ly, e.x, e.y, e.z, e.w, h)) {
-            have = true;
-            break;
-          }
-        }
-      }
-      __syncwarp();
-      if constexpr (kQuadPack) {
-        PairGeo g{};
-        have = have && pair_geo_row(lx, ly, h, ih, e, g);
-        quad_pairs<typename Pack::template Kern<0>>(have, g, acc_t);
-      } else if (have) {
-        PairGeo g;
-        if (pair_geo_row(lx, ly, h, ih, e, g)) {
-          if constexpr (PREC == WSB_PREC_FP32)
-            pack_pair_f32<Pack, 0>(g, acc_t);
-          else
-            pack_pair<Pack, PREC, 0>(g, acc_t);
-        }
-      }
-    }
+    pair_walk<Pack, PREC>(S, G, sub, r.lx, r.ly, r.h, r.kb, r.ke, r.m0, r.m1, acc_t, s_next + threadIdx.x);
     const bool write = ok && sub == 0;
     if constexpr (STAGED)
       pack_stage<Pack, 0>(acc_t, G, write, wacc + w * (Pack::kN * 12));
     else
-      pack_finish<Pack, 0>(acc_t, G, write, i, write ? ind[i] : 0.0, h, pose, assign, out);
+      pack_finish<Pack, 0>(acc_t, G, write, r.row, write ? ind[r.row] : 0.0, r.h, pose, assign, out);
+  }
+}
+
+// ------------------------------------------------------------------------------------------------ one launch for few rows
+// The whole aggregate of up to kThreads consecutive rows by one block: body frame and broadphase (a thread per row), the
+// row information of the rows in cells with edges (four or eight lanes a row), a counting sort of the rows with pairs by
+// their number in shared memory, the pair walk over them (the lanes of a row as in k_agg_pairs, so the same sums in the
+// same order) and the outputs.  For launches of few rows, which the seven launches of the sorted route leave waiting for
+// one another (one_launch gives the times).  Above some 10^5 rows the sorted route is faster: there a warp's rows have equal
+// pair counts.
+struct BlockRow {
+  double lx, ly, h, ind;
+  uint64_t m0, m1;
+  int32_t kb, ke;
+};
+
+template <class Pack, int PREC>
+__global__ void __launch_bounds__(kThreads, pack_min_blocks(Pack::kN) < 5 ? pack_min_blocks(Pack::kN) : 5)
+    k_agg_block(SurfView S, const double* __restrict__ pos, const double* __restrict__ sup,
+                const int32_t* __restrict__ allowed, int64_t n, const double* __restrict__ pose, double4 obb,
+                int unbounded, bool assign, const PackOut out, int rows) {
+  constexpr bool kQuadPack = Pack::kN == 1 && Pack::template Kern<0>::kQuad;
+  constexpr int kInfo = 4;                                          // lanes per row of the row information
+  extern __shared__ double4 s_dyn[];
+  double* const s_acc = reinterpret_cast<double*>(s_dyn + kThreads);
+  __shared__ BlockRow s_row[kThreads];
+  __shared__ int32_t s_cell[kThreads];                              // rows in cells with edges, compacted: their cell
+  __shared__ int16_t s_cand[kThreads], s_order[kThreads];           // their place in the block; the rows with pairs, sorted
+  __shared__ int32_t s_hist[kKeys], s_count[2];
+  const int t = threadIdx.x, lane = t & 31;
+  const int64_t row0 = (int64_t)blockIdx.x * rows;
+  const int here = (int)min((int64_t)rows, n - row0);
+  for (int k = t; k < kKeys; k += kThreads) s_hist[k] = 0;
+  if (t < 2) s_count[t] = 0;
+  __syncthreads();
+  // body frame, broadphase, cell; rows without candidates are settled (as in k_agg_prep)
+  int flag = 0;                                                     // 0 not a candidate, 1 constant row, 2 candidates
+  double w = 0.0;
+  if (t < here) {
+    const int64_t i = row0 + t;
+    double lx, ly;
+    to_local_rn(pos[2 * i], pos[2 * i + 1], pose[0], pose[1], pose[2], pose[3], lx, ly);
+    const double h = sup[i];
+    bool valid = allowed ? (allowed[i] != 0) : true;
+    if (valid && !unbounded) {
+      const double dx = __dadd_rn(fmax(__dsub_rn(obb.x, lx), 0.0), fmax(__dsub_rn(lx, obb.z), 0.0));
+      const double dy = __dadd_rn(fmax(__dsub_rn(obb.y, ly), 0.0), fmax(__dsub_rn(ly, obb.w), 0.0));
+      valid = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy))) < h;
+    }
+    int32_t b = -1;
+    if (valid) {
+      flag = 1;
+      if (!cell_of(S, lx, ly, b))
+        w = S.background;
+      else if (S.cempty[b])
+        w = S.cind[b];
+      else
+        flag = 2;
+    }
+    if (flag == 2) {
+      const int c = atomicAdd(&s_count[0], 1);                      // (the order is irrelevant: every row is its own)
+      s_cand[c] = (int16_t)t;
+      s_cell[c] = b;
+      s_row[t].lx = lx;
+      s_row[t].ly = ly;
+      s_row[t].h = h;
+    }
+  }
+  __syncthreads();
+  // the row information: neighbour mask and count, indicator (as in k_agg_rowinfo)
+  const int ncand = s_count[0];
+  for (int c0 = 0; c0 < ncand; c0 += kThreads / kInfo) {
+    const int c = c0 + t / kInfo, sub = t % kInfo;
+    const bool cand = c < ncand;
+    int r = 0, cnt = 0, cross = 0, bad = 0, k0 = 0, k1 = 0;
+    int32_t b = 0;
+    uint64_t m0 = 0, m1 = 0;
+    double lx = 0.0, ly = 0.0, h = 1.0;
+    if (cand) {
+      r = s_cand[c];
+      b = s_cell[c];
+      lx = s_row[r].lx;
+      ly = s_row[r].ly;
+      h = s_row[r].h;
+      const int32_t cx = b / S.ny, cy = b % S.ny;
+      const double rx = __dadd_rn(S.lo_x, __dmul_rn(__dadd_rn((double)cx, 0.5), S.cell));
+      const double ry = __dadd_rn(S.lo_y, __dmul_rn(__dadd_rn((double)cy, 0.5), S.cell));
+      bool degenerate = S.cok[b] == 0;
+      k0 = S.cstart[b];
+      k1 = S.cstart[b + 1];
+      for (int k = k0 + sub; k < k1; k += kInfo) {
+        const double4 e = ldg4(S.crec + k);
+        if (seg_within_fast(lx, ly, e.x, e.y, e.z, e.w, h)) {
+          ++cnt;
+          const int q = k - k0;
+          if (q < 64)
+            m0 |= 1ull << q;
+          else if (q < kMaskBits)
+            m1 |= 1ull << (q - 64);
+        }
+        if (!degenerate) cross += segment_crossing(rx, ry, lx, ly, e, &degenerate);
+      }
+      bad = degenerate ? 1 : 0;
+    }
+#pragma unroll
+    for (int o = 1; o < kInfo; o <<= 1) {
+      cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+      cross += __shfl_xor_sync(0xffffffffu, cross, o);
+      bad |= __shfl_xor_sync(0xffffffffu, bad, o);
+      m0 |= __shfl_xor_sync(0xffffffffu, m0, o);
+      m1 |= __shfl_xor_sync(0xffffffffu, m1, o);
+    }
+    if (cand && sub == 0) {
+      BlockRow& q = s_row[r];
+      q.ind = bad ? indicator_at(S, lx, ly, h, true, b) : S.cind[b] + (double)cross;
+      q.m0 = m0;
+      q.m1 = m1;
+      q.kb = k0;
+      q.ke = k1;
+      const int key = cnt > 0 ? 63 - min(cnt, 63) : kKeys - 1;
+      // the row's key and its rank among the block's rows of that key
+      s_cell[c] = key | (atomicAdd(&s_hist[key], 1) << 8);
+    }
+  }
+  __syncthreads();
+  // exclusive prefix of the key counts (64 keys of rows with pairs), by one warp
+  if (t < 32) {
+    const int a = s_hist[lane], b = s_hist[lane + 32];
+    int sa = a, sb = b;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int ta = __shfl_up_sync(0xffffffffu, sa, o), tb = __shfl_up_sync(0xffffffffu, sb, o);
+      if (lane >= o) {
+        sa += ta;
+        sb += tb;
+      }
+    }
+    const int tot = __shfl_sync(0xffffffffu, sa, 31);
+    __syncwarp();
+    s_hist[lane] = sa - a;
+    s_hist[lane + 32] = tot + sb - b;
+    if (lane == 31) s_hist[64] = tot + sb;
+  }
+  __syncthreads();
+  if (t < ncand) {
+    const int key = s_cell[t] & 255;
+    if (key < kKeys - 1) s_order[s_hist[key] + (s_cell[t] >> 8)] = s_cand[t];
+  }
+  // the rows without pairs: the indicator times the whole-plane channels
+  if (t < ncand && (s_cell[t] & 255) == kKeys - 1) {
+    const int r = s_cand[t];
+    pack_constant_row<Pack, 0>(row0 + r, s_row[r].ind, s_row[r].h, pose, assign, out);
+  }
+  if (t < here && flag < 2 && (flag == 1 || assign)) pack_constant_row<Pack, 0>(row0 + t, w, sup[row0 + t], pose, assign, out);
+  __syncthreads();
+  // the rows with pairs, as k_agg_pairs takes them
+  constexpr int kWarps = kThreads / 32, kLongRows = 32 / kLongLanes, kShortRows = 32 / kShortLanes;
+  const int nwork = s_hist[64], nlong = s_hist[kKeys - 1 - (kQuadPack ? kLongQuad : kLongPairs)];
+  const int tlong = (nlong + kLongRows - 1) / kLongRows, tasks = tlong + (nwork - nlong + kShortRows - 1) / kShortRows;
+  for (int task = t / 32; task < tasks; task += kWarps) {
+    const bool lng = task < tlong;
+    const int G = lng ? kLongLanes : kShortLanes, sub = lane % G;
+    const int at = lng ? task * kLongRows + lane / kLongLanes : nlong + (task - tlong) * kShortRows + lane / kShortLanes;
+    const bool ok = at < (lng ? nlong : nwork);
+    BlockRow q{};
+    q.h = 1.0;
+    int r = 0;
+    if (ok) {
+      r = s_order[at];
+      q = s_row[r];
+    }
+    double* const acc_t = s_acc + t;
+    pair_walk<Pack, PREC>(S, G, sub, q.lx, q.ly, q.h, q.kb, q.ke, q.m0, q.m1, acc_t, s_dyn + t);
+    pack_finish<Pack, 0>(acc_t, G, ok && sub == 0, row0 + r, q.ind, q.h, pose, assign, out);
   }
 }
 
@@ -991,6 +1161,58 @@ static int launch_pack(const SurfView& v, const double* sup, const Workspace& w,
                           (const double*)w.ind, (const int32_t*)w.key, (const double*)w.wacc, n, pose, assign, out));
   }
   return WSB_OK;
+}
+
+// Whether an aggregate takes the one-launch route.  Device time on B200, sorted against one launch: w4 among 64 star
+// polygons 4096 rows 59 / 40 us, 65 536 82 / 56, 131 072 88 / 88, 262 144 113 / 135; four kernels 4096 84 / 62, 65 536
+// 121 / 130 (host side 144 / 131), 131 072 143 / 214; the delta+ groups 65 536 237 / 177, 131 072 272 / 282.  One kernel
+// over a surface of few cells (a 256-gon of 300: the sort's counters collide) 262 144 rows 150 / 74, 2^20 477 / 262; with
+// several kernels the sorted rows win there too.  The results are the same bits, so the rule may look at the launch.
+static bool one_launch(const Surface* s, int n_groups, int64_t n) {
+  if (n_groups > 1) return n <= (1 << 16);
+  return n <= (1 << 17) || n >= 256 * (int64_t)s->n_nonempty;
+}
+
+// its blocks hold 16 to 128 rows, so that the launch has at least two blocks per SM where it has the rows
+struct RowArgs {
+  const double *pos, *sup;
+  const int32_t* allowed;
+  int64_t n;
+  const double *pose, *obb;
+  int unbounded;
+};
+
+template <class Pack, int PREC>
+static int launch_block(const SurfView& v, const RowArgs& a, bool assign, const PackOut& out, cudaStream_t st) {
+  constexpr size_t smem = pack_smem_bytes<Pack>();
+  auto kern = k_agg_block<Pack, PREC>;
+  if (smem > 32 * 1024) {       // with the static arrays above the default limit: opt in once per device
+    static std::atomic<uint64_t> opted{0};
+    int dev = 0;
+    WSB_CUDA(cudaGetDevice(&dev));
+    const uint64_t bit = 1ull << (dev & 63);
+    if (!(opted.load() & bit)) {
+      WSB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      opted.fetch_or(bit);
+    }
+  }
+  int rows = kThreads;
+  while (rows > 16 && a.n < (int64_t)rows * 148 * 2) rows /= 2;
+  if (g_pair_ev[0]) WSB_CUDA(cudaEventRecord(g_pair_ev[0], st));
+  kern<<<(unsigned)((a.n + rows - 1) / rows), kThreads, smem, st>>>(v, a.pos, a.sup, a.allowed, a.n, a.pose,
+                                                                   make_double4(a.obb[0], a.obb[1], a.obb[2], a.obb[3]),
+                                                                   a.unbounded, assign, out, rows);
+  WSB_CUDA(cudaGetLastError());
+  if (g_pair_ev[1]) WSB_CUDA(cudaEventRecord(g_pair_ev[1], st));
+  return WSB_OK;
+}
+
+// a pack over a prepared workspace, or (rows != nullptr) over rows in one launch
+template <class Pack, int PREC>
+static int launch_any(const SurfView& v, const double* sup, const Workspace& w, int64_t n, const double* pose, bool assign,
+                      const PackOut& out, const RowArgs* rows, cudaStream_t st) {
+  return rows ? launch_block<Pack, PREC>(v, *rows, assign, out, st)
+              : launch_pack<Pack, PREC>(v, sup, w, n, pose, assign, out, st);
 }
 
 // ------------------------------------------------------------------------------------------------ adjoint
@@ -1563,10 +1785,9 @@ extern "C" int wsb_aggregate_prepare(const wsb_surface* s_, const double* pos, c
   return sort_rows(s, pos, sup, allowed, n, pose, obb, unbounded, w, (cudaStream_t)stream);
 }
 
-extern "C" int wsb_aggregate_evaluate(const wsb_surface* s_, int kernel, int precision, const double* sup, int64_t n,
-                                      const double* pose, int out_mask, double* lam, double* G, double* cov,
-                                      double* m1, double* m2, const void* workspace, size_t workspace_bytes,
-                                      void* stream) {
+static int evaluate(const wsb_surface* s_, int kernel, int precision, const double* sup, int64_t n, const double* pose,
+                    int out_mask, double* lam, double* G, double* cov, double* m1, double* m2, const void* workspace,
+                    size_t workspace_bytes, const RowArgs* rows, void* stream) {
   const Surface* s = reinterpret_cast<const Surface*>(s_);
   if (!s) return fail(WSB_ERR_ARG, "wsb_aggregate_evaluate: NULL surface");
   if (!aggregate_kernel_ok(kernel)) return fail(WSB_ERR_UNSUPPORTED, "wsb_aggregate_evaluate: unknown kernel id");
@@ -1595,9 +1816,9 @@ extern "C" int wsb_aggregate_evaluate(const wsb_surface* s_, int kernel, int pre
   o.m2[0] = M2;
   auto launch1 = [&](auto kt) {
     using P1 = KPack<decltype(kt)>;
-    if (precision == WSB_PREC_MIXED) return launch_pack<P1, WSB_PREC_MIXED>(v, sup, w, n, pose, assign, o, st);
-    if (precision == WSB_PREC_FP32) return launch_pack<P1, WSB_PREC_FP32>(v, sup, w, n, pose, assign, o, st);
-    return launch_pack<P1, WSB_PREC_FP64>(v, sup, w, n, pose, assign, o, st);
+    if (precision == WSB_PREC_MIXED) return launch_any<P1, WSB_PREC_MIXED>(v, sup, w, n, pose, assign, o, rows, st);
+    if (precision == WSB_PREC_FP32) return launch_any<P1, WSB_PREC_FP32>(v, sup, w, n, pose, assign, o, rows, st);
+    return launch_any<P1, WSB_PREC_FP64>(v, sup, w, n, pose, assign, o, rows, st);
   };
   int rc = 0;
   if (kernel == Kern_w2p5::kId)
@@ -1609,6 +1830,14 @@ extern "C" int wsb_aggregate_evaluate(const wsb_surface* s_, int kernel, int pre
   if (rc) return rc;
   WSB_CUDA(cudaGetLastError());
   return WSB_OK;
+}
+
+extern "C" int wsb_aggregate_evaluate(const wsb_surface* s, int kernel, int precision, const double* sup, int64_t n,
+                                      const double* pose, int out_mask, double* lam, double* G, double* cov,
+                                      double* m1, double* m2, const void* workspace, size_t workspace_bytes,
+                                      void* stream) {
+  return evaluate(s, kernel, precision, sup, n, pose, out_mask, lam, G, cov, m1, m2, workspace, workspace_bytes, nullptr,
+                  stream);
 }
 
 // The kernel sets evaluated in one pass over the neighbour pairs, largest first: the smoothing-kernel families, and
@@ -1636,11 +1865,10 @@ static bool match_pack(const int32_t* kernels, int n_groups, const int32_t* pack
   return true;
 }
 
-extern "C" int wsb_aggregate_evaluate_groups(const wsb_surface* s_, int n_groups, const int32_t* kernels,
-                                             int precision, const double* sup, int64_t n, const double* pose,
-                                             int out_mask, double* const* lam, double* const* G, double* const* cov,
-                                             double* const* m1, double* const* m2, const void* workspace,
-                                             size_t workspace_bytes, void* stream) {
+static int evaluate_groups(const wsb_surface* s_, int n_groups, const int32_t* kernels, int precision, const double* sup,
+                           int64_t n, const double* pose, int out_mask, double* const* lam, double* const* G,
+                           double* const* cov, double* const* m1, double* const* m2, const void* workspace,
+                           size_t workspace_bytes, const RowArgs* rows, void* stream) {
   const Surface* s = reinterpret_cast<const Surface*>(s_);
   if (!s) return fail(WSB_ERR_ARG, "wsb_aggregate_evaluate_groups: NULL surface");
   if (n_groups < 1 || n_groups > WSB_MAX_GROUPS || !kernels)
@@ -1668,9 +1896,9 @@ extern "C" int wsb_aggregate_evaluate_groups(const wsb_surface* s_, int n_groups
   for (int p = 0; p < m; ++p) in_pack[perm[p]] = true;
   for (int g = 0; g < n_groups; ++g) {                              // the groups outside the pack: one pass each
     if (in_pack[g]) continue;
-    const int rc = wsb_aggregate_evaluate(s_, kernels[g], precision, sup, n, pose, out_mask, pick(lam, g, WSB_OUT_LAM),
-                                          pick(G, g, WSB_OUT_G), pick(cov, g, WSB_OUT_COV), pick(m1, g, WSB_OUT_M1),
-                                          pick(m2, g, WSB_OUT_M2), workspace, workspace_bytes, stream);
+    const int rc = evaluate(s_, kernels[g], precision, sup, n, pose, out_mask, pick(lam, g, WSB_OUT_LAM),
+                            pick(G, g, WSB_OUT_G), pick(cov, g, WSB_OUT_COV), pick(m1, g, WSB_OUT_M1),
+                            pick(m2, g, WSB_OUT_M2), workspace, workspace_bytes, rows, stream);
     if (rc) return rc;
   }
   if (which < 0) return WSB_OK;
@@ -1692,9 +1920,9 @@ extern "C" int wsb_aggregate_evaluate_groups(const wsb_surface* s_, int n_groups
   }
   auto run = [&](auto pack) {
     using P = decltype(pack);
-    if (precision == WSB_PREC_MIXED) return launch_pack<P, WSB_PREC_MIXED>(v, sup, w, n, pose, assign, o, st);
-    if (precision == WSB_PREC_FP32) return launch_pack<P, WSB_PREC_FP32>(v, sup, w, n, pose, assign, o, st);
-    return launch_pack<P, WSB_PREC_FP64>(v, sup, w, n, pose, assign, o, st);
+    if (precision == WSB_PREC_MIXED) return launch_any<P, WSB_PREC_MIXED>(v, sup, w, n, pose, assign, o, rows, st);
+    if (precision == WSB_PREC_FP32) return launch_any<P, WSB_PREC_FP32>(v, sup, w, n, pose, assign, o, rows, st);
+    return launch_any<P, WSB_PREC_FP64>(v, sup, w, n, pose, assign, o, rows, st);
   };
   int rc;
   switch (which) {
@@ -1707,6 +1935,30 @@ extern "C" int wsb_aggregate_evaluate_groups(const wsb_surface* s_, int n_groups
   }
   if (rc) return rc;
   WSB_CUDA(cudaGetLastError());
+  return WSB_OK;
+}
+
+extern "C" int wsb_aggregate_evaluate_groups(const wsb_surface* s, int n_groups, const int32_t* kernels,
+                                             int precision, const double* sup, int64_t n, const double* pose,
+                                             int out_mask, double* const* lam, double* const* G, double* const* cov,
+                                             double* const* m1, double* const* m2, const void* workspace,
+                                             size_t workspace_bytes, void* stream) {
+  return evaluate_groups(s, n_groups, kernels, precision, sup, n, pose, out_mask, lam, G, cov, m1, m2, workspace,
+                         workspace_bytes, nullptr, stream);
+}
+
+// the front half of an aggregate: nothing where the rows take the one-launch route, else the sorted rows; the checks of
+// wsb_aggregate_prepare in both
+static int front(const wsb_surface* s_, int n_groups, const RowArgs& a, void* workspace, size_t workspace_bytes,
+                 void* stream, const RowArgs** rows) {
+  *rows = one_launch(reinterpret_cast<const Surface*>(s_), n_groups, a.n) ? &a : nullptr;
+  if (!*rows)
+    return wsb_aggregate_prepare(s_, a.pos, a.sup, a.allowed, a.n, a.pose, a.obb, a.unbounded, workspace, workspace_bytes,
+                                 stream);
+  const size_t need = carve(reinterpret_cast<const Surface*>(s_), a.n, workspace).total;
+  if (!workspace || workspace_bytes < need)
+    return fail(WSB_ERR_SIZE, "wsb_aggregate_prepare: workspace of " + std::to_string(workspace_bytes) + " bytes, need " +
+                                  std::to_string(need));
   return WSB_OK;
 }
 
@@ -1724,10 +1976,11 @@ extern "C" int wsb_aggregate(const wsb_surface* s_, int kernel, int precision, c
     WSB_CUDA(cudaSetDevice(s->device));
     WSB_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t), (cudaStream_t)stream));
   }
-  rc = wsb_aggregate_prepare(s_, pos, sup, allowed, n, pose, obb, unbounded, workspace, workspace_bytes, stream);
+  const RowArgs args{pos, sup, allowed, n, pose, obb, unbounded}, *rows = nullptr;
+  rc = front(s_, 1, args, workspace, workspace_bytes, stream, &rows);
   if (rc) return rc;
-  return wsb_aggregate_evaluate(s_, kernel, precision, sup, n, pose, out_mask, lam, G, cov, m1, m2, workspace,
-                                workspace_bytes, stream);
+  return evaluate(s_, kernel, precision, sup, n, pose, out_mask, lam, G, cov, m1, m2, workspace, workspace_bytes, rows,
+                  stream);
 }
 
 extern "C" int wsb_aggregate_groups(const wsb_surface* s_, int n_groups, const int32_t* kernels, int precision,
@@ -1746,10 +1999,11 @@ extern "C" int wsb_aggregate_groups(const wsb_surface* s_, int n_groups, const i
   if (precision != WSB_PREC_FP64 && precision != WSB_PREC_MIXED && precision != WSB_PREC_FP32)
     return fail(WSB_ERR_UNSUPPORTED, "wsb_aggregate_groups: unknown precision mode");
   if (n == 0) return WSB_OK;
-  rc = wsb_aggregate_prepare(s_, pos, sup, allowed, n, pose, obb, unbounded, workspace, workspace_bytes, stream);
+  const RowArgs args{pos, sup, allowed, n, pose, obb, unbounded}, *rows = nullptr;
+  rc = front(s_, n_groups, args, workspace, workspace_bytes, stream, &rows);
   if (rc) return rc;
-  return wsb_aggregate_evaluate_groups(s_, n_groups, kernels, precision, sup, n, pose, out_mask, lam, G, cov, m1, m2,
-                                       workspace, workspace_bytes, stream);
+  return evaluate_groups(s_, n_groups, kernels, precision, sup, n, pose, out_mask, lam, G, cov, m1, m2, workspace,
+                         workspace_bytes, rows, stream);
 }
 
 extern "C" int wsb_aggregate_backward(const wsb_surface* s_, int kernel, const double* pos, const double* sup,
