@@ -31,17 +31,18 @@ class BoundaryMoments(torch.autograd.Function):
         supc = sup.detach().to(F64).contiguous()
         ns = rep.native(support, dev)
         ws, need = ns.workspace(N)
-        lam = torch.zeros(N, dtype=F64, device=dev)
-        G = torch.zeros((N, 2), dtype=F64, device=dev)
-        Cov = torch.zeros((N, 2, 2), dtype=F64, device=dev)
-        m1 = torch.zeros((N, 2), dtype=F64, device=dev)
-        m2 = torch.zeros((N, 2, 2), dtype=F64, device=dev)
+        lam = torch.empty(N, dtype=F64, device=dev)              # the call assigns every row
+        G = torch.empty((N, 2), dtype=F64, device=dev)
+        Cov = torch.empty((N, 2, 2), dtype=F64, device=dev)
+        m1 = torch.empty((N, 2), dtype=F64, device=dev)
+        m2 = torch.empty((N, 2, 2), dtype=F64, device=dev)
         pose = body.pose_tensor(dev)
-        obb = (_lib.ctypes.c_double * 4)(*body.obb())
+        obb, unbounded = body.broadphase()
         check(lib.wsb_aggregate(ns.handle, kid, _PREC[precision], ptr(posc), ptr(supc), None, N, ptr(pose), obb,
-                                int(body.unbounded()), _lib.OUT_ALL, ptr(lam), ptr(G), ptr(Cov), ptr(m1), ptr(m2),
+                                unbounded, _lib.OUT_ALL | _lib.OUT_ASSIGN, ptr(lam), ptr(G), ptr(Cov), ptr(m1), ptr(m2),
                                 ptr(ws), need, None, _stream()), "wsb_aggregate")
         ctx.save_for_backward(posc, supc)
+        ctx.set_materialize_grads(False)       # an output the loss does not use has no gradient tensor to fill and test
         ctx.body, ctx.rep, ctx.kid, ctx.support, ctx.nverts = body, rep, kid, support, len(verts)
         ctx.verts_device, ctx.verts_dtype = verts.device, verts.dtype
         return lam, m1, m2, G, Cov
@@ -58,17 +59,18 @@ class BoundaryMoments(torch.autograd.Function):
         ns = ctx.rep.native(ctx.support, dev)
         ws, need = ns.workspace(N)
         d_pos = torch.zeros((N, 2), dtype=F64, device=dev)
-        d_verts = torch.zeros((ctx.nverts, 2), dtype=F64, device=dev)
+        # the vertices' adjoint (four atomic sums a pair) only where it is asked for
+        d_verts = torch.zeros((ctx.nverts, 2), dtype=F64, device=dev) if ctx.needs_input_grad[1] else None
         gl = None if g_lam is None else g_lam.to(F64).contiguous()
         g1 = None if g_m1 is None else g_m1.to(F64).contiguous()
         g2 = None if g_m2 is None else g_m2.to(F64).contiguous()
         pose = ctx.body.pose_tensor(dev)
-        obb = (_lib.ctypes.c_double * 4)(*ctx.body.obb())
+        obb, unbounded = ctx.body.broadphase()
         check(lib.wsb_aggregate_backward(ns.handle, ctx.kid, ptr(posc), ptr(supc), None, N, ptr(pose), obb,
-                                         int(ctx.body.unbounded()), ptr(gl), ptr(g1), ptr(g2), ptr(d_pos),
+                                         unbounded, ptr(gl), ptr(g1), ptr(g2), ptr(d_pos),
                                          ptr(d_verts), ptr(ws), need, _stream()), "wsb_aggregate_backward")
-        return (d_pos.to(posc.dtype), d_verts.to(ctx.verts_device, ctx.verts_dtype), None, None, None, None, None,
-                None)
+        return (d_pos.to(posc.dtype), None if d_verts is None else d_verts.to(ctx.verts_device, ctx.verts_dtype), None,
+                None, None, None, None, None)
 
 
 def aggregate_moments(body, rep, pos, sup, kernel, support, precision="fp64"):

@@ -145,24 +145,28 @@ class FusedWall(WallAggregate):
         N = self.N
         al = None if allowed is None else allowed.to(torch.int32).contiguous()
         names = ("lam", "G", "Cov", "m1", "m2")
+        # what every body's call shares: the stream, the addresses of the inputs, the outputs' first addresses and their
+        # bytes per body; a call of a few thousand rows is bound by this bookkeeping
+        stream = torch.cuda.current_stream(self.dev).cuda_stream
+        st, p_pos, p_sup, p_al = _lib.c_void_p(stream), ptr(pos), ptr(sup), ptr(al)
+        base = {k: [(out[k].data_ptr(), 8 * out[k].stride(0)) for out in outs] for k in names}
+        ptr_array, kernel_ids, prec = _lib.c_void_p * len(kids), _lib.int32s(kids), _PREC[self.precision]
         for bi, body in enumerate(self.scene.bodies):
             if not body.reps:
                 for out in outs:
                     for t in out.values():
                         t[bi].zero_()
                 continue
-            pose = body.pose_tensor(self.dev)
-            obb = (_lib.ctypes.c_double * 4)(*body.obb())
+            p_pose = ptr(body.pose_tensor(self.dev))
+            at = {k: [b + bi * step for b, step in base[k]] for k in names}
             for ri, rep in enumerate(body.fused_reps(self.support, self.dev)):
                 mode = _lib.OUT_ALL | (_lib.OUT_ASSIGN if ri == 0 else 0)     # the first representation assigns
                 if isinstance(rep, DiskArrayRep):
                     nd = rep.native(self.support, self.dev)
-                    dws, dneed = nd.workspace(N)
+                    dws, dneed = nd.workspace(N, stream)
                     for gi, kid in enumerate(kids):
-                        o = outs[gi]
-                        check(lib.wsb_disk_aggregate(nd.handle, kid, ptr(pos), ptr(sup), ptr(al), N, ptr(pose), mode,
-                                                     ptr(o["lam"][bi]), ptr(o["G"][bi]), ptr(o["Cov"][bi]),
-                                                     ptr(o["m1"][bi]), ptr(o["m2"][bi]), ptr(dws), dneed, _stream()),
+                        check(lib.wsb_disk_aggregate(nd.handle, kid, p_pos, p_sup, p_al, N, p_pose, mode,
+                                                     *[at[k][gi] for k in names], ptr(dws), dneed, st),
                               "wsb_disk_aggregate")
                     continue
                 ns = rep.native(self.support, self.dev)
@@ -170,23 +174,22 @@ class FusedWall(WallAggregate):
                     ws = self.workspaces[id(rep)]
                     need = ws.numel()
                 else:
-                    ws, need = ns.workspace(N)
+                    ws, need = ns.workspace(N, stream)
+                obb, unbounded = body.broadphase()
                 if rep._triangle is None:
-                    tgt = {k: _lib.ptrs([out[k][bi] for out in outs]) for k in names}
-                    check(lib.wsb_aggregate_groups(ns.handle, len(kids), _lib.int32s(kids), _PREC[self.precision],
-                                                   ptr(pos), ptr(sup), ptr(al), N, ptr(pose), obb,
-                                                   int(body.unbounded()), mode, tgt["lam"], tgt["G"], tgt["Cov"],
-                                                   tgt["m1"], tgt["m2"], ptr(ws), need, _stream()),
+                    tgt = [ptr_array(*at[k]) for k in names]
+                    check(lib.wsb_aggregate_groups(ns.handle, len(kids), kernel_ids, prec, p_pos, p_sup, p_al, N, p_pose,
+                                                   obb, unbounded, mode, *tgt, ptr(ws), need, st),
                           "wsb_aggregate_groups")
                     continue
+                pose = body.pose_tensor(self.dev)
                 for gi, kid in enumerate(kids):
                     # closed form into scratch, then the rows the quadrature takes are overridden while combining
                     self._group = gi
                     tgt = {k: torch.empty_like(outs[gi][k][bi]) for k in names}
-                    check(lib.wsb_aggregate(ns.handle, kid, _PREC[self.precision], ptr(pos), ptr(sup), ptr(al), N,
-                                            ptr(pose), obb, int(body.unbounded()), _lib.OUT_ALL | _lib.OUT_ASSIGN,
-                                            ptr(tgt["lam"]), ptr(tgt["G"]), ptr(tgt["Cov"]), ptr(tgt["m1"]),
-                                            ptr(tgt["m2"]), ptr(ws), need, None, _stream()), "wsb_aggregate")
+                    check(lib.wsb_aggregate(ns.handle, kid, prec, p_pos, p_sup, p_al, N, p_pose, obb, unbounded,
+                                            _lib.OUT_ALL | _lib.OUT_ASSIGN, *[ptr(tgt[k]) for k in names], ptr(ws), need,
+                                            None, st), "wsb_aggregate")
                     self._conditioned(body, bi, ri, rep, pos, sup, al, kid, pose, tgt, outs[gi])
 
     def _conditioned(self, body, bi, ri, rep, pos, sup, al, kid, pose, closed, out, tolerance=2e-12,

@@ -100,6 +100,7 @@ class RadialEvaluator:
             ids = [i for i, a in enumerate(r.alpha) for _ in range(a)] + list(r.derivative)
             meta.append([sum(r.alpha), *(ids + [0, 0])[:2], len(r.derivative)])
         self.metadata = np.ascontiguousarray(np.array(meta, dtype=np.int32).reshape(-1, 4))
+        self._metadata_ptr = self.metadata.ctypes.data_as(_lib.POINTER(_lib.c_int32))
         self._kind_id = _lib.RADIAL_SPHERE if kind == "sphere" else _lib.RADIAL_PLANE
         self._kernel_id = KERNEL_IDS[kernel]
         self._prec_id = _PRECISIONS[precision]
@@ -167,18 +168,25 @@ class RadialBatch:
         return sum(t.numel() * t.element_size() for t in (self.distances, self.normals, self.supports, self.radii,
                                                            self.work, self.values, self.status))
 
+    def _launch(self, stream):
+        """the native call, on the device that is current."""
+        ev = self.evaluator
+        check(lib.wsb_radial_channels(ev._kind_id, ev._kernel_id, ev._prec_id, ptr(self.distances),
+                                      ptr(self.radii) if ev.kind == "sphere" else None, ptr(self.normals),
+                                      ptr(self.supports), self.count, ev._metadata_ptr, len(ev.requests),
+                                      ptr(self.values), ptr(self.work), ptr(self.status),
+                                      _lib.c_void_p(stream.cuda_stream)), "wsb_radial_channels")
+
     def launch(self, stream=None):
         ev = self.evaluator
         if self.count and len(ev.requests):
             st = stream if stream is not None else torch.cuda.current_stream(ev.device)
-            meta = ev.metadata
-            with torch.cuda.device(ev.device):
-                check(lib.wsb_radial_channels(ev._kind_id, ev._kernel_id, ev._prec_id, ptr(self.distances),
-                                              ptr(self.radii) if ev.kind == "sphere" else None, ptr(self.normals),
-                                              ptr(self.supports), self.count,
-                                              meta.ctypes.data_as(_lib.POINTER(_lib.c_int32)), len(ev.requests),
-                                              ptr(self.values), ptr(self.work), ptr(self.status),
-                                              _lib.c_void_p(st.cuda_stream)), "wsb_radial_channels")
+            dev = ev.device.index
+            if dev is None or dev == torch.cuda.current_device():
+                self._launch(st)
+            else:
+                with torch.cuda.device(dev):
+                    self._launch(st)
         return self.values
 
     def numpy(self):

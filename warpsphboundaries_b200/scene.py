@@ -74,14 +74,20 @@ class NativeSurface:
         self.K = int(info.K)
         self.support_max = float(support_max)
         self._ws = {}
+        self._need = (-1, 0)
 
-    def workspace(self, n):
-        """the workspace for n rows on the current stream: one buffer per stream, grown geometrically and reused for
-        any smaller row count (the library carves it per call and allocates nothing itself)."""
+    def workspace(self, n, stream=None):
+        """the workspace for n rows on the current stream (or the raw `stream` the caller found current): one buffer per
+        stream, grown geometrically and reused for any smaller row count (the library carves it per call and allocates
+        nothing itself)."""
         # with the staging region: the evaluations store every row's outputs in one coalesced pass
-        need = int(lib.wsb_aggregate_workspace_size(self.handle, int(n)) +
-                   lib.wsb_aggregate_staging_size(self.handle, int(n)))
-        key = torch.cuda.current_stream(self.device).cuda_stream
+        last = self._need                              # (n, bytes) of the last call, replaced as one object
+        if last[0] != n:
+            last = (n, int(lib.wsb_aggregate_workspace_size(self.handle, int(n)) +
+                           lib.wsb_aggregate_staging_size(self.handle, int(n))))
+            self._need = last
+        need = last[1]
+        key = torch.cuda.current_stream(self.device).cuda_stream if stream is None else stream
         ws = self._ws.get(key)
         if ws is None or ws.numel() < need:
             ws = torch.empty(max(need, int(1.5 * ws.numel()) if ws is not None else need, 1), dtype=torch.uint8,
@@ -389,10 +395,11 @@ class NativeDisks:
         self.handle = h
         self._ws = {}
 
-    def workspace(self, n):
-        """the work-list buffer for n rows on the current stream (one per stream, grown geometrically)."""
+    def workspace(self, n, stream=None):
+        """the work-list buffer for n rows on the current stream, or the raw `stream` the caller found current (one per
+        stream, grown geometrically)."""
         need = int(lib.wsb_disk_workspace_size(self.handle, int(n)))
-        key = torch.cuda.current_stream(self.device).cuda_stream
+        key = torch.cuda.current_stream(self.device).cuda_stream if stream is None else stream
         ws = self._ws.get(key)
         if ws is None or ws.numel() < need:
             ws = torch.empty(max(need, int(1.5 * ws.numel()) if ws is not None else need, 1), dtype=torch.uint8,
@@ -753,6 +760,15 @@ class Body:
         return any((isinstance(r, SurfaceRep) and r.background) or
                    (isinstance(r, (ImplicitRep, SdfRep)) and r.unbounded()) for r in self.reps)
 
+    def broadphase(self):
+        """(obb, unbounded) as the library takes them: four C doubles (formed once per box), an int."""
+        box = self.obb()
+        c = self.__dict__.get("_boxCache")
+        if c is None or c[0] != box:
+            c = (box, (ctypes.c_double * 4)(*box))
+            self._boxCache = c
+        return c[1], int(self.unbounded())
+
     def fusable(self):
         from .implicit import DiskBody
         return all(isinstance(r, (SurfaceRep, SdfRep, DiskArrayRep)) or
@@ -779,10 +795,10 @@ class Body:
 
     def pose_tensor(self, device):
         """(cx, cy, cos, sin) on the device, cached while the pose is unchanged."""
-        c, s = self.pose._cs()
-        key = (self.center.data_ptr(), self.center._version, c, s, str(device))
+        key = (self.center.data_ptr(), self.center._version, float(self.angle), device)
         hit = self.__dict__.get("_poseCache")
         if hit is None or hit[0] != key:
+            c, s = self.pose._cs()
             t = torch.cat([self.center.to(device, F64).reshape(2), torch.tensor([c, s], dtype=F64, device=device)])
             hit = (key, t)
             self._poseCache = hit
