@@ -259,13 +259,14 @@ TreeView tree_of(const Surface* s) {
 // box, finer than the leaves need)
 void edge_tree(const std::vector<double4>& erec, std::vector<double4>& box, std::vector<int32_t>& id) {
   const int64_t n = (int64_t)erec.size();
-  double lo[2] = {INFINITY, INFINITY}, hi[2] = {-INFINITY, -INFINITY};
-  for (const double4& r : erec) {
-    const double m[2] = {0.5 * r.x + 0.5 * r.z, 0.5 * r.y + 0.5 * r.w};
-    for (int k = 0; k < 2; ++k) {
-      lo[k] = std::min(lo[k], m[k]);
-      hi[k] = std::max(hi[k], m[k]);
-    }
+  const double4* rec = erec.data();
+  double lx = INFINITY, ly = INFINITY, hx = -INFINITY, hy = -INFINITY;
+  for (int64_t e = 0; e < n; ++e) {
+    const double mx = 0.5 * rec[e].x + 0.5 * rec[e].z, my = 0.5 * rec[e].y + 0.5 * rec[e].w;
+    lx = std::min(lx, mx);
+    ly = std::min(ly, my);
+    hx = std::max(hx, mx);
+    hy = std::max(hy, my);
   }
   auto spread = [](uint32_t v) {
     v = (v | (v << 8)) & 0x00ff00ffu;
@@ -273,49 +274,62 @@ void edge_tree(const std::vector<double4>& erec, std::vector<double4>& box, std:
     v = (v | (v << 2)) & 0x33333333u;
     return (v | (v << 1)) & 0x55555555u;
   };
-  double scale[2];
-  for (int k = 0; k < 2; ++k) scale[k] = hi[k] > lo[k] ? 2047.0 / (hi[k] - lo[k]) : 0.0;
+  const double sx = hx > lx ? 2047.0 / (hx - lx) : 0.0, sy = hy > ly ? 2047.0 / (hy - ly) : 0.0;
   std::vector<uint64_t> key((size_t)n), tmp((size_t)n);
-  std::vector<uint32_t> count(2 * 2048, 0);
+  uint64_t* kp = key.data();
   for (int64_t e = 0; e < n; ++e) {
-    const double4& r = erec[(size_t)e];
-    const double m[2] = {0.5 * r.x + 0.5 * r.z, 0.5 * r.y + 0.5 * r.w};
-    uint32_t q[2];
-    for (int k = 0; k < 2; ++k) q[k] = (uint32_t)std::min(2047.0, std::max(0.0, (m[k] - lo[k]) * scale[k]));
-    const uint32_t code = spread(q[0]) | (spread(q[1]) << 1);
-    ++count[code & 2047];
-    ++count[2048 + (code >> 11)];
-    key[(size_t)e] = ((uint64_t)code << 32) | (uint64_t)e;
+    const double mx = 0.5 * rec[e].x + 0.5 * rec[e].z, my = 0.5 * rec[e].y + 0.5 * rec[e].w;
+    const uint32_t qx = (uint32_t)(int32_t)std::min(2047.0, std::max(0.0, (mx - lx) * sx));
+    const uint32_t qy = (uint32_t)(int32_t)std::min(2047.0, std::max(0.0, (my - ly) * sy));
+    kp[e] = ((uint64_t)(spread(qx) | (spread(qy) << 1)) << 32) | (uint64_t)e;
   }
+  std::vector<uint32_t> count(2 * 2048, 0);
+  uint32_t* c0 = count.data();
+  for (int64_t e = 0; e < n; ++e) {
+    ++c0[(kp[e] >> 32) & 2047];
+    ++c0[2048 + (kp[e] >> 43)];
+  }
+  uint64_t *a = kp, *b = tmp.data();
   for (int pass = 0; pass < 2; ++pass) {               // radix sort of the 22-bit codes
-    uint32_t* c = count.data() + 2048 * pass;
+    uint32_t* c = c0 + 2048 * pass;
     uint32_t sum = 0;
-    for (int b = 0; b < 2048; ++b) {
-      const uint32_t v = c[b];
-      c[b] = sum;
+    for (int k = 0; k < 2048; ++k) {
+      const uint32_t v = c[k];
+      c[k] = sum;
       sum += v;
     }
-    for (uint64_t k : key) tmp[c[(k >> (32 + 11 * pass)) & 2047]++] = k;
-    key.swap(tmp);
+    for (int64_t e = 0; e < n; ++e) b[c[(a[e] >> (32 + 11 * pass)) & 2047]++] = a[e];
+    std::swap(a, b);
   }
   id.resize((size_t)n);
-  for (int64_t i = 0; i < n; ++i) id[(size_t)i] = (int32_t)(uint32_t)key[(size_t)i];
-  box.clear();
-  for (int64_t i = 0; i < n; i += kGroup) {
-    double4 b = make_double4(INFINITY, INFINITY, -INFINITY, -INFINITY);
-    for (int64_t k = i; k < std::min<int64_t>(i + kGroup, n); ++k) {
-      const double4& r = erec[(size_t)id[(size_t)k]];
-      b = make_double4(std::min(b.x, std::min(r.x, r.z)), std::min(b.y, std::min(r.y, r.w)),
-                       std::max(b.z, std::max(r.x, r.z)), std::max(b.w, std::max(r.y, r.w)));
-    }
-    box.push_back(b);
+  int32_t* ip = id.data();
+  for (int64_t i = 0; i < n; ++i) ip[i] = (int32_t)(uint32_t)a[i];
+  size_t n_box = 0;
+  for (int64_t m = n; m > 1 || n_box == 0;) {
+    m = (m + kGroup - 1) / kGroup;
+    n_box += (size_t)m;
   }
-  for (size_t start = 0, end = box.size(); end - start > 1; start = end, end = box.size()) {
-    for (size_t i = start; i < end; i += kGroup) {
-      double4 b = box[i];
-      for (size_t k = i + 1; k < std::min(i + kGroup, end); ++k)
-        b = make_double4(std::min(b.x, box[k].x), std::min(b.y, box[k].y), std::max(b.z, box[k].z), std::max(b.w, box[k].w));
-      box.push_back(b);
+  box.resize(n_box);
+  double4* bp = box.data();
+  size_t end = 0;
+  for (int64_t i = 0; i < n; i += kGroup) {
+    double x0 = INFINITY, y0 = INFINITY, x1 = -INFINITY, y1 = -INFINITY;
+    const int64_t last = std::min<int64_t>(i + kGroup, n);
+    for (int64_t k = i; k < last; ++k) {
+      const double4& r = rec[ip[k]];
+      x0 = std::min(x0, std::min(r.x, r.z));
+      y0 = std::min(y0, std::min(r.y, r.w));
+      x1 = std::max(x1, std::max(r.x, r.z));
+      y1 = std::max(y1, std::max(r.y, r.w));
+    }
+    bp[end++] = make_double4(x0, y0, x1, y1);
+  }
+  for (size_t start = 0, stop = end; stop - start > 1; start = stop, stop = end) {
+    for (size_t i = start; i < stop; i += kGroup) {
+      double4 v = bp[i];
+      for (size_t k = i + 1; k < std::min(i + kGroup, stop); ++k)
+        v = make_double4(std::min(v.x, bp[k].x), std::min(v.y, bp[k].y), std::max(v.z, bp[k].z), std::max(v.w, bp[k].w));
+      bp[end++] = v;
     }
   }
 }
