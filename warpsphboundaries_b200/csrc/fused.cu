@@ -44,13 +44,13 @@ static_assert(sizeof(WorkRec) == 64 && offsetof(WorkRec, h) == 16 && offsetof(Wo
 struct Workspace {
   int32_t* key;      // [n] cell of a row in a cell with edges (sorted by it), -1 for rows settled by k_agg_prep
   double* lpos;      // [2n] body-frame positions
-  int32_t* counts;   // [nbk + 1]   } zeroed together (buckets: the cells with edges, by compact index)
-  int32_t* cursor;   // [nbk]       }
+  int32_t* counts;   // [nbk + 1] rows per bucket (the cells with edges, by compact index)
   int32_t* offs;     // [nbk + 1] exclusive prefix sums of counts
   int32_t* order;    // [n] rows sorted by bucket
   double* ind;       // [n] indicator of a row (by row index)
   int32_t* flag;     // [n] 0 not a candidate, 1 candidate without neighbour pairs, 2 row with pairs (by row index)
-  int32_t* rkey;     // [n] count key of a sorted row: 63 - min(pairs, 63) for rows with pairs, 64 otherwise
+  int32_t* rkey;     // [n] a row's rank in its bucket until the sort, then the count key of a sorted row: 63 - min(pairs, 63) for
+                     // rows with pairs, 64 otherwise (of the sorted rows only)
   uint64_t* mask;    // [2n] by sorted row: bit k set when candidate k (< kMaskBits) of the row's cell is a neighbour
   int32_t* khist;    // [kKeys] rows per key   } zeroed together
   int32_t* kcur;     // [kKeys] fill cursors   }
@@ -74,8 +74,7 @@ static Workspace carve(const Surface* s, int64_t n, void* base) {
   };
   w.key = (int32_t*)take(sizeof(int32_t) * std::max<int64_t>(n, 1));
   w.lpos = (double*)take(sizeof(double) * 2 * std::max<int64_t>(n, 1));
-  w.counts = (int32_t*)take(sizeof(int32_t) * (2 * nbk + 1));
-  w.cursor = w.counts + nbk + 1;
+  w.counts = (int32_t*)take(sizeof(int32_t) * (nbk + 1));
   w.offs = (int32_t*)take(sizeof(int32_t) * (nbk + 1));
   w.order = (int32_t*)take(sizeof(int32_t) * std::max<int64_t>(n, 1));
   w.ind = (double*)take(sizeof(double) * std::max<int64_t>(n, 1));
@@ -99,11 +98,14 @@ static void attach_staging(Workspace& w, void* base, size_t workspace_bytes) {
   w.wacc = (p && workspace_bytes >= w.total + w.staging && ((uintptr_t)p & 31u) == 0) ? (double*)p : nullptr;
 }
 
-// body-frame position (bit-for-bit Pose.toLocal), broadphase (fixedadj.py:257-265) and the bucket of every row
+// body-frame position (bit-for-bit Pose.toLocal), broadphase (fixedadj.py:257-265), the bucket of every row and its rank
+// there (the order inside a bucket is arbitrary: no row's result depends on it); one atomic a row, where ranks drawn by a
+// second kernel cost another
 __global__ void k_agg_prep(SurfView S, const double* __restrict__ pos, const double* __restrict__ sup,
                            const int32_t* __restrict__ allowed, int64_t n, const double* __restrict__ pose,
                            double4 obb, int unbounded, int32_t* __restrict__ key, double* __restrict__ lpos,
-                           int32_t* __restrict__ counts, double* __restrict__ ind, int32_t* __restrict__ flag) {
+                           int32_t* __restrict__ counts, double* __restrict__ ind, int32_t* __restrict__ flag,
+                           int32_t* __restrict__ rank) {
   pdl_wait();      // the preceding kernel of the stream has completed and its writes are visible
   pdl_trigger();   // the next kernel of the stream may be scheduled into the SMs this grid frees
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -126,9 +128,10 @@ __global__ void k_agg_prep(SurfView S, const double* __restrict__ pos, const dou
     int32_t cid;
     b = cell_of(S, lx, ly, cid) ? cid : ncells;
   }
-  if (b < ncells && S.cempty[b] == 0) {        // a cell with candidates: the row is sorted and row info takes it
+  const int32_t c = b < ncells ? S.ccompact[b] : -1;
+  if (c >= 0) {                                  // a cell with candidates: the row is sorted and row info takes it
     key[i] = b;
-    atomicAdd(&counts[S.ccompact[b]], 1);        // bucketed by the cell's index among the cells with edges
+    rank[i] = atomicAdd(&counts[c], 1);          // bucketed by the cell's index among the cells with edges
     return;
   }
   // no candidates: not a candidate of the body (flag 0), outside the grid (the background), or an edge-free cell, whose
@@ -139,16 +142,13 @@ __global__ void k_agg_prep(SurfView S, const double* __restrict__ pos, const dou
 }
 
 __global__ void k_agg_scatter(SurfView S, const int32_t* __restrict__ key, int64_t n, const int32_t* __restrict__ offs,
-                              int32_t* __restrict__ cursor, int32_t* __restrict__ order) {
+                              const int32_t* __restrict__ rank, int32_t* __restrict__ order) {
   pdl_wait();      // the preceding kernel of the stream has completed and its writes are visible
   pdl_trigger();   // the next kernel of the stream may be scheduled into the SMs this grid frees
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int32_t b = key[i];
-  if (b >= 0) {
-    const int32_t c = S.ccompact[b];
-    order[offs[c] + atomicAdd(&cursor[c], 1)] = (int32_t)i;
-  }
+  if (b >= 0) order[offs[S.ccompact[b]] + rank[i]] = (int32_t)i;
 }
 
 // index of the lowest set bit of the 128-bit mask (m0 low word), cleared; -1 when the mask is empty
@@ -213,7 +213,9 @@ __device__ __forceinline__ double4 ldg4(const double4* p) {
 // eight lanes: cells of small polygons list ten times the mean, and launches of a few hundred thousand rows waited for
 // their rows' serial walk.  The others take short_lanes each: one where the rows fill the GPU, more in launches that leave
 // it idle (info_lanes; the results are integers and do not depend on it).  (B200: 300 001 rows, cells of up to 161 candidates, 22 us against
-// 103 with a lane per row in cell order; 2^20 rows 58 against 66; four lanes for every row 41 and 80.)
+// 103 with a lane per row in cell order; 2^20 rows 58 against 66; four lanes for every row 41 and 80.)  Bound by the latency
+// of the candidates' records, at 24 warps per SM: with each record loaded one test ahead 51 us against 62 (2^20 rows,
+// 350 000 of them with candidates) and 19 against 22.
 constexpr int kListLanes = 8;
 constexpr int kInfoWarps = kThreads / 32;
 
@@ -260,8 +262,11 @@ __global__ void __launch_bounds__(kThreads, 6) k_agg_rowinfo(SurfView S, const d
       const double ry = __dadd_rn(S.lo_y, __dmul_rn(__dadd_rn((double)cy, 0.5), S.cell));
       degenerate = S.cok[b] == 0;
       const int k0 = S.cstart[b], k1 = S.cstart[b + 1];
+      // (the next record is loaded ahead of this one's tests)
+      double4 next = k0 + sub < k1 ? ldg4(S.crec + k0 + sub) : double4{};
       for (int k = k0 + sub; k < k1; k += G) {
-        const double4 e = ldg4(S.crec + k);
+        const double4 e = next;
+        if (k + G < k1) next = ldg4(S.crec + k + G);
         if (seg_within_fast(lx, ly, e.x, e.y, e.z, e.w, h)) {
           ++cnt;
           const int r = k - k0;
@@ -297,9 +302,6 @@ __global__ void __launch_bounds__(kThreads, 6) k_agg_rowinfo(SurfView S, const d
     const unsigned peers = __match_any_sync(0xffffffffu, ckey);
     if (ckey >= 0 && lane == __ffs(peers) - 1) atomicAdd(&s_hist[ckey], __popc(peers));
   }
-  // the positions past the sorted rows hold no row
-  for (int64_t j = nrows + blockIdx.x * (int64_t)kThreads + threadIdx.x; j < n; j += (int64_t)gridDim.x * kThreads)
-    rkey[j] = kKeys - 1;
   // one global add per key the block has: a global atomic per warp and key would serialise on the few hot keys of
   // millions of rows
   __syncthreads();
@@ -1425,80 +1427,95 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_block(const int32_t* __re
   }
 }
 
-// rows with pairs into `work`, grouped by count key (decreasing pair count): the prefix of the key histogram per
-// block, then warp-aggregated cursor atomics (the order inside a key group is arbitrary; every row's result is
-// independent of it)
-__global__ void k_key_scatter(SurfView S, const int32_t* __restrict__ rkey, int64_t n, const int32_t* __restrict__ khist,
-                              int32_t* __restrict__ kcur, const int32_t* __restrict__ order,
-                              int32_t* __restrict__ bucket, const double* __restrict__ lpos,
-                              const double* __restrict__ sup, const uint64_t* __restrict__ mask,
-                              WorkRec* __restrict__ wrec, int32_t* __restrict__ nwork) {
+// rows with pairs into `wrec`, grouped by count key (decreasing pair count): the prefix of the key histogram per block, the
+// rows' ranks among the block's rows of their key, one global cursor add per key the block has (the order inside a key group
+// is arbitrary; every row's result is independent of it).  A block takes kScatterRows sorted rows and returns at once where
+// there are none; what a record holds is loaded before the cursor adds are waited for.  Bound by those loads and the cursor
+// adds on a few hot keys: 2^20 rows 18 us, against 24 with a row a thread, blocks for all rows and the loads after the adds.
+constexpr int kScatterRows = 2 * kThreads;
+
+__global__ void __launch_bounds__(kThreads) k_key_scatter(SurfView S, const int32_t* __restrict__ rkey,
+                                                          const int32_t* __restrict__ offs,
+                                                          const int32_t* __restrict__ khist, int32_t* __restrict__ kcur,
+                                                          const int32_t* __restrict__ order, int32_t* __restrict__ bucket,
+                                                          const double* __restrict__ lpos, const double* __restrict__ sup,
+                                                          const uint64_t* __restrict__ mask, WorkRec* __restrict__ wrec,
+                                                          int32_t* __restrict__ nwork) {
   pdl_wait();      // the preceding kernel of the stream has completed and its writes are visible
   pdl_trigger();   // the next kernel of the stream may be scheduled into the SMs this grid frees
-  constexpr int kWork = kKeys - 1;                                  // keys of rows with pairs: 0 .. 63
+  constexpr int kWork = kKeys - 1, kItems = kScatterRows / kThreads;  // keys of rows with pairs: 0 .. 63
   static_assert(kWork == 64, "two keys a lane in the prefix scan");
-  __shared__ int32_t s_pre[kWork + 1];                              // exclusive prefix of the key counts
+  __shared__ int32_t s_pre[kWork];                                  // exclusive prefix of the key counts
   __shared__ int32_t s_cnt[kWork];                                  // this block's rows per key, then its base
+  const int64_t nrows = offs[S.nne], j0 = blockIdx.x * (int64_t)kScatterRows + threadIdx.x;
+  if (blockIdx.x > 0 && j0 - threadIdx.x >= nrows) return;
+  const int lane = threadIdx.x & 31;
+  int key[kItems], rank[kItems];
+#pragma unroll
+  for (int q = 0; q < kItems; ++q) {
+    const int64_t j = j0 + q * kThreads;
+    key[q] = j < nrows ? rkey[j] : kWork;
+  }
   if (threadIdx.x < 32) {
     // the prefix of the 64 key counts by one warp: lane l scans keys l and l + 32
-    const int l = threadIdx.x;
-    const int a = khist[l], b = khist[l + 32];
+    const int a = khist[lane], b = khist[lane + 32];
     int sa = a, sb = b;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int ta = __shfl_up_sync(0xffffffffu, sa, o), tb = __shfl_up_sync(0xffffffffu, sb, o);
-      if (l >= o) {
+      if (lane >= o) {
         sa += ta;
         sb += tb;
       }
     }
     const int tot_a = __shfl_sync(0xffffffffu, sa, 31), tot_b = __shfl_sync(0xffffffffu, sb, 31);
-    s_pre[l] = sa - a;
-    s_pre[l + 32] = tot_a + sb - b;
+    s_pre[lane] = sa - a;
+    s_pre[lane + 32] = tot_a + sb - b;
     // (the first key of a shorter row: the prefix up to it counts the long ones)
     constexpr int ka = kWork - kLongPairs, kb = kWork - kLongQuad;
-    if (blockIdx.x == 0 && l == ka % 32) nwork[1] = ka < 32 ? sa - a : tot_a + sb - b;
-    if (blockIdx.x == 0 && l == kb % 32) nwork[2] = kb < 32 ? sa - a : tot_a + sb - b;
-    if (l == 0) {
-      s_pre[kWork] = tot_a + tot_b;
-      if (blockIdx.x == 0) nwork[0] = tot_a + tot_b;                // rows with key < 64
+    if (blockIdx.x == 0 && lane == ka % 32) nwork[1] = ka < 32 ? sa - a : tot_a + sb - b;
+    if (blockIdx.x == 0 && lane == kb % 32) nwork[2] = kb < 32 ? sa - a : tot_a + sb - b;
+    if (blockIdx.x == 0 && lane == 0) nwork[0] = tot_a + tot_b;     // rows with key < 64
+  } else if (threadIdx.x - 32 < 32) {
+    s_cnt[lane] = s_cnt[lane + 32] = 0;
+  }
+  __syncthreads();
+  WorkRec r[kItems];
+#pragma unroll
+  for (int q = 0; q < kItems; ++q) {
+    const unsigned peers = __match_any_sync(0xffffffffu, key[q]);
+    const int leader = __ffs(peers) - 1;
+    rank[q] = 0;
+    if (key[q] < kWork && lane == leader) rank[q] = atomicAdd(&s_cnt[key[q]], __popc(peers));
+    rank[q] = __shfl_sync(0xffffffffu, rank[q], leader) + __popc(peers & ((1u << lane) - 1));
+    if (key[q] < kWork) {
+      const int64_t j = j0 + q * kThreads;
+      const int32_t i = order[j], b = bucket[i];
+      const ulonglong2 mm = reinterpret_cast<const ulonglong2*>(mask)[j];
+      r[q].lx = lpos[2 * i];
+      r[q].ly = lpos[2 * i + 1];
+      r[q].h = sup[i];
+      r[q].row = i;
+      r[q].kb = S.cstart[b];
+      r[q].ke = S.cstart[b + 1];
+      r[q].pad[0] = r[q].pad[1] = r[q].pad[2] = 0;
+      r[q].m0 = mm.x;
+      r[q].m1 = mm.y;
     }
   }
-  for (int k = threadIdx.x; k < kWork; k += kThreads) s_cnt[k] = 0;
   __syncthreads();
-  const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int key = j < n ? rkey[j] : -1;
-  const bool mine = key >= 0 && key < kWork;
-  // the row's rank among the block's rows of its key (warp-aggregated shared atomics), then one global cursor add
-  // per key the block has: the block's base in that key's range
-  const unsigned peers = __match_any_sync(0xffffffffu, mine ? key : -1);
-  const int lane = threadIdx.x & 31;
-  const int leader = __ffs(peers) - 1;
-  int rank = 0;
-  if (mine && lane == leader) rank = atomicAdd(&s_cnt[key], __popc(peers));
-  rank = __shfl_sync(0xffffffffu, rank, leader) + __popc(peers & ((1u << lane) - 1));
+  if (threadIdx.x < kWork) {
+    const int c = s_cnt[threadIdx.x];
+    if (c) s_cnt[threadIdx.x] = s_pre[threadIdx.x] + atomicAdd(&kcur[threadIdx.x], c);
+  }
   __syncthreads();
-  for (int k = threadIdx.x; k < kWork; k += kThreads)
-    if (s_cnt[k]) s_cnt[k] = atomicAdd(&kcur[k], s_cnt[k]);
-  __syncthreads();
-  if (mine) {
-    // gather the row's record once here, so the evaluations read one coalesced record per work row
-    const int32_t i = order[j];
-    const int32_t b = bucket[i];
-    const ulonglong2 mm = reinterpret_cast<const ulonglong2*>(mask)[j];
-    WorkRec r;
-    r.lx = lpos[2 * i];
-    r.ly = lpos[2 * i + 1];
-    r.h = sup[i];
-    r.row = i;
-    r.kb = S.cstart[b];
-    r.ke = S.cstart[b + 1];
-    r.pad[0] = r.pad[1] = r.pad[2] = 0;
-    r.m0 = mm.x;
-    r.m1 = mm.y;
-    const int32_t slot = s_pre[key] + s_cnt[key] + rank;
-    wrec[slot] = r;
-    bucket[i] = slot;            // from here on a work row's key is its work slot (read by the staged expansion)
+#pragma unroll
+  for (int q = 0; q < kItems; ++q) {
+    if (key[q] < kWork) {
+      const int32_t slot = s_cnt[key[q]] + rank[q];
+      wrec[slot] = r[q];
+      bucket[r[q].row] = slot;   // from here on a work row's key is its work slot (read by the staged expansion)
+    }
   }
 }
 
@@ -1706,7 +1723,8 @@ static cudaError_t launch_dep(void (*k)(P...), unsigned grid, unsigned block, si
 
 // lanes per row of a short list, by the launch's lanes in waves of the row-info kernel (6 CTAs on 148 SMs; a third of the
 // rows of a domain are in cells with edges).  B200, one lane against the choice: 4096 rows of a 256-gon (30 candidates
-// each) 17.3 against 8.0 us, 2^18 rows 26 against 16, 300 001 rows 31 against 22; 2^20 rows 58 with one, 74 with two.
+// each) 17.3 against 8.0 us, 2^18 rows 26 against 16, 300 001 rows 31 against 22; 2^20 rows 58 with one, 74 with two (each
+// before the record's load went one test ahead).
 static int info_lanes(int64_t n) {
   const int64_t wave = (int64_t)148 * 6 * kThreads;
   return n * 8 <= 4 * wave ? 8 : (n * 4 <= 10 * wave ? 4 : (n * 2 <= 10 * wave ? 2 : 1));
@@ -1715,20 +1733,20 @@ static int info_lanes(int64_t n) {
 static int sort_rows(const Surface* s, const double* pos, const double* sup, const int32_t* allowed, int64_t n,
                      const double* pose, const double* obb, int unbounded, const Workspace& w, cudaStream_t st) {
   const int64_t nbk = (int64_t)s->n_nonempty + 2;   // buckets: the cells with edges
-  WSB_CUDA(cudaMemsetAsync(w.counts, 0, sizeof(int32_t) * (2 * nbk + 1), st));
+  WSB_CUDA(cudaMemsetAsync(w.counts, 0, sizeof(int32_t) * (nbk + 1), st));
   WSB_CUDA(cudaMemsetAsync(w.khist, 0, sizeof(int32_t) * 2 * kKeys, st));
   const SurfView v = view_of(s);
   const unsigned grid = (unsigned)((n + kThreads - 1) / kThreads);
   k_agg_prep<<<grid, kThreads, 0, st>>>(v, pos, sup, allowed, n, pose, make_double4(obb[0], obb[1], obb[2], obb[3]),
-                                        unbounded, w.key, w.lpos, w.counts, w.ind, w.flag);
+                                        unbounded, w.key, w.lpos, w.counts, w.ind, w.flag, w.rkey);
   WSB_CUDA(launch_dep(k_scan_block, 1, kScanThreads, 0, st, (const int32_t*)w.counts, w.offs, nbk + 1));
   WSB_CUDA(launch_dep(k_agg_scatter, grid, kThreads, 0, st, v, (const int32_t*)w.key, n, (const int32_t*)w.offs,
-                      w.cursor, w.order));
+                      (const int32_t*)w.rkey, w.order));
   const int lanes = info_lanes(n);
   WSB_CUDA(launch_dep(k_agg_rowinfo, (unsigned)((n * lanes + kThreads - 1) / kThreads), kThreads, 0, st, v, sup, (const int32_t*)w.key, (const double*)w.lpos,
                       (const int32_t*)w.offs, (const int32_t*)w.order, n, w.ind, w.flag, w.rkey, w.mask, w.khist, lanes));
-  WSB_CUDA(launch_dep(k_key_scatter, grid, kThreads, 0, st, v, (const int32_t*)w.rkey, n, (const int32_t*)w.khist,
-                      w.kcur, (const int32_t*)w.order, w.key, (const double*)w.lpos, sup, (const uint64_t*)w.mask,
+  WSB_CUDA(launch_dep(k_key_scatter, (unsigned)((n + kScatterRows - 1) / kScatterRows), kThreads, 0, st, v,
+                      (const int32_t*)w.rkey, (const int32_t*)w.offs, (const int32_t*)w.khist, w.kcur, (const int32_t*)w.order, w.key, (const double*)w.lpos, sup, (const uint64_t*)w.mask,
                       w.wrec, w.nwork));
   WSB_CUDA(cudaGetLastError());
   return WSB_OK;
