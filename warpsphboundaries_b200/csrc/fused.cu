@@ -1043,42 +1043,32 @@ __global__ void __launch_bounds__(kThreads, pack_min_blocks(Pack::kN) < 5 ? pack
   }
 }
 
-// Staged expansion: one thread per row, consecutive rows in consecutive threads, so every output array is written in
-// full coalesced sectors -- a work row's outputs from its staged channel sums (key[i] is its work slot), any other row
-// the indicator times the whole-plane channels.  A work row's outputs, every kernel of the pack, from its staged sums
-// (already loaded: a[kernel * 12 + c]).
+// Staged expansion: one thread per row and kernel, consecutive rows in consecutive threads, so every output array is
+// written in full coalesced sectors -- a work row's outputs from its staged channel sums (key[i] is its work slot), any
+// other row the indicator times the whole-plane channels.  Kernel `which` of the pack, its sums already loaded.
 template <class Pack, int K, int VEC>
-__device__ __forceinline__ void pack_expand_row(const double* a, int64_t i, double w, double h, const double* pose,
-                                                bool assign, const PackOut& o) {
+__device__ __forceinline__ void pack_expand_row(int which, double acc[12], int64_t i, double w, double h,
+                                                const double* pose, bool assign, const PackOut& o) {
   if constexpr (K < Pack::kN) {
-    using KT = typename Pack::template Kern<K>;
-    double acc[12];
-#pragma unroll
-    for (int c = 0; c < 12; ++c) acc[c] = a[K * 12 + c];
-    if constexpr (KT::kQuad)
-      finish_row_quad<VEC>(acc, h, pose, i, assign, o.lam[K], o.G[K], o.cov[K], o.m1[K], o.m2[K]);
-    else
-      finish_row<VEC>(acc, w, KT::kMass, KT::kPlane2, h, pose, i, assign, o.lam[K], o.G[K], o.cov[K], o.m1[K],
-                      o.m2[K]);
-    pack_expand_row<Pack, K + 1, VEC>(a, i, w, h, pose, assign, o);
+    if (which == K) {
+      using KT = typename Pack::template Kern<K>;
+      if constexpr (KT::kQuad)
+        finish_row_quad<VEC>(acc, h, pose, i, assign, o.lam[K], o.G[K], o.cov[K], o.m1[K], o.m2[K]);
+      else
+        finish_row<VEC>(acc, w, KT::kMass, KT::kPlane2, h, pose, i, assign, o.lam[K], o.G[K], o.cov[K], o.m1[K],
+                        o.m2[K]);
+    } else {
+      pack_expand_row<Pack, K + 1, VEC>(which, acc, i, w, h, pose, assign, o);
+    }
   }
 }
 
-// a work row's staged sums, every kernel: 3 Pack::kN 32-byte loads issued together (a row's slot is 96 bytes a
-// kernel, 32-byte aligned: each load reads one whole sector), so their latencies overlap instead of each kernel's
-// loads following the previous kernel's stores (measured on B200, four-kernel pack on the 2^20-particle scene: the
-// expansion from 148 to 140 us)
-template <class Pack>
-__device__ __forceinline__ void load_staged(const double* src, double* a) {
-#pragma unroll
-  for (int c = 0; c < Pack::kN * 3; ++c) ld4_nc(src + 4 * c, a[4 * c], a[4 * c + 1], a[4 * c + 2], a[4 * c + 3]);
-}
-
 // VEC (write_outputs): 2 when G / m1 are 16-byte and cov / m2 32-byte aligned, so every store of a warp writes whole
-// 32-byte sectors (no read-modify-write of partly written sectors); 1 when all are 16-byte aligned; 0 otherwise
-// (121 registers, 4 CTAs per SM: capping the registers at 5 / 6 / 8 CTAs measured 0.340 / 0.356 / 0.390 ms for the
-// grouped pass on the 2^20-particle scene against 0.306 ms -- the spilled staged sums cost more than the occupancy
-// gains)
+// 32-byte sectors (no read-modify-write of partly written sectors); 1 when all are 16-byte aligned; 0 otherwise.
+// The kernels of a pack are neighbouring blocks, so a row's flag, indicator, slot and support come from L2 after the first,
+// and a thread holds one kernel's sums.  Bound by the output stores: four kernels of 2^20 rows (436 MB of outputs, 70 MB of
+// staged sums) 111 us, 4.6 TB/s, against 114 with all kernels in a thread (121 registers) and 122 with one kernel's blocks
+// after the other's; three kernels of 300 001 rows 22.5 us against 25.7.
 template <class Pack, int VEC>
 __global__ void __launch_bounds__(kThreads) k_agg_expand(const double* __restrict__ sup,
                                                          const int32_t* __restrict__ flag,
@@ -1089,18 +1079,23 @@ __global__ void __launch_bounds__(kThreads) k_agg_expand(const double* __restric
                                                          const PackOut out) {
   pdl_wait();      // the preceding kernel of the stream has completed and its writes are visible
   pdl_trigger();   // the next kernel of the stream may be scheduled into the SMs this grid frees
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t i = blockIdx.x / Pack::kN * (int64_t)blockDim.x + threadIdx.x;
+  const int which = blockIdx.x % Pack::kN;
   if (i >= n) return;
   const int32_t f = flag[i];
   if (f == 0 && !assign) return;                                   // not a candidate, outputs added to: nothing
   // one code path for every row, so a warp issues each of its output stores once (work and constant rows of a warp
   // in separate branches would store every sector twice with partial masks): a constant row is a work row with zero
   // sums and the same finish (the indicator terms, w = 0 for a non-candidate)
-  double a[Pack::kN * 12];
+  double a[12];
 #pragma unroll
-  for (int c = 0; c < Pack::kN * 12; ++c) a[c] = 0.0;
-  if (f == 2) load_staged<Pack>(wacc + (int64_t)slot[i] * (Pack::kN * 12), a);
-  pack_expand_row<Pack, 0, VEC>(a, i, f != 0 ? ind[i] : 0.0, sup[i], pose, assign, out);
+  for (int c = 0; c < 12; ++c) a[c] = 0.0;
+  if (f == 2) {
+    const double* src = wacc + ((int64_t)slot[i] * Pack::kN + which) * 12;   // 96 bytes, 32-byte aligned: whole sectors
+#pragma unroll
+    for (int c = 0; c < 3; ++c) ld4_nc(src + 4 * c, a[4 * c], a[4 * c + 1], a[4 * c + 2], a[4 * c + 3]);
+  }
+  pack_expand_row<Pack, 0, VEC>(which, a, i, f != 0 ? ind[i] : 0.0, sup[i], pose, assign, out);
 }
 
 static int pack_out_vec(const PackOut& o, int n) {
@@ -1153,13 +1148,13 @@ static int launch_pack(const SurfView& v, const double* sup, const Workspace& w,
   if (staged) {
     const int vec = pack_out_vec(out, Pack::kN);
     if (vec == 2)
-      WSB_CUDA(launch_dep(k_agg_expand<Pack, 2>, rows, kThreads, 0, st, sup, (const int32_t*)w.flag,
+      WSB_CUDA(launch_dep(k_agg_expand<Pack, 2>, rows * Pack::kN, kThreads, 0, st, sup, (const int32_t*)w.flag,
                           (const double*)w.ind, (const int32_t*)w.key, (const double*)w.wacc, n, pose, assign, out));
     else if (vec == 1)
-      WSB_CUDA(launch_dep(k_agg_expand<Pack, 1>, rows, kThreads, 0, st, sup, (const int32_t*)w.flag,
+      WSB_CUDA(launch_dep(k_agg_expand<Pack, 1>, rows * Pack::kN, kThreads, 0, st, sup, (const int32_t*)w.flag,
                           (const double*)w.ind, (const int32_t*)w.key, (const double*)w.wacc, n, pose, assign, out));
     else
-      WSB_CUDA(launch_dep(k_agg_expand<Pack, 0>, rows, kThreads, 0, st, sup, (const int32_t*)w.flag,
+      WSB_CUDA(launch_dep(k_agg_expand<Pack, 0>, rows * Pack::kN, kThreads, 0, st, sup, (const int32_t*)w.flag,
                           (const double*)w.ind, (const int32_t*)w.key, (const double*)w.wacc, n, pose, assign, out));
   }
   return WSB_OK;
