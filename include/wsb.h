@@ -60,7 +60,10 @@ enum { WSB_RADIAL_PLANE = 0, WSB_RADIAL_SPHERE = 1 };
 
 /* output selection bits of wsb_aggregate */
 enum { WSB_OUT_LAM = 1, WSB_OUT_G = 2, WSB_OUT_COV = 4, WSB_OUT_M1 = 8, WSB_OUT_M2 = 16, WSB_OUT_ALL = 31,
-       WSB_OUT_ASSIGN = 32 /* overwrite the outputs (rows that are not candidates get zeros) instead of adding */ };
+       WSB_OUT_ASSIGN = 32 /* overwrite the outputs (rows that are not candidates get zeros) instead of adding */,
+       WSB_WS_SCRATCH = 64 /* wsb_aggregate, wsb_aggregate_groups: nothing is read from the workspace after the call; it
+                            * need not be left as wsb_aggregate_prepare leaves it, and launches of few rows take one
+                            * kernel (the same results) */ };
 
 typedef struct wsb_surface wsb_surface;
 
@@ -164,7 +167,7 @@ int wsb_aggregate_evaluate(const wsb_surface* s, int kernel, int precision, cons
  * {w2, w4, w6}, {w2, cone, lw2}, {w4, cone, lw4}, {w2, cone}, {w4, cone} that the groups contain (each kernel once,
  * any order) is evaluated in one pass over the neighbour pairs, sharing each pair's chord, special functions and
  * monomial integrals between kernel blocks of equal support radius; every other group runs its own pass.
- * At most WSB_MAX_GROUPS groups.  _groups = _prepare + _evaluate_groups. */
+ * At most WSB_MAX_GROUPS groups.  _groups = _prepare + _evaluate_groups (without WSB_WS_SCRATCH in out_mask). */
 enum { WSB_MAX_GROUPS = 8 };
 int wsb_aggregate_evaluate_groups(const wsb_surface* s, int n_groups, const int32_t* kernels, int precision,
                                   const double* sup, int64_t n, const double* pose, int out_mask, double* const* lam,

@@ -39,7 +39,7 @@ class BoundaryMoments(torch.autograd.Function):
         pose = body.pose_tensor(dev)
         obb, unbounded = body.broadphase()
         check(lib.wsb_aggregate(ns.handle, kid, _PREC[precision], ptr(posc), ptr(supc), None, N, ptr(pose), obb,
-                                unbounded, _lib.OUT_ALL | _lib.OUT_ASSIGN, ptr(lam), ptr(G), ptr(Cov), ptr(m1), ptr(m2),
+                                unbounded, _lib.OUT_ALL | _lib.OUT_ASSIGN | _lib.WS_SCRATCH, ptr(lam), ptr(G), ptr(Cov), ptr(m1), ptr(m2),
                                 ptr(ws), need, None, _stream()), "wsb_aggregate")
         ctx.save_for_backward(posc, supc)
         ctx.set_materialize_grads(False)       # an output the loss does not use has no gradient tensor to fill and test

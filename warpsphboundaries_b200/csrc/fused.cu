@@ -1960,11 +1960,12 @@ extern "C" int wsb_aggregate_evaluate_groups(const wsb_surface* s, int n_groups,
                          workspace_bytes, nullptr, stream);
 }
 
-// the front half of an aggregate: nothing where the rows take the one-launch route, else the sorted rows; the checks of
-// wsb_aggregate_prepare in both
-static int front(const wsb_surface* s_, int n_groups, const RowArgs& a, void* workspace, size_t workspace_bytes,
+// the front half of an aggregate: nothing where the rows take the one-launch route (the caller has the workspace as
+// scratch), else the sorted rows; the checks of wsb_aggregate_prepare in both
+static int front(const wsb_surface* s_, int n_groups, const RowArgs& a, int out_mask, void* workspace, size_t workspace_bytes,
                  void* stream, const RowArgs** rows) {
-  *rows = one_launch(reinterpret_cast<const Surface*>(s_), n_groups, a.n) ? &a : nullptr;
+  const bool one = (out_mask & WSB_WS_SCRATCH) != 0 && one_launch(reinterpret_cast<const Surface*>(s_), n_groups, a.n);
+  *rows = one ? &a : nullptr;
   if (!*rows)
     return wsb_aggregate_prepare(s_, a.pos, a.sup, a.allowed, a.n, a.pose, a.obb, a.unbounded, workspace, workspace_bytes,
                                  stream);
@@ -1990,7 +1991,7 @@ extern "C" int wsb_aggregate(const wsb_surface* s_, int kernel, int precision, c
     WSB_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t), (cudaStream_t)stream));
   }
   const RowArgs args{pos, sup, allowed, n, pose, obb, unbounded}, *rows = nullptr;
-  rc = front(s_, 1, args, workspace, workspace_bytes, stream, &rows);
+  rc = front(s_, 1, args, out_mask, workspace, workspace_bytes, stream, &rows);
   if (rc) return rc;
   return evaluate(s_, kernel, precision, sup, n, pose, out_mask, lam, G, cov, m1, m2, workspace, workspace_bytes, rows,
                   stream);
@@ -2013,7 +2014,7 @@ extern "C" int wsb_aggregate_groups(const wsb_surface* s_, int n_groups, const i
     return fail(WSB_ERR_UNSUPPORTED, "wsb_aggregate_groups: unknown precision mode");
   if (n == 0) return WSB_OK;
   const RowArgs args{pos, sup, allowed, n, pose, obb, unbounded}, *rows = nullptr;
-  rc = front(s_, n_groups, args, workspace, workspace_bytes, stream, &rows);
+  rc = front(s_, n_groups, args, out_mask, workspace, workspace_bytes, stream, &rows);
   if (rc) return rc;
   return evaluate_groups(s_, n_groups, kernels, precision, sup, n, pose, out_mask, lam, G, cov, m1, m2, workspace,
                          workspace_bytes, rows, stream);
@@ -2156,6 +2157,6 @@ extern "C" int wsb_aggregate_noalloc(const wsb_surface* s_, int kernel, int prec
   void* scratch = nullptr;
   rc = noalloc_scratch(s->device, &scratch);
   if (rc) return rc;
-  return wsb_aggregate(s_, kernel, precision, pos, sup, allowed, n, pose, obb, unbounded, out_mask, lam, G, cov, m1, m2,
-                       scratch, kNoAllocScratchBytes, status, stream);
+  return wsb_aggregate(s_, kernel, precision, pos, sup, allowed, n, pose, obb, unbounded, out_mask | WSB_WS_SCRATCH, lam, G,
+                       cov, m1, m2, scratch, kNoAllocScratchBytes, status, stream);
 }

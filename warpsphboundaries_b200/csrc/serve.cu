@@ -147,7 +147,7 @@ static int scene_aggregate(const wsb_scene* sc, int n_groups, const int32_t* ker
       continue;
     }
     for (size_t ri = 0; ri < body.surfaces.size(); ++ri) {
-      const int mode = WSB_OUT_ALL | (ri == 0 ? WSB_OUT_ASSIGN : 0);     // the first surface assigns, the rest add
+      const int mode = WSB_OUT_ALL | WSB_WS_SCRATCH | (ri == 0 ? WSB_OUT_ASSIGN : 0);     // the first surface assigns, the rest add
       const int rc = wsb_aggregate_groups(body.surfaces[ri], n_groups, kernels, precision, pos, sup, allowed, n,
                                           sc->d_pose + 4 * b, body.obb, body.unbounded, mode, ptr[0].data(),
                                           ptr[1].data(), ptr[2].data(), ptr[3].data(), ptr[4].data(), ws, ws_bytes, st);

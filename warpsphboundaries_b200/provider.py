@@ -160,7 +160,7 @@ class FusedWall(WallAggregate):
             p_pose = ptr(body.pose_tensor(self.dev))
             at = {k: [b + bi * step for b, step in base[k]] for k in names}
             for ri, rep in enumerate(body.fused_reps(self.support, self.dev)):
-                mode = _lib.OUT_ALL | (_lib.OUT_ASSIGN if ri == 0 else 0)     # the first representation assigns
+                mode = _lib.OUT_ALL | _lib.WS_SCRATCH | (_lib.OUT_ASSIGN if ri == 0 else 0)     # the first representation assigns
                 if isinstance(rep, DiskArrayRep):
                     nd = rep.native(self.support, self.dev)
                     dws, dneed = nd.workspace(N, stream)
@@ -188,7 +188,7 @@ class FusedWall(WallAggregate):
                     self._group = gi
                     tgt = {k: torch.empty_like(outs[gi][k][bi]) for k in names}
                     check(lib.wsb_aggregate(ns.handle, kid, prec, p_pos, p_sup, p_al, N, p_pose, obb, unbounded,
-                                            _lib.OUT_ALL | _lib.OUT_ASSIGN, *[ptr(tgt[k]) for k in names], ptr(ws), need,
+                                            _lib.OUT_ALL | _lib.OUT_ASSIGN | _lib.WS_SCRATCH, *[ptr(tgt[k]) for k in names], ptr(ws), need,
                                             None, st), "wsb_aggregate")
                     self._conditioned(body, bi, ri, rep, pos, sup, al, kid, pose, tgt, outs[gi])
 

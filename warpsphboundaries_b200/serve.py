@@ -364,7 +364,7 @@ class BoundaryServer:
 
     # ------------------------------------------------------------------ the loop
     # device seconds a row, by request class (measured on B200 at large batches: 2-D one kernel with prepare, the
-    # adjoint about as much again; closed surfaces of the 3-D configuration; sphere rows), for the lane choice only
+    # adjoint about as much again; closed surfaces with every row near the surface; sphere rows), for the lane choice only
     _ROW_COST = {"2d": 2.5e-10, "2d_grad": 5e-10, "3d_surface": 6.5e-9, "3d_spheres": 2.5e-10}
 
     def _cost(self, r):
@@ -591,7 +591,7 @@ class BoundaryServer:
         for bi, (pose, obb, unbounded, reps) in enumerate(plan):
             o = [ptr(outs[k][bi]) for k in OUT_KEYS]
             for ri, ns in enumerate(reps):
-                mode = _lib.OUT_ALL | (_lib.OUT_ASSIGN if ri == 0 else 0)
+                mode = _lib.OUT_ALL | _lib.WS_SCRATCH | (_lib.OUT_ASSIGN if ri == 0 else 0)
                 check(lib.wsb_aggregate(ns.handle, kid, prec, ptr(pos), ptr(sup), ptr(allowed), n, ptr(pose), obb,
                                         unbounded, mode, *o, ptr(ws), ws.numel(), None, st), "wsb_aggregate")
 
