@@ -794,15 +794,16 @@ class Body:
         return cache[key]
 
     def pose_tensor(self, device):
-        """(cx, cy, cos, sin) on the device, cached while the pose is unchanged."""
-        key = (self.center.data_ptr(), self.center._version, float(self.angle), device)
+        """(cx, cy, cos, sin) on the device, cached while the pose is unchanged (the centre's tensor is held, so that another
+        one is never taken for it)."""
+        centre, key = self.center, (self.center._version, float(self.angle), device)
         hit = self.__dict__.get("_poseCache")
-        if hit is None or hit[0] != key:
+        if hit is None or hit[0] is not centre or hit[1] != key:
             c, s = self.pose._cs()
-            t = torch.cat([self.center.to(device, F64).reshape(2), torch.tensor([c, s], dtype=F64, device=device)])
-            hit = (key, t)
+            t = torch.cat([centre.to(device, F64).reshape(2), torch.tensor([c, s], dtype=F64, device=device)])
+            hit = (centre, key, t)
             self._poseCache = hit
-        return hit[1]
+        return hit[2]
 
     def state_row(self):
         """(cx, cy, cos, sin, vx, vy, omega, ax, ay, alpha) of the kinematics kernel."""
