@@ -332,11 +332,11 @@ def serving_run(n_requests, dev, pair_density, seed=0, start_load=0.9, max_strea
     # burst capacity; while a stream leaves the device outside that window, the next one's rate is scaled by the busy
     # fraction towards 84 % (at most 6x a step, max_streams streams in all).  The burst's capacity is only a starting point: with several streams and
     # the host issuing one batch at a time it understates what the device absorbs under a stream.
-    # Where a higher rate makes the device no busier, the host's launches are the limit: the stream before it, the last that
-    # kept up, is the one reported.
+    # Where a stream ends well after its last arrival with the device below the window, the host's launches are the limit: the
+    # last stream that kept up is the one reported.
     tried = []
     load = start_load
-    kept = None                                                # the stream before: (load, rate, wall, stats, busy)
+    kept = None                                                # the last that kept up: (load, rate, wall, stats)
     for attempt in range(max_streams):
         rate, wall, st = stream(load)
         busy = st.get("gpu_busy") or 0.0
@@ -345,10 +345,12 @@ def serving_run(n_requests, dev, pair_density, seed=0, start_load=0.9, max_strea
                       "host": st.get("host")})
         if 0.8 <= busy <= 0.9:
             break
-        if kept and kept[4] < 0.8 and kept[0] < load and busy < kept[4] + 0.02:
-            load, rate, wall, st, busy = kept
-            break
-        kept = (load, rate, wall, st, busy)
+        if busy < 0.8:
+            if wall <= 1.02 * float(np.sum(unit)) / rate:
+                kept = (load, rate, wall, st)
+            elif kept:
+                load, rate, wall, st = kept
+                break
         if attempt + 1 == max_streams:
             break
         # busy is close to proportional to the arrival rate below saturation; above 90 % the queue grows (an overloaded

@@ -747,12 +747,12 @@ __device__ __forceinline__ void pack_stage(const double* acc_t, int G, bool writ
 // split g, g + G, ... and found by the float-prefiltered predicate.  G = 2, and 8 for the rows of kLongPairs pairs or
 // more (kLongQuad for a quadrature kernel), which come first: two lanes would evaluate some 46 pairs one after the other
 // on small polygons, and launches of a few hundred thousand rows waited for them.  (B200, 300 001 rows of the delta+ groups:
-// 100 -> 37 us; 2^20 rows, w4 109 -> 82 us, four kernels 204 -> 203.  From 16 pairs on: 36 / 87 / 219; from 48: 52 / 81 /
-// 200; w2p5 144 from 16 pairs on, 199 from 32, 247 from 48.)  G follows from the row alone.  Work rows are sorted by pair
-// count, so the lanes of a warp evaluate nearly the same number of closed forms.  The G partial sums are combined by an
-// xor butterfly (the same additions on every lane, commutative, so the result is deterministic and identical on the G
-// lanes).  The channel sums live in shared memory ([kernel][channel][thread]), which keeps the registers for the closed
-// form.
+// 100 -> 37 us; 2^20 rows, w4 110 -> 86 us, four kernels, whose lanes clear and combine 48 sums each, 202 -> 213.  The limit:
+// from 16 pairs on 36 / 87 / 219 where 32 gave 37 / 82 / 203, from 48 on 52 / 81 / 200; w2p5 144 from 16 pairs on, 199 from
+// 32, 247 from 48.)  G follows from the row alone.  Work rows are sorted by pair count, so the lanes of a warp evaluate
+// nearly the same number of closed forms.  The G partial sums are combined by an xor butterfly (the same additions on every
+// lane, commutative, so the result is deterministic and identical on the G lanes).  The channel sums live in shared memory
+// ([kernel][channel][thread]), which keeps the registers for the closed form.
 constexpr int kShortLanes = 2, kLongLanes = 8;
 
 // the pairs of a warp's rows (every lane takes part; lane `sub` of the G that share a row; no row: kb = e1 = 0, an empty
