@@ -78,3 +78,30 @@ def test_short_edges_and_planes_through_the_query(kernel):
         for k in range(len(Q_)):
             ref = _unit(M3.channels(V_, F_, Q_[k], h_[k], kernel), h_[k])
             assert np.abs(_unit(g_[k], h_[k]) - ref).max() <= 1e-9 * (1 + np.abs(ref).max()), k
+
+
+@pytest.mark.parametrize("kernel", ["cubic", "w2", "w4", "w6"])
+def test_a_vertex_just_inside_the_support(kernel):
+    """faces that reach into the support by a vertex only, by 1e-7 to 1e-9 supports, the foot of the query outside them:
+    the edges' angles beyond the support are of order one and cancel to the angle of that depth."""
+    rng = np.random.default_rng(21)
+    apex, axis = np.array([0.1, -0.2, 0.05]), np.array([0.48, 0.6, 0.64])
+    base = np.linalg.svd(axis[None])[2][1:]                      # two directions across the axis
+    ring = [0.2 * (np.cos(t) * base[0] + np.sin(t) * base[1]) for t in (0.3, 2.1, 4.6)]
+    V = np.concatenate([[apex], apex - axis * np.array([[0.25], [0.4], [0.3]]) + ring])
+    Fc = np.array([[0, 1, 2], [0, 2, 3], [0, 3, 1], [1, 3, 2]])
+    if np.dot(np.cross(V[1] - V[0], V[2] - V[0]), V[3] - V[0]) > 0:
+        Fc = Fc[:, ::-1].copy()                                  # outward normals
+    u = axis + rng.uniform(0.3, 1.2, (24, 1)) * _directions(rng, 24, base)
+    u /= np.linalg.norm(u, axis=1, keepdims=True)
+    Q = np.concatenate([apex + (1.0 - depth) * u for depth in (1e-7, 1e-8, 1e-9)])
+    h = np.ones(len(Q))
+    got = _channels(ClosedMesh(V, Fc, 1.0, DEV), Q, h, kernel)
+    for k in range(len(Q)):
+        ref = M3.channels(V, Fc, Q[k], 1.0, kernel)
+        assert np.abs(got[k] - ref).max() <= 1e-10 * (1 + np.abs(ref).max()), k
+
+
+def _directions(rng, n, base):
+    t = rng.uniform(0, 2 * np.pi, n)
+    return np.cos(t)[:, None] * base[0] + np.sin(t)[:, None] * base[1]

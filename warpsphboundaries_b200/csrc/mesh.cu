@@ -362,6 +362,7 @@ __device__ __forceinline__ void face_block(const double* __restrict__ F, const d
   for (int n = 0; n <= B::kLine; ++n) M[n] = 0.0;
   double lam = 0.0, om = 0.0, th = 0.0, s3 = 0.0, ox = 1.0, oy = 0.0;
   float turn = 0.0f;
+  bool beyond = false;                  // some edge has a part beyond R
   const double zz = z * z;
 #pragma unroll 1
   for (int e = 0; e < 3; ++e) {
@@ -381,7 +382,7 @@ __device__ __forceinline__ void face_block(const double* __restrict__ F, const d
     const bool in = s1 > s0;
     // the angle under which the foot of the query sees the part of the edge beyond R: the parts' rotations multiplied
     // (their sum lies in (-pi, pi), with the sign of w), and those of the three edges: one atan2 a face; the float sum
-    // of the edges' angles tells the full turns
+    // of the edges' angles only tells the full turns (it may cancel to 0 where the angle is 1e-7)
     if (w != 0.0 && (!in || lo < s0 || s1 < hi)) {
       const double ww = w * w;
       double x, y;
@@ -398,6 +399,7 @@ __device__ __forceinline__ void face_block(const double* __restrict__ F, const d
       const double m = 1.0 / (fabs(x) + fabs(y));
       x *= m;
       y *= m;
+      beyond = true;
       turn += atan2f((float)y, (float)x);
       const double t0 = ox * x - oy * y;
       oy = ox * y + oy * x;
@@ -465,7 +467,7 @@ __device__ __forceinline__ void face_block(const double* __restrict__ F, const d
         A.kk[k] += mu[i] * (mu[j] * wk + t[j] * hk) + t[i] * (mu[j] * hk);
   }
   double out = 0.0;
-  if (turn != 0.0f) {
+  if (beyond) {
     out = atan2(oy, ox);
     out += kTwoPi * rint((turn - out) * (1.0 / kTwoPi));
   }
