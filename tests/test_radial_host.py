@@ -1,5 +1,7 @@
 """Host logic of the radial family (no GPU): the request contract, argument checks, C-ABI argument errors."""
+import copy
 import ctypes
+import pickle
 
 import numpy as np
 import pytest
@@ -78,3 +80,17 @@ def test_whole_support_constants_match_the_oracle():
         full = np.array([float(x) for x in K._radial_full(name)])
         assert np.abs(full - OR.invariants(-1.5, name)).max() < 1e-10
         assert np.abs(full - OR.invariants(-1.0, name, radius=3.0)).max() < 1e-10
+
+
+@pytest.mark.parametrize("requests", [None, [Request((1, 0, 1)), Request((0, 0, 0), (2,))]])
+def test_evaluator_is_copied_and_pickled(requests):
+    """before and after a launch has formed the C view of its request rows, which stays its own."""
+    ev = RadialEvaluator("sphere", requests, kernel="w4")
+    for used in (False, True):
+        if used:
+            ev._request_rows()
+        for other in (copy.copy(ev), copy.deepcopy(ev), pickle.loads(pickle.dumps(ev))):
+            assert other.kind == "sphere" and other.requests == ev.requests and other.device == ev.device
+            rows = other._request_rows()
+            assert [rows[k] for k in range(other.metadata.size)] == ev.metadata.ravel().tolist()
+            assert ctypes.addressof(rows.contents) == other.metadata.ctypes.data

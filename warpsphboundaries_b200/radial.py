@@ -100,11 +100,23 @@ class RadialEvaluator:
             ids = [i for i, a in enumerate(r.alpha) for _ in range(a)] + list(r.derivative)
             meta.append([sum(r.alpha), *(ids + [0, 0])[:2], len(r.derivative)])
         self.metadata = np.ascontiguousarray(np.array(meta, dtype=np.int32).reshape(-1, 4))
-        self._metadata_ptr = self.metadata.ctypes.data_as(_lib.POINTER(_lib.c_int32))
         self._kind_id = _lib.RADIAL_SPHERE if kind == "sphere" else _lib.RADIAL_PLANE
         self._kernel_id = KERNEL_IDS[kernel]
         self._prec_id = _PRECISIONS[precision]
         self.accuracy_status = "reference 70-digit radial and sphere fixtures pass on the GPU (float64)"
+
+    def _request_rows(self):
+        """the request rows as the library takes them, formed once per array (1-2 us of a small call)."""
+        held = self.__dict__.get("_rows")
+        if held is None or held[0] is not self.metadata:
+            held = (self.metadata, self.metadata.ctypes.data_as(_lib.POINTER(_lib.c_int32)))
+            self._rows = held
+        return held[1]
+
+    def __getstate__(self):
+        state = dict(self.__dict__)
+        state.pop("_rows", None)               # a C pointer can be neither copied nor pickled
+        return state
 
     def prepare(self, distances, normals, supports, *, radii=None):
         """validated, frozen device arrays of one batch (radial.py:151-185)."""
@@ -173,7 +185,7 @@ class RadialBatch:
         ev = self.evaluator
         check(lib.wsb_radial_channels(ev._kind_id, ev._kernel_id, ev._prec_id, ptr(self.distances),
                                       ptr(self.radii) if ev.kind == "sphere" else None, ptr(self.normals),
-                                      ptr(self.supports), self.count, ev._metadata_ptr, len(ev.requests),
+                                      ptr(self.supports), self.count, ev._request_rows(), len(ev.requests),
                                       ptr(self.values), ptr(self.work), ptr(self.status),
                                       _lib.c_void_p(stream.cuda_stream)), "wsb_radial_channels")
 
