@@ -145,6 +145,12 @@ def ptrs(tensors):
     return (c_void_p * len(tensors))(*[None if t is None else t.data_ptr() for t in tensors])
 
 
+class Double4(ctypes.Array):
+    """four C doubles (a named type: the anonymous c_double * 4 cannot be pickled)."""
+    _type_ = c_double
+    _length_ = 4
+
+
 def int32s(values):
     """a host int32 array."""
     return (c_int32 * len(values))(*values)

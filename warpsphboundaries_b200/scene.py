@@ -765,7 +765,7 @@ class Body:
         box = self.obb()
         c = self.__dict__.get("_boxCache")
         if c is None or c[0] != box:
-            c = (box, (ctypes.c_double * 4)(*box))
+            c = (box, _lib.Double4(*box))
             self._boxCache = c
         return c[1], int(self.unbounded())
 
