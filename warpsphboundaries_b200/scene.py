@@ -14,6 +14,7 @@ from typing import List, Optional
 
 import numpy as np
 import torch
+from torch.autograd.forward_ad import unpack_dual
 
 from . import _lib
 from ._lib import check, lib, ptr
@@ -970,9 +971,19 @@ class Scene:
                 if not isinstance(rep, SurfaceRep):
                     continue
                 ns = rep.native(supportMax, self.device) if supportMax is not None else rep._default_native(self.device)
+                # the kernel writes by address: never into a tensor whose derivative by the points is tracked (an earlier
+                # representation's closed form); the rows the surface takes have no derivative
+                d, n = best, normal
+                tracked = d.requires_grad or n.requires_grad or unpack_dual(d).tangent is not None
+                if tracked:
+                    d, n = d.detach().clone(), n.detach().clone()
                 check(lib.wsb_body_distance(ns.handle, ptr(pts), M, ptr(bd.pose_tensor(self.device)),
-                                            float(supportMax) if supportMax else 0.0, int(first), bi, ptr(best),
-                                            ptr(normal), ptr(bidx), _stream()), "wsb_body_distance")
+                                            float(supportMax) if supportMax else 0.0, int(first), bi, ptr(d), ptr(n),
+                                            ptr(bidx), _stream()), "wsb_body_distance")
+                if tracked:
+                    better = d < best
+                    best = torch.where(better, d, best)
+                    normal = torch.where(better[:, None], n, normal)
                 first = False
         hit = torch.full((M,), not first, dtype=torch.bool, device=self.device)
         if first:
