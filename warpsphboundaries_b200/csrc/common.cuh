@@ -6,7 +6,9 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <string>
+#include <vector>
 
 #include "../../include/wsb.h"
 #include "kernel_tables.h"
@@ -64,13 +66,13 @@ struct Surface {
   int32_t* bitems = nullptr;    // [n_bitems]
   double4* erec = nullptr;      // [n_edges] (ax, ay, bx, by) by edge id
   double4* brec = nullptr;      // [n_bitems] the records of the y-bin items, bin order
-  // bounding-box tree over the edges (signed distance), one allocation: node boxes by level, edge records and ids in
-  // tree order
-  double4* tbox = nullptr;
-  double4* trec = nullptr;      // [n_edges]
-  int32_t* tid = nullptr;       // [n_edges]
-  // host copies (tests, signed distance set-up)
-  std::string err;
+  // bounding-box tree over the edges, built by the first signed distance (edge_tree_of) from the host's edge records; one
+  // device allocation: node boxes by level, edge records and ids in tree order
+  mutable std::mutex tree_mu;
+  mutable std::vector<double4> herec;            // [n_edges] until the tree is built
+  mutable double4* tbox = nullptr;               // guarded by tree_mu, never changed once set
+  mutable const double4* trec = nullptr;         // [n_edges]
+  mutable const int32_t* tid = nullptr;          // [n_edges]
 };
 
 // ----------------------------------------------------------------------------------------------- rounding-exact helpers

@@ -3,6 +3,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <cstring>
+#include <new>
 #include <vector>
 
 #include "common.cuh"
@@ -235,7 +237,7 @@ __global__ void __launch_bounds__(kDistThreads, 16) k_body_distance(SurfView S, 
   if (bidx) bidx[i] = better ? body : -1;
 }
 
-TreeView tree_of(const Surface* s) {
+TreeView view_of_tree(const Surface* s) {
   TreeView T{};
   T.box = s->tbox;
   T.rec = s->trec;
@@ -252,8 +254,6 @@ TreeView tree_of(const Surface* s) {
   }
   return T;
 }
-
-}  // namespace
 
 // the tree's host arrays: boxes by level, edge ids in Morton order (11 bits an axis over the midpoints'
 // box, finer than the leaves need)
@@ -334,6 +334,48 @@ void edge_tree(const std::vector<double4>& erec, std::vector<double4>& box, std:
   }
 }
 
+// The tree of a surface, built by the first signed distance asked of it: 0.26 ms on the host for 17 400 edges, which the
+// surfaces of callers that ask for none (aggregates, adjoints, a geometry rebuilt each step) do not pay.  Safe from any
+// thread; a stream that is being captured is not touched (a stream of its own, host-synchronised before the tree is
+// published), and allocations during another stream's capture are permitted for the length of the call.
+int edge_tree_of(const Surface* s, TreeView* out) try {
+  std::lock_guard<std::mutex> lock(s->tree_mu);
+  if (!s->tbox) {
+    std::vector<double4> box;
+    std::vector<int32_t> id;
+    edge_tree(s->herec, box, id);
+    const size_t nb = box.size(), n = (size_t)s->n_edges;
+    std::vector<double4> all(nb + n + (n * sizeof(int32_t) + sizeof(double4) - 1) / sizeof(double4));
+    std::copy(box.begin(), box.end(), all.begin());
+    for (size_t i = 0; i < n; ++i) all[nb + i] = s->herec[(size_t)id[i]];
+    std::memcpy(all.data() + nb + n, id.data(), n * sizeof(int32_t));
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    WSB_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    double4* dev = nullptr;
+    cudaStream_t st = nullptr;
+    cudaError_t e = cudaMalloc((void**)&dev, all.size() * sizeof(double4));
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dev, all.data(), all.size() * sizeof(double4), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (st) cudaStreamDestroy(st);
+    if (e != cudaSuccess && dev) cudaFree(dev);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) {
+      cudaGetLastError();                              // (an allocation that failed is not the next launch's error)
+      return cuda_fail(e, "signed distance: edge tree");
+    }
+    s->trec = dev + nb;
+    s->tid = reinterpret_cast<const int32_t*>(dev + nb + n);
+    s->tbox = dev;
+    std::vector<double4>().swap(s->herec);
+  }
+  *out = view_of_tree(s);
+  return WSB_OK;
+} catch (const std::bad_alloc&) {
+  return fail(WSB_ERR_DEVICE, "signed distance: no host memory for the edge tree");
+}
+
+}  // namespace
 }  // namespace wsb
 
 using namespace wsb;
@@ -346,8 +388,10 @@ extern "C" int wsb_signed_distance(const wsb_surface* s_, const double* lpos, in
   if (m == 0) return WSB_OK;
   if (!lpos || !d || !cp || !n_loc || !edge) return fail(WSB_ERR_ARG, "wsb_signed_distance: NULL array");
   WSB_CUDA(cudaSetDevice(s->device));
+  TreeView tree;
+  if (const int rc = edge_tree_of(s, &tree)) return rc;
   k_signed_distance<<<(unsigned)((m * kGroup + kDistThreads - 1) / kDistThreads), kDistThreads, 0, (cudaStream_t)stream>>>(
-      view_of(s), tree_of(s), lpos, m, norm_support, d, cp, n_loc, edge);
+      view_of(s), tree, lpos, m, norm_support, d, cp, n_loc, edge);
   WSB_CUDA(cudaGetLastError());
   return WSB_OK;
 }
@@ -361,8 +405,10 @@ extern "C" int wsb_body_distance(const wsb_surface* s_, const double* pos, int64
   if (m == 0) return WSB_OK;
   if (!pos || !pose || !best || !normal) return fail(WSB_ERR_ARG, "wsb_body_distance: NULL array");
   WSB_CUDA(cudaSetDevice(s->device));
+  TreeView tree;
+  if (const int rc = edge_tree_of(s, &tree)) return rc;
   k_body_distance<<<(unsigned)((m * kGroup + kDistThreads - 1) / kDistThreads), kDistThreads, 0, (cudaStream_t)stream>>>(
-      view_of(s), tree_of(s), pos, m, pose, norm_support, first, body, best, normal, body_index);
+      view_of(s), tree, pos, m, pose, norm_support, first, body, best, normal, body_index);
   WSB_CUDA(cudaGetLastError());
   return WSB_OK;
 }

@@ -10,9 +10,6 @@
 
 namespace wsb {
 
-// distance.cu
-void edge_tree(const std::vector<double4>& erec, std::vector<double4>& box, std::vector<int32_t>& id);
-
 static thread_local std::string g_last_error;
 
 void set_error(const std::string& msg) { g_last_error = msg; }
@@ -113,17 +110,6 @@ static int upload(T** dst, const T* src, int64_t n) {
 template <typename T>
 static int upload(T** dst, const std::vector<T>& src) {
   return upload(dst, src.data(), (int64_t)src.size());
-}
-
-// the edge tree in one allocation: boxes, records (gathered later), ids
-static int upload_tree(Surface* s, const std::vector<double4>& box, const std::vector<int32_t>& id, int64_t n_edges) {
-  const size_t nb = box.size() * sizeof(double4), nr = (size_t)n_edges * sizeof(double4);
-  WSB_CUDA(cudaMalloc((void**)&s->tbox, nb + nr + id.size() * sizeof(int32_t)));
-  s->trec = s->tbox + box.size();
-  s->tid = (int32_t*)(s->trec + n_edges);
-  WSB_CUDA(cudaMemcpy(s->tbox, box.data(), nb, cudaMemcpyHostToDevice));
-  WSB_CUDA(cudaMemcpy(s->tid, id.data(), id.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
-  return WSB_OK;
 }
 
 static void free_surface(Surface* s) {
@@ -258,16 +244,13 @@ extern "C" int wsb_surface_create(const double* verts, int64_t n_verts, const in
   s->dy = dy;
   s->n_bitems = (int64_t)bitems.size();
   std::memcpy(s->bbox, bb, sizeof(bb));
-  std::vector<double4> tbox;
-  std::vector<int32_t> tid;
-  edge_tree(erec, tbox, tid);
-  // the records in cell-list, y-bin and tree order are gathered on the device (5 MB instead of 0.6 MB of pageable copies for
+  // the records in cell-list and y-bin order are gathered on the device (5 MB instead of 0.6 MB of pageable copies for
   // 17 400 edges), the cell indicators written by their kernel
   int rc = WSB_OK;
   if ((rc = upload(&s->verts, verts, 2 * n_verts)) || (rc = upload(&s->edges, edges, 2 * n_edges)) ||
       (rc = upload(&s->cstart, start)) || (rc = upload(&s->citems, items)) || (rc = upload(&s->cempty, cempty)) ||
       (rc = upload(&s->ccompact, ccompact)) || (rc = upload(&s->bstart, bstart)) || (rc = upload(&s->bitems, bitems)) ||
-      (rc = upload(&s->erec, erec)) || (rc = upload_tree(s, tbox, tid, n_edges)) ||
+      (rc = upload(&s->erec, erec)) ||
       (rc = upload(&s->crec, (const double4*)nullptr, n_items)) ||
       (rc = upload(&s->brec, (const double4*)nullptr, s->n_bitems)) ||
       (rc = upload(&s->cind, (const double*)nullptr, ncells)) || (rc = upload(&s->cok, (const int32_t*)nullptr, ncells))) {
@@ -275,7 +258,6 @@ extern "C" int wsb_surface_create(const double* verts, int64_t n_verts, const in
     delete s;
     return rc;
   }
-  k_gather_records<<<(unsigned)((n_edges + 255) / 256), 256>>>(s->erec, s->tid, n_edges, s->trec);
   if (n_items) k_gather_records<<<(unsigned)((n_items + 255) / 256), 256>>>(s->erec, s->citems, n_items, s->crec);
   if (s->n_bitems)
     k_gather_records<<<(unsigned)((s->n_bitems + 255) / 256), 256>>>(s->erec, s->bitems, s->n_bitems, s->brec);
@@ -288,6 +270,7 @@ extern "C" int wsb_surface_create(const double* verts, int64_t n_verts, const in
     delete s;
     return cuda_fail(e, "wsb_surface_create: cell indicator");
   }
+  s->herec = std::move(erec);
   *out = s;
   return WSB_OK;
 }
