@@ -75,3 +75,47 @@ def test_workspace_is_left_prepared_without_the_flag():
     loops, X, h = _rows(1000)
     got, again = _call(loops, X, h, ("w2", "w4", "w6"), _lib.OUT_ASSIGN, after=True)
     assert _same(got, again)
+
+
+def _polygon(n, radius, h):
+    """a wavy n-gon and its rms candidate-list length."""
+    t = 2 * np.pi * np.arange(n) / n
+    r = radius * (1 + 0.02 * np.sin(9 * t))
+    P = np.stack([r * np.cos(t), r * np.sin(t)], 1)
+    scene, rep, _ = make_scene([P], center=(0.1, -0.3), angle=0.7)
+    length = np.diff(rep.native(h, DEV).cells()[0]).astype(float)
+    return P, float(np.sqrt((length[length > 0] ** 2).mean()))
+
+
+@pytest.mark.parametrize("edges,radius,h,n,kernels,one", [
+    (256, 0.45, 0.03, 1 << 16, ("w4",), True), (256, 0.45, 0.03, 1 << 18, ("w4",), True),
+    (600, 0.05, 0.1, 1 << 14, ("w4",), True), (600, 0.05, 0.1, 1 << 16, ("w4",), False),
+    (1000, 0.2, 0.05, 1 << 16, ("w4",), False), (1000, 0.2, 0.05, 1 << 16, ("w2", "w4", "w6"), False),
+    (256, 0.45, 0.03, 1 << 16, ("cubic", "w2", "w4", "w6"), True),
+    (1000, 0.2, 0.05, 1 << 12, ("cubic", "w2", "w4", "w6"), True),
+    (1000, 0.2, 0.05, 1 << 14, ("cubic", "w2", "w4", "w6"), False),
+    (256, 0.2, 0.05, 1 << 17, ("w2p5",), False), (256, 0.45, 0.03, 1 << 17, ("w2p5",), True),
+    (600, 0.3, 0.05, 1 << 15, ("w4", "cubic"), False), (600, 0.3, 0.05, 1 << 15, ("w4", "cone", "lw4"), True)])
+def test_long_lists_go_to_the_sorted_rows(edges, radius, h, n, kernels, one):
+    """the one-launch route leaves the workspace alone, the sorted route fills it: which of them a call takes follows its
+    rows, its kernels and the length of the candidate lists; same bits either way."""
+    P, length = _polygon(edges, radius, h)
+    rng = np.random.default_rng(5)
+    X = rng.uniform(-1.4 * radius - h, 1.4 * radius + h, (n, 2)) + np.array([0.1, -0.3])
+    scene, rep, body = make_scene([P], center=(0.1, -0.3), angle=0.7)
+    ns = rep.native(h, DEV)
+    pos = torch.tensor(X, dtype=torch.float64, device=DEV)
+    sup = torch.full((n,), h, dtype=torch.float64, device=DEV)
+    obb, unbounded = body.broadphase()
+    ws, need = ns.workspace(n)
+    got = []
+    for flags in (_lib.OUT_ASSIGN | _lib.WS_SCRATCH, _lib.OUT_ASSIGN):
+        ws.fill_(0x5a)
+        out = [{k: torch.empty((n,) + w, dtype=torch.float64, device=DEV) for k, w in WIDTH.items()} for _ in kernels]
+        _lib.check(_lib.lib.wsb_aggregate_groups(
+            ns.handle, len(kernels), _lib.int32s([IDS[k] for k in kernels]), _lib.PREC_FP64, _lib.ptr(pos), _lib.ptr(sup),
+            None, n, _lib.ptr(body.pose_tensor(DEV)), obb, unbounded, _lib.OUT_ALL | flags,
+            *[_lib.ptrs([o[k] for o in out]) for k in WIDTH], _lib.ptr(ws), need, _stream()), "groups")
+        got.append((bool((ws == 0x5a).all()), out))
+    assert (got[0][0], got[1][0]) == (one, False), length
+    assert all(torch.equal(torch.nan_to_num(a[k]), torch.nan_to_num(b[k])) for a, b in zip(got[0][1], got[1][1]) for k in WIDTH)

@@ -62,6 +62,7 @@ struct Surface {
   int32_t* ccompact = nullptr;  // [nx*ny] index of a cell among the cells with edges (longest list first), -1 for an empty one
   int32_t n_nonempty = 0;       // cells with edges
   int32_t n_long = 0;           // of those, cells of kLongList edges or more
+  double list_rms = 0;          // root mean square of their lists' lengths
   int32_t* bstart = nullptr;    // [nb+1]
   int32_t* bitems = nullptr;    // [n_bitems]
   double4* erec = nullptr;      // [n_edges] (ax, ay, bx, by) by edge id

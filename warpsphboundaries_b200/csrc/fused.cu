@@ -1160,17 +1160,75 @@ static int launch_pack(const SurfView& v, const double* sup, const Workspace& w,
   return WSB_OK;
 }
 
-// Whether an aggregate takes the one-launch route.  Device time on B200, sorted against one launch: w4 among 64 star
-// polygons 4096 rows 59 / 40 us, 65 536 82 / 56, 131 072 88 / 88, 262 144 113 / 135; four kernels 4096 84 / 62, 65 536
-// 121 / 130 (host side 144 / 131), 131 072 143 / 214; the delta+ groups 65 536 237 / 177, 131 072 272 / 282.  One kernel
-// over a surface of few cells (a 256-gon of 300: the sort's counters collide) 262 144 rows 150 / 74, 2^20 477 / 262; with
-// several kernels the sorted rows win there too.  The results are the same bits, so the rule may look at the launch.
-static bool one_launch(const Surface* s, int n_groups, int64_t n) {
-  if (n_groups > 1) return n <= (1 << 16);
-  return n <= (1 << 17) || n >= 256 * (int64_t)s->n_nonempty;
+static bool is_quad_kernel(int k) { return k == Kern_w2p5::kId || k == Kern_w4p5::kId; }
+
+// The kernel sets evaluated in one pass over the neighbour pairs, largest first: the smoothing-kernel families, and
+// the exact groups of the delta+ layout (scheme kernel, cone, wall-Laplacian kernel).  The first set contained in the
+// groups (each of its kernels exactly once, any order) runs as one pack; every other group runs its own pass.
+static const int32_t kPackCW[4] = {WSB_KERNEL_CUBIC, WSB_KERNEL_W2, WSB_KERNEL_W4, WSB_KERNEL_W6};
+static const int32_t kPackW[3] = {WSB_KERNEL_W2, WSB_KERNEL_W4, WSB_KERNEL_W6};
+static const int32_t kPackD2L[3] = {WSB_KERNEL_W2, WSB_KERNEL_CONE, WSB_KERNEL_LW2};
+static const int32_t kPackD4L[3] = {WSB_KERNEL_W4, WSB_KERNEL_CONE, WSB_KERNEL_LW4};
+static const int32_t kPackD2[2] = {WSB_KERNEL_W2, WSB_KERNEL_CONE};
+static const int32_t kPackD4[2] = {WSB_KERNEL_W4, WSB_KERNEL_CONE};
+
+// perm[p] = the group holding pack kernel p when each of the pack's kernels is exactly one of the groups
+static bool match_pack(const int32_t* kernels, int n_groups, const int32_t* pack, int m, int* perm) {
+  if (n_groups < m) return false;
+  for (int p = 0; p < m; ++p) {
+    perm[p] = -1;
+    for (int g = 0; g < n_groups; ++g)
+      if (kernels[g] == pack[p]) {
+        if (perm[p] >= 0) return false;
+        perm[p] = g;
+      }
+    if (perm[p] < 0) return false;
+  }
+  return true;
 }
 
-// its blocks hold 16 to 128 rows, so that the launch has at least two blocks per SM where it has the rows
+// the set of the groups that runs as one pack (its place in the order below; its kernels' groups in perm), -1 for none
+constexpr int kPackSizes[6] = {4, 3, 3, 3, 2, 2};
+static int find_pack(const int32_t* kernels, int n_groups, int* perm) {
+  static const int32_t* const packs[6] = {kPackCW, kPackW, kPackD2L, kPackD4L, kPackD2, kPackD4};
+  for (int k = 0; k < 6; ++k)
+    if (match_pack(kernels, n_groups, packs[k], kPackSizes[k], perm)) return k;
+  return -1;
+}
+
+// Whether an aggregate takes the one-launch route: by its rows, the kernels and the root mean square length of the cells'
+// candidate lists.  A block takes consecutive rows, so a warp waits for its longest list and its highest pair count, which
+// the sorted rows avoid; the sorted route waits for seven launches one after the other.  Device time on B200, us, sorted
+// against one launch:
+//   list length (rms)         w4: 2^14       2^16        2^17        2^18    | w2p5: 2^14       2^16         2^17
+//   8    (256-gon)               40 / 18     43 / 22     61 / 36     83 / 52 |       68 / 34     90 / 50    130 / 90
+//   21   (64 star polygons)      59 / 44     63 / 56     89 / 87    111 / -  |      130 / 75    155 / 105   227 / 178
+//   28   (256-gon, wide h)       46 / 31     83 / 46    113 / 83    162 / 129|      105 / 63    174 / 129   208 / 236
+//   43   (600-gon)               53 / 46     82 / 71    132 / 126   177 / 199|      117 / 73    154 / 151   195 / 269
+//   65   (600-gon)               67 / 56    102 / 112   172 / 201   256 / 313|      124 / 88    212 / 208   279 / 385
+//   109  (1000-gon)              90 / 79    148 / 167   216 / 313   370 / 491|      161 / 134   288 / 328   403 / 600
+//   455  (600 edges, 15 cells)  434 / 285   513 / 717   716 / 1234 1257 / 1947|     742 / 572  1042 / 1445 1572 / 2411
+//   and for several kernels   w2,w4,w6: 2^14   2^16  | w4,cubic: 2^14   2^16  | delta+: 2^14   2^16  | all four: 2^12  2^14   2^16
+//   8                            38 / 23    52 / 30  |      48 / 34    64 / 42 |     85 / 58  118 / 81 |    40 / 28  42 / 46   61 / 58
+//   21                           68 / 59    77 / 71  |      95 / 93   105 / 119|    169 / 133  200 / 178|    80 / 63  83 / 87   95 / 132
+//   28                           54 / 42    99 / 64  |      74 / 66   129 / 97 |    138 / 106  235 / 196|    60 / 51  65 / 90  112 / 126
+//   43                           64 / 63   118 / 100 |      90 / 95   135 / 154|    159 / 135  229 / 253|    73 / 69  80 / 119 138 / 186
+//   109                         110 / 108  181 / 225 |     157 / 159  241 / 350|    244 / 243  425 / 563|   101 / 75 129 / 173 198 / 427
+// Four kernels stay in one launch a little past the device's crossing: launching the sorted route takes the host 118 us a
+// call, one launch 100 (16 001 rows among 64 star polygons, calls one after the other: 120 against 103).
+// The results are the same bits, so the rule may look at the launch.
+static bool one_launch(const Surface* s, int n_groups, const int32_t* kernels, int64_t n) {
+  int perm[kMaxPack];
+  const int which = find_pack(kernels, n_groups, perm);
+  const double work = (double)n * s->list_rms;
+  if (which >= 0 && kPackSizes[which] >= 4) return n <= (1 << 12) || (n <= (1 << 16) && work <= 0.85e6);
+  if (n <= (1 << 14)) return true;
+  if (n_groups > 1) return n <= (1 << 16) && work <= (which >= 0 ? 2e6 : 1e6);
+  // one kernel; over few cells the sort's counters collide, so many rows stay here: 256-gon of 378 cells 2^20 rows 204 / 183
+  if (n > (1 << 17) && n < 256 * (int64_t)s->n_nonempty) return false;
+  return work <= 3e6 || (s->list_rms <= 30.0 && !is_quad_kernel(kernels[0]));
+}
+
 struct RowArgs {
   const double *pos, *sup;
   const int32_t* allowed;
@@ -1193,6 +1251,7 @@ static int launch_block(const SurfView& v, const RowArgs& a, bool assign, const 
       opted.fetch_or(bit);
     }
   }
+  // blocks of 16 to 128 rows, so that the launch has at least two blocks per SM where it has the rows
   int rows = kThreads;
   while (rows > 16 && a.n < (int64_t)rows * 148 * 2) rows /= 2;
   if (g_pair_ev[0]) WSB_CUDA(cudaEventRecord(g_pair_ev[0], st));
@@ -1748,7 +1807,6 @@ static int sort_rows(const Surface* s, const double* pos, const double* sup, con
 }
 
 // kernel ids the fused aggregate serves: the exact-table kernels and the quadrature kernels (the tensile group)
-static bool is_quad_kernel(int k) { return k == Kern_w2p5::kId || k == Kern_w4p5::kId; }
 static bool aggregate_kernel_ok(int k) { return (k >= 0 && k < kNumKernels) || is_quad_kernel(k); }
 
 static int check_common(const Surface* s, int kernel, const double* pos, const double* sup, int64_t n,
@@ -1853,31 +1911,6 @@ extern "C" int wsb_aggregate_evaluate(const wsb_surface* s, int kernel, int prec
                   stream);
 }
 
-// The kernel sets evaluated in one pass over the neighbour pairs, largest first: the smoothing-kernel families, and
-// the exact groups of the delta+ layout (scheme kernel, cone, wall-Laplacian kernel).  The first set contained in the
-// groups (each of its kernels exactly once, any order) runs as one pack; every other group runs its own pass.
-static const int32_t kPackCW[4] = {WSB_KERNEL_CUBIC, WSB_KERNEL_W2, WSB_KERNEL_W4, WSB_KERNEL_W6};
-static const int32_t kPackW[3] = {WSB_KERNEL_W2, WSB_KERNEL_W4, WSB_KERNEL_W6};
-static const int32_t kPackD2L[3] = {WSB_KERNEL_W2, WSB_KERNEL_CONE, WSB_KERNEL_LW2};
-static const int32_t kPackD4L[3] = {WSB_KERNEL_W4, WSB_KERNEL_CONE, WSB_KERNEL_LW4};
-static const int32_t kPackD2[2] = {WSB_KERNEL_W2, WSB_KERNEL_CONE};
-static const int32_t kPackD4[2] = {WSB_KERNEL_W4, WSB_KERNEL_CONE};
-
-// perm[p] = the group holding pack kernel p when each of the pack's kernels is exactly one of the groups
-static bool match_pack(const int32_t* kernels, int n_groups, const int32_t* pack, int m, int* perm) {
-  if (n_groups < m) return false;
-  for (int p = 0; p < m; ++p) {
-    perm[p] = -1;
-    for (int g = 0; g < n_groups; ++g)
-      if (kernels[g] == pack[p]) {
-        if (perm[p] >= 0) return false;
-        perm[p] = g;
-      }
-    if (perm[p] < 0) return false;
-  }
-  return true;
-}
-
 static int evaluate_groups(const wsb_surface* s_, int n_groups, const int32_t* kernels, int precision, const double* sup,
                            int64_t n, const double* pose, int out_mask, double* const* lam, double* const* G,
                            double* const* cov, double* const* m1, double* const* m2, const void* workspace,
@@ -1897,14 +1930,7 @@ static int evaluate_groups(const wsb_surface* s_, int n_groups, const int32_t* k
   if (!sup || !pose) return fail(WSB_ERR_ARG, "wsb_aggregate_evaluate_groups: NULL array");
   auto pick = [&](double* const* a, int g, int bit) { return (a && (out_mask & bit)) ? a[g] : nullptr; };
   int perm[kMaxPack];
-  int which = -1, m = 0;
-  const int32_t* packs[6] = {kPackCW, kPackW, kPackD2L, kPackD4L, kPackD2, kPackD4};
-  const int sizes[6] = {4, 3, 3, 3, 2, 2};
-  for (int k = 0; k < 6 && which < 0; ++k)
-    if (match_pack(kernels, n_groups, packs[k], sizes[k], perm)) {
-      which = k;
-      m = sizes[k];
-    }
+  const int which = find_pack(kernels, n_groups, perm), m = which < 0 ? 0 : kPackSizes[which];
   bool in_pack[WSB_MAX_GROUPS] = {false};
   for (int p = 0; p < m; ++p) in_pack[perm[p]] = true;
   for (int g = 0; g < n_groups; ++g) {                              // the groups outside the pack: one pass each
@@ -1962,9 +1988,10 @@ extern "C" int wsb_aggregate_evaluate_groups(const wsb_surface* s, int n_groups,
 
 // the front half of an aggregate: nothing where the rows take the one-launch route (the caller has the workspace as
 // scratch), else the sorted rows; the checks of wsb_aggregate_prepare in both
-static int front(const wsb_surface* s_, int n_groups, const RowArgs& a, int out_mask, void* workspace, size_t workspace_bytes,
-                 void* stream, const RowArgs** rows) {
-  const bool one = (out_mask & WSB_WS_SCRATCH) != 0 && one_launch(reinterpret_cast<const Surface*>(s_), n_groups, a.n);
+static int front(const wsb_surface* s_, int n_groups, const int32_t* kernels, const RowArgs& a, int out_mask, void* workspace,
+                 size_t workspace_bytes, void* stream, const RowArgs** rows) {
+  const bool one =
+      (out_mask & WSB_WS_SCRATCH) != 0 && one_launch(reinterpret_cast<const Surface*>(s_), n_groups, kernels, a.n);
   *rows = one ? &a : nullptr;
   if (!*rows)
     return wsb_aggregate_prepare(s_, a.pos, a.sup, a.allowed, a.n, a.pose, a.obb, a.unbounded, workspace, workspace_bytes,
@@ -1991,7 +2018,8 @@ extern "C" int wsb_aggregate(const wsb_surface* s_, int kernel, int precision, c
     WSB_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t), (cudaStream_t)stream));
   }
   const RowArgs args{pos, sup, allowed, n, pose, obb, unbounded}, *rows = nullptr;
-  rc = front(s_, 1, args, out_mask, workspace, workspace_bytes, stream, &rows);
+  const int32_t kernels[1] = {kernel};
+  rc = front(s_, 1, kernels, args, out_mask, workspace, workspace_bytes, stream, &rows);
   if (rc) return rc;
   return evaluate(s_, kernel, precision, sup, n, pose, out_mask, lam, G, cov, m1, m2, workspace, workspace_bytes, rows,
                   stream);
@@ -2014,7 +2042,7 @@ extern "C" int wsb_aggregate_groups(const wsb_surface* s_, int n_groups, const i
     return fail(WSB_ERR_UNSUPPORTED, "wsb_aggregate_groups: unknown precision mode");
   if (n == 0) return WSB_OK;
   const RowArgs args{pos, sup, allowed, n, pose, obb, unbounded}, *rows = nullptr;
-  rc = front(s_, n_groups, args, out_mask, workspace, workspace_bytes, stream, &rows);
+  rc = front(s_, n_groups, kernels, args, out_mask, workspace, workspace_bytes, stream, &rows);
   if (rc) return rc;
   return evaluate_groups(s_, n_groups, kernels, precision, sup, n, pose, out_mask, lam, G, cov, m1, m2, workspace,
                          workspace_bytes, rows, stream);

@@ -199,6 +199,8 @@ extern "C" int wsb_surface_create(const double* verts, int64_t n_verts, const in
   std::vector<int32_t> ccompact(ncells);
   // the cells with edges in decreasing order of their lists' length (a counting sort; cell order within a length)
   int32_t nne = 0, nlc = 0;
+  double len2 = 0.0;
+  for (int64_t c = 0; c < ncells; ++c) len2 += (double)(start[c + 1] - start[c]) * (double)(start[c + 1] - start[c]);
   {
     std::vector<int32_t> of((size_t)K + 2, 0);
     for (int64_t c = 0; c < ncells; ++c) ++of[K - (start[c + 1] - start[c]) + 1];
@@ -238,6 +240,7 @@ extern "C" int wsb_surface_create(const double* verts, int64_t n_verts, const in
   s->K = K;
   s->n_nonempty = nne;
   s->n_long = nlc;
+  s->list_rms = std::sqrt(len2 / std::max(nne, 1));
   s->n_items = n_items;
   s->nb = nb;
   s->y0 = y0;
