@@ -981,8 +981,13 @@ int mesh_lists(Mesh* m, const BoxLists& L, int64_t ncells, int32_t** len) {
   return WSB_OK;
 }
 
-// the workspace of n queries: the listed rows, their number and that of the rows with faces, the indicator (where the
-// caller wants none), the rows with faces and their masks
+// Queries are taken kMeshSlice at a time, so the workspace stops growing there (80 bytes a query and 8 per mask word past
+// the first: 0.34 to 0.57 GB; 21 GB for 2^28 queries at once).  A slice of that size takes some milliseconds, its three launches
+// a few microseconds.
+constexpr int64_t kMeshSlice = 1 << 22;
+
+// the workspace of n queries (of one slice): the listed rows, their number and that of the rows with faces, the indicator
+// (where the caller wants none), the rows with faces and their masks
 struct MeshWork {
   int32_t *near, *counts, *ind;
   MeshRow* rows;
@@ -992,7 +997,7 @@ struct MeshWork {
 MeshWork carve_mesh(const Mesh* m, int64_t n, void* base) {
   MeshWork w{};
   const uintptr_t p = ((uintptr_t)base + 255) & ~(uintptr_t)255;
-  const size_t k = (size_t)std::max<int64_t>(n, 1);
+  const size_t k = (size_t)std::min<int64_t>(std::max<int64_t>(n, 1), kMeshSlice);
   size_t off = 0;
   auto take = [&](size_t bytes) {
     const size_t o = off;
@@ -1009,22 +1014,28 @@ MeshWork carve_mesh(const Mesh* m, int64_t n, void* base) {
 }
 
 template <class M>
-int launch_mesh(const Mesh* m, const double* pos, const double* sup, int64_t n, double* out, int32_t* ind,
+int launch_mesh(const Mesh* m, const double* pos_all, const double* sup_all, int64_t n_all, double* out_all, int32_t* inside,
                 const MeshWork& w, cudaStream_t st) {
   const MeshView v = view_of(m);
-  const unsigned grid = (unsigned)((n + kMeshThreads - 1) / kMeshThreads);
-  WSB_CUDA(cudaMemsetAsync(w.counts, 0, 2 * sizeof(int32_t), st));
-  k_mesh_rowinfo<M><<<grid, kMeshThreads, 0, st>>>(v, pos, sup, n, ind, w.near, w.counts, out);
-  WSB_CUDA(cudaGetLastError());
   const int warps = kMeshThreads / 32;
-  const auto grid_of = [&](int blocks) {           // the resident warps, striding over the rows; no more warps than rows
-    return (unsigned)std::min<int64_t>((n + warps - 1) / warps, (int64_t)148 * blocks);
-  };
-  k_mesh_search<M><<<grid_of(kSearchBlocks), kMeshThreads, 0, st>>>(v, pos, sup, w.near, w.counts, m->words, ind, w.rows,
-                                                                    w.mask, out);
-  WSB_CUDA(cudaGetLastError());
-  k_mesh_eval<M><<<grid_of(kEvalBlocks), kMeshThreads, 0, st>>>(v, w.rows, w.mask, m->words, w.counts + 1, out);
-  WSB_CUDA(cudaGetLastError());
+  for (int64_t at = 0; at < n_all; at += kMeshSlice) {
+    const int64_t n = std::min(kMeshSlice, n_all - at);
+    const double *pos = pos_all + 3 * at, *sup = sup_all + at;
+    double* out = out_all + 28 * at;
+    int32_t* ind = inside ? inside + at : w.ind;
+    const unsigned grid = (unsigned)((n + kMeshThreads - 1) / kMeshThreads);
+    const auto grid_of = [&](int blocks) {         // the resident warps, striding over the rows; no more warps than rows
+      return (unsigned)std::min<int64_t>((n + warps - 1) / warps, (int64_t)148 * blocks);
+    };
+    WSB_CUDA(cudaMemsetAsync(w.counts, 0, 2 * sizeof(int32_t), st));
+    k_mesh_rowinfo<M><<<grid, kMeshThreads, 0, st>>>(v, pos, sup, n, ind, w.near, w.counts, out);
+    WSB_CUDA(cudaGetLastError());
+    k_mesh_search<M><<<grid_of(kSearchBlocks), kMeshThreads, 0, st>>>(v, pos, sup, w.near, w.counts, m->words, ind, w.rows,
+                                                                      w.mask, out);
+    WSB_CUDA(cudaGetLastError());
+    k_mesh_eval<M><<<grid_of(kEvalBlocks), kMeshThreads, 0, st>>>(v, w.rows, w.mask, m->words, w.counts + 1, out);
+    WSB_CUDA(cudaGetLastError());
+  }
   return WSB_OK;
 }
 
@@ -1270,12 +1281,11 @@ extern "C" int wsb_mesh_channels(const wsb_mesh* m, int kernel, const double* po
     return fail(WSB_ERR_SIZE, "wsb_mesh_channels: workspace smaller than wsb_mesh_workspace_size");
   WSB_CUDA(cudaSetDevice(m->device));
   const MeshWork w = carve_mesh(m, n, workspace);
-  int32_t* ind = inside ? inside : w.ind;
   cudaStream_t st = (cudaStream_t)stream;
   switch (kernel) {
-    case WSB_KERNEL_CUBIC: return launch_mesh<Mesh_cubic>(m, pos, sup, n, out, ind, w, st);
-    case WSB_KERNEL_W2: return launch_mesh<Mesh_w2>(m, pos, sup, n, out, ind, w, st);
-    case WSB_KERNEL_W4: return launch_mesh<Mesh_w4>(m, pos, sup, n, out, ind, w, st);
-    default: return launch_mesh<Mesh_w6>(m, pos, sup, n, out, ind, w, st);
+    case WSB_KERNEL_CUBIC: return launch_mesh<Mesh_cubic>(m, pos, sup, n, out, inside, w, st);
+    case WSB_KERNEL_W2: return launch_mesh<Mesh_w2>(m, pos, sup, n, out, inside, w, st);
+    case WSB_KERNEL_W4: return launch_mesh<Mesh_w4>(m, pos, sup, n, out, inside, w, st);
+    default: return launch_mesh<Mesh_w6>(m, pos, sup, n, out, inside, w, st);
   }
 }
