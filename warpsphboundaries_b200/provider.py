@@ -157,7 +157,8 @@ class FusedWall(WallAggregate):
                     for t in out.values():
                         t[bi].zero_()
                 continue
-            p_pose = ptr(body.pose_tensor(self.dev))
+            pose = body.pose_tensor(self.dev)        # held until the body's calls are made: the body may replace its own
+            p_pose = ptr(pose)
             at = {k: [b + bi * step for b, step in base[k]] for k in names}
             for ri, rep in enumerate(body.fused_reps(self.support, self.dev)):
                 mode = _lib.OUT_ALL | _lib.WS_SCRATCH | (_lib.OUT_ASSIGN if ri == 0 else 0)     # the first representation assigns
@@ -182,7 +183,6 @@ class FusedWall(WallAggregate):
                                                    obb, unbounded, mode, *tgt, ptr(ws), need, st),
                           "wsb_aggregate_groups")
                     continue
-                pose = body.pose_tensor(self.dev)
                 for gi, kid in enumerate(kids):
                     # closed form into scratch, then the rows the quadrature takes are overridden while combining
                     self._group = gi

@@ -977,9 +977,9 @@ class Scene:
                 tracked = d.requires_grad or n.requires_grad or unpack_dual(d).tangent is not None
                 if tracked:
                     d, n = d.detach().clone(), n.detach().clone()
-                check(lib.wsb_body_distance(ns.handle, ptr(pts), M, ptr(bd.pose_tensor(self.device)),
-                                            float(supportMax) if supportMax else 0.0, int(first), bi, ptr(d), ptr(n),
-                                            ptr(bidx), _stream()), "wsb_body_distance")
+                pose = bd.pose_tensor(self.device)     # held until the call is made: the body may replace its own
+                check(lib.wsb_body_distance(ns.handle, ptr(pts), M, ptr(pose), float(supportMax) if supportMax else 0.0,
+                                            int(first), bi, ptr(d), ptr(n), ptr(bidx), _stream()), "wsb_body_distance")
                 if tracked:
                     better = d < best
                     best = torch.where(better, d, best)
