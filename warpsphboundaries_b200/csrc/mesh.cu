@@ -55,6 +55,7 @@ struct Mesh {
   int64_t n_items = 0, n_col_items = 0;
   double* fdata = nullptr;     // [n_faces * kFaceDoubles]
   int32_t words = 1;           // 64-bit words of a row's hit mask (at most kMaxWords)
+  int32_t eval_rows = 32;      // rows a warp of the evaluation takes at most (fewer where their faces would pass 2^31)
   int64_t* nstart = nullptr;   // [nx*ny*nz + 1]
   int32_t* nitems = nullptr;   // per cell the faces a query of the cell may reach (each once)
   double col = 1;              // size of an (x, y) column: half a cell (a cell where that would list too many faces)
@@ -844,11 +845,13 @@ __device__ __forceinline__ int select_bit(uint64_t m, int k) {
 // spread the quadrature nodes of one edge after the other over its lanes (7.0 ms with the search).
 constexpr int kEvalBlocks = 3;        // resident CTAs per SM (168 registers)
 constexpr int kEvalRows = 32;
+static_assert((INT32_MAX / 8) * (int64_t)kBatch < ((int64_t)1 << 31) && ((int64_t)1 << 26) * kEvalRows <= ((int64_t)1 << 31),
+              "the flattened lists of a batch fit 32 bits: at most INT32_MAX / 8 faces a list");
 constexpr int kPairStride = 29;       // doubles per pair in shared memory (28 and one against bank conflicts)
 
 template <class M>
 __global__ void __launch_bounds__(kMeshThreads, kEvalBlocks)
-    k_mesh_eval(MeshView Mv, const MeshRow* __restrict__ rows, const uint64_t* __restrict__ mask, int words,
+    k_mesh_eval(MeshView Mv, const MeshRow* __restrict__ rows, const uint64_t* __restrict__ mask, int words, int most,
                 const int32_t* __restrict__ nrows, double* __restrict__ out) {
   __shared__ double s_val[kMeshThreads / 32][32 * kPairStride];
   __shared__ double s_h[kMeshThreads / 32][32];               // the round's supports and tags
@@ -856,7 +859,7 @@ __global__ void __launch_bounds__(kMeshThreads, kEvalBlocks)
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   double* const val = s_val[wib];
   const Channel ch = channel_of(lane);
-  const int n = *nrows, warps = gridDim.x * (kMeshThreads / 32), per = batch_rows(n, warps, kEvalRows);
+  const int n = *nrows, warps = gridDim.x * (kMeshThreads / 32), per = batch_rows(n, warps, most);
   for (int it = (blockIdx.x * (kMeshThreads / 32) + wib) * per; it < n; it += warps * per) {
     unsigned pairs = 0;
     if (lane < per && it + lane < n) {
@@ -969,8 +972,7 @@ int mesh_lists(Mesh* m, const BoxLists& L, int64_t ncells, int32_t** len) {
   int64_t total = 0;
   int32_t longest = 0;
   WSB_CUDA(cudaMemcpy(&longest, *len + ncells, sizeof(longest), cudaMemcpyDeviceToHost));
-  if (longest > (1 << 26))   // the passes flatten up to 32 lists in 32 bits
-    return fail(WSB_ERR_SIZE, "wsb_mesh_create: more than 2^26 faces within reach of one cell");
+  m->eval_rows = longest > (1 << 26) ? kBatch : kEvalRows;   // the lists of a batch are flattened in 32 bits
   m->words = std::min(kMaxWords, std::max(1, (longest + 63) / 64));
   WSB_CUDA(cudaMemcpy(&total, m->nstart + ncells, sizeof(total), cudaMemcpyDeviceToHost));
   WSB_CUDA(cudaMalloc((void**)&m->nitems, sizeof(int32_t) * (size_t)std::max<int64_t>(total, 1)));
@@ -1033,7 +1035,7 @@ int launch_mesh(const Mesh* m, const double* pos_all, const double* sup_all, int
     k_mesh_search<M><<<grid_of(kSearchBlocks), kMeshThreads, 0, st>>>(v, pos, sup, w.near, w.counts, m->words, ind, w.rows,
                                                                       w.mask, out);
     WSB_CUDA(cudaGetLastError());
-    k_mesh_eval<M><<<grid_of(kEvalBlocks), kMeshThreads, 0, st>>>(v, w.rows, w.mask, m->words, w.counts + 1, out);
+    k_mesh_eval<M><<<grid_of(kEvalBlocks), kMeshThreads, 0, st>>>(v, w.rows, w.mask, m->words, m->eval_rows, w.counts + 1, out);
     WSB_CUDA(cudaGetLastError());
   }
   return WSB_OK;
