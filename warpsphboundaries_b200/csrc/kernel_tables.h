@@ -2335,18 +2335,18 @@ template <> __host__ __device__ __forceinline__ void Rad_w6::eval<0, float>(floa
 // ---- 3-D closed surfaces: compact potentials per truncated block (unit support, W~ = c3*pi * shape); rows:
 //      0 A_K0, 1 A_K1, 2 A_K2, 3 A_W, 4 A_L, 5 A2_K2
 struct MeshBlock_cubic_0 {
-  static constexpr double kR = 1.0;
+  static constexpr double kR = 1.0, kRho = 0.5;
   static constexpr int kTop = 7;      // highest power of A2_K2
   static constexpr int kLine = 5;     // highest power of the other potentials
   static constexpr double kNu[6] = {0.26666666666666666, 0.05714285714285714, 0.01904761904761905, 0.0, 0.0, -0.01904761904761905};
-  static constexpr double kC[6][kTop + 1] = {{-0.8, 0.0, 2.6666666666666665, -4.0, 2.4, -0.5333333333333333, 0.0, 0.0}, {-0.4, 0.0, 2.0, -3.2, 2.0, -0.45714285714285713, 0.0, 0.0}, {-0.26666666666666666, 0.0, 1.6, -2.6666666666666665, 1.7142857142857142, -0.4, 0.0, 0.0}, {-0.8, 0.0, 8.0, -16.0, 12.0, -3.2, 0.0, 0.0}, {16.0, -48.0, 48.0, -16.0, 0.0, 0.0, 0.0, 0.0}, {0.05714285714285714, 0.0, -0.13333333333333333, 0.0, 0.4, -0.5333333333333333, 0.2857142857142857, -0.05714285714285714}};
+  static constexpr double kC[6][kTop + 1] = {{-0.5, 0.7, -0.4, -0.5333333333333333, 1.0666666666666667, -0.5333333333333333, 0.0, 0.0}, {-0.18928571428571428, 0.45714285714285713, -0.37142857142857144, -0.34285714285714286, 0.8571428571428571, -0.45714285714285713, 0.0, 0.0}, {-0.10535714285714286, 0.33214285714285713, -0.32857142857142857, -0.23809523809523808, 0.7142857142857143, -0.4, 0.0, 0.0}, {-0.15, 1.0, -2.0, 0.0, 4.0, -3.2, 0.0, 0.0}, {2.0, -12.0, 24.0, -16.0, 0.0, 0.0, 0.0, 0.0}, {0.03616071428571429, -0.05267857142857143, 0.030357142857142857, 0.055952380952380955, -0.11190476190476191, 0.023809523809523808, 0.08571428571428572, -0.05714285714285714}};
 };
 struct MeshBlock_cubic_1 {
-  static constexpr double kR = 0.5;
+  static constexpr double kR = 0.5, kRho = 0.25;
   static constexpr int kTop = 7;      // highest power of A2_K2
   static constexpr int kLine = 5;     // highest power of the other potentials
   static constexpr double kNu[6] = {-0.016666666666666666, -0.0017857142857142857, -0.00029761904761904765, 0.0, 0.0, 0.00029761904761904765};
-  static constexpr double kC[6][kTop + 1] = {{0.1, 0.0, -1.3333333333333333, 4.0, -4.8, 2.1333333333333333, 0.0, 0.0}, {0.05, 0.0, -1.0, 3.2, -4.0, 1.8285714285714285, 0.0, 0.0}, {0.03333333333333333, 0.0, -0.8, 2.6666666666666665, -3.4285714285714284, 1.6, 0.0, 0.0}, {0.1, 0.0, -4.0, 16.0, -24.0, 12.8, 0.0, 0.0}, {-8.0, 48.0, -96.0, 64.0, 0.0, 0.0, 0.0, 0.0}, {-0.0017857142857142857, 0.0, 0.016666666666666666, 0.0, -0.2, 0.5333333333333333, -0.5714285714285714, 0.22857142857142856}};
+  static constexpr double kC[6][kTop + 1] = {{0.0625, -0.175, 0.2, 0.5333333333333333, -2.1333333333333333, 2.1333333333333333, 0.0, 0.0}, {0.023660714285714285, -0.11428571428571428, 0.18571428571428572, 0.34285714285714286, -1.7142857142857142, 1.8285714285714285, 0.0, 0.0}, {0.013169642857142857, -0.08303571428571428, 0.16428571428571428, 0.23809523809523808, -1.4285714285714286, 1.6, 0.0, 0.0}, {0.01875, -0.25, 1.0, 0.0, -8.0, 12.8, 0.0, 0.0}, {-1.0, 12.0, -48.0, 64.0, 0.0, 0.0, 0.0, 0.0}, {-0.0011300223214285715, 0.0032924107142857143, -0.003794642857142857, -0.013988095238095239, 0.055952380952380955, -0.023809523809523808, -0.17142857142857143, 0.22857142857142856}};
 };
 struct Mesh_cubic {
   static constexpr int kBlocks = 2;
@@ -2354,11 +2354,11 @@ struct Mesh_cubic {
   template <int B> using Block = std::tuple_element_t<B, std::tuple<MeshBlock_cubic_0, MeshBlock_cubic_1>>;
 };
 struct MeshBlock_w2_0 {
-  static constexpr double kR = 1.0;
+  static constexpr double kR = 1.0, kRho = 0.5;
   static constexpr int kTop = 9;      // highest power of A2_K2
   static constexpr int kLine = 7;     // highest power of the other potentials
   static constexpr double kNu[6] = {0.25, 0.052083333333333336, 0.016666666666666666, 0.0, 0.0, -0.016666666666666666};
-  static constexpr double kC[6][kTop + 1] = {{-0.75, 0.0, 1.75, 0.0, -5.25, 7.0, -3.75, 0.75, 0.0, 0.0}, {-0.375, 0.0, 1.3125, 0.0, -4.375, 6.0, -3.28125, 0.6666666666666666, 0.0, 0.0}, {-0.25, 0.0, 1.05, 0.0, -3.75, 5.25, -2.9166666666666665, 0.6, 0.0, 0.0}, {-0.75, 0.0, 5.25, 0.0, -26.25, 42.0, -26.25, 6.0, 0.0, 0.0}, {10.5, 0.0, -105.0, 210.0, -157.5, 42.0, 0.0, 0.0, 0.0, 0.0}, {0.052083333333333336, 0.0, -0.125, 0.0, 0.2625, 0.0, -0.625, 0.75, -0.3645833333333333, 0.06666666666666667}};
+  static constexpr double kC[6][kTop + 1] = {{-0.474609375, 0.69140625, -0.3984375, -0.734375, 1.46875, -0.3125, -1.125, 0.75, 0.0, 0.0}, {-0.17887369791666666, 0.4576822916666667, -0.388671875, -0.4947916666666667, 1.2369791666666667, -0.34375, -0.9479166666666666, 0.6666666666666666, 0.0, 0.0}, {-0.09869791666666666, 0.334375, -0.353125, -0.3541666666666667, 1.0625, -0.35, -0.8166666666666667, 0.6, 0.0, 0.0}, {-0.12890625, 0.984375, -2.296875, 0.0, 6.5625, -5.25, -5.25, 6.0, 0.0, 0.0}, {1.96875, -13.125, 26.25, 0.0, -52.5, 42.0, 0.0, 0.0, 0.0, 0.0}, {0.03203938802083333, -0.04934895833333333, 0.03424479166666667, 0.05260416666666667, -0.13255208333333332, 0.035416666666666666, 0.14791666666666667, -0.10833333333333334, -0.06458333333333334, 0.06666666666666667}};
 };
 struct Mesh_w2 {
   static constexpr int kBlocks = 1;
@@ -2366,11 +2366,11 @@ struct Mesh_w2 {
   template <int B> using Block = std::tuple_element_t<B, std::tuple<MeshBlock_w2_0>>;
 };
 struct MeshBlock_w4_0 {
-  static constexpr double kR = 1.0;
+  static constexpr double kR = 1.0, kRho = 0.5;
   static constexpr int kTop = 12;      // highest power of A2_K2
   static constexpr int kLine = 10;     // highest power of the other potentials
   static constexpr double kNu[6] = {0.25, 0.045572916666666664, 0.01282051282051282, 0.0, 0.0, -0.01282051282051282};
-  static constexpr double kC[6][kTop + 1] = {{-0.859375, 0.0, 2.578125, 0.0, -7.21875, 0.0, 25.78125, -41.25, 30.078125, -11.0, 1.640625, 0.0, 0.0}, {-0.4296875, 0.0, 1.93359375, 0.0, -6.015625, 0.0, 22.55859375, -36.666666666666664, 27.0703125, -10.0, 1.50390625, 0.0, 0.0}, {-0.2864583333333333, 0.0, 1.546875, 0.0, -5.15625, 0.0, 20.052083333333332, -33.0, 24.609375, -9.166666666666666, 1.3882211538461537, 0.0, 0.0}, {-0.859375, 0.0, 7.734375, 0.0, -36.09375, 0.0, 180.46875, -330.0, 270.703125, -110.0, 18.046875, 0.0, 0.0}, {15.46875, 0.0, -144.375, 0.0, 1082.8125, -2310.0, 2165.625, -990.0, 180.46875, 0.0, 0.0, 0.0, 0.0}, {0.045572916666666664, 0.0, -0.14322916666666666, 0.0, 0.38671875, 0.0, -0.859375, 0.0, 2.5065104166666665, -3.6666666666666665, 2.4609375, -0.8333333333333334, 0.11568509615384616}};
+  static constexpr double kC[6][kTop + 1] = {{-0.4878387451171875, 0.81622314453125, -0.79656982421875, -0.4814453125, 2.65478515625, -2.376953125, -2.013671875, 4.671875, -0.96484375, -2.796875, 1.640625, 0.0, 0.0}, {-0.16856511433919272, 0.5148061116536459, -0.7085418701171875, -0.18513997395833334, 2.1547444661458335, -2.23876953125, -1.5437825520833333, 4.173177083333333, -1.0107421875, -2.48046875, 1.50390625, 0.0, 0.0}, {-0.08692149626903045, 0.3620746319110577, -0.6124220628004807, -0.03317808493589743, 1.7914287860576923, -2.0833834134615383, -1.2118890224358974, 3.7608173076923075, -1.0231370192307692, -2.2255608974358974, 1.3882211538461537, 0.0, 0.0}, {-0.0797271728515625, 0.83587646484375, -3.11187744140625, 3.3837890625, 7.33154296875, -20.302734375, 2.255859375, 33.515625, -21.26953125, -19.765625, 18.046875, 0.0, 0.0}, {1.6717529296875, -15.791015625, 51.884765625, -45.1171875, -112.79296875, 252.65625, -36.09375, -268.125, 180.46875, 0.0, 0.0, 0.0, 0.0}, {0.0251620121491261, -0.043460748134515226, 0.0470579098432492, 0.018621200170272436, -0.15725277631710738, 0.17250726161858973, 0.12495617988782051, -0.384189703525641, 0.08356495392628205, 0.3610276442307692, -0.2135917467948718, -0.13922275641025642, 0.11568509615384616}};
 };
 struct Mesh_w4 {
   static constexpr int kBlocks = 1;
@@ -2378,11 +2378,11 @@ struct Mesh_w4 {
   template <int B> using Block = std::tuple_element_t<B, std::tuple<MeshBlock_w4_0>>;
 };
 struct MeshBlock_w6_0 {
-  static constexpr double kR = 1.0;
+  static constexpr double kR = 1.0, kRho = 0.5;
   static constexpr int kTop = 15;      // highest power of A2_K2
   static constexpr int kLine = 13;     // highest power of the other potentials
   static constexpr double kNu[6] = {0.25, 0.041015625, 0.010416666666666666, 0.0, 0.0, -0.010416666666666666};
-  static constexpr double kC[6][kTop + 1] = {{-0.95703125, 0.0, 3.5546875, 0.0, -11.73046875, 0.0, 33.515625, 0.0, -136.85546875, 250.25, -223.9453125, 113.75, -31.58203125, 3.75, 0.0, 0.0}, {-0.478515625, 0.0, 2.666015625, 0.0, -9.775390625, 0.0, 29.326171875, 0.0, -123.169921875, 227.5, -205.283203125, 105.0, -29.326171875, 3.5, 0.0, 0.0}, {-0.3190104166666667, 0.0, 2.1328125, 0.0, -8.37890625, 0.0, 26.067708333333332, 0.0, -111.97265625, 208.54166666666666, -189.4921875, 97.5, -27.37109375, 3.28125, 0.0, 0.0}, {-0.95703125, 0.0, 10.6640625, 0.0, -58.65234375, 0.0, 234.609375, 0.0, -1231.69921875, 2502.5, -2463.3984375, 1365.0, -410.56640625, 52.5, 0.0, 0.0}, {21.328125, 0.0, -234.609375, 0.0, 1407.65625, 0.0, -9853.59375, 22522.5, -24633.984375, 15015.0, -4926.796875, 682.5, 0.0, 0.0, 0.0, 0.0}, {0.041015625, 0.0, -0.15950520833333334, 0.0, 0.533203125, 0.0, -1.396484375, 0.0, 3.2584635416666665, 0.0, -11.197265625, 18.958333333333332, -15.791015625, 7.5, -1.955078125, 0.21875}};
+  static constexpr double kC[6][kTop + 1] = {{-0.4940614700317383, 0.8928604125976562, -1.1504592895507812, 0.127838134765625, 3.1809844970703125, -5.720458984375, 0.443603515625, 10.6337890625, -10.270263671875, -6.341796875, 14.638671875, -2.6171875, -7.20703125, 3.75, 0.0, 0.0}, {-0.15748357772827148, 0.5346717834472656, -0.9687538146972656, 0.4102630615234375, 2.4110031127929688, -5.1448974609375, 1.0074462890625, 9.21826171875, -9.7437744140625, -5.2294921875, 13.4599609375, -2.70703125, -6.576171875, 3.5, 0.0, 0.0}, {-0.07599163055419922, 0.360687255859375, -0.8074874877929688, 0.5185445149739584, 1.8810272216796875, -4.6253662109375, 1.3369954427083333, 8.0830078125, -9.210205078125, -4.368489583333333, 12.439453125, -2.7421875, -6.04296875, 3.28125, 0.0, 0.0}, {-0.047631263732910156, 0.6352615356445312, -3.2596206665039062, 6.873321533203125, 1.6037750244140625, -32.991943359375, 40.323486328125, 43.9892578125, -120.970458984375, 9.775390625, 146.630859375, -74.6484375, -69.31640625, 52.5, 0.0, 0.0}, {1.2705230712890625, -15.57952880859375, 72.39898681640625, -131.9677734375, -65.98388671875, 615.849609375, -615.849609375, -703.828125, 1583.61328125, -234.609375, -1173.046875, 682.5, 0.0, 0.0, 0.0, 0.0}, {0.020642638206481934, -0.03799581527709961, 0.05217599868774414, -0.014352162679036459, -0.1370538075764974, 0.29181162516276044, -0.07194264729817708, -0.5652669270833334, 0.6723124186197916, 0.3864339192708333, -1.1394449869791667, 0.16829427083333334, 0.92236328125, -0.443359375, -0.314453125, 0.21875}};
 };
 struct Mesh_w6 {
   static constexpr int kBlocks = 1;

@@ -19,19 +19,22 @@
 //    int_f u F = sum_e mu_e int_e A_F ds,  int_f u u^T F = sum_e mu_e (x) int_e u A_F ds - P int_f A_F
 //    (w_e: signed distance of the foot point to the edge line, mu_e: in-plane outward edge normal, P = I - N N^T).
 //  * edges.  Beyond the block's radius the first integrand is -A_F(|z|) / rho^2: an angle.  Inside, every integrand has
-//    a closed form in r = sqrt(c^2 + s^2), c^2 = z^2 + w^2, a = |z|: the line integrals of A_F are moments
-//    I_n = int r^n ds (n >= -1, -2, -3), and in the divided difference
-//      (r^(2m) - a^(2m)) / (r^2 - a^2)   = sum_(i<m) r^(2i) a^(2(m-1-i)),
-//      (r^(2m+1) - a^(2m+1)) / (r^2 - a^2) = sum_(i<m) r^(2i+1) a^(2(m-1-i)) + a^(2m) / (r + a),
-//    so a face needs its edges' w-weighted moments sum_e w_e I_n and Lambda = sum_e w_e int ds / (r + a) only, each
-//    potential one dot product with them (synthetic division by r^2 - a^2, once per face).  With
+//    a closed form in r = sqrt(c^2 + s^2), c^2 = z^2 + w^2, a = |z|.  A_F is taken in powers of t = r - R/2 (and its one
+//    negative power of r); with P_n = int t^n ds, Q_n = int t^n / r ds, p = R/2 (`rho` in the code):
+//      (n + 1) P_n = [s t^n] - n p P_(n-1) + n c^2 Q_(n-1),   Q_n = P_(n-1) - p Q_(n-1),   P_0 = D,  Q_0 = L,
+//    errors shrink by p a step, and the line integrals of A_F are dot products with the P_n.  In the divided difference
+//    (A(r) - A(a)) / (r - a) is a polynomial in t (synthetic division at a - p), so a face needs its edges' w-weighted
+//    sums alone: V_k = sum_e w_e int t^k / (r + a) ds, V_k = sum_e w_e P_(k-1) - (a + p) V_(k-1), V_0 = Lambda.  With
 //    Y = (s1 r0 - s0 r1) / c^2 (formed without cancellation), U = c^2 Y + c D, B = (r1 + c)(r0 + c), kappa = w / (c + a):
-//      int ds / r = log1p(2 U / ((r1 - s1 + c) (r0 + s0 + c))) = L,   int c ds / r^2 = 2 atan(U / (B + s0 s1)) = Theta,
+//      L = int ds / r = 2 atanh(D / (r0 + r1)),   int c ds / r^2 = 2 atan(U / (B + s0 s1)) = Theta,
 //      int ds / r^3 = Y / (r0 r1),                int w ds / (r (r + a)) = 2 atan(kappa U / (B + kappa^2 s0 s1)) = Omega,
-//      w int ds / (r + a) = w L - a Omega,  I_n = (E_n + n c^2 I_(n-2)) / (n + 1),  E_n = [s r^n],
-//      E_n = D/2 (r1^n + r0^n + S^2 / (r0 + r1) T_n),  T_n = (r1^n - r0^n) / (r1 - r0)      (D = s1 - s0, S = s1 + s0):
-//    sums of terms of one sign throughout, so a short edge keeps its relative accuracy.  The rounding of a channel is
-//    that of the potentials' monomial form (sum |c_n| / max |A|).
+//      Lambda = sum_e (w L - a Omega),
+//      [s t^n] = D/2 (t1^n + t0^n + S^2 / (r0 + r1) T_n),  T_n = (t1^n - t0^n) / (t1 - t0)      (D = s1 - s0, S = s1 + s0).
+//    Why about R/2: in powers of r itself the terms of A cancel to one part in 445 (w4) or 3718 (w6), about R/2 to one in 3
+//    or 4 (in V_k, which meets t = -a - p, to one in 19 or 54 at a = 0.3), so the rounding of a channel was four to twelve
+//    times that of 32 quadrature nodes an edge and is now the same (rms over 1200 rows near a surface, units of the support:
+//    w2 8e-15 -> 4e-15, w4 1.2e-13 -> 4e-14, w6 1.5e-12 -> 3.5e-13; the quadrature 4e-15, 4.5e-14, 4e-13), for 4 % of the
+//    time (2^21 queries, 2.6 M pairs of a row and a face: 729 -> 757 us).
 //    Powers z^p multiply the profiles whose potentials hold r^-m (m <= p) so that every face term stays bounded as
 //    the query approaches the face plane.
 //  * kernels of several pieces are sums of truncated blocks P(r) 1[r <= R] (the decomposition of the 2-D tables); every
@@ -329,7 +332,7 @@ __device__ __forceinline__ double zpow(double z) {
   else return z * z * z;
 }
 
-// coefficient n of potential f of block B, and the coefficient of its negative power
+// coefficient of (r - R/2)^n of potential f of block B, and the coefficient of its negative power of r
 template <class B, int f, int n>
 struct MeshC {
   static constexpr double v = B::kC[f][n];
@@ -338,6 +341,13 @@ template <class B, int f>
 struct MeshNu {
   static constexpr double v = B::kNu[f];
 };
+
+// the highest power of potential f of block B
+template <class B, int f, int n = B::kTop>
+constexpr int mesh_degree() {
+  if constexpr (n == 0 || MeshC<B, f, n>::v != 0.0) return n;
+  else return mesh_degree<B, f, n - 1>();
+}
 
 // the power z^p that multiplies each potential (rows of the block tables) and its one negative power r^-m
 constexpr int kZPow[6] = {1, 2, 3, 0, 0, 1};
@@ -355,10 +365,10 @@ struct FaceSums {
 template <class B>
 __device__ __forceinline__ void face_block(const double* __restrict__ F, const double q[3], double ih,
                                            const double N[3], double z, FaceSums& A) {
-  constexpr double R = B::kR;
+  constexpr double R = B::kR, rho = B::kRho;
   const double a = fabs(z), sg = z > 0.0 ? 1.0 : (z < 0.0 ? -1.0 : 0.0);
   if (!(a < R)) return;                 // no point of the plane within R: no chord, and the potentials vanish at |z|
-  double M[B::kLine + 1];               // sum_e w_e I_n
+  double M[B::kLine + 1];               // sum_e w_e P_n
 #pragma unroll
   for (int n = 0; n <= B::kLine; ++n) M[n] = 0.0;
   double lam = 0.0, om = 0.0, th = 0.0, s3 = 0.0, ox = 1.0, oy = 0.0;
@@ -412,44 +422,40 @@ __device__ __forceinline__ void face_block(const double* __restrict__ F, const d
     const bool same = s0 > 0.0 || s1 < 0.0;                       // the chord on one side of the foot
     const double Y = (same ? D * S : s1 * r0 - s0 * r1) / (same ? s1 * r0 + s0 * r1 : c2);
     const double U = fma(Y, c2, c * D), Bc = (r1 + c) * (r0 + c), s01 = s0 * s1, ca = c + a;
-    const double as = log1p(2.0 * U / ((r1 - s1 + c) * (r0 + s0 + c)));
     const double ica = 1.0 / (c * ca), ic = ica * ca, kap = w * (ica * c);
     const double rr = r0 * r1, rs = r0 + r1, irs = 1.0 / (rr * rs), ir = irs * rs, Y3 = Y * ir;
+    // int ds / r = 2 atanh(D / rs) = log1p(2 D / (rs - D)); towards D = rs in the form that does not cancel
+    const bool mid = D < 0.75 * rs;
+    const double as = log1p(2.0 * (mid ? D : U) / (mid ? rs - D : (r1 - s1 + c) * (r0 + s0 + c)));
     const double Om = 2.0 * atan(kap * U / fmax(fma(kap * kap, s01, Bc), 1e-300));
     const double Th = 2.0 * atan(U / fmax(Bc + s01, 1e-300));
     om += Om;
     lam += w * as - a * Om;
     th += w * ic * Th;
     s3 += a * w * Y3;
-    const double sr = S * (irs * rr), qs = S * sr, eh = 0.5 * D;
-    double pb = r1, pa = r0, T = 1.0, nc2 = c2;
-    double Im = D;                                                // I_(n-1), I_n
-    double I = 0.5 * fma(eh, rs + qs, c2 * as);
+    const double sr = S * (irs * rr), qs = S * sr, eh = 0.5 * D, t1 = r1 - rho, t0 = r0 - rho;
+    double pb = 1.0, pa = 1.0, T = 0.0, nc2 = 0.0;                // t1^n, t0^n, T_n, n c^2
+    double Pm = D, Qm = as;                                       // P_(n-1), Q_(n-1)
     M[0] = fma(w, D, M[0]);
-    M[1] = fma(w, I, M[1]);
     // the four line integrals of the potentials and (A2_K2(r1) - A2_K2(r0)) / (r1 - r0)
     double k1 = fma(MeshC<B, 1, 0>::v, D, MeshNu<B, 1>::v * Th * ic), k2 = fma(MeshC<B, 2, 0>::v, D, MeshNu<B, 2>::v * Y3);
-    double lw = MeshC<B, 3, 0>::v * D, ll = MeshC<B, 4, 0>::v * D, t2 = MeshC<B, 5, 1>::v - MeshNu<B, 5>::v * ir;
-    if constexpr (MeshC<B, 1, 1>::v != 0.0) k1 = fma(MeshC<B, 1, 1>::v, I, k1);
-    if constexpr (MeshC<B, 2, 1>::v != 0.0) k2 = fma(MeshC<B, 2, 1>::v, I, k2);
-    if constexpr (MeshC<B, 3, 1>::v != 0.0) lw = fma(MeshC<B, 3, 1>::v, I, lw);
-    if constexpr (MeshC<B, 4, 1>::v != 0.0) ll = fma(MeshC<B, 4, 1>::v, I, ll);
-    static_for<2, B::kTop + 1>([&](auto nn) {
+    double lw = MeshC<B, 3, 0>::v * D, ll = MeshC<B, 4, 0>::v * D, t2 = -MeshNu<B, 5>::v * ir;
+    static_for<1, B::kTop + 1>([&](auto nn) {
       constexpr int n = decltype(nn)::value;
-      T = fma(r1, T, pa);
-      if constexpr (MeshC<B, 5, n>::v != 0.0) t2 = fma(MeshC<B, 5, n>::v, T, t2);
-      pa *= r0;
+      T = fma(t1, T, pa);
+      t2 = fma(MeshC<B, 5, n>::v, T, t2);
+      pa *= t0;
       if constexpr (n <= B::kLine) {
-        pb *= r1;
+        pb *= t1;
         nc2 += c2;
-        const double In = fma(nc2, Im, eh * fma(qs, T, pb + pa)) * (1.0 / (n + 1));
-        M[n] = fma(w, In, M[n]);
-        if constexpr (MeshC<B, 1, n>::v != 0.0) k1 = fma(MeshC<B, 1, n>::v, In, k1);
-        if constexpr (MeshC<B, 2, n>::v != 0.0) k2 = fma(MeshC<B, 2, n>::v, In, k2);
-        if constexpr (MeshC<B, 3, n>::v != 0.0) lw = fma(MeshC<B, 3, n>::v, In, lw);
-        if constexpr (MeshC<B, 4, n>::v != 0.0) ll = fma(MeshC<B, 4, n>::v, In, ll);
-        Im = I;
-        I = In;
+        const double Pn = fma(nc2, Qm, fma(-n * rho, Pm, eh * fma(qs, T, pb + pa))) * (1.0 / (n + 1));
+        Qm = fma(-rho, Qm, Pm);
+        Pm = Pn;
+        M[n] = fma(w, Pn, M[n]);
+        k1 = fma(MeshC<B, 1, n>::v, Pn, k1);
+        k2 = fma(MeshC<B, 2, n>::v, Pn, k2);
+        lw = fma(MeshC<B, 3, n>::v, Pn, lw);
+        if constexpr (MeshC<B, 4, n>::v != 0.0) ll = fma(MeshC<B, 4, n>::v, Pn, ll);
       }
     });
     const double lk1 = z * k1, lk2b = z * k2, lk2 = z * lk2b, hk = 0.5 * z * (D * sr * t2), wk = w * lk2b, hl = 0.5 * ll;
@@ -472,26 +478,28 @@ __device__ __forceinline__ void face_block(const double* __restrict__ F, const d
     out = atan2(oy, ox);
     out += kTwoPi * rint((turn - out) * (1.0 / kTwoPi));
   }
+  // V_k = sum_e w_e int (r - rho)^k / (r + a) ds, in the place of the M_k
+  double vk = lam;
+  static_for<0, B::kLine + 1>([&](auto kk) {
+    constexpr int k = decltype(kk)::value;
+    const double next = fma(-(a + rho), vk, M[k]);
+    M[k] = vk;
+    vk = next;
+  });
+  const double ta = a - rho;
   static_for<0, 6>([&](auto ff) {
     constexpr int f = decltype(ff)::value, p = kZPow[f], m = kNeg[f];
-    constexpr int top = f == 5 ? B::kTop : B::kLine;
-    double J = 0.0, Aa = 0.0, b = 0.0;
-    // even powers, then odd ones: synthetic division in r^2 by r^2 - z^2
-    static_for<0, top / 2>([&](auto kk) {
-      constexpr int i = top / 2 - decltype(kk)::value;
-      b = fma(zz, b, MeshC<B, f, 2 * i>::v);
-      J = fma(b, M[2 * i - 2], J);
+    constexpr int top = mesh_degree<B, f>();
+    static_assert(top <= B::kLine + 2, "powers of the quotient");
+    // (A(r) - A(a)) / (r - a) in powers of r - rho by synthetic division, the remainder A(a)
+    double J = 0.0, g = MeshC<B, f, top>::v;
+    static_for<0, top>([&](auto kk) {
+      constexpr int k = top - 1 - decltype(kk)::value;
+      J = fma(g, k > B::kLine ? vk : M[k > B::kLine ? 0 : k], J);
+      g = fma(ta, g, MeshC<B, f, k>::v);
     });
-    Aa = fma(zz, b, MeshC<B, f, 0>::v);
-    b = 0.0;
-    static_for<0, (top + 1) / 2 - 1>([&](auto kk) {
-      constexpr int i = (top + 1) / 2 - 1 - decltype(kk)::value;
-      b = fma(zz, b, MeshC<B, f, 2 * i + 1>::v);
-      J = fma(b, M[2 * i - 1], J);
-    });
-    b = fma(zz, b, MeshC<B, f, 1>::v);
-    J = fma(b, lam, J) * zpow<p>(z);
-    Aa = fma(a, b, Aa) * zpow<p>(z);                             // z^p A_F(|z|)
+    J *= zpow<p>(z);
+    double Aa = g * zpow<p>(z);                                  // z^p A_F(|z|)
     if constexpr (m > 0) {
       constexpr double nu = MeshNu<B, f>::v;
       const double zr = zpow<p - m>(z);

@@ -809,9 +809,19 @@ def mesh_blocks(name: str):
     return tuple(out)
 
 
+def mesh_shifted(f, rho, top):
+    """the coefficients of the powers 0 .. top of r - rho of a Laurent polynomial's part of powers >= 0."""
+    out = [F(0)] * (top + 1)
+    for e, c in f.items():
+        for k in range(e + 1) if e >= 0 else ():
+            out[k] += c * comb(e, k) * rho ** (e - k)
+    return out
+
+
 def emit_mesh() -> list:
-    """generated tables of the closed-surface family: per kernel and block the radius, the coefficients of the six
-    compact potentials (powers 0, 1, ... of r) and the coefficients of their negative powers."""
+    """generated tables of the closed-surface family: per kernel and block the radius R, rho = R / 2, the coefficients of
+    the six compact potentials (powers 0, 1, ... of r - rho: in powers of r they cancel to one part in 445 (w4) or 3718
+    (w6), sum |c_n| R^n / max |A|, about rho to one in 3 or 4) and the coefficients of their negative powers of r."""
     out = ["// ---- 3-D closed surfaces: compact potentials per truncated block (unit support, W~ = c3*pi * shape); rows:",
            "//      0 A_K0, 1 A_K1, 2 A_K2, 3 A_W, 4 A_L, 5 A2_K2"]
     for name in RADIAL_KERNELS:
@@ -821,13 +831,14 @@ def emit_mesh() -> list:
             top = max(max(f) for f in fs)
             line = max(max(f) for f in fs[:5])
             out.append(f"struct MeshBlock_{name}_{b} {{")
-            out.append(f"  static constexpr double kR = {_lit(t['R'])};")
+            rho = F(t["R"]) / 2
+            out.append(f"  static constexpr double kR = {_lit(t['R'])}, kRho = {_lit(rho)};")
             out.append(f"  static constexpr int kTop = {top};      // highest power of A2_K2")
             out.append(f"  static constexpr int kLine = {line};     // highest power of the other potentials")
             out.append("  static constexpr double kNu[6] = {" +
                        ", ".join(_lit(f.get(-m, F(0)) if m else F(0)) for f, m in zip(fs, MESH_NEGATIVE)) + "};")
             out.append("  static constexpr double kC[6][kTop + 1] = {" + ", ".join(
-                "{" + ", ".join(_lit(f.get(n, F(0))) for n in range(top + 1)) + "}" for f in fs) + "};")
+                "{" + ", ".join(map(_lit, mesh_shifted(f, rho, top))) + "}" for f in fs) + "};")
             out.append("};")
         q = [sum(t["Q"][k] for t in blocks) for k in range(3)]
         out.append(f"struct Mesh_{name} {{")
