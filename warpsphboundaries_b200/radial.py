@@ -104,6 +104,7 @@ class RadialEvaluator:
         self._kernel_id = KERNEL_IDS[kernel]
         self._prec_id = _PRECISIONS[precision]
         self.accuracy_status = "reference 70-digit radial and sphere fixtures pass on the GPU (float64)"
+        self._request_rows()
 
     def _request_rows(self):
         """the request rows as the library takes them, formed once per array (1-2 us of a small call)."""
