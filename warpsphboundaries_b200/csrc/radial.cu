@@ -11,7 +11,7 @@
 // The reference integrates products of linear factors in Bernstein form; here each radial sub-interval (per kernel
 // piece: the full-ball region [0, min(1, -d)] and the cap region [|d|, min(1, 2R + d)]) is integrated by the
 // Gauss-Legendre rule that is exact for its polynomial integrands (w2 7 nodes in the cap region, w4 8, w6 10; 12 nodes
-// leave < 1e-17 relative on cubic's outer Laurent piece, r >= 1/2).  Cancellation is avoided by factoring the angular
+// leave < 1e-17 relative on cubic's outer Laurent piece, r >= 1/2; float32 takes 12 throughout).  Cancellation is avoided by factoring the angular
 // terms, with the factor r kept inside so that no node divides:
 //   ru = r (1 + cap) = (r - d)(2R + d - r) / (2 D),  rv = r (1 - cap) = (r + d)(r + d + 2R) / (2 D)   (sphere)
 //   ru = r - d,                                      rv = r + d                                       (half-space)
@@ -34,12 +34,19 @@ struct Inv9 {
   T v[9];
 };
 
+// nodes of a region: those that are exact for it in float64; in float32 always 12, over which the roundings of the profile's
+// values average out (with 7 to 10 the error of w4 and w6 is 1.1 to 1.2 times as large)
+template <typename T>
+constexpr int radial_nodes(int exact) {
+  return sizeof(T) == 4 ? 12 : exact;
+}
+
 // one piece's contribution: the full-ball region [lo, hi] (cap = 1) and the cap region [clo, chi]
 template <class KR, int P, typename T>
 __device__ __forceinline__ void radial_piece(T d, T R, T inv2D, bool sphere, T full_end, T cap_end, Inv9<T>& acc) {
   const T plo = T(KR::kLo[P]), phi = T(KR::kHi[P]);
   {
-    constexpr int N = KR::kBall[P];
+    constexpr int N = radial_nodes<T>(KR::kBall[P]);
     const T lo = plo, hi = fmin(phi, full_end);
     if (hi > lo) {
       const T c = T(0.5) * (hi + lo), hw = T(0.5) * (hi - lo);
@@ -65,11 +72,11 @@ __device__ __forceinline__ void radial_piece(T d, T R, T inv2D, bool sphere, T f
     }
   }
   {
-    constexpr int N = KR::kCap[P];
+    constexpr int N = radial_nodes<T>(KR::kCap[P]);
     const T lo = fmax(plo, fabs(d)), hi = fmin(phi, cap_end);
     if (hi > lo) {
       const T c = T(0.5) * (hi + lo), hw = T(0.5) * (hi - lo);
-      T s[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+      T s[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
       for (int g = 0; g < N; ++g) {
         const T r = fma_t(hw, T(radial_gx<N>(g)), c), wg = T(radial_gw<N>(g));
@@ -81,7 +88,7 @@ __device__ __forceinline__ void radial_piece(T d, T R, T inv2D, bool sphere, T f
           rv *= (rv + T(2) * R) * inv2D;
         }
         const T rc = T(0.5) * (ru - rv), a1 = ru * rv, at = ru * ru * (r + rv), an = ru * fma_t(rc, rc - r, r * r);
-        const T wr = wg * r, ww = wr * w, wl = wr * l, wd = wg * dl;
+        const T wr = wg * r, ww = wr * w, wl = wr * l, lu = wl * ru, wd = wg * T(1.0 / 6.0) * dl;
         s[0] = fma_t(ww, ru, s[0]);
         s[1] = fma_t(ww, a1, s[1]);
         s[2] = fma_t(ww, at, s[2]);
@@ -89,9 +96,9 @@ __device__ __forceinline__ void radial_piece(T d, T R, T inv2D, bool sphere, T f
         s[4] = fma_t(wl, a1, s[4]);
         s[5] = fma_t(wl, at, s[5]);
         s[6] = fma_t(wl, an, s[6]);
-        s[7] = fma_t(wl, ru, s[7]);
-        s[8] = fma_t(wd, at, s[8]);
-        s[9] = fma_t(wd, an, s[9]);
+        // (the Hessian's two terms cancel: they are combined at the node, not in sums of their own)
+        s[7] += fma_t(wd, at, lu);
+        s[8] += fma_t(T(2) * wd, an, lu);
       }
       const T h3 = hw * T(1.0 / 3.0);
       acc.v[0] += T(2) * hw * s[0];
@@ -101,8 +108,8 @@ __device__ __forceinline__ void radial_piece(T d, T R, T inv2D, bool sphere, T f
       acc.v[4] += hw * s[4];
       acc.v[5] -= h3 * s[5];
       acc.v[6] -= T(2) * h3 * s[6];
-      acc.v[7] += fma_t(T(2) * hw, s[7], h3 * s[8]);
-      acc.v[8] += fma_t(T(2) * hw, s[7], T(2) * h3 * s[9]);
+      acc.v[7] += T(2) * hw * s[7];
+      acc.v[8] += T(2) * hw * s[8];
     }
   }
 }
@@ -158,8 +165,8 @@ __device__ __forceinline__ void baseline_row(const double inv[9], const double n
 // invariants, x 9) are one contiguous range each: every thread puts its row into shared memory (odd strides against bank
 // conflicts), then the block stores the range coalesced.  FULL: the 28 baseline requests in their order -- written
 // straight from the invariants; other sets look up each request's row of the table (half of the instructions of a full
-// row before).  2^21 sphere rows (w4) on B200: 0.136 ms (5.0 TB/s of DRAM traffic) with 8 + 7 nodes a row and no division in a node; 0.47 ms with 12 + 12
-// nodes, a division each, and the table for every set.
+// row before).  2^21 sphere rows (w4) on B200: 0.131 ms with 8 + 7 nodes a row and no division in a node (float32, 12 + 12
+// nodes: 0.132); 0.47 ms with 12 + 12 nodes, a division each, and the table for every set.
 template <class KR, typename T, bool FULL>
 __global__ void __launch_bounds__(kRadialThreads, 6) k_radial(const double* __restrict__ dist,
                                                               const double* __restrict__ radii,
