@@ -272,7 +272,8 @@ __global__ void __launch_bounds__(kDiskThreads) k_disk_rows(const int32_t* __res
 // Pass 2, the listed particles, 32 to a warp, lane r for particle r: the disks of its cell in cell-list order -- one that
 // covers the support adds its constants, one with an arc waits for the warp: the arcs of the 32 particles are cut into
 // items of 12 quadrature nodes, flattened on the lanes (1 to some 20 panels an arc: a lane per arc would wait for the
-// longest), and lane r adds up its arc's items in order, so a particle's result does not depend on its neighbours.
+// longest), and lane r adds up its arc's items in order, so a particle's result does not depend on its neighbours (nor on
+// how many a warp takes: fewer than 32 where there are few, 3000 particles among 40 disks, cubic, 75 -> 60 us a call).
 // On B200, 1024 disks and 2^20 particles (w4, 0.52 M arcs): 0.25 ms, 52 % of the FP64 pipe.  A warp per particle, the nodes of one panel after the
 // other over its lanes and eight butterfly sums per disk, took 1.25 ms; a thread per particle 4.79.
 template <int KID>
@@ -285,11 +286,13 @@ __global__ void __launch_bounds__(kDiskThreads, kDiskBlocks)
   __shared__ DiskArc s_arc[kDiskThreads / 32][32];
   __shared__ double s_sum[kDiskThreads / 32][32][9];          // an item's eight sums (9: against bank conflicts)
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int64_t n0 = counts[0], n1 = counts[1], b0 = (n0 + 31) / 32, batches = b0 + (n1 + 31) / 32;
-  const int64_t warps = (int64_t)gridDim.x * (kDiskThreads / 32);
+  // particles a warp takes at a time: 32, fewer where that would leave warps of the grid without any
+  const int64_t n0 = counts[0], n1 = counts[1], warps = (int64_t)gridDim.x * (kDiskThreads / 32);
+  const int64_t per = min((n0 + n1 + warps - 1) / warps, (int64_t)32);
+  const int64_t b0 = per ? (n0 + per - 1) / per : 0, batches = per ? b0 + (n1 + per - 1) / per : 0;
   for (int64_t b = (int64_t)blockIdx.x * (kDiskThreads / 32) + wib; b < batches; b += warps) {
-    const int64_t j = b < b0 ? b * 32 + lane : (b - b0) * 32 + lane;
-    const bool mine = j < (b < b0 ? n0 : n1);
+    const int64_t j = (b < b0 ? b : b - b0) * per + lane;
+    const bool mine = lane < per && j < (b < b0 ? n0 : n1);
     const int64_t i = mine ? work[b < b0 ? j : n - 1 - j] : 0;
     double lx = 0.0, ly = 0.0, h = 1.0, acc[12];
     int32_t cid = 0, k = 0, k1 = 0;
@@ -681,12 +684,11 @@ extern "C" int wsb_disk_aggregate(const wsb_disks* d_, int kernel, const double*
   int32_t* counts = reinterpret_cast<int32_t*>(static_cast<char*>(workspace) + need - 256);
   WSB_CUDA(cudaMemsetAsync(counts, 0, 2 * sizeof(int32_t), st));
   const unsigned grid = (unsigned)((n + kDiskThreads - 1) / kDiskThreads);
-  // the resident warps, striding over batches of 32 listed particles; no more warps than batches
+  // the resident warps, striding over batches of listed particles; no more warps than particles
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device);
   constexpr int W = kDiskThreads / 32;
-  const int64_t batches = (n + 31) / 32 + 1;
-  const unsigned wgrid = (unsigned)std::min<int64_t>((batches + W - 1) / W, (int64_t)sms * kDiskBlocks);
+  const unsigned wgrid = (unsigned)std::min<int64_t>((n + W - 1) / W, (int64_t)sms * kDiskBlocks);
   auto launch = [&](auto kid) {
     constexpr int K = decltype(kid)::value;
     k_disk_rows<K><<<grid, kDiskThreads, 0, st>>>(d->cstart, d->items, d->nx, d->ny, d->lo_x, d->lo_y, d->cell, pos, sup,
