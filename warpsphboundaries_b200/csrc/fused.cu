@@ -692,7 +692,7 @@ __device__ __forceinline__ void pack_constant_row(int64_t i, double w, double h,
 }
 
 // a work row, every kernel of the pack: the G lanes' sums combined by an xor butterfly (every lane of the warp takes
-// part), then the lane that writes adds the indicator terms and stores the outputs
+// part; G = 1: already combined), then the lane that writes adds the indicator terms and stores the outputs
 template <class Pack, int K>
 __device__ __forceinline__ void pack_finish(const double* acc_t, int G, bool write, int64_t i, double w, double h,
                                             const double* pose, bool assign, const PackOut& o) {
@@ -745,15 +745,38 @@ __device__ __forceinline__ void pack_stage(const double* acc_t, int G, bool writ
 // row and splits its neighbours: the row's neighbour mask (set by k_agg_rowinfo) lists them among the first kMaskBits
 // candidates of its cell, and lane g takes those of rank g, g + G, ... in candidate order; candidates past the mask are
 // split g, g + G, ... and found by the float-prefiltered predicate.  G = 2, and 8 for the rows of kLongPairs pairs or
-// more (kLongQuad for a quadrature kernel), which come first: two lanes would evaluate some 46 pairs one after the other
-// on small polygons, and launches of a few hundred thousand rows waited for them.  (B200, 300 001 rows of the delta+ groups:
-// 100 -> 37 us; 2^20 rows, w4 110 -> 86 us, four kernels, whose lanes clear and combine 48 sums each, 202 -> 213.  The limit:
-// from 16 pairs on 36 / 87 / 219 where 32 gave 37 / 82 / 203, from 48 on 52 / 81 / 200; w2p5 144 from 16 pairs on, 199 from
-// 32, 247 from 48.)  G follows from the row alone.  Work rows are sorted by pair count, so the lanes of a warp evaluate
-// nearly the same number of closed forms.  The G partial sums are combined by an xor butterfly (the same additions on every
-// lane, commutative, so the result is deterministic and identical on the G lanes).  The channel sums live in shared memory
-// ([kernel][channel][thread]), which keeps the registers for the closed form.
+// more (kLongQuad for a quadrature kernel), which come first and whose lane g takes the neighbours at places g, g + 8, ...
+// of the mask: two lanes would evaluate some 46 pairs one after the other on small polygons, and launches of a few hundred
+// thousand rows waited for them.  G follows from the row alone.  Work rows are sorted by pair count, so the lanes of a warp
+// evaluate nearly the same number of closed forms.  The partial sums are combined in a fixed order: two lanes' by an
+// exchange, eight lanes' through shared memory, where each lane adds up its share of the channels (an xor butterfly over
+// the eight, 144 exchanges for four kernels, and eight mask pops a pair made large launches of long rows slower than two
+// lanes had been: 2^20 rows around a 1000-gon, four kernels, 2388 us a call, 2090 with two lanes, now 2121; one kernel 1303,
+// 1246, 1211).  The limit, 32 pairs against 48, 63 and no split, the pair pass of four kernels among 64 star polygons: 2^20
+// rows 192 / 190 / 190 / 190 us, 300 001 rows 68 / 88 / 102 / 111, 100 001 rows 55 / 78 / 96 / 102; one kernel 2^20 rows 110 us
+// without, 74 now; tensile 144 us from 16 pairs on, 199 from 32, 247 from 48.  The channel sums live in shared memory ([kernel][channel][thread]), which keeps the registers for the
+// closed form.
 constexpr int kShortLanes = 2, kLongLanes = 8;
+
+// the sums over the eight lanes of each of a warp's long rows, put(channel, sum) by lane channel % 8 of the row; `acc` the
+// warp's part of the channel sums (every lane takes part; the lanes start at different slots: no bank conflicts)
+template <class Pack, class F>
+__device__ __forceinline__ void long_sums(const double* acc, F&& put) {
+  const int lane = threadIdx.x & 31, q = lane % kLongLanes;
+  __syncwarp();
+#pragma unroll
+  for (int c0 = 0; c0 < Pack::kN * 12; c0 += kLongLanes) {
+    const int c = c0 + q;
+    if (c < Pack::kN * 12) {
+      const double* a = acc + c * kThreads + (lane - q);
+      double v[kLongLanes];
+#pragma unroll
+      for (int j = 0; j < kLongLanes; ++j) v[j] = a[(j + q) % kLongLanes];
+      put(c, ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])));
+    }
+  }
+  __syncwarp();
+}
 
 // the pairs of a warp's rows (every lane takes part; lane `sub` of the G that share a row; no row: kb = e1 = 0, an empty
 // mask): the channel sums of the lane's share into acc_t
@@ -762,9 +785,15 @@ __device__ __forceinline__ void pair_walk(const SurfView& S, int G, int sub, dou
                                           uint64_t mk0, uint64_t mk1, double* acc_t, double4* slot) {
   constexpr bool kQuadPack = Pack::kN == 1 && Pack::template Kern<0>::kQuad;
   int kt = kb + kMaskBits + sub;                                    // past the mask: lane sub scans kt, kt + G, ...
-  // lane sub takes the neighbours of rank sub, sub + G, ... of the mask (in candidate order), then its share of the
-  // candidates past the mask by the predicate
-  for (int s = 0; s < sub; ++s) pop_bit(mk0, mk1);
+  // lane sub's neighbours of the mask, then its share of the candidates past the mask by the predicate
+  static_assert(kShortLanes == 2 && kLongLanes == 8, "the lanes' shares of the mask");
+  const bool lng = G == kLongLanes;
+  if (lng) {
+    mk0 &= 0x0101010101010101ull << sub;
+    mk1 &= 0x0101010101010101ull << sub;
+  } else if (sub) {
+    pop_bit(mk0, mk1);
+  }
   int nb = pop_bit(mk0, mk1);
   const double ih = 1.0 / h;
 #pragma unroll
@@ -783,7 +812,7 @@ __device__ __forceinline__ void pair_walk(const SurfView& S, int G, int sub, dou
       cp_async_wait_all();
       e = *slot;
       have = true;
-      for (int s = 1; s < G; ++s) pop_bit(mk0, mk1);
+      if (!lng) pop_bit(mk0, mk1);                                  // (the other lane's)
       nb = pop_bit(mk0, mk1);
       if (nb >= 0)
         cp_async_rec(slot, S.crec + kb + nb);
@@ -862,10 +891,17 @@ __global__ void __launch_bounds__(kThreads, MINB) k_agg_pairs(SurfView S, const 
     double* const acc_t = s_acc + threadIdx.x;
     pair_walk<Pack, PREC>(S, G, sub, r.lx, r.ly, r.h, r.kb, r.ke, r.m0, r.m1, acc_t, s_next + threadIdx.x);
     const bool write = ok && sub == 0;
-    if constexpr (STAGED)
-      pack_stage<Pack, 0>(acc_t, G, write, wacc + w * (Pack::kN * 12));
-    else
-      pack_finish<Pack, 0>(acc_t, G, write, r.row, write ? ind[r.row] : 0.0, r.h, pose, assign, out);
+    double* const acc_w = s_acc + (threadIdx.x - lane);
+    if constexpr (STAGED) {
+      double* const dst = wacc + w * (Pack::kN * 12);
+      if (lng)
+        long_sums<Pack>(acc_w, [&](int c, double v) { if (ok) dst[c] = __dmul_rn(v, kInvPi); });
+      else
+        pack_stage<Pack, 0>(acc_t, G, write, dst);
+    } else {
+      if (lng) long_sums<Pack>(acc_w, [&](int c, double v) { acc_w[c * kThreads + lane - sub] = v; });
+      pack_finish<Pack, 0>(acc_t, lng ? 1 : G, write, r.row, write ? ind[r.row] : 0.0, r.h, pose, assign, out);
+    }
   }
 }
 
@@ -1039,7 +1075,11 @@ __global__ void __launch_bounds__(kThreads, pack_min_blocks(Pack::kN) < 5 ? pack
     }
     double* const acc_t = s_acc + t;
     pair_walk<Pack, PREC>(S, G, sub, q.lx, q.ly, q.h, q.kb, q.ke, q.m0, q.m1, acc_t, s_dyn + t);
-    pack_finish<Pack, 0>(acc_t, G, ok && sub == 0, row0 + r, q.ind, q.h, pose, assign, out);
+    if (lng) {
+      double* const acc_w = s_acc + (t - lane);
+      long_sums<Pack>(acc_w, [&](int c, double v) { acc_w[c * kThreads + lane - sub] = v; });
+    }
+    pack_finish<Pack, 0>(acc_t, lng ? 1 : G, ok && sub == 0, row0 + r, q.ind, q.h, pose, assign, out);
   }
 }
 
@@ -1108,9 +1148,6 @@ static int pack_out_vec(const PackOut& o, int n) {
   return v16 ? (v32 ? 2 : 1) : 0;
 }
 
-// the pair kernel of a pack over a prepared workspace (two lanes per work row: measured fastest on the 2^20-particle
-// scene, 1 / 2 lanes give 10.4 / 11.3e9 pairs/s with one kernel, 1 / 2 / 4 lanes 0.448 / 0.421 / 0.471 ms for the
-// four-kernel pack, which also beat the four kernels as two two-kernel packs, 0.426 ms)
 // instrumentation: events recorded on the launching stream right before and after each fused pair kernel (set by
 // wsb_set_pair_events; NULL: none)
 static cudaEvent_t g_pair_ev[2] = {nullptr, nullptr};
@@ -1120,6 +1157,7 @@ constexpr size_t pack_smem_bytes() {
   return sizeof(double4) * kThreads + sizeof(double) * Pack::kN * 12 * kThreads;
 }
 
+// the pair kernel of a pack over a prepared workspace, and the expansion of its staged sums
 template <class Pack, int PREC>
 static int launch_pack(const SurfView& v, const double* sup, const Workspace& w, int64_t n, const double* pose,
                        bool assign, const PackOut& out, cudaStream_t st) {
