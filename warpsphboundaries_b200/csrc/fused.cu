@@ -1252,6 +1252,7 @@ static int find_pack(const int32_t* kernels, int n_groups, int* perm) {
 //   28                           54 / 42    99 / 64  |      74 / 66   129 / 97 |    138 / 106  235 / 196|    60 / 51  65 / 90  112 / 126
 //   43                           64 / 63   118 / 100 |      90 / 95   135 / 154|    159 / 135  229 / 253|    73 / 69  80 / 119 138 / 186
 //   109                         110 / 108  181 / 225 |     157 / 159  241 / 350|    244 / 243  425 / 563|   101 / 75 129 / 173 198 / 427
+// (w4 at 2^15 rows: 107 / 112 for 109, 428 / 423 for 455; w4 and w2p5 at 100 000 rows of length 35 123 / 117 and 291 / 270.)
 // Four kernels stay in one launch a little past the device's crossing: launching the sorted route takes the host 118 us a
 // call, one launch 100 (16 001 rows among 64 star polygons, calls one after the other: 120 against 103).
 // The results are the same bits, so the rule may look at the launch.
@@ -1260,11 +1261,12 @@ static bool one_launch(const Surface* s, int n_groups, const int32_t* kernels, i
   const int which = find_pack(kernels, n_groups, perm);
   const double work = (double)n * s->list_rms;
   if (which >= 0 && kPackSizes[which] >= 4) return n <= (1 << 12) || (n <= (1 << 16) && work <= 0.85e6);
-  if (n <= (1 << 14)) return true;
+  const bool closed = n_groups == 1 && !is_quad_kernel(kernels[0]);
+  if (n <= (closed ? 1 << 15 : 1 << 14)) return true;
   if (n_groups > 1) return n <= (1 << 16) && work <= (which >= 0 ? 2e6 : 1e6);
   // one kernel; over few cells the sort's counters collide, so many rows stay here: 256-gon of 378 cells 2^20 rows 204 / 183
   if (n > (1 << 17) && n < 256 * (int64_t)s->n_nonempty) return false;
-  return work <= 3e6 || (s->list_rms <= 30.0 && !is_quad_kernel(kernels[0]));
+  return closed ? work <= 4e6 || s->list_rms <= 30.0 : work <= 3.5e6;
 }
 
 struct RowArgs {
