@@ -223,8 +223,9 @@ int wsb_aggregate_backward(const wsb_surface* s, int kernel, const double* pos, 
 
 /* Signed distance of body-frame points lpos [m*2] to the surface: d [m] (> 0 in the fluid), closest point cp [m*2],
  * unit normal n_loc [m*2] into the fluid, edge [m] int32.  norm_support > 0: the indicator uses that support
- * normalisation (the sync-free route), else none.  Replaces the SurfaceRep branch of Scene.signed_distance
- * (src/warpSPHBoundaries/scene/scene.py:1312-1350). */
+ * normalisation (the sync-free route), else none.  The first distance of a surface (this call or the next) builds its
+ * edge tree: some host work and one allocation, from any thread and under stream capture as well.  Replaces the
+ * SurfaceRep branch of Scene.signed_distance (src/warpSPHBoundaries/scene/scene.py:1312-1350). */
 int wsb_signed_distance(const wsb_surface* s, const double* lpos, int64_t m, double norm_support, double* d,
                         double* cp, double* n_loc, int32_t* edge, void* stream);
 
@@ -384,7 +385,7 @@ int wsb_mesh_create(const double* verts, int64_t n_verts, const int32_t* faces, 
                     int device, wsb_mesh** out);
 int wsb_mesh_destroy(wsb_mesh* m);
 
-/* bytes of the workspace wsb_mesh_channels needs for n queries */
+/* bytes of the workspace wsb_mesh_channels needs for n queries (the same from 2^22 on: longer calls run in slices) */
 size_t wsb_mesh_workspace_size(const wsb_mesh* m, int64_t n);
 
 /* 1 where the query pos [n*3] (device) lies inside the solid, else 0 (parity of a vertical ray's crossings with

@@ -848,7 +848,7 @@ __device__ __forceinline__ int select_bit(uint64_t m, int k) {
 // pair, whatever row it belongs to, so the lanes stay full although a row has some 20 faces.  The 28 terms of each pair
 // go through shared memory to the lanes k < 28, which add accumulator k of the row pair after pair in the list's order
 // and finish the row when the next row's first pair comes: the result does not depend on the other rows.
-// On the 2^21-particle scene of 20480 faces (w4, 106 825 rows with faces, 2.6 M pairs): 0.43 ms on B200, 20011 near queries (w2) 0.10 ms; 12 warps per
+// On the 2^21-particle scene of 20480 faces (w4, 106 825 rows with faces, 2.6 M pairs): 0.46 ms on B200, 20011 near queries (w2) 0.105 ms; 12 warps per
 // SM, bound by the latency of the float64 chains (38 % of the pipe, issue 43 %; 4 CTAs at 128 registers: no gain).  Before, a warp took one row and
 // spread the quadrature nodes of one edge after the other over its lanes (7.0 ms with the search).
 constexpr int kEvalBlocks = 3;        // resident CTAs per SM (168 registers)
