@@ -752,10 +752,10 @@ __device__ __forceinline__ void pack_stage(const double* acc_t, int G, bool writ
 // exchange, eight lanes' through shared memory, where each lane adds up its share of the channels (an xor butterfly over
 // the eight, 144 exchanges for four kernels, and eight mask pops a pair made large launches of long rows slower than two
 // lanes had been: 2^20 rows around a 1000-gon, four kernels, 2388 us a call, 2090 with two lanes, now 2121; one kernel 1303,
-// 1246, 1211).  The limit, 32 pairs against 48, 63 and no split, the pair pass of four kernels among 64 star polygons: 2^20
-// rows 192 / 190 / 190 / 190 us, 300 001 rows 68 / 88 / 102 / 111, 100 001 rows 55 / 78 / 96 / 102; one kernel 2^20 rows 110 us
-// without, 74 now; tensile 144 us from 16 pairs on, 199 from 32, 247 from 48.  The channel sums live in shared memory ([kernel][channel][thread]), which keeps the registers for the
-// closed form.
+// 1246, 1211).  The limit, 32 pairs against 48, 63 and no split, the pair pass of four kernels among 64 star polygons:
+// 2^20 rows 192 / 190 / 190 / 190 us, 300 001 rows 68 / 88 / 102 / 111, 100 001 rows 55 / 78 / 96 / 102; one kernel 2^20 rows
+// 110 us without, 74 now; tensile 144 us from 16 pairs on, 199 from 32, 247 from 48.  The channel sums live in shared
+// memory ([kernel][channel][thread]), which keeps the registers for the closed form.
 constexpr int kShortLanes = 2, kLongLanes = 8;
 
 // the sums over the eight lanes of each of a warp's long rows, put(channel, sum) by lane channel % 8 of the row; `acc` the
@@ -1246,12 +1246,13 @@ static int find_pack(const int32_t* kernels, int n_groups, int* perm) {
 //   65   (600-gon)               67 / 56    102 / 112   172 / 201   256 / 313|      124 / 88    212 / 208   279 / 385
 //   109  (1000-gon)              90 / 79    148 / 167   216 / 313   370 / 491|      161 / 134   288 / 328   403 / 600
 //   455  (600 edges, 15 cells)  434 / 285   513 / 717   716 / 1234 1257 / 1947|     742 / 572  1042 / 1445 1572 / 2411
-//   and for several kernels   w2,w4,w6: 2^14   2^16  | w4,cubic: 2^14   2^16  | delta+: 2^14   2^16  | all four: 2^12  2^14   2^16
-//   8                            38 / 23    52 / 30  |      48 / 34    64 / 42 |     85 / 58  118 / 81 |    40 / 28  42 / 46   61 / 58
-//   21                           68 / 59    77 / 71  |      95 / 93   105 / 119|    169 / 133  200 / 178|    80 / 63  83 / 87   95 / 132
-//   28                           54 / 42    99 / 64  |      74 / 66   129 / 97 |    138 / 106  235 / 196|    60 / 51  65 / 90  112 / 126
-//   43                           64 / 63   118 / 100 |      90 / 95   135 / 154|    159 / 135  229 / 253|    73 / 69  80 / 119 138 / 186
-//   109                         110 / 108  181 / 225 |     157 / 159  241 / 350|    244 / 243  425 / 563|   101 / 75 129 / 173 198 / 427
+//   several kernels, 2^14 and 2^16 rows (all four: 2^12 too)
+//   length    w2,w4,w6            w4,cubic            delta+               all four
+//   8         38/23    52/30      48/34    64/42       85/58   118/81      40/28    42/46    61/58
+//   21        68/59    77/71      95/93   105/119     169/133  200/178     80/63    83/87    95/132
+//   28        54/42    99/64      74/66   129/97      138/106  235/196     60/51    65/90   112/126
+//   43        64/63   118/100     90/95   135/154     159/135  229/253     73/69    80/119  138/186
+//   109      110/108  181/225    157/159  241/350     244/243  425/563    101/75   129/173  198/427
 // (w4 at 2^15 rows: 107 / 112 for 109, 428 / 423 for 455; w4 and w2p5 at 100 000 rows of length 35 123 / 117 and 291 / 270.)
 // Four kernels stay in one launch a little past the device's crossing: launching the sorted route takes the host 118 us a
 // call, one launch 100 (16 001 rows among 64 star polygons, calls one after the other: 120 against 103).

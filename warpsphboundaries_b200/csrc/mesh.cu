@@ -848,9 +848,10 @@ __device__ __forceinline__ int select_bit(uint64_t m, int k) {
 // pair, whatever row it belongs to, so the lanes stay full although a row has some 20 faces.  The 28 terms of each pair
 // go through shared memory to the lanes k < 28, which add accumulator k of the row pair after pair in the list's order
 // and finish the row when the next row's first pair comes: the result does not depend on the other rows.
-// On the 2^21-particle scene of 20480 faces (w4, 106 825 rows with faces, 2.6 M pairs): 0.46 ms on B200, 20011 near queries (w2) 0.105 ms; 12 warps per
-// SM, bound by the latency of the float64 chains (38 % of the pipe, issue 43 %; 4 CTAs at 128 registers: no gain).  Before, a warp took one row and
-// spread the quadrature nodes of one edge after the other over its lanes (7.0 ms with the search).
+// On the 2^21-particle scene of 20480 faces (w4, 106 825 rows with faces, 2.6 M pairs): 0.46 ms on B200, 20011 near queries
+// (w2) 0.105 ms; 12 warps per SM, bound by the latency of the float64 chains (38 % of the pipe, issue 44 %; 4 CTAs at 128
+// registers: no gain).  Before, a warp took one row and spread the quadrature nodes of one edge after the other over its
+// lanes (7.0 ms with the search).
 constexpr int kEvalBlocks = 3;        // resident CTAs per SM (168 registers)
 constexpr int kEvalRows = 32;
 static_assert((INT32_MAX / 8) * (int64_t)kBatch < ((int64_t)1 << 31) && ((int64_t)1 << 26) * kEvalRows <= ((int64_t)1 << 31),
@@ -992,8 +993,8 @@ int mesh_lists(Mesh* m, const BoxLists& L, int64_t ncells, int32_t** len) {
 }
 
 // Queries are taken kMeshSlice at a time, so the workspace stops growing there (80 bytes a query and 8 per mask word past
-// the first: 0.34 to 0.57 GB; 21 GB for 2^28 queries at once).  A slice of that size takes some milliseconds, its three launches
-// a few microseconds.
+// the first: 0.34 to 0.57 GB; 21 GB for 2^28 queries at once).  A slice of that size takes some milliseconds, its three
+// launches a few microseconds.
 constexpr int64_t kMeshSlice = 1 << 22;
 
 // the workspace of n queries (of one slice): the listed rows, their number and that of the rows with faces, the indicator
@@ -1043,7 +1044,8 @@ int launch_mesh(const Mesh* m, const double* pos_all, const double* sup_all, int
     k_mesh_search<M><<<grid_of(kSearchBlocks), kMeshThreads, 0, st>>>(v, pos, sup, w.near, w.counts, m->words, ind, w.rows,
                                                                       w.mask, out);
     WSB_CUDA(cudaGetLastError());
-    k_mesh_eval<M><<<grid_of(kEvalBlocks), kMeshThreads, 0, st>>>(v, w.rows, w.mask, m->words, m->eval_rows, w.counts + 1, out);
+    k_mesh_eval<M><<<grid_of(kEvalBlocks), kMeshThreads, 0, st>>>(v, w.rows, w.mask, m->words, m->eval_rows, w.counts + 1,
+                                                                  out);
     WSB_CUDA(cudaGetLastError());
   }
   return WSB_OK;

@@ -11,8 +11,8 @@
 // The reference integrates products of linear factors in Bernstein form; here each radial sub-interval (per kernel
 // piece: the full-ball region [0, min(1, -d)] and the cap region [|d|, min(1, 2R + d)]) is integrated by the
 // Gauss-Legendre rule that is exact for its polynomial integrands (w2 7 nodes in the cap region, w4 8, w6 10; 12 nodes
-// leave < 1e-17 relative on cubic's outer Laurent piece, r >= 1/2; float32 takes 12 throughout).  Cancellation is avoided by factoring the angular
-// terms, with the factor r kept inside so that no node divides:
+// leave < 1e-17 relative on cubic's outer Laurent piece, r >= 1/2; float32 takes 12 throughout).  Cancellation is avoided
+// by factoring the angular terms, with the factor r kept inside so that no node divides:
 //   ru = r (1 + cap) = (r - d)(2R + d - r) / (2 D),  rv = r (1 - cap) = (r + d)(r + d + 2R) / (2 D)   (sphere)
 //   ru = r - d,                                      rv = r + d                                       (half-space)
 //   r a0 = 2 ru, r^2 a1 = -ru rv, r^3 at = ru^2 (r + rv) / 3, r^3 an = 2/3 ru (rc^2 - r rc + r^2), rc = r cap
